@@ -109,17 +109,36 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* e
     return ok != 0;
 }
 
-// Ring position: slot index and the parity of its current use.
+// Ring position: slot index and the parity of its current use.  The positions
+// are carried along in 32 bits: forming them from a stage counter took two
+// 64-bit divisions per ring and stage in every role, several hundred cycles
+// of each handshake (column pass at n = 20 000: 1821 cycles per stage).
 struct Ring {
     uint32_t slot, phase;
-    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {
+    __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {  // by: a few slots
         slot += by;
         while (slot >= n) {
             slot -= n;
             phase ^= 1u;
         }
     }
+    __device__ __forceinline__ void jump(uint32_t by, uint32_t n) {  // by: any number (once per unit)
+        const uint32_t t = slot + by, laps = t / n;
+        slot = t - laps * n;
+        phase ^= laps & 1u;
+    }
 };
+
+// Waits for the copies of every slot a producer has filled (`next`: the
+// position it would fill next; `lapped`: it has filled every slot at least
+// once), so that no CTA leaves with copies in flight into its shared memory.
+__device__ __forceinline__ void drain_ring(uint64_t* full, const Ring& next, bool lapped, uint32_t n, int* err,
+                                           int code) {
+    for (uint32_t s = 0; s < n; ++s) {
+        if (s < next.slot) mbar_wait(full + s, next.phase, err, code);
+        else if (lapped) mbar_wait(full + s, next.phase ^ 1u, err, code);
+    }
+}
 
 // MMA issue loop of one of the two MMA warps.  Measured properties of the
 // issuing thread shape it: (1) it is latency bound on operand arithmetic
@@ -134,16 +153,12 @@ struct Ring {
 //
 // This warp's K blocks of one work unit: [start, start + len0), then groups
 // of G, each followed by `skip` K blocks that belong to the other warp.  The
-// unit's first K block is stage g0 of the CTA's stage sequence (the rings run
-// on across the CTA's units: stage g sits in A slot g % S, W slot g % SW).
-__device__ __forceinline__ Ring ring_at(uint64_t g, uint32_t n) {
-    return Ring{(uint32_t)(g % n), (uint32_t)((g / n) & 1u)};
-}
-
+// unit's first K block sits at A ring position st and W ring position sw (the
+// rings run on across the CTA's units).
 template <int NCH, bool MAIN, bool IND, int G>
 __device__ __forceinline__ bool tc8_mma_loop(const Tc8Args& a, uint32_t tmem, uint32_t d_main, uint32_t bsm_addr,
                                              uint64_t* full_b, uint64_t* full_a, uint64_t* a_empty,
-                                             uint64_t* b_empty, uint64_t g0, uint32_t nkb, uint32_t start,
+                                             uint64_t* b_empty, Ring st, Ring sw, uint32_t nkb, uint32_t start,
                                              uint32_t len0, uint32_t skip) {
     const uint32_t S = a.stages, SW = a.wstages;
     const uint32_t chunk = a.n_main / NCH;
@@ -156,7 +171,8 @@ __device__ __forceinline__ bool tc8_mma_loop(const Tc8Args& a, uint32_t tmem, ui
     const uint64_t hstep = (uint64_t)a.n_total * (128 >> 4);  // next 128-sample half of the stage
     const uint32_t d_ind = tmem + a.n_main;
     const uint32_t a0 = tmem + a.a_base;
-    Ring st = ring_at(g0 + start, S), sw = ring_at(g0 + start, SW);  // A ring (TMEM), W ring (shared memory)
+    st.advance(start, S);
+    sw.advance(start, SW);
     uint32_t i = start, len = len0;
     while (i < nkb) {
         const uint32_t g = min(len, nkb - i);
@@ -203,15 +219,15 @@ __device__ __forceinline__ bool tc8_mma_loop(const Tc8Args& a, uint32_t tmem, ui
 template <int NCH, bool MAIN, bool IND>
 __device__ __forceinline__ bool tc8_mma_dispatch(const Tc8Args& a, uint32_t tmem, uint32_t d_main, uint32_t bsm_addr,
                                                  uint64_t* full_b, uint64_t* full_a, uint64_t* a_empty,
-                                                 uint64_t* b_empty, uint64_t g0, uint32_t nkb, uint32_t start,
+                                                 uint64_t* b_empty, Ring st, Ring sw, uint32_t nkb, uint32_t start,
                                                  uint32_t len0, uint32_t skip) {
     if (a.group == 4)
-        return tc8_mma_loop<NCH, MAIN, IND, 4>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, g0, nkb,
+        return tc8_mma_loop<NCH, MAIN, IND, 4>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
                                                start, len0, skip);
     if (a.group == 2)
-        return tc8_mma_loop<NCH, MAIN, IND, 2>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, g0, nkb,
+        return tc8_mma_loop<NCH, MAIN, IND, 2>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
                                                start, len0, skip);
-    return tc8_mma_loop<NCH, MAIN, IND, 1>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, g0, nkb,
+    return tc8_mma_loop<NCH, MAIN, IND, 1>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
                                            start, len0, skip);
 }
 
@@ -298,58 +314,56 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
     } else if (warp == 0) {
         if (lane == 0) {
             // packed-code producer: runs up to P stages ahead of the unpackers,
-            // across units; each (tile, stage) operand is one contiguous bulk copy
-            uint64_t g = 0, issued = 0;
-            bool ok = true;
+            // across units; each (tile, stage) operand is one contiguous bulk copy.
+            // (A slot's first fill waits for the phase before a fresh
+            // barrier's first one, which is complete.)
+            Ring pr{0, 0};
+            bool ok = true, lapped = false;
             for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const uint32_t nkb = unit_nkb(u), rot = unit_rot(u, nkb);
                 const uint8_t* src =
                     a.tiles + (uint64_t)(u % a.gx) * a.tile_bytes + (uint64_t)unit_kb0(u) * kStageBytes;
-                for (uint32_t i = 0; i < nkb; ++i, ++g) {
-                    const uint32_t ks = i + rot < nkb ? i + rot : i + rot - nkb;
-                    const Ring pr = ring_at(g, P);
-                    if (g >= P && !mbar_wait(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21)) {
+                uint32_t ks = rot;
+                for (uint32_t i = 0; i < nkb; ++i) {
+                    if (!mbar_wait(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21)) {
                         ok = false;
                         break;
                     }
                     mbar_arrive_tx(p_full + pr.slot, kStageBytes);
                     bulk_g2s(psm + pr.slot * kStageBytes, src + (uint64_t)ks * kStageBytes, kStageBytes,
                              p_full + pr.slot);
-                    issued = g + 1;
+                    if (++ks == nkb) ks = 0;
+                    pr.advance(1, P);
+                    lapped = lapped || pr.slot == 0;
                 }
             }
-            // never leave with copies in flight into this CTA's shared memory
-            for (uint64_t q = issued > P ? issued - P : 0; q < issued; ++q) {
-                const Ring pr = ring_at(q, P);
-                mbar_wait(p_full + pr.slot, pr.phase, a.err, 22);
-            }
+            drain_ring(p_full, pr, lapped, P, a.err, 22);
         }
     } else if (warp == 2) {
         // each spinning role has a warp of its own: lanes of one warp that
         // spin in different loops starve each other
         if (lane == 0) {
             // W producer: one bulk copy per stage, across units
-            uint64_t g = 0, issued = 0;
-            bool ok = true;
+            Ring wr{0, 0};
+            bool ok = true, lapped = false;
             for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-                const uint32_t nkb = unit_nkb(u), rot = unit_rot(u, nkb), kb0 = unit_kb0(u);
-                for (uint32_t i = 0; i < nkb; ++i, ++g) {
-                    const uint32_t ks = i + rot < nkb ? i + rot : i + rot - nkb;
-                    const Ring wr = ring_at(g, SW);
-                    if (g >= SW && !mbar_wait(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23)) {
+                const uint32_t nkb = unit_nkb(u), rot = unit_rot(u, nkb);
+                const uint8_t* src = a.wop + (uint64_t)unit_kb0(u) * a.b_stage_bytes;
+                uint32_t ks = rot;
+                for (uint32_t i = 0; i < nkb; ++i) {
+                    if (!mbar_wait(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23)) {
                         ok = false;
                         break;
                     }
                     mbar_arrive_tx(full_b + wr.slot, a.b_stage_bytes);
-                    bulk_g2s(bsm + wr.slot * a.b_stage_bytes, a.wop + (uint64_t)(kb0 + ks) * a.b_stage_bytes,
-                             a.b_stage_bytes, full_b + wr.slot);
-                    issued = g + 1;
+                    bulk_g2s(bsm + wr.slot * a.b_stage_bytes, src + (uint64_t)ks * a.b_stage_bytes, a.b_stage_bytes,
+                             full_b + wr.slot);
+                    if (++ks == nkb) ks = 0;
+                    wr.advance(1, SW);
+                    lapped = lapped || wr.slot == 0;
                 }
             }
-            for (uint64_t q = issued > SW ? issued - SW : 0; q < issued; ++q) {
-                const Ring wr = ring_at(q, SW);
-                mbar_wait(full_b + wr.slot, wr.phase, a.err, 24);
-            }
+            drain_ring(full_b, wr, lapped, SW, a.err, 24);
         }
     } else if (warp == 1 || warp == 3) {
         if (lane == 0) {
@@ -357,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             const uint32_t bsm_addr = smem_u32(bsm);
             const uint32_t G = a.group;
             const int nch = a.n_main > 256 ? 2 : 1;  // host guarantees an even split into <= 256-wide MMAs
-            uint64_t g0 = 0;
+            Ring st{0, 0}, sw{0, 0};  // A ring (TMEM) and W ring (shared memory) at the unit's first stage
             uint32_t k = 0;  // this CTA's units so far
             bool ok = true;
             for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++k) {
@@ -372,43 +386,44 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
                     if (m == 0) {
                         if (nch == 1)
                             ok = tc8_mma_dispatch<1, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, g0, nkb, 0, G, 0);
+                                                                  b_empty, st, sw, nkb, 0, G, 0);
                         else
                             ok = tc8_mma_dispatch<2, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, g0, nkb, 0, G, 0);
+                                                                  b_empty, st, sw, nkb, 0, G, 0);
                     } else {
                         ok = tc8_mma_dispatch<1, false, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, g0, nkb, 0, G > 1 ? G / 2 : 1, 0);
+                                                              b_empty, st, sw, nkb, 0, G > 1 ? G / 2 : 1, 0);
                     }
                 } else if (ok && a.kcopies == 2) {
                     // alternate groups of G K blocks into accumulator copies m
                     const uint32_t d_main = tmem + m * a.d_cols;
                     if (nch == 1)
                         ok = tc8_mma_dispatch<1, true, false>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, g0, nkb, m * G, G, G);
+                                                              b_empty, st, sw, nkb, m * G, G, G);
                     else
                         ok = tc8_mma_dispatch<2, true, false>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, g0, nkb, m * G, G, G);
+                                                              b_empty, st, sw, nkb, m * G, G, G);
                 } else if (ok && m == 0) {
                     // one MMA warp does everything
                     if (nch == 1) {
                         if (ind)
                             ok = tc8_mma_dispatch<1, true, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                 b_empty, g0, nkb, 0, G, 0);
+                                                                 b_empty, st, sw, nkb, 0, G, 0);
                         else
                             ok = tc8_mma_dispatch<1, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, g0, nkb, 0, G, 0);
+                                                                  b_empty, st, sw, nkb, 0, G, 0);
                     } else {
                         if (ind)
                             ok = tc8_mma_dispatch<2, true, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                 b_empty, g0, nkb, 0, G, 0);
+                                                                 b_empty, st, sw, nkb, 0, G, 0);
                         else
                             ok = tc8_mma_dispatch<2, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, g0, nkb, 0, G, 0);
+                                                                  b_empty, st, sw, nkb, 0, G, 0);
                     }
                 }
                 mma_commit(tmem_full);  // both MMA warps arrive per unit (an idle one at once)
-                g0 += nkb;
+                st.jump(nkb, S);
+                sw.jump(nkb, SW);
             }
         }
     } else {
@@ -419,15 +434,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
         const uint32_t row = q * 32 + lane;
         const uint32_t lane_base = tmem + ((q * 32) << 16);
         const uint32_t nsets = a.usets;
-        uint64_t g0 = 0;
+        Ring pr{set, 0}, st{set, 0};  // this set's next stage (usets <= stages, pstages)
+        uint32_t ahead = set;         // its distance from the unit's first stage
         uint32_t k = 0;
         bool ok = true;
         for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++k) {
             const uint32_t nkb = unit_nkb(u);
-            for (uint32_t i = 0; i < nkb && set < nsets; ++i) {
-                const uint64_t g = g0 + i;
-                if (g % nsets != set) continue;
-                const Ring pr = ring_at(g, P), st = ring_at(g, S);
+            for (; ahead < nkb && set < nsets; ahead += nsets) {
                 // one lane polls each barrier and the warp follows it (the warp
                 // barrier orders the other lanes after its observation)
                 if (!warp_wait(p_full + pr.slot, pr.phase, a.err, 27)) {
@@ -466,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
                 }
                 keep32(gv);  // expanded before the stage wait: only the stores follow it
                 keep32(h);
-                if (g >= S && !warp_wait(a_empty + st.slot, st.phase ^ 1u, a.err, 28)) {
+                if (!warp_wait(a_empty + st.slot, st.phase ^ 1u, a.err, 28)) {
                     ok = false;
                     break;
                 }
@@ -492,8 +505,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
                 fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_a + st.slot);
+                pr.advance(nsets, P);
+                st.advance(nsets, S);
             }
             if (!ok) break;
+            ahead -= nkb;
             // epilogue of unit u: the sets take 16-column groups round robin
             ok = warp_wait(tmem_full, k & 1u, a.err, 29);
             // the second accumulator copy holds data only if its first group exists
@@ -552,7 +568,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty);
-            g0 += nkb;
         }
     }
     fence_before();
