@@ -45,7 +45,7 @@ constexpr int kHalves = 2;                         // tile blocks per pipeline s
 constexpr int kStageK = kTileK * kHalves;          // 256 samples per stage
 constexpr int kStageBytes = kTileBytes * kHalves;  // packed bytes per stage
 constexpr int kUnpackSets = 2;   // sets of four unpack warps taking K blocks round robin
-constexpr int kThreads = 128 + 128 * kUnpackSets;  // code-copy, 2 MMA, W-copy warps + unpack sets
+constexpr int kThreads = 128 + 128 * kUnpackSets;  // code-copy, MMA, W-copy (and one idle) warps + unpack sets
 constexpr int kMainTerms = 4;
 constexpr int kIndTerms = 3;
 constexpr uint32_t kTabGeno = 0x40380000u;  // code 00,01 -> 0; 10 -> 1.0; 11 -> 2.0 (E4M3 bytes)
@@ -63,9 +63,8 @@ struct Tc8Args {
     uint32_t stages, tmem_cols;  // stages: A operand ring depth (TMEM)
     uint32_t wstages;       // W operand ring depth (shared memory), >= stages
     uint32_t pstages;       // packed-code prefetch depth
-    uint32_t group;         // K blocks an MMA warp waits for at once (1, 2, 4; divides stages)
-    uint32_t kcopies;       // accumulator copies (2: MMA warps take alternate K groups)
-    uint32_t nsplit;        // 1: MMA warp 0 issues the genotype MMAs, warp 1 the indicator MMAs
+    uint32_t group;         // K blocks per group of an accumulator copy (1, 2, 4; divides stages)
+    uint32_t kcopies;       // accumulator copies (2: alternate K groups)
     uint32_t a_base;        // first TMEM column of the A stages
     uint32_t usets;         // unpack sets in use: at most `stages`, so that a set never waits on a stage
                             // two uses ahead (an mbarrier parity wait cannot tell those apart)
@@ -109,6 +108,27 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* e
     return ok != 0;
 }
 
+// The same bounded wait polled by every lane, with warp votes as the only
+// branch conditions: the compiler then knows that the warp stays converged
+// and keeps the loop around it (ring positions, descriptors) in uniform
+// registers, which the tensor-core and bulk-copy instructions take their
+// operands from.
+__device__ __forceinline__ bool warp_wait_uniform(uint64_t* bar, uint32_t parity, int* err, int code) {
+    const uint32_t addr = smem_u32(bar);
+    if (__all_sync(0xffffffffu, mbar_try(addr, parity))) return true;
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        if (__all_sync(0xffffffffu, mbar_try(addr, parity))) return true;
+        if ((it & 1023u) == 0) {
+            const bool stop = *(volatile int*)err != 0 || clock64() - t0 > kWaitCycles;
+            if (__any_sync(0xffffffffu, stop)) {
+                if ((threadIdx.x & 31) == 0) atomicCAS(err, 0, code);
+                return false;
+            }
+        }
+    }
+}
+
 // Ring position: slot index and the parity of its current use.  The positions
 // are carried along in 32 bits: forming them from a stage counter took two
 // 64-bit divisions per ring and stage in every role, several hundred cycles
@@ -135,31 +155,27 @@ struct Ring {
 __device__ __forceinline__ void drain_ring(uint64_t* full, const Ring& next, bool lapped, uint32_t n, int* err,
                                            int code) {
     for (uint32_t s = 0; s < n; ++s) {
-        if (s < next.slot) mbar_wait(full + s, next.phase, err, code);
-        else if (lapped) mbar_wait(full + s, next.phase ^ 1u, err, code);
+        if (s < next.slot) warp_wait_uniform(full + s, next.phase, err, code);
+        else if (lapped) warp_wait_uniform(full + s, next.phase ^ 1u, err, code);
     }
 }
 
-// MMA issue loop of one of the two MMA warps.  Measured properties of the
-// issuing thread shape it: (1) it is latency bound on operand arithmetic
-// between MMAs, so descriptors / TMEM addresses are per-stage bases plus
-// compile-time offsets; (2) an mbarrier wait by the issuing thread returns only
-// after the MMAs it issued before have (nearly) drained from the tensor pipe,
-// so a single issuing warp leaves the pipe idle at every wait.  Two MMA warps
-// whose waits fall at different K blocks keep it busy: without the indicator
-// they take alternate groups of G K blocks into two accumulator copies (summed
-// in the epilogue); with it one issues the genotype MMAs and the other the
-// indicator MMAs of every K block, their group boundaries G/2 apart.
+// MMA issue of one work unit (nkb stages from ring positions st, sw, which are
+// carried on).  The whole warp runs the loop and each tcgen05 instruction is
+// predicated on one elected lane: with the loop under `lane == 0` instead,
+// every MMA took at least 116 cycles to issue whatever its width, since its
+// operands went from vector to uniform registers one instruction at a time
+// (measured, one thread, 128 x N x 32 E4M3: 116 cycles at N = 32 ... 192;
+// this form N / 2 cycles, the pipe's rate: 64 at N = 128).  One warp then
+// keeps the pipe full.
 //
-// This warp's K blocks of one work unit: [start, start + len0), then groups
-// of G, each followed by `skip` K blocks that belong to the other warp.  The
-// unit's first K block sits at A ring position st and W ring position sw (the
-// rings run on across the CTA's units).
-template <int NCH, bool MAIN, bool IND, int G>
-__device__ __forceinline__ bool tc8_mma_loop(const Tc8Args& a, uint32_t tmem, uint32_t d_main, uint32_t bsm_addr,
-                                             uint64_t* full_b, uint64_t* full_a, uint64_t* a_empty,
-                                             uint64_t* b_empty, Ring st, Ring sw, uint32_t nkb, uint32_t start,
-                                             uint32_t len0, uint32_t skip) {
+// With two accumulator copies (kcopies) alternate groups of a.group K blocks
+// go to copies 0 and 1, summed in the epilogue; the indicator MMAs of a K block
+// follow its genotype MMAs.
+template <int NCH, bool IND>
+__device__ __forceinline__ bool tc8_mma_unit(const Tc8Args& a, uint32_t tmem, uint32_t bsm_addr, uint64_t* full_b,
+                                             uint64_t* full_a, uint64_t* a_empty, uint64_t* b_empty, Ring& st,
+                                             Ring& sw, uint32_t nkb, uint32_t elected) {
     const uint32_t S = a.stages, SW = a.wstages;
     const uint32_t chunk = a.n_main / NCH;
     const uint32_t id_main = instr_desc_e4m3(chunk);
@@ -171,64 +187,34 @@ __device__ __forceinline__ bool tc8_mma_loop(const Tc8Args& a, uint32_t tmem, ui
     const uint64_t hstep = (uint64_t)a.n_total * (128 >> 4);  // next 128-sample half of the stage
     const uint32_t d_ind = tmem + a.n_main;
     const uint32_t a0 = tmem + a.a_base;
-    st.advance(start, S);
-    sw.advance(start, SW);
-    uint32_t i = start, len = len0;
-    while (i < nkb) {
-        const uint32_t g = min(len, nkb - i);
-        bool ok = true;
-        Ring w = st, wb = sw;
-        for (uint32_t j = 0; j < g && ok; ++j) {
-            ok = mbar_wait(full_b + wb.slot, wb.phase, a.err, 25) && mbar_wait(full_a + w.slot, w.phase, a.err, 26);
-            w.advance(1, S);
-            wb.advance(1, SW);
-        }
-        if (!ok) return false;
+    uint32_t copy = 0, in_group = 0;   // accumulator copy of this stage, its place in the group
+    for (uint32_t i = 0; i < nkb; ++i) {
+        if (!warp_wait_uniform(full_b + sw.slot, sw.phase, a.err, 25)) return false;
+        if (!warp_wait_uniform(full_a + st.slot, st.phase, a.err, 26)) return false;
         fence_after();
+        const uint64_t bd = bdesc0 + sw.slot * bstep;
+        const uint32_t ad = a0 + st.slot * a.a_cols;
+        const uint32_t d_main = tmem + copy * a.d_cols;
+        const uint32_t acc0 = i > copy * a.group ? 1u : 0u;  // the copy's first stage clears it
 #pragma unroll
-        for (int j = 0; j < G; ++j) {
-            if ((uint32_t)j < g) {
-                const uint64_t bd = bdesc0 + sw.slot * bstep;
-                const uint32_t ad = a0 + st.slot * a.a_cols;
-                const uint32_t acc0 = (i + j) > start ? 1u : 0u;
+        for (int kk = 0; kk < kStageK / 32; ++kk) {
+            const uint32_t acc = kk > 0 ? 1u : acc0;
+            const uint64_t bk = bd + (kk >> 2) * hstep + (kk & 3) * 2;
 #pragma unroll
-                for (int kk = 0; kk < kStageK / 32; ++kk) {
-                    const uint32_t acc = kk > 0 ? 1u : acc0;
-                    const uint64_t bk = bd + (kk >> 2) * hstep + (kk & 3) * 2;
-                    if (MAIN) {
-#pragma unroll
-                        for (int ch = 0; ch < NCH; ++ch)
-                            mma_ts_f8(d_main + ch * chunk, ad + kk * 8, bk + ch * chstep, id_main, acc);
-                    }
-                    if (IND) mma_ts_f8(d_ind, ad + kStageK / 4 + kk * 8, bk + indoff, id_ind, acc);
-                }
-                mma_commit(a_empty + st.slot);
-                mma_commit(b_empty + sw.slot);
-                st.advance(1, S);
-                sw.advance(1, SW);
-            }
+            for (int ch = 0; ch < NCH; ++ch)
+                mma_ts_f8(d_main + ch * chunk, ad + kk * 8, bk + ch * chstep, id_main, acc, elected);
+            if (IND) mma_ts_f8(d_ind, ad + kStageK / 4 + kk * 8, bk + indoff, id_ind, acc, elected);
         }
-        i += g + skip;
-        st.advance(skip, S);
-        sw.advance(skip, SW);
-        len = G;
+        mma_commit(a_empty + st.slot, elected);
+        mma_commit(b_empty + sw.slot, elected);
+        st.advance(1, S);
+        sw.advance(1, SW);
+        if (a.kcopies == 2 && ++in_group == a.group) {
+            in_group = 0;
+            copy ^= 1u;
+        }
     }
     return true;
-}
-
-template <int NCH, bool MAIN, bool IND>
-__device__ __forceinline__ bool tc8_mma_dispatch(const Tc8Args& a, uint32_t tmem, uint32_t d_main, uint32_t bsm_addr,
-                                                 uint64_t* full_b, uint64_t* full_a, uint64_t* a_empty,
-                                                 uint64_t* b_empty, Ring st, Ring sw, uint32_t nkb, uint32_t start,
-                                                 uint32_t len0, uint32_t skip) {
-    if (a.group == 4)
-        return tc8_mma_loop<NCH, MAIN, IND, 4>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
-                                               start, len0, skip);
-    if (a.group == 2)
-        return tc8_mma_loop<NCH, MAIN, IND, 2>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
-                                               start, len0, skip);
-    return tc8_mma_loop<NCH, MAIN, IND, 1>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
-                                           start, len0, skip);
 }
 
 // One CTA per SM runs work units u = blockIdx.x, blockIdx.x + gridDim.x, ...
@@ -248,17 +234,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
     float* scl = reinterpret_cast<float*>(psm + P * kStageBytes);             // up to 512 floats
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scl) + 2048);
     uint64_t* full_b = bars;                 // [SW] W stage landed (TMA tx)
-    uint64_t* b_empty = bars + SW;           // [SW] every MMA warp's MMAs on the W stage done
+    uint64_t* b_empty = bars + SW;           // [SW] the MMAs reading the W stage done
     uint64_t* full_a = bars + 2 * SW;        // [S] A operand written to TMEM (128 arrivals)
     uint64_t* a_empty = full_a + S;          // [S] the MMAs reading the A stage done
     uint64_t* p_full = a_empty + S;          // [P] packed codes landed (TMA tx)
     uint64_t* p_empty = p_full + P;          // [P] packed codes consumed (4 warp arrivals)
-    uint64_t* tmem_full = p_empty + P;       // a unit's MMAs done (both MMA warps commit)
+    uint64_t* tmem_full = p_empty + P;       // a unit's MMAs done
     uint64_t* d_empty = tmem_full + 1;       // a unit's epilogue has read D (8 unpack warps)
     uint64_t* never = d_empty + 1;           // test hook: a barrier nothing arrives at
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(never + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // warp index through a shuffle: known to be the same in every lane
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const bool ind = a.n_ind != 0;
     auto unit_kb0 = [&](uint32_t u) { return (u / a.gx) * a.kb_per_split; };
     auto unit_nkb = [&](uint32_t u) {
@@ -277,17 +264,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < SW; ++s) {
             mbar_init(full_b + s, 1);
-            mbar_init(b_empty + s, a.nsplit ? 2 : 1);   // every MMA warp that reads the stage commits
+            mbar_init(b_empty + s, 1);
         }
         for (uint32_t s = 0; s < S; ++s) {
             mbar_init(full_a + s, 4);     // one arrival per unpack warp
-            mbar_init(a_empty + s, a.nsplit ? 2 : 1);
+            mbar_init(a_empty + s, 1);
         }
         for (uint32_t p = 0; p < P; ++p) {
             mbar_init(p_full + p, 1);
             mbar_init(p_empty + p, 4);
         }
-        mbar_init(tmem_full, 2);
+        mbar_init(tmem_full, 1);
         mbar_init(d_empty, 4 * kUnpackSets);
         mbar_init(never, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -312,121 +299,79 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
     if (a.expire_cycles > 0) {
         if (threadIdx.x == 0) mbar_wait_for(never, 0, a.err, 30, a.expire_cycles);
     } else if (warp == 0) {
-        if (lane == 0) {
-            // packed-code producer: runs up to P stages ahead of the unpackers,
-            // across units; each (tile, stage) operand is one contiguous bulk copy.
-            // (A slot's first fill waits for the phase before a fresh
-            // barrier's first one, which is complete.)
-            Ring pr{0, 0};
-            bool ok = true, lapped = false;
-            for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-                const uint32_t nkb = unit_nkb(u), rot = unit_rot(u, nkb);
-                const uint8_t* src =
-                    a.tiles + (uint64_t)(u % a.gx) * a.tile_bytes + (uint64_t)unit_kb0(u) * kStageBytes;
-                uint32_t ks = rot;
-                for (uint32_t i = 0; i < nkb; ++i) {
-                    if (!mbar_wait(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_arrive_tx(p_full + pr.slot, kStageBytes);
-                    bulk_g2s(psm + pr.slot * kStageBytes, src + (uint64_t)ks * kStageBytes, kStageBytes,
-                             p_full + pr.slot);
-                    if (++ks == nkb) ks = 0;
-                    pr.advance(1, P);
-                    lapped = lapped || pr.slot == 0;
-                }
+        // packed-code producer: runs up to P stages ahead of the unpackers,
+        // across units; each (tile, stage) operand is one contiguous bulk copy.
+        // (A slot's first fill waits for the phase before a fresh barrier's
+        // first one, which is complete.)
+        const uint32_t elected = elect_one();
+        Ring pr{0, 0};
+        bool ok = true, lapped = false;
+        for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+            const uint32_t nkb = unit_nkb(u);
+            const uint8_t* src = a.tiles + (uint64_t)(u % a.gx) * a.tile_bytes + (uint64_t)unit_kb0(u) * kStageBytes;
+            uint32_t ks = unit_rot(u, nkb);
+            for (uint32_t i = 0; i < nkb; ++i) {
+                ok = warp_wait_uniform(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21);
+                if (!ok) break;
+                bulk_g2s_tx(psm + pr.slot * kStageBytes, src + (uint64_t)ks * kStageBytes, kStageBytes,
+                            p_full + pr.slot, elected);
+                if (++ks == nkb) ks = 0;
+                pr.advance(1, P);
+                lapped = lapped || pr.slot == 0;
             }
-            drain_ring(p_full, pr, lapped, P, a.err, 22);
         }
+        drain_ring(p_full, pr, lapped, P, a.err, 22);
     } else if (warp == 2) {
         // each spinning role has a warp of its own: lanes of one warp that
         // spin in different loops starve each other
-        if (lane == 0) {
-            // W producer: one bulk copy per stage, across units
-            Ring wr{0, 0};
-            bool ok = true, lapped = false;
-            for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-                const uint32_t nkb = unit_nkb(u), rot = unit_rot(u, nkb);
-                const uint8_t* src = a.wop + (uint64_t)unit_kb0(u) * a.b_stage_bytes;
-                uint32_t ks = rot;
-                for (uint32_t i = 0; i < nkb; ++i) {
-                    if (!mbar_wait(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_arrive_tx(full_b + wr.slot, a.b_stage_bytes);
-                    bulk_g2s(bsm + wr.slot * a.b_stage_bytes, src + (uint64_t)ks * a.b_stage_bytes, a.b_stage_bytes,
-                             full_b + wr.slot);
-                    if (++ks == nkb) ks = 0;
-                    wr.advance(1, SW);
-                    lapped = lapped || wr.slot == 0;
-                }
-            }
-            drain_ring(full_b, wr, lapped, SW, a.err, 24);
-        }
-    } else if (warp == 1 || warp == 3) {
-        if (lane == 0) {
-            const uint32_t m = warp == 1 ? 0u : 1u;  // MMA warp index
-            const uint32_t bsm_addr = smem_u32(bsm);
-            const uint32_t G = a.group;
-            const int nch = a.n_main > 256 ? 2 : 1;  // host guarantees an even split into <= 256-wide MMAs
-            Ring st{0, 0}, sw{0, 0};  // A ring (TMEM) and W ring (shared memory) at the unit's first stage
-            uint32_t k = 0;  // this CTA's units so far
-            bool ok = true;
-            for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++k) {
-                const uint32_t nkb = unit_nkb(u);
-                // D is free once the previous unit's epilogue has read it
-                if (k > 0) {
-                    ok = mbar_wait(d_empty, (k - 1) & 1u, a.err, 31);
-                    fence_after();
-                }
-                if (ok && a.nsplit) {
-                    // genotype MMAs on warp 0, indicator MMAs on warp 1, boundaries G/2 apart
-                    if (m == 0) {
-                        if (nch == 1)
-                            ok = tc8_mma_dispatch<1, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, st, sw, nkb, 0, G, 0);
-                        else
-                            ok = tc8_mma_dispatch<2, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, st, sw, nkb, 0, G, 0);
-                    } else {
-                        ok = tc8_mma_dispatch<1, false, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, st, sw, nkb, 0, G > 1 ? G / 2 : 1, 0);
-                    }
-                } else if (ok && a.kcopies == 2) {
-                    // alternate groups of G K blocks into accumulator copies m
-                    const uint32_t d_main = tmem + m * a.d_cols;
-                    if (nch == 1)
-                        ok = tc8_mma_dispatch<1, true, false>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, st, sw, nkb, m * G, G, G);
-                    else
-                        ok = tc8_mma_dispatch<2, true, false>(a, tmem, d_main, bsm_addr, full_b, full_a, a_empty,
-                                                              b_empty, st, sw, nkb, m * G, G, G);
-                } else if (ok && m == 0) {
-                    // one MMA warp does everything
-                    if (nch == 1) {
-                        if (ind)
-                            ok = tc8_mma_dispatch<1, true, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                 b_empty, st, sw, nkb, 0, G, 0);
-                        else
-                            ok = tc8_mma_dispatch<1, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, st, sw, nkb, 0, G, 0);
-                    } else {
-                        if (ind)
-                            ok = tc8_mma_dispatch<2, true, true>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                 b_empty, st, sw, nkb, 0, G, 0);
-                        else
-                            ok = tc8_mma_dispatch<2, true, false>(a, tmem, tmem, bsm_addr, full_b, full_a, a_empty,
-                                                                  b_empty, st, sw, nkb, 0, G, 0);
-                    }
-                }
-                mma_commit(tmem_full);  // both MMA warps arrive per unit (an idle one at once)
-                st.jump(nkb, S);
-                sw.jump(nkb, SW);
+        // W producer: one bulk copy per stage, across units
+        const uint32_t elected = elect_one();
+        Ring wr{0, 0};
+        bool ok = true, lapped = false;
+        for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+            const uint32_t nkb = unit_nkb(u);
+            const uint8_t* src = a.wop + (uint64_t)unit_kb0(u) * a.b_stage_bytes;
+            uint32_t ks = unit_rot(u, nkb);
+            for (uint32_t i = 0; i < nkb; ++i) {
+                ok = warp_wait_uniform(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23);
+                if (!ok) break;
+                bulk_g2s_tx(bsm + wr.slot * a.b_stage_bytes, src + (uint64_t)ks * a.b_stage_bytes, a.b_stage_bytes,
+                            full_b + wr.slot, elected);
+                if (++ks == nkb) ks = 0;
+                wr.advance(1, SW);
+                lapped = lapped || wr.slot == 0;
             }
         }
-    } else {
+        drain_ring(full_b, wr, lapped, SW, a.err, 24);
+    } else if (warp == 1) {
+        const uint32_t elected = elect_one();
+        const uint32_t bsm_addr = smem_u32(bsm);
+        const bool wide = a.n_main > 256;  // host guarantees an even split into <= 256-wide MMAs
+        Ring st{0, 0}, sw{0, 0};           // A ring (TMEM), W ring (shared memory)
+        uint32_t k = 0;                    // this CTA's units so far
+        bool ok = true;
+        for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++k) {
+            const uint32_t nkb = unit_nkb(u);
+            // D is free once the previous unit's epilogue has read it
+            if (k > 0) {
+                ok = warp_wait_uniform(d_empty, (k - 1) & 1u, a.err, 31);
+                fence_after();
+            }
+            if (ok) {
+                if (ind)
+                    ok = wide ? tc8_mma_unit<2, true>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
+                                                      elected)
+                              : tc8_mma_unit<1, true>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
+                                                      elected);
+                else
+                    ok = wide ? tc8_mma_unit<2, false>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw,
+                                                       nkb, elected)
+                              : tc8_mma_unit<1, false>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw,
+                                                       nkb, elected);
+            }
+            mma_commit(tmem_full, elected);
+        }
+    } else if (warp >= 4) {
         // kUnpackSets sets of four unpack warps take the stages of the CTA's
         // sequence round robin; warp % 4 is the TMEM lane quarter a warp may access
         const uint32_t set = (uint32_t)(warp - 4) >> 2;
@@ -1379,7 +1324,6 @@ static int tc8_launch(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t ro
     a.pstages = pl.pstages;
     a.group = pl.group;
     a.kcopies = pl.kcopies;
-    a.nsplit = pl.nsplit;
     a.a_base = pl.a_base;
     a.usets = std::min<uint32_t>(kUnpackSets, std::min(pl.stages, pl.pstages));
     a.tmem_cols = pl.tmem_cols;
