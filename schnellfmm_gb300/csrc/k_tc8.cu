@@ -44,8 +44,15 @@ constexpr int kTileBytes = kM * kTileK / 4;        // 4 KiB: 128 rows x 32 B
 constexpr int kHalves = 2;                         // tile blocks per pipeline stage
 constexpr int kStageK = kTileK * kHalves;          // 256 samples per stage
 constexpr int kStageBytes = kTileBytes * kHalves;  // packed bytes per stage
-constexpr int kUnpackSets = 2;   // sets of four unpack warps taking K blocks round robin
-constexpr int kThreads = 128 + 128 * kUnpackSets;  // code-copy, MMA, W-copy (and one idle) warps + unpack sets
+// Warps: code copies, W copies, two for the MMAs, then the unpack sets of four,
+// then the epilogue, two per TMEM lane quarter.  Three and four unpack sets were
+// slower (80 registers a thread: column pass 2.66 ms against 2.54 ms with two
+// sets at 1 M SNPs x 20 000 samples), and so were four epilogue warps where a
+// unit is short (5003 samples: row pass 375 us against 283 us).
+constexpr int kUnpackSets = 2;
+constexpr int kEpiWarps = 8;
+constexpr int kCtlWarps = 4;
+constexpr int kThreads = 32 * (kCtlWarps + 4 * kUnpackSets + kEpiWarps);
 constexpr int kMainTerms = 4;
 constexpr int kIndTerms = 3;
 constexpr uint32_t kTabGeno = 0x40380000u;  // code 00,01 -> 0; 10 -> 1.0; 11 -> 2.0 (E4M3 bytes)
@@ -59,15 +66,16 @@ struct Tc8Args {
     uint32_t n_total;       // B rows (n_main + n_ind, or n_main when ind_shared)
     uint32_t ind_shared;    // indicator MMAs read B rows [0, n_ind) of the main terms
     uint32_t d_cols;        // TMEM columns reserved for D
-    uint32_t a_cols;        // TMEM columns per A stage (32, or 64 with the indicator)
-    uint32_t stages, tmem_cols;  // stages: A operand ring depth (TMEM)
-    uint32_t wstages;       // W operand ring depth (shared memory), >= stages
+    uint32_t a_cols;        // TMEM columns per A slot: a stage's genotypes, or half a stage's with the indicator
+    uint32_t parts;         // A slots per stage: 1, or 2 (a slot per half, with the indicator)
+    uint32_t slots, tmem_cols;   // A operand ring depth in slots (TMEM)
+    uint32_t wstages;       // W operand ring depth (shared memory)
     uint32_t pstages;       // packed-code prefetch depth
-    uint32_t group;         // K blocks per group of an accumulator copy (1, 2, 4; divides stages)
+    uint32_t group;         // K blocks per group of an accumulator copy
     uint32_t kcopies;       // accumulator copies (2: alternate K groups)
     uint32_t a_base;        // first TMEM column of the A stages
-    uint32_t usets;         // unpack sets in use: at most `stages`, so that a set never waits on a stage
-                            // two uses ahead (an mbarrier parity wait cannot tell those apart)
+    uint32_t usets;         // unpack sets in use
+    uint32_t none;          // 0 (see tc8_unpack)
     uint32_t b_stage_bytes; // n_total * 256: one stage of the stage-major W operand
     const float* inv_scale; // n_total: 2^-(e0 + 4t) per B row
     const uint8_t* wop;     // stage-major, pre-swizzled W operand (wop_offset)
@@ -97,23 +105,13 @@ __device__ __forceinline__ void keep32(const uint32_t (&v)[32]) {
                  "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]));
 }
 
-// Warp-wide bounded wait: lane 0 polls the barrier, the result is broadcast
-// and __syncwarp orders the other lanes after lane 0's observation.  One
-// poller per warp keeps the barrier word's traffic low.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, err, code) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();
-    return ok != 0;
-}
-
-// The same bounded wait polled by every lane, with warp votes as the only
+// Warp-wide bounded wait polled by every lane, with warp votes as the only
 // branch conditions: the compiler then knows that the warp stays converged
 // and keeps the loop around it (ring positions, descriptors) in uniform
 // registers, which the tensor-core and bulk-copy instructions take their
-// operands from.
-__device__ __forceinline__ bool warp_wait_uniform(uint64_t* bar, uint32_t parity, int* err, int code) {
+// operands from.  (A wait polled by lane 0 and passed on by a shuffle took
+// about 250 cycles on a barrier that was already complete.)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
     const uint32_t addr = smem_u32(bar);
     if (__all_sync(0xffffffffu, mbar_try(addr, parity))) return true;
     const long long t0 = clock64();
@@ -142,11 +140,6 @@ struct Ring {
             phase ^= 1u;
         }
     }
-    __device__ __forceinline__ void jump(uint32_t by, uint32_t n) {  // by: any number (once per unit)
-        const uint32_t t = slot + by, laps = t / n;
-        slot = t - laps * n;
-        phase ^= laps & 1u;
-    }
 };
 
 // Waits for the copies of every slot a producer has filled (`next`: the
@@ -155,66 +148,227 @@ struct Ring {
 __device__ __forceinline__ void drain_ring(uint64_t* full, const Ring& next, bool lapped, uint32_t n, int* err,
                                            int code) {
     for (uint32_t s = 0; s < n; ++s) {
-        if (s < next.slot) warp_wait_uniform(full + s, next.phase, err, code);
-        else if (lapped) warp_wait_uniform(full + s, next.phase ^ 1u, err, code);
+        if (s < next.slot) warp_wait(full + s, next.phase, err, code);
+        else if (lapped) warp_wait(full + s, next.phase ^ 1u, err, code);
     }
 }
 
-// MMA issue of one work unit (nkb stages from ring positions st, sw, which are
-// carried on).  The whole warp runs the loop and each tcgen05 instruction is
-// predicated on one elected lane: with the loop under `lane == 0` instead,
-// every MMA took at least 116 cycles to issue whatever its width, since its
-// operands went from vector to uniform registers one instruction at a time
-// (measured, one thread, 128 x N x 32 E4M3: 116 cycles at N = 32 ... 192;
-// this form N / 2 cycles, the pipe's rate: 64 at N = 128).  One warp then
-// keeps the pipe full.
+// MMA issue of one warp's share of a work unit (nkb stages from ring positions
+// st, sw, which are carried on).  The whole warp runs the loop and each tcgen05
+// instruction is predicated on one elected lane: with the loop under
+// `lane == 0` instead, every MMA took at least 116 cycles to issue whatever its
+// width, since its operands went from vector to uniform registers one
+// instruction at a time (measured, 128 x N x 32 E4M3: 116 cycles at N = 32 ...
+// 192; this form N / 2 cycles, the pipe's rate).
 //
-// With two accumulator copies (kcopies) alternate groups of a.group K blocks
-// go to copies 0 and 1, summed in the epilogue; the indicator MMAs of a K block
-// follow its genotype MMAs.
-template <int NCH, bool IND>
-__device__ __forceinline__ bool tc8_mma_unit(const Tc8Args& a, uint32_t tmem, uint32_t bsm_addr, uint64_t* full_b,
-                                             uint64_t* full_a, uint64_t* a_empty, uint64_t* b_empty, Ring& st,
-                                             Ring& sw, uint32_t nkb, uint32_t elected) {
-    const uint32_t S = a.stages, SW = a.wstages;
-    const uint32_t chunk = a.n_main / NCH;
-    const uint32_t id_main = instr_desc_e4m3(chunk);
-    const uint32_t id_ind = IND ? instr_desc_e4m3(a.n_ind) : 0u;
-    const uint64_t bdesc0 = smem_desc(bsm_addr);
-    const uint64_t bstep = a.b_stage_bytes >> 4;          // descriptor address units per stage
-    const uint64_t chstep = (uint64_t)chunk * (128 >> 4);  // per main chunk of B rows
-    const uint64_t indoff = a.ind_shared ? 0ull : (uint64_t)a.n_main * (128 >> 4);
+// Two warps issue.  A barrier wait of a warp comes back only once the MMAs that
+// it issued before have left its queue, so the pipe runs dry at every wait of
+// a single issuer (875 of 1390 cycles per stage busy); the other warp's MMAs
+// fill that time.  The warps' accumulators are disjoint and each sees its own
+// in K order: with two accumulator copies they take alternate groups of
+// a.group stages; with the indicator one takes the genotype and one the
+// indicator MMAs; otherwise each takes half of the output columns.
+struct MmaShare {
+    uint32_t idesc;      // instruction descriptor (its N)
+    uint32_t d;          // first accumulator column
+    uint32_t a_off;      // TMEM column offset of its operand in an A slot
+    uint32_t b_off;      // first B row of its operand, in descriptor units
+    uint32_t copy;       // its accumulator copy (kcopies == 2)
+};
+
+template <int PARTS>
+__device__ __forceinline__ bool tc8_mma_unit(const Tc8Args& a, const MmaShare& m, uint32_t a0, uint64_t bdesc0,
+                                             uint64_t* full_b, uint64_t* full_a, uint64_t* a_empty,
+                                             uint64_t* b_empty, Ring& st, Ring& sw, uint32_t nkb,
+                                             uint32_t elected) {
+    constexpr int kSteps = kStageK / 32 / PARTS;           // MMA K steps per A slot
+    const uint32_t S = a.slots, SW = a.wstages;
+    const uint64_t bstep = a.b_stage_bytes >> 4;           // descriptor address units per stage
     const uint64_t hstep = (uint64_t)a.n_total * (128 >> 4);  // next 128-sample half of the stage
-    const uint32_t d_ind = tmem + a.n_main;
-    const uint32_t a0 = tmem + a.a_base;
-    uint32_t copy = 0, in_group = 0;   // accumulator copy of this stage, its place in the group
+    const bool alternate = a.kcopies == 2;
+    uint32_t copy = 0, in_group = 0, acc = 0;  // copy of this stage, its place in the group; 0 clears D
     for (uint32_t i = 0; i < nkb; ++i) {
-        if (!warp_wait_uniform(full_b + sw.slot, sw.phase, a.err, 25)) return false;
-        if (!warp_wait_uniform(full_a + st.slot, st.phase, a.err, 26)) return false;
-        fence_after();
-        const uint64_t bd = bdesc0 + sw.slot * bstep;
-        const uint32_t ad = a0 + st.slot * a.a_cols;
-        const uint32_t d_main = tmem + copy * a.d_cols;
-        const uint32_t acc0 = i > copy * a.group ? 1u : 0u;  // the copy's first stage clears it
+        if (!alternate || copy == m.copy) {
+            const uint64_t bd = bdesc0 + sw.slot * bstep + m.b_off;
 #pragma unroll
-        for (int kk = 0; kk < kStageK / 32; ++kk) {
-            const uint32_t acc = kk > 0 ? 1u : acc0;
-            const uint64_t bk = bd + (kk >> 2) * hstep + (kk & 3) * 2;
+            for (int part = 0; part < PARTS; ++part) {
+                if (part == 0 && !warp_wait(full_b + sw.slot, sw.phase, a.err, 25)) return false;
+                if (!warp_wait(full_a + st.slot, st.phase, a.err, 26)) return false;
+                fence_after();
+                const uint32_t ad = a0 + st.slot * a.a_cols + m.a_off;
 #pragma unroll
-            for (int ch = 0; ch < NCH; ++ch)
-                mma_ts_f8(d_main + ch * chunk, ad + kk * 8, bk + ch * chstep, id_main, acc, elected);
-            if (IND) mma_ts_f8(d_ind, ad + kStageK / 4 + kk * 8, bk + indoff, id_ind, acc, elected);
+                for (int s = 0; s < kSteps; ++s) {
+                    const int kk = part * kSteps + s;
+                    mma_ts_f8(m.d, ad + s * 8, bd + (kk >> 2) * hstep + (kk & 3) * 2, m.idesc, acc, elected);
+                    acc = 1u;
+                }
+                mma_commit(a_empty + st.slot, elected);
+                st.advance(1, S);
+            }
+            mma_commit(b_empty + sw.slot, elected);
+        } else {
+            st.advance(PARTS, S);
         }
-        mma_commit(a_empty + st.slot, elected);
-        mma_commit(b_empty + sw.slot, elected);
-        st.advance(1, S);
         sw.advance(1, SW);
-        if (a.kcopies == 2 && ++in_group == a.group) {
+        if (alternate && ++in_group == a.group) {
             in_group = 0;
             copy ^= 1u;
         }
     }
     return true;
+}
+
+// Half a row (128 codes, 32 B) of a stage.
+__device__ __forceinline__ void load_half(const uint8_t* tile, uint32_t row, uint32_t* w) {
+    const uint4* rp = reinterpret_cast<const uint4*>(tile + row * (kTileK / 4));
+    const uint4 x = rp[0], y = rp[1];
+    w[0] = x.x;
+    w[1] = x.y;
+    w[2] = x.z;
+    w[3] = x.w;
+    w[4] = y.x;
+    w[5] = y.y;
+    w[6] = y.z;
+    w[7] = y.w;
+}
+
+// The E4M3 bytes of half a row (128 codes): a 32-bit word holds 16 two-bit
+// codes; masking the even / odd codes into nibbles gives PRMT selectors
+// directly (4 codes per PRMT), and the B operand stores K in the matching
+// even-then-odd order.  With IND also the missing-call indicator's bytes.
+template <bool IND>
+__device__ __forceinline__ void expand_half(const uint32_t* w, uint32_t (&gv)[32], uint32_t (&mv)[32]) {
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const uint32_t e0 = w[t] & 0x33333333u, o0 = (w[t] >> 2) & 0x33333333u;
+        const uint32_t e1 = e0 >> 16, o1 = o0 >> 16;
+        gv[4 * t] = __byte_perm(kTabGeno, 0u, e0);
+        gv[4 * t + 1] = __byte_perm(kTabGeno, 0u, e1);
+        gv[4 * t + 2] = __byte_perm(kTabGeno, 0u, o0);
+        gv[4 * t + 3] = __byte_perm(kTabGeno, 0u, o1);
+        if (IND) {
+            mv[4 * t] = __byte_perm(kTabMiss, 0u, e0);
+            mv[4 * t + 1] = __byte_perm(kTabMiss, 0u, e1);
+            mv[4 * t + 2] = __byte_perm(kTabMiss, 0u, o0);
+            mv[4 * t + 3] = __byte_perm(kTabMiss, 0u, o1);
+        }
+    }
+}
+
+// One unpack warp's part of the CTA's items (all its units in sequence), a row
+// per lane expanded into TMEM.  An item, one A slot, is a stage's genotypes or,
+// with the indicator, half a stage's genotypes and indicator: that doubles the
+// ring where TMEM holds two stages only (D takes 224 of its 512 columns at 32
+// outputs).  A set takes items set, set + usets, ...  Everything is expanded
+// before the wait for the slot, so a freed slot is refilled by its stores alone.
+//
+// A packed slot is released once its codes are in registers.  The arrival's
+// count depends on them (`none` is 0), so it cannot be issued before the loads
+// have returned: released right behind the loads, the refill has been seen to
+// overtake them.
+template <bool IND>
+__device__ __forceinline__ void tc8_unpack(const Tc8Args& a, uint32_t a0, const uint8_t* psm, uint32_t row,
+                                           uint64_t* p_full, uint64_t* p_empty, uint64_t* full_a, uint64_t* a_empty,
+                                           uint32_t set, uint32_t stages) {
+    const uint32_t S = a.slots, P = a.pstages, nsets = a.usets;
+    const bool lane0 = (threadIdx.x & 31) == 0;
+    constexpr uint32_t kPerStage = IND ? 2 : 1;
+    const uint32_t items = stages * kPerStage;
+    Ring pr{set / kPerStage, 0}, st{set, 0};
+    for (uint32_t i = set; i < items; i += nsets) {
+        uint32_t w[IND ? 8 : 16], x[32], y[32];
+        if (!warp_wait(p_full + pr.slot, pr.phase, a.err, 27)) return;
+        const uint8_t* tile = psm + pr.slot * kStageBytes;
+        uint32_t seen;
+        if constexpr (IND) {
+            load_half(tile + (i & 1u) * kTileBytes, row, w);
+            seen = w[0] | w[4];
+        } else {
+            load_half(tile, row, w);
+            load_half(tile + kTileBytes, row, w + 8);
+            seen = w[0] | w[4] | w[8] | w[12];
+        }
+        __syncwarp();
+        if (lane0) mbar_arrive_n(p_empty + pr.slot, 1u + (seen & a.none));
+        pr.advance((i + nsets) / kPerStage - i / kPerStage, P);
+        if constexpr (IND) {
+            expand_half<true>(w, x, y);
+        } else {
+            expand_half<false>(w, x, x);
+            expand_half<false>(w + 8, y, y);
+        }
+        keep32(x);  // expanded before the slot wait: only the stores follow it
+        keep32(y);
+        const uint32_t a_col = a0 + st.slot * a.a_cols;
+        if (!warp_wait(a_empty + st.slot, st.phase ^ 1u, a.err, 28)) return;
+        tmem_st_x32(a_col, x);
+        tmem_st_x32(a_col + 32, y);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        fence_before();
+        __syncwarp();
+        if (lane0) mbar_arrive(full_a + st.slot);
+        st.advance(nsets, S);
+    }
+}
+
+__device__ __forceinline__ void fma16(const float* scl, const float (&v)[16], float (&acc)[16]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 f = reinterpret_cast<const float4*>(scl)[q];
+        acc[4 * q] = fmaf(f.x, v[4 * q], acc[4 * q]);
+        acc[4 * q + 1] = fmaf(f.y, v[4 * q + 1], acc[4 * q + 1]);
+        acc[4 * q + 2] = fmaf(f.z, v[4 * q + 2], acc[4 * q + 2]);
+        acc[4 * q + 3] = fmaf(f.w, v[4 * q + 3], acc[4 * q + 3]);
+    }
+}
+
+// 16 columns c0 .. of a warp's 32 rows from the accumulators: pm = sum_t
+// scale_t (sum of the copies), pi the indicator's terms.
+__device__ __forceinline__ void read_terms(const Tc8Args& a, uint32_t d0, const float* scl, uint32_t c0,
+                                           bool second_copy, float (&pm)[16], float (&pi)[16]) {
+    float v[16], v2[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) pm[k] = pi[k] = 0.f;
+    if (second_copy) {
+#pragma unroll 1
+        for (int t = 0; t < kMainTerms; ++t) {
+            const uint32_t col = t * a.wpad + c0;
+            tmem_ld_x16_async(d0 + col, v);
+            tmem_ld_x16_async(d0 + a.d_cols + col, v2);
+            tmem_ld_wait();
+            pin16(v);
+            pin16(v2);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] += v2[k];
+            fma16(scl + col, v, pm);
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int t = 0; t < kMainTerms; t += 2) {
+        const uint32_t col = t * a.wpad + c0;
+        tmem_ld_x16_async(d0 + col, v);
+        tmem_ld_x16_async(d0 + col + a.wpad, v2);
+        tmem_ld_wait();
+        pin16(v);
+        pin16(v2);
+        fma16(scl + col, v, pm);
+        fma16(scl + col + a.wpad, v2, pm);
+    }
+    if (a.n_ind) {
+        const uint32_t dcol = a.n_main + c0, scol = (a.ind_shared ? 0u : a.n_main) + c0;
+        tmem_ld_x16_async(d0 + dcol, v);
+        tmem_ld_x16_async(d0 + dcol + a.wpad, v2);
+        tmem_ld_wait();
+        pin16(v);
+        pin16(v2);
+        fma16(scl + scol, v, pi);
+        tmem_ld_x16_async(d0 + dcol + 2 * a.wpad, v);
+        fma16(scl + scol + a.wpad, v2, pi);
+        tmem_ld_wait();
+        pin16(v);
+        fma16(scl + scol + 2 * a.wpad, v, pi);
+    }
 }
 
 // One CTA per SM runs work units u = blockIdx.x, blockIdx.x + gridDim.x, ...
@@ -228,19 +382,19 @@ __device__ __forceinline__ bool tc8_mma_unit(const Tc8Args& a, uint32_t tmem, ui
 __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant__ Tc8Args a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t S = a.stages, SW = a.wstages, P = a.pstages;
+    const uint32_t S = a.slots, SW = a.wstages, P = a.pstages;
     uint8_t* bsm = smem;
     uint8_t* psm = bsm + SW * a.b_stage_bytes;
     float* scl = reinterpret_cast<float*>(psm + P * kStageBytes);             // up to 512 floats
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scl) + 2048);
     uint64_t* full_b = bars;                 // [SW] W stage landed (TMA tx)
     uint64_t* b_empty = bars + SW;           // [SW] the MMAs reading the W stage done
-    uint64_t* full_a = bars + 2 * SW;        // [S] A operand written to TMEM (128 arrivals)
-    uint64_t* a_empty = full_a + S;          // [S] the MMAs reading the A stage done
+    uint64_t* full_a = bars + 2 * SW;        // [S] A slot written to TMEM (4 warps)
+    uint64_t* a_empty = full_a + S;          // [S] the MMAs reading the A slot done
     uint64_t* p_full = a_empty + S;          // [P] packed codes landed (TMA tx)
-    uint64_t* p_empty = p_full + P;          // [P] packed codes consumed (4 warp arrivals)
+    uint64_t* p_empty = p_full + P;          // [P] packed codes in registers (4 or 8 warps)
     uint64_t* tmem_full = p_empty + P;       // a unit's MMAs done
-    uint64_t* d_empty = tmem_full + 1;       // a unit's epilogue has read D (8 unpack warps)
+    uint64_t* d_empty = tmem_full + 1;       // a unit's epilogue has read D (its warps)
     uint64_t* never = d_empty + 1;           // test hook: a barrier nothing arrives at
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(never + 1);
 
@@ -264,18 +418,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < SW; ++s) {
             mbar_init(full_b + s, 1);
-            mbar_init(b_empty + s, 1);
+            mbar_init(b_empty + s, a.kcopies == 2 ? 1 : 2);  // every MMA warp that reads the stage
         }
         for (uint32_t s = 0; s < S; ++s) {
             mbar_init(full_a + s, 4);     // one arrival per unpack warp
-            mbar_init(a_empty + s, 1);
+            mbar_init(a_empty + s, a.kcopies == 2 ? 1 : 2);
         }
         for (uint32_t p = 0; p < P; ++p) {
             mbar_init(p_full + p, 1);
-            mbar_init(p_empty + p, 4);
+            mbar_init(p_empty + p, 4 * a.parts);  // every unpack warp that reads the slot
         }
-        mbar_init(tmem_full, 1);
-        mbar_init(d_empty, 4 * kUnpackSets);
+        mbar_init(tmem_full, 2);
+        mbar_init(d_empty, kEpiWarps);
         mbar_init(never, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -311,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             const uint8_t* src = a.tiles + (uint64_t)(u % a.gx) * a.tile_bytes + (uint64_t)unit_kb0(u) * kStageBytes;
             uint32_t ks = unit_rot(u, nkb);
             for (uint32_t i = 0; i < nkb; ++i) {
-                ok = warp_wait_uniform(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21);
+                ok = warp_wait(p_empty + pr.slot, pr.phase ^ 1u, a.err, 21);
                 if (!ok) break;
                 bulk_g2s_tx(psm + pr.slot * kStageBytes, src + (uint64_t)ks * kStageBytes, kStageBytes,
                             p_full + pr.slot, elected);
@@ -333,7 +487,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             const uint8_t* src = a.wop + (uint64_t)unit_kb0(u) * a.b_stage_bytes;
             uint32_t ks = unit_rot(u, nkb);
             for (uint32_t i = 0; i < nkb; ++i) {
-                ok = warp_wait_uniform(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23);
+                ok = warp_wait(b_empty + wr.slot, wr.phase ^ 1u, a.err, 23);
                 if (!ok) break;
                 bulk_g2s_tx(bsm + wr.slot * a.b_stage_bytes, src + (uint64_t)ks * a.b_stage_bytes, a.b_stage_bytes,
                             full_b + wr.slot, elected);
@@ -343,10 +497,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             }
         }
         drain_ring(full_b, wr, lapped, SW, a.err, 24);
-    } else if (warp == 1) {
+    } else if (warp == 1 || warp == 3) {
         const uint32_t elected = elect_one();
-        const uint32_t bsm_addr = smem_u32(bsm);
-        const bool wide = a.n_main > 256;  // host guarantees an even split into <= 256-wide MMAs
+        const uint32_t second = warp == 3 ? 1u : 0u;
+        MmaShare m;
+        m.copy = second;
+        if (ind) {
+            m.idesc = instr_desc_e4m3(second ? a.n_ind : a.n_main);
+            m.d = tmem + (second ? a.n_main : 0u);
+            m.a_off = second ? a.a_cols / 2 : 0u;
+            m.b_off = second && !a.ind_shared ? a.n_main * (128 >> 4) : 0u;
+        } else {
+            const uint32_t n = a.kcopies == 2 ? a.n_main : a.n_main / 2;
+            m.idesc = instr_desc_e4m3(n);
+            m.d = tmem + second * (a.kcopies == 2 ? a.d_cols : n);
+            m.a_off = 0;
+            m.b_off = a.kcopies == 2 ? 0u : second * n * (128 >> 4);
+        }
+        const uint32_t a0 = tmem + a.a_base;
+        const uint64_t bdesc0 = smem_desc(smem_u32(bsm));
         Ring st{0, 0}, sw{0, 0};           // A ring (TMEM), W ring (shared memory)
         uint32_t k = 0;                    // this CTA's units so far
         bool ok = true;
@@ -354,165 +523,75 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
             const uint32_t nkb = unit_nkb(u);
             // D is free once the previous unit's epilogue has read it
             if (k > 0) {
-                ok = warp_wait_uniform(d_empty, (k - 1) & 1u, a.err, 31);
+                ok = warp_wait(d_empty, (k - 1) & 1u, a.err, 31);
                 fence_after();
             }
-            if (ok) {
-                if (ind)
-                    ok = wide ? tc8_mma_unit<2, true>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
-                                                      elected)
-                              : tc8_mma_unit<1, true>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw, nkb,
-                                                      elected);
-                else
-                    ok = wide ? tc8_mma_unit<2, false>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw,
-                                                       nkb, elected)
-                              : tc8_mma_unit<1, false>(a, tmem, bsm_addr, full_b, full_a, a_empty, b_empty, st, sw,
-                                                       nkb, elected);
-            }
-            mma_commit(tmem_full, elected);
+            if (ok)
+                ok = ind ? tc8_mma_unit<2>(a, m, a0, bdesc0, full_b, full_a, a_empty, b_empty, st, sw, nkb, elected)
+                         : tc8_mma_unit<1>(a, m, a0, bdesc0, full_b, full_a, a_empty, b_empty, st, sw, nkb, elected);
+            mma_commit(tmem_full, elected);  // both warps arrive per unit (an idle one at once)
         }
-    } else if (warp >= 4) {
-        // kUnpackSets sets of four unpack warps take the stages of the CTA's
-        // sequence round robin; warp % 4 is the TMEM lane quarter a warp may access
-        const uint32_t set = (uint32_t)(warp - 4) >> 2;
-        const uint32_t q = (uint32_t)warp & 3u;
-        const uint32_t row = q * 32 + lane;
-        const uint32_t lane_base = tmem + ((q * 32) << 16);
-        const uint32_t nsets = a.usets;
-        Ring pr{set, 0}, st{set, 0};  // this set's next stage (usets <= stages, pstages)
-        uint32_t ahead = set;         // its distance from the unit's first stage
+    } else if (warp >= kCtlWarps && warp < kCtlWarps + 4 * kUnpackSets) {
+        // sets of four unpack warps; warp % 4 is the TMEM lane quarter a warp
+        // may access
+        const uint32_t set = (uint32_t)(warp - kCtlWarps) >> 2;
+        if (set < a.usets) {
+            uint32_t stages = 0;  // of the CTA
+            for (uint32_t u = blockIdx.x; u < a.units; u += gridDim.x) stages += unit_nkb(u);
+            const uint32_t row = ((uint32_t)warp & 3u) * 32 + lane;
+            const uint32_t a0 = tmem + ((((uint32_t)warp & 3u) * 32) << 16) + a.a_base;
+            if (ind) tc8_unpack<true>(a, a0, psm, row, p_full, p_empty, full_a, a_empty, set, stages);
+            else tc8_unpack<false>(a, a0, psm, row, p_full, p_empty, full_a, a_empty, set, stages);
+        }
+    } else if (warp >= kCtlWarps + 4 * kUnpackSets) {
+        // epilogue warps: a unit's accumulators are read as soon as its MMAs
+        // are done and handed back (d_empty) before the results are formed and
+        // stored, while the unpack and MMA warps go on with the next unit
+        const uint32_t row = ((uint32_t)warp & 3u) * 32 + lane;
+        const uint32_t d0 = tmem + ((((uint32_t)warp & 3u) * 32) << 16);
+        const uint32_t cfirst = ((uint32_t)(warp - kCtlWarps - 4 * kUnpackSets) >> 2) * 16;  // 16-column groups in turn
         uint32_t k = 0;
-        bool ok = true;
-        for (uint32_t u = blockIdx.x; u < a.units && ok; u += gridDim.x, ++k) {
+        for (uint32_t u = blockIdx.x; u < a.units; u += gridDim.x, ++k) {
             const uint32_t nkb = unit_nkb(u);
-            for (; ahead < nkb && set < nsets; ahead += nsets) {
-                // one lane polls each barrier and the warp follows it (the warp
-                // barrier orders the other lanes after its observation)
-                if (!warp_wait(p_full + pr.slot, pr.phase, a.err, 27)) {
-                    ok = false;
-                    break;
-                }
-                // this row's 256 codes: 32 B in each of the stage's two tile blocks
-                const uint8_t* rp = psm + pr.slot * kStageBytes + row * (kTileK / 4);
-                const uint4 p0 = reinterpret_cast<const uint4*>(rp)[0], p1 = reinterpret_cast<const uint4*>(rp)[1];
-                const uint4 p2 = reinterpret_cast<const uint4*>(rp + kTileBytes)[0];
-                const uint4 p3 = reinterpret_cast<const uint4*>(rp + kTileBytes)[1];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_empty + pr.slot);   // codes are in registers: release the slot
-                // a 32-bit word holds 16 two-bit codes; masking the even / odd codes
-                // into nibbles gives PRMT selectors directly (4 codes per PRMT), and
-                // the B operand stores K in the matching even-then-odd order
-                const uint32_t w16[16] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w,
-                                          p2.x, p2.y, p2.z, p2.w, p3.x, p3.y, p3.z, p3.w};
-                uint32_t ev[16], od[16];
-#pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    ev[t] = w16[t] & 0x33333333u;
-                    od[t] = (w16[t] >> 2) & 0x33333333u;
-                }
-                uint32_t gv[32], h[32];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    gv[4 * t] = __byte_perm(kTabGeno, 0u, ev[t]);
-                    gv[4 * t + 1] = __byte_perm(kTabGeno, 0u, ev[t] >> 16);
-                    gv[4 * t + 2] = __byte_perm(kTabGeno, 0u, od[t]);
-                    gv[4 * t + 3] = __byte_perm(kTabGeno, 0u, od[t] >> 16);
-                    h[4 * t] = __byte_perm(kTabGeno, 0u, ev[8 + t]);
-                    h[4 * t + 1] = __byte_perm(kTabGeno, 0u, ev[8 + t] >> 16);
-                    h[4 * t + 2] = __byte_perm(kTabGeno, 0u, od[8 + t]);
-                    h[4 * t + 3] = __byte_perm(kTabGeno, 0u, od[8 + t] >> 16);
-                }
-                keep32(gv);  // expanded before the stage wait: only the stores follow it
-                keep32(h);
-                if (!warp_wait(a_empty + st.slot, st.phase ^ 1u, a.err, 28)) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t a_col = lane_base + a.a_base + st.slot * a.a_cols;
-                tmem_st_x32(a_col, gv);
-                tmem_st_x32(a_col + 32, h);
-                if (ind) {
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) {
-                        gv[4 * t] = __byte_perm(kTabMiss, 0u, ev[t]);
-                        gv[4 * t + 1] = __byte_perm(kTabMiss, 0u, ev[t] >> 16);
-                        gv[4 * t + 2] = __byte_perm(kTabMiss, 0u, od[t]);
-                        gv[4 * t + 3] = __byte_perm(kTabMiss, 0u, od[t] >> 16);
-                        h[4 * t] = __byte_perm(kTabMiss, 0u, ev[8 + t]);
-                        h[4 * t + 1] = __byte_perm(kTabMiss, 0u, ev[8 + t] >> 16);
-                        h[4 * t + 2] = __byte_perm(kTabMiss, 0u, od[8 + t]);
-                        h[4 * t + 3] = __byte_perm(kTabMiss, 0u, od[8 + t] >> 16);
-                    }
-                    tmem_st_x32(a_col + 64, gv);
-                    tmem_st_x32(a_col + 96, h);
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_a + st.slot);
-                pr.advance(nsets, P);
-                st.advance(nsets, S);
-            }
-            if (!ok) break;
-            ahead -= nkb;
-            // epilogue of unit u: the sets take 16-column groups round robin
-            ok = warp_wait(tmem_full, k & 1u, a.err, 29);
-            // the second accumulator copy holds data only if its first group exists
-            const bool second_copy = a.kcopies == 2 && nkb > a.group;
-            fence_after();
             const uint32_t grow = (u % a.gx) * kM + row;
-            const bool live = ok && grow < a.rows;
+            const bool live = grow < a.rows;
             double rm = 0.0, rs = 0.0;
             if (a.mode == 1 && live) {
                 rm = a.row_mean[grow];
                 rs = a.row_scale[grow];
             }
             float* dst = a.out + (uint64_t)(u / a.gx) * a.split_stride + (uint64_t)grow * a.ldo;
-            for (uint32_t c0 = set * 16; c0 < a.wpad && ok; c0 += 16 * kUnpackSets) {
-                float pm[16], pi[16], v[16];
-#pragma unroll
-                for (int kk = 0; kk < 16; ++kk) pm[kk] = pi[kk] = 0.f;
-                for (int t = 0; t < kMainTerms; ++t) {
-                    const uint32_t col = t * a.wpad + c0;
-                    tmem_ld_x16(lane_base + col, v);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (second_copy) {
-                        float v2[16];
-                        tmem_ld_x16(lane_base + a.d_cols + col, v2);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int kk = 0; kk < 16; ++kk) v[kk] += v2[kk];
-                    }
-#pragma unroll
-                    for (int kk = 0; kk < 16; ++kk) pm[kk] = fmaf(scl[col + kk], v[kk], pm[kk]);
+            if (!warp_wait(tmem_full, k & 1u, a.err, 29)) break;
+            // the second accumulator copy holds data only if its first group exists
+            const bool second_copy = a.kcopies == 2 && nkb > a.group;
+            fence_after();
+            for (uint32_t c0 = cfirst;; c0 += 4 * kEpiWarps) {
+                float pm[16], pi[16];
+                if (c0 < a.wpad) read_terms(a, d0, scl, c0, second_copy, pm, pi);
+                if (c0 + 4 * kEpiWarps >= a.wpad) {
+                    // this warp's last read: D may be overwritten by the next unit's MMAs
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty);
                 }
-                if (ind) {
-                    for (int t = 0; t < kIndTerms; ++t) {
-                        const uint32_t col = a.n_main + t * a.wpad + c0;
-                        const uint32_t scol = (a.ind_shared ? 0u : a.n_main) + t * a.wpad + c0;
-                        tmem_ld_x16(lane_base + col, v);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int kk = 0; kk < 16; ++kk) pi[kk] = fmaf(scl[scol + kk], v[kk], pi[kk]);
-                    }
-                }
-                if (live) {
-#pragma unroll
-                    for (int kk = 0; kk < 16; ++kk) {
-                        if (a.mode == 1)
-                            v[kk] = (float)(rs * ((double)pm[kk] - rm * (a.cs[c0 + kk] - (double)pi[kk])));
-                        else
-                            v[kk] = pm[kk] + pi[kk];
-                    }
+                if (c0 < a.wpad && live) {
                     float4* d4 = reinterpret_cast<float4*>(dst + c0);
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) d4[t] = make_float4(v[4 * t], v[4 * t + 1], v[4 * t + 2], v[4 * t + 3]);
+                    for (int t = 0; t < 4; ++t) {
+                        float o[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int kk = 4 * t + q;
+                            if (a.mode == 1)
+                                o[q] = (float)(rs * ((double)pm[kk] - rm * (a.cs[c0 + kk] - (double)pi[kk])));
+                            else
+                                o[q] = pm[kk] + pi[kk];
+                        }
+                        d4[t] = make_float4(o[0], o[1], o[2], o[3]);
+                    }
                 }
+                if (c0 + 4 * kEpiWarps >= a.wpad) break;
             }
-            // D may be overwritten by the next unit's MMAs
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(d_empty);
         }
     }
     fence_before();
@@ -812,9 +891,9 @@ static int env_int(const char* name, int dflt) {
     return v && *v ? std::atoi(v) : dflt;
 }
 
-// The plan with explicit caps on the packed-code ring (pmax), the W ring
-// (smax) and the MMA wait group (gmax); fp8_plan takes them from the
-// environment (defaults 8, 8, 4).
+// The plan with explicit caps on the packed-code ring (pmax), the A ring (smax
+// stages), the K blocks per group of an accumulator copy (gmax: 1 or 2) and the
+// W ring (wmax); fp8_plan takes them from the environment.
 Fp8Plan fp8_plan_knobs(int wpad, bool ind, uint64_t tiles, int pmax_in, int smax, int gmax_in, int wmax,
                        bool ind_shared) {
     Fp8Plan p{};
@@ -824,51 +903,55 @@ Fp8Plan fp8_plan_knobs(int wpad, bool ind, uint64_t tiles, int pmax_in, int smax
     p.ind_shared = (ind && ind_shared) ? 1u : 0u;
     p.n_total = p.ind_shared ? p.n_main : p.n_main + p.n_ind;      // B rows
     p.d_cols = (uint32_t)round_up(p.n_main + p.n_ind, 32);       // accumulator columns
-    p.a_cols = (ind ? 2 : 1) * (kStageK / 4);  // TMEM columns of one stage's A operand(s)
+    const uint32_t a_stage = (ind ? 2 : 1) * (kStageK / 4);  // TMEM columns of one stage's A operand(s)
     p.b_stage_bytes = p.n_total * 128 * kHalves;  // one bulk copy: 16-byte multiple, below the 1 MB tx limit
-    // one CTA per SM: all of TMEM; the packed-code ring gives up depth (8, 4,
-    // then 2 stages) until shared memory holds at least two W stages
-    p.tmem_cols = 512;
+    p.tmem_cols = 512;  // one CTA per SM: all of TMEM
     const size_t fixed = 1024 + 2048 + 128 * 8 + 64;
-    // MMA warp roles: with the indicator, genotype and indicator MMAs on
-    // separate warps; without it, two accumulator copies when TMEM holds them
-    // next to at least three A stages
-    p.nsplit = ind ? 1 : 0;
-    p.kcopies = (!ind && 2 * p.d_cols + 3 * p.a_cols <= 512) ? 2 : 1;
+    // without the indicator two accumulator copies when TMEM holds them next to
+    // at least three A stages; alternate pairs of K blocks go to them
+    p.kcopies = (!ind && 2 * p.d_cols + 3 * a_stage <= 512) ? 2 : 1;
+    p.group = gmax_in >= 2 ? 2 : 1;
     p.a_base = p.kcopies * p.d_cols;
-    const uint32_t by_tmem = p.a_base < 512 ? (512 - p.a_base) / p.a_cols : 0;
-    // A ring: as deep as TMEM allows (cap smax).  W ring: its own depth in
-    // shared memory, at least one stage more than the A ring and at least 3
-    // where it fits (cap wmax): a W stage is refilled only after the MMAs on
-    // it complete, and the refill comes from L2 (the same W for every CTA).
-    // The packed-code ring gives up depth (pmax, halving down to 2) for it.
-    p.stages = std::min<uint32_t>(by_tmem, (uint32_t)std::max(1, smax));
-    const uint32_t pmax = (uint32_t)std::min(16, std::max(2, pmax_in));
+    // A ring: as deep as TMEM allows (cap smax stages), whole stages or, with
+    // the indicator, half stages, an even number of them
+    p.parts = ind ? 2 : 1;
+    p.a_cols = a_stage / p.parts;
+    const uint32_t by_tmem = p.a_base < 512 ? (512 - p.a_base) / a_stage : 0;
+    const uint32_t cap = (uint32_t)std::max(1, smax) * p.parts;
+    p.slots = p.a_base < 512 ? std::min<uint32_t>((512 - p.a_base) / p.a_cols / p.parts * p.parts, cap) : 0;
+    // Shared memory: 4, 3 or 2 W stages (caps wmax, and pmax for the codes), then
+    // packed-code stages, up to 8, then more W stages if they fit.  Four of
+    // each where they fit: 32 KB W stages and 8 KB code stages stream at 435
+    // cycles per stage with 4 + 8 and 507 with 5 + 4 (the MMAs take 512).
+    const uint32_t pmax = (uint32_t)std::min(16, std::max(2, pmax_in)) & ~1u;
     const uint32_t wcap = (uint32_t)std::max(1, std::min(16, wmax));
-    const uint32_t wwant = std::min(wcap, std::max(p.stages + 1, 3u));
-    uint32_t by_smem = 0;
-    for (p.pstages = pmax;; p.pstages /= 2) {
-        const size_t budget = 225 * 1024 - fixed - (size_t)p.pstages * kStageBytes;
-        by_smem = (uint32_t)(budget / p.b_stage_bytes);
-        if (by_smem >= wwant || p.pstages <= 2) break;
+    const size_t budget = 225 * 1024 - fixed;
+    uint32_t pfit = 0;
+    for (p.wstages = std::min(wcap, 4u);; --p.wstages) {
+        const size_t wb = (size_t)p.wstages * p.b_stage_bytes;
+        pfit = wb < budget ? (uint32_t)((budget - wb) / kStageBytes) & ~1u : 0u;
+        if (pfit >= 4 || p.wstages <= 2) break;
     }
-    p.wstages = std::min(by_smem, wcap);
-    p.stages = std::min(p.stages, p.wstages);
-    // MMA wait groups: up to 16 MMAs per wait and warp, at least two groups in the ring
-    const uint32_t nch = p.n_main > 256 ? 2 : 1;
-    const uint32_t per_stage = (kStageK / 32) * (p.nsplit || p.kcopies == 2 ? nch : nch + (ind ? 1 : 0));
-    p.group = 1;
-    const uint32_t gmax = (uint32_t)gmax_in;
-    for (uint32_t gsz : {4u, 2u})
-        if (gsz <= gmax && gsz * per_stage <= 16 && p.stages >= 2 * gsz) {
-            p.group = gsz;
-            break;
-        }
-    p.stages -= p.stages % p.group;
+    p.pstages = std::max(2u, std::min(pfit, pmax));
+    while (p.wstages < wcap &&
+           (size_t)(p.wstages + 1) * p.b_stage_bytes + (size_t)p.pstages * kStageBytes <= budget)
+        ++p.wstages;
+    // A wait by phase parity must know the use before the awaited one to be
+    // over.  Two accumulator copies are worked on by two MMA warps that run
+    // independently, in turns of group stages: their A and W slots stay with one
+    // warp (a multiple of two turns deep; both fit whatever the caps).  With one
+    // copy the MMAs complete in item order, and at most one unpack set per A
+    // slot suffices.
+    if (p.kcopies == 2) {
+        p.slots = 4;
+        p.wstages = std::max(4u, p.wstages & ~3u);
+    }
+    p.usets = std::min<uint32_t>(kUnpackSets, std::max(p.slots, 1u));
     p.smem = fixed + (size_t)p.pstages * kStageBytes + (size_t)p.wstages * p.b_stage_bytes;
     (void)tiles;
-    p.ok = p.n_total % 8 == 0 && p.stages >= 2 && p.n_main % ceil_div(p.n_main, 256) == 0 && (p.n_main / ceil_div(p.n_main, 256)) % 16 == 0 &&
-           p.n_ind <= 256;
+    p.ok = p.n_total % 8 == 0 && by_tmem >= 2 && p.slots >= 2 * p.parts && p.wstages >= 2 &&
+           (size_t)p.wstages * p.b_stage_bytes + (size_t)p.pstages * kStageBytes <= budget &&
+           p.n_main <= 512 && p.n_ind <= 256;
     return p;
 }
 
@@ -1246,7 +1329,7 @@ static Fp8Plan tc8_tuned_plan(Ctx& c, const Fp8Plan& pl, const TileView& tv, uin
     for (int pmax : {2, 4, 8, 16})
         for (int smax : {2, 3, 4, 8}) {
             const Fp8Plan q = rebuild(pmax, smax);
-            if (!q.ok || q.group != pl.group || q.kcopies != pl.kcopies || q.nsplit != pl.nsplit) continue;
+            if (!q.ok || q.group != pl.group || q.kcopies != pl.kcopies) continue;
             float ms = 1e30f;
             for (int rep = 0; rep < 2; ++rep) {
                 SLFMM_CUDA(cudaEventRecord(e0, c.stream));
@@ -1319,13 +1402,15 @@ static int tc8_launch(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t ro
     a.ind_shared = pl.ind_shared;
     a.d_cols = pl.d_cols;
     a.a_cols = pl.a_cols;
-    a.stages = pl.stages;
+    a.parts = pl.parts;
+    a.slots = pl.slots;
     a.wstages = pl.wstages;
     a.pstages = pl.pstages;
     a.group = pl.group;
     a.kcopies = pl.kcopies;
     a.a_base = pl.a_base;
-    a.usets = std::min<uint32_t>(kUnpackSets, std::min(pl.stages, pl.pstages));
+    a.usets = pl.usets;
+    a.none = 0;
     a.tmem_cols = pl.tmem_cols;
     a.b_stage_bytes = pl.b_stage_bytes;
     a.inv_scale = inv_scale;
@@ -1363,9 +1448,9 @@ static int tc8_launch(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t ro
         cudaGetLastError();
         char buf[320];
         snprintf(buf, sizeof buf,
-                 "split-FP8 contraction launch failed (%s): units %u x %u, smem %zu, stages %u/%u, pstages %u, "
+                 "split-FP8 contraction launch failed (%s): units %u x %u, smem %zu, slots %u, stages %u, pstages %u, "
                  "group %u, n_total %u, rows %llu, K %llu",
-                 cudaGetErrorString(le), gx, gy, pl.smem, pl.stages, pl.wstages, pl.pstages, pl.group, pl.n_total,
+                 cudaGetErrorString(le), gx, gy, pl.smem, pl.slots, pl.wstages, pl.pstages, pl.group, pl.n_total,
                  (unsigned long long)rows, (unsigned long long)K);
         throw Error(SLFMM_ERR_CUDA, buf);
     }

@@ -290,8 +290,8 @@ void launch_scale_product(Ctx& c, const double* a, const double* b, uint64_t n, 
 // k_tc8.cu : split-FP8 tcgen05 contractions with optional missing-call
 // indicator operand
 struct Fp8Plan {
-    uint32_t wpad, n_main, n_ind, n_total, d_cols, a_cols, stages, wstages, pstages, group, tmem_cols, b_stage_bytes;
-    uint32_t kcopies, nsplit, a_base;
+    uint32_t wpad, n_main, n_ind, n_total, d_cols, a_cols, parts, slots, wstages, pstages, group, tmem_cols, b_stage_bytes;
+    uint32_t kcopies, a_base, usets;
     uint32_t ind_shared;  // indicator MMAs read the leading main terms (B holds n_main rows)
     size_t smem;
     bool ok;
