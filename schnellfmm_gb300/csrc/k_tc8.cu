@@ -924,7 +924,7 @@ Fp8Plan fp8_plan_knobs(int wpad, bool ind, uint64_t tiles, int pmax_in, int smax
     // each where they fit: 32 KB W stages and 8 KB code stages stream at 435
     // cycles per stage with 4 + 8 and 507 with 5 + 4 (the MMAs take 512).
     const uint32_t pmax = (uint32_t)std::min(16, std::max(2, pmax_in)) & ~1u;
-    const uint32_t wcap = (uint32_t)std::max(1, std::min(16, wmax));
+    const uint32_t wcap = (uint32_t)std::max(p.kcopies == 2 ? 4 : 1, std::min(16, wmax));
     const size_t budget = 225 * 1024 - fixed;
     uint32_t pfit = 0;
     for (p.wstages = std::min(wcap, 4u);; --p.wstages) {
@@ -944,7 +944,7 @@ Fp8Plan fp8_plan_knobs(int wpad, bool ind, uint64_t tiles, int pmax_in, int smax
     // slot suffices.
     if (p.kcopies == 2) {
         p.slots = 4;
-        p.wstages = std::max(4u, p.wstages & ~3u);
+        p.wstages &= ~3u;
     }
     p.usets = std::min<uint32_t>(kUnpackSets, std::max(p.slots, 1u));
     p.smem = fixed + (size_t)p.pstages * kStageBytes + (size_t)p.wstages * p.b_stage_bytes;
