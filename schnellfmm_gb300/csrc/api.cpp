@@ -787,16 +787,19 @@ void step0(Ctx& c, const double* x_host, uint64_t n, int d, double lambda, bool 
     SLFMM_CUDA(cudaMemcpyAsync(gtmp.get(), gx.get(), d * d * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
     launch_jacobi_svd(c, gtmp.get(), d, V.get(), sig.get());
     // ridge: (X^T X + lambda I)^-1 with safe_inv semantics
-    std::vector<double> gxh = fetch(c, gx.get(), (size_t)d * d);
-    for (int j = 0; j < d; ++j) gxh[j * d + j] += lambda;
-    DBuf<double> gl = upload(c, gxh.data(), gxh.size());
     s.ridge_inv.alloc(d * d, c.stream);
     DBuf<int> st(1, c.stream);
     DBuf<double> eps(1, c.stream);
-    launch_inverse(c, gl.get(), d, s.ridge_inv.get(), st.get(), eps.get());
-    std::vector<double> Vh = fetch(c, V.get(), (size_t)d * d);
-    std::vector<double> ev = fetch(c, sig.get(), (size_t)d);
-    safe_inv_report(fetch(c, st.get(), 1)[0], fetch(c, eps.get(), 1)[0], "X^T X + \u03bbI (ridge)");
+    const InverseJob ridge{gx.get(), d, lambda, s.ridge_inv.get(), st.get(), eps.get()};
+    launch_inverses(c, &ridge, 1);
+    std::vector<double> Vh((size_t)d * d), ev(d), epsh(1);
+    std::vector<int> sth(1);
+    d2h(c, Vh.data(), V.get(), Vh.size());
+    d2h(c, ev.data(), sig.get(), ev.size());
+    d2h(c, sth.data(), st.get(), 1);
+    d2h(c, epsh.data(), eps.get(), 1);
+    sync(c);
+    safe_inv_report(sth[0], epsh[0], "X^T X + \u03bbI (ridge)");
     // kept directions: sigma_j^2 = eigenvalue of X^T X
     std::vector<int> keep;
     const double emax = ev.empty() ? 0.0 : ev[0];
@@ -852,21 +855,18 @@ void cholqr2_f32(Ctx& c, float* Z, uint64_t m, int a, int ld) {
     DBuf<int> st(1, c.stream);
     for (int round = 0; round < 2; ++round) {
         launch_gram_f32(c, Z, ld, m, a, G.get());
-        launch_cholesky(c, G.get(), a, st.get());
-        launch_tri_inv_lower(c, G.get(), a, Linv.get());
+        launch_chol_inv(c, G.get(), a, Linv.get(), false, st.get());
         launch_trmul_f32(c, Z, ld, m, a, Linv.get());
     }
 }
 
 void cholqr2_f64(Ctx& c, double* A, uint64_t m, int a, int ld) {
     ProfScope ps(c, "cholqr2", 2.0 * m * a * 8, 4.0 * m * a * a);
-    DBuf<double> G(a * a, c.stream), Linv(a * a, c.stream), LinvT(a * a, c.stream), tmp(m * a, c.stream);
+    DBuf<double> G(a * a, c.stream), LinvT(a * a, c.stream), tmp(m * a, c.stream);
     DBuf<int> st(1, c.stream);
     for (int round = 0; round < 2; ++round) {
         launch_atb(c, A, ld, A, ld, m, a, a, G.get());
-        launch_cholesky(c, G.get(), a, st.get());
-        launch_tri_inv_lower(c, G.get(), a, Linv.get());
-        launch_transpose(c, Linv.get(), a, a, LinvT.get());
+        launch_chol_inv(c, G.get(), a, LinvT.get(), true, st.get());
         launch_gemm_small(c, A, ld, m, a, LinvT.get(), a, a, 1.0, 0.0, tmp.get(), a);
         SLFMM_CUDA(cudaMemcpy2DAsync(A, ld * sizeof(double), tmp.get(), a * sizeof(double), a * sizeof(double), m,
                                      cudaMemcpyDeviceToDevice, c.stream));
@@ -979,22 +979,23 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     // by 1/sqrt(eps)).  RSS, SS_cov and beta depend only on span(C), which
     // the column-dropping factorisation spans exactly.
     double ctc_eps = 0.0;
-    {
-        DBuf<double> inv((size_t)w * w, c.stream), epsd(1, c.stream);
-        DBuf<int> sti(1, c.stream);
-        if (d > 0) {
-            DBuf<double> xtx((size_t)d * d, c.stream);
-            launch_atb(c, s0.xs.get(), d, s0.xs.get(), d, n, d, d, xtx.get());
-            launch_inverse(c, xtx.get(), d, inv.get(), sti.get(), epsd.get());
-            safe_inv_report(fetch(c, sti.get(), 1)[0], fetch(c, epsd.get(), 1)[0], "X^T X for sequential R^2");
-        }
-        launch_inverse(c, G.get(), w, inv.get(), sti.get(), epsd.get());
-        const int status = fetch(c, sti.get(), 1)[0];
-        const double eps = fetch(c, epsd.get(), 1)[0];
-        safe_inv_report(status, eps, "C^T C  where C = [1 | X | U_hat]");
-        if (status == 1) ctc_eps = eps;
-    }
-    std::vector<double> Gh = fetch(c, G.get(), (size_t)w * w);
+    DBuf<double> UtU(K * K, c.stream), UtUi(K * K, c.stream), xtx((size_t)d * d, c.stream), epsd(3, c.stream);
+    DBuf<int> std3(3, c.stream);
+    launch_atb(c, s0.xs.get(), d, s0.xs.get(), d, n, d, d, xtx.get());
+    launch_atb(c, u_hat_dev, K, u_hat_dev, K, n, K, K, UtU.get());
+    const InverseJob jobs[3] = {{xtx.get(), d, 0.0, nullptr, std3.get(), epsd.get()},
+                                {G.get(), w, 0.0, nullptr, std3.get() + 1, epsd.get() + 1},
+                                {UtU.get(), K, 0.0, UtUi.get(), std3.get() + 2, epsd.get() + 2}};
+    launch_inverses(c, jobs, 3);
+    std::vector<double> Gh((size_t)w * w), epsh(3);
+    std::vector<int> sth(3);
+    d2h(c, Gh.data(), G.get(), Gh.size());
+    d2h(c, sth.data(), std3.get(), 3);
+    d2h(c, epsh.data(), epsd.get(), 3);
+    sync(c);
+    safe_inv_report(sth[0], epsh[0], "X^T X for sequential R^2");
+    safe_inv_report(sth[1], epsh[1], "C^T C  where C = [1 | X | U_hat]");
+    if (sth[1] == 1) ctc_eps = epsh[1];
     const std::vector<double> Graw = Gh;  // unnormalised C^T C
     std::vector<double> f(w);
     for (int k = 0; k < w; ++k) f[k] = Gh[k * w + k] > 0 ? 1.0 / std::sqrt(Gh[k * w + k]) : 0.0;
@@ -1006,9 +1007,8 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
         if (f[k] == 0.0) Gh[k * w + k] = 0.0;
     DBuf<double> L = upload(c, Gh.data(), Gh.size());
     DBuf<int> st1(1, c.stream), dropped(w, c.stream);
-    launch_cholesky(c, L.get(), w, st1.get(), 1e-10, dropped.get());
     DBuf<double> Linv(w * w, c.stream);
-    launch_tri_inv_lower(c, L.get(), w, Linv.get());
+    launch_chol_inv(c, L.get(), w, Linv.get(), false, st1.get(), 1e-10, dropped.get());
     std::vector<double> Li = fetch(c, Linv.get(), (size_t)w * w);
     std::vector<int> dr = fetch(c, dropped.get(), (size_t)w);
     for (int k = 0; k < w; ++k)
@@ -1109,19 +1109,15 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     }
     // beta rows: R ((I - P_U) X)^T Q_C  (src/testing.rs:285-296, 360-362)
     {
-        DBuf<double> UtU(K * K, c.stream), UtUi(K * K, c.stream), M1(K * d, c.stream), M2(K * d, c.stream),
-            F(n * d, c.stream), FtQ(d * w, c.stream), Bpp(d * w, c.stream);
-        DBuf<int> sti(1, c.stream);
-        DBuf<double> epsd(1, c.stream);
-        launch_atb(c, u_hat_dev, K, u_hat_dev, K, n, K, K, UtU.get());
-        launch_inverse(c, UtU.get(), K, UtUi.get(), sti.get(), epsd.get());
+        DBuf<double> M1(K * d, c.stream), M2(K * d, c.stream), F(n * d, c.stream), FtQ(d * w, c.stream),
+            Bpp(d * w, c.stream);
         launch_atb(c, u_hat_dev, K, s0.xs.get(), d, n, K, d, M1.get());
         launch_gemm_small(c, UtUi.get(), K, K, K, M1.get(), d, d, 1.0, 0.0, M2.get(), d);
         SLFMM_CUDA(cudaMemcpyAsync(F.get(), s0.xs.get(), n * d * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
         launch_gemm_small(c, u_hat_dev, K, n, K, M2.get(), d, d, -1.0, 1.0, F.get(), d);
         launch_atb(c, F.get(), d, QC.get(), w, n, d, w, FtQ.get());
         launch_gemm_small(c, s0.ridge_inv.get(), d, d, d, FtQ.get(), w, w, 1.0, 0.0, Bpp.get(), w);
-        safe_inv_report(fetch(c, sti.get(), 1)[0], fetch(c, epsd.get(), 1)[0], "U_hat^T U_hat");
+        safe_inv_report(sth[2], epsh[2], "U_hat^T U_hat");
         std::vector<double> Bh = fetch(c, Bpp.get(), (size_t)d * w);
         for (int jj = 0; jj < d; ++jj)
             for (int k = 1; k < w; ++k) bt[jj * wu + (k - 1)] = (float)Bh[jj * w + k];

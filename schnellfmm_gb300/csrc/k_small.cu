@@ -405,51 +405,72 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __re
 }
 
 // A (m x a, a <= 32, lda % 4 == 0, rows 16-byte aligned) <- A Linv^T in
-// place for a lower-triangular Linv, one row per thread: the row is read as
-// 16-byte loads (elements past a zero), out[c] = sum_{k <= c} row[k] R[c][k]
-// with R = Linv in FP32 passed as a kernel parameter -- every FMA takes its R
-// operand from the constant bank, the same for the whole warp -- and the row
-// is written back.
-struct Mat32 {
-    float v[32][32];
-};
+// place for a lower-triangular Linv, two rows per thread: a row is read as
+// 16-byte loads, out[c] = sum_{k <= c} row[k] Linv[c][k] in the order of k, and
+// written back.  Linv sits in shared memory in FP32, transposed, so that the
+// factors of four outputs are one broadcast 16-byte load for both rows (144
+// loads per 1056 products).  Taken from device memory: as a kernel parameter it
+// cost a copy to the host and a synchronisation per call, six per fit.
+constexpr int kTrmulRows = 2;
 __global__ void __launch_bounds__(256) k_trmul_rows(float* __restrict__ A, int lda, uint64_t m, int a,
-                                                    const __grid_constant__ Mat32 R) {
-    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < m; i += (uint64_t)gridDim.x * 256) {
-        float* row = A + i * lda;
-        float x[32];
+                                                    const double* __restrict__ Linv) {
+    __shared__ __align__(16) float Rt[32][32];  // Rt[k][c] = Linv[c][k], zero padded
+    for (int e = threadIdx.x; e < 32 * 32; e += 256) {
+        const int k = e >> 5, c = e & 31;
+        Rt[k][c] = (k <= c && c < a) ? (float)Linv[c * a + k] : 0.f;
+    }
+    __syncthreads();
+    const uint64_t step = (uint64_t)gridDim.x * 256;
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < m; i += kTrmulRows * step) {
+        float o[kTrmulRows][32];
+#pragma unroll
+        for (int r = 0; r < kTrmulRows; ++r)
+#pragma unroll
+            for (int c = 0; c < 32; ++c) o[r][c] = 0.f;
 #pragma unroll
         for (int kq = 0; kq < 8; ++kq) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (4 * kq < a) {
-                v = reinterpret_cast<const float4*>(row)[kq];
-                if (4 * kq + 4 > a) {
-                    v.y = 4 * kq + 1 < a ? v.y : 0.f;
-                    v.z = 4 * kq + 2 < a ? v.z : 0.f;
-                    v.w = 4 * kq + 3 < a ? v.w : 0.f;
+            if (4 * kq >= a) break;
+            float x[kTrmulRows][4];
+#pragma unroll
+            for (int r = 0; r < kTrmulRows; ++r) {
+                const uint64_t row = i + r * step;
+                const float4 v = row < m ? row_quad(A + row * lda, kq, a) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[r][0] = v.x;
+                x[r][1] = v.y;
+                x[r][2] = v.z;
+                x[r][3] = v.w;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const int k = 4 * kq + kk;
+#pragma unroll
+                for (int cq = kq; cq < 8; ++cq) {
+                    const float4 f = reinterpret_cast<const float4*>(Rt[k])[cq];
+                    const float ff[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (4 * cq + j >= k)
+#pragma unroll
+                            for (int r = 0; r < kTrmulRows; ++r)
+                                o[r][4 * cq + j] = fmaf(x[r][kk], ff[j], o[r][4 * cq + j]);
                 }
             }
-            x[4 * kq] = v.x;
-            x[4 * kq + 1] = v.y;
-            x[4 * kq + 2] = v.z;
-            x[4 * kq + 3] = v.w;
         }
-        float o[32];
 #pragma unroll
-        for (int c = 0; c < 32; ++c) o[c] = 0.f;
-        // Linv is lower triangular: R[c][k] = 0 for k > c (528 products)
+        for (int r = 0; r < kTrmulRows; ++r) {
+            const uint64_t row = i + r * step;
+            if (row >= m) break;
+            float* dst = A + row * lda;
 #pragma unroll
-        for (int k = 0; k < 32; ++k)
+            for (int cq = 0; cq < 8; ++cq) {
+                if (4 * cq + 4 <= a) {
+                    reinterpret_cast<float4*>(dst)[cq] =
+                        make_float4(o[r][4 * cq], o[r][4 * cq + 1], o[r][4 * cq + 2], o[r][4 * cq + 3]);
+                } else if (4 * cq < a) {
 #pragma unroll
-            for (int c = k; c < 32; ++c) o[c] = fmaf(x[k], R.v[c][k], o[c]);
-#pragma unroll
-        for (int cq = 0; cq < 8; ++cq) {
-            if (4 * cq + 4 <= a) {
-                reinterpret_cast<float4*>(row)[cq] = make_float4(o[4 * cq], o[4 * cq + 1], o[4 * cq + 2], o[4 * cq + 3]);
-            } else if (4 * cq < a) {
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj)
-                    if (4 * cq + jj < a) row[4 * cq + jj] = o[4 * cq + jj];
+                    for (int jj = 0; jj < 4; ++jj)
+                        if (4 * cq + jj < a) dst[4 * cq + jj] = o[r][4 * cq + jj];
+                }
             }
         }
     }
@@ -600,6 +621,146 @@ __global__ void k_tri_inv_lower(const double* __restrict__ L, int a, double* __r
     }
 }
 
+// Cholesky factor and its inverse in one pass: X = L^-1 of G = L L^T (G read
+// only), with the pivot rules of k_cholesky.  A thread keeps its elements (i, j),
+// j <= i, of the packed lower triangle in registers: element (i, j) is S_ij
+// until step j makes it L_ij, then the running right-hand side s_ij of X's
+// forward substitution, which step i divides by the pivot.  Step k updates every
+// element below row k by one FMA with the same operand pair in both roles,
+//   S_ij -= L_ik L_jk (j > k),   s_ij -= L_ik X_kj (j <= k),
+// so both recurrences run their terms in the order of k_cholesky and
+// k_tri_inv_lower and give the same bits.
+//
+// One SM issues an FP64 warp instruction per scheduler every 64 cycles
+// (sqrt about 690 cycles, a division 570, measured), so a step is the chain
+// sqrt, division, FMA, whatever the width up to 32: the division of all a
+// elements of the step's column and row is one warp instruction stream.  The
+// two kernels it replaces also divided integers per element and ran the
+// substitution as one dependent FMA chain per column: 20 x 20 27 + 20 us,
+// 30 x 30 28 + 24 us, against 15 and 26 us.
+template <int T, int R>
+__global__ void __launch_bounds__(T, 1) k_chol_inv(const double* __restrict__ G, int a, double* __restrict__ X,
+                                                int transposed, int* __restrict__ status, double drop_tol,
+                                                int* __restrict__ dropped) {
+    __shared__ double vec[2][kMaxDesign];  // step k's column below the diagonal, row up to it
+    __shared__ double res[kMaxDesign];     // L_ik (i > k) and X_kj (j <= k)
+    __shared__ double diag[kMaxDesign];
+    __shared__ double wmax[T / 32];
+    const int tid = threadIdx.x, ne = a * (a + 1) / 2;
+    int ij[R];  // i << 16 | j; -1: no element
+    double val[R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+        const int e = tid + T * m;
+        int i = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+        while (i * (i + 1) / 2 > e) --i;
+        while ((i + 1) * (i + 2) / 2 <= e) ++i;
+        const int j = e - i * (i + 1) / 2;
+        ij[m] = e < ne ? (i << 16 | j) : -1;
+        val[m] = e < ne ? G[i * a + j] : 0.0;
+        if (e < ne && j == 0) vec[0][i] = val[m];
+    }
+    double dm = 0.0;
+    for (int k = tid; k < a; k += T) {
+        diag[k] = G[k * a + k];
+        dm = fmax(dm, fabs(diag[k]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+    if ((tid & 31) == 0) wmax[tid >> 5] = dm;
+    __syncthreads();
+    double dmax = 0.0;
+    for (int w = 0; w < T / 32; ++w) dmax = fmax(dmax, wmax[w]);
+    int bad = 0;
+    for (int k = 0; k < a; ++k) {
+        const double* v = vec[k & 1];
+        if (tid < ((a + 31) & ~31)) {  // whole warps: the pivot is formed by each of them
+            double pv = v[k];
+            bool drop = false;
+            if (drop_tol >= 0.0) {
+                if (!(pv > drop_tol * fabs(diag[k])) || !(pv > 1e-300)) { drop = true; ++bad; pv = 1.0; }
+            } else if (!(pv > 1e-300 + 1e-28 * dmax)) {
+                pv = 1e-28 * dmax + 1e-300;
+                ++bad;
+            }
+            const double piv = sqrt(pv);
+            if (tid < a) {
+                double q = (tid == k ? 1.0 : v[tid]) / piv;
+                if (drop && tid > k) q = 0.0;
+                res[tid] = q;
+                const double x = tid <= k ? q : 0.0;
+                if (transposed) X[tid * a + k] = x;
+                else X[k * a + tid] = x;
+                if (tid == k && dropped) dropped[k] = drop ? 1 : 0;
+            }
+        }
+        __syncthreads();
+        double* nv = vec[(k + 1) & 1];
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+            const int i = ij[m] >> 16, j = ij[m] & 0xffff;
+            if (i > k) {
+                val[m] = fma(-res[i], res[j], j == k ? 0.0 : val[m]);
+                if (i == k + 1) nv[j] = val[m];
+                else if (j == k + 1) nv[i] = val[m];
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0 && status) status[0] = bad;
+}
+
+// k_chol_inv for wide matrices: the packed triangle in shared memory, a warp
+// per row and step (lanes over its columns); bound by the a^3 / 3 FMAs on one
+// SM's FP64 pipe.
+__global__ void __launch_bounds__(1024, 1) k_chol_inv_wide(const double* __restrict__ G, int a,
+                                                           double* __restrict__ X, int transposed,
+                                                           int* __restrict__ status, double drop_tol,
+                                                           int* __restrict__ dropped) {
+    extern __shared__ double P[];          // packed lower triangle
+    __shared__ double res[kMaxDesign];
+    __shared__ double diag[kMaxDesign];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int i = warp; i < a; i += 32)
+        for (int j = lane; j <= i; j += 32) P[i * (i + 1) / 2 + j] = G[i * a + j];
+    for (int k = tid; k < a; k += blockDim.x) diag[k] = G[k * a + k];
+    __syncthreads();
+    double dmax = 0.0;
+    for (int k = 0; k < a; ++k) dmax = fmax(dmax, fabs(diag[k]));
+    int bad = 0;
+    for (int k = 0; k < a; ++k) {
+        if (tid < ((a + 31) & ~31)) {
+            double pv = P[k * (k + 1) / 2 + k];
+            bool drop = false;
+            if (drop_tol >= 0.0) {
+                if (!(pv > drop_tol * fabs(diag[k])) || !(pv > 1e-300)) { drop = true; ++bad; pv = 1.0; }
+            } else if (!(pv > 1e-300 + 1e-28 * dmax)) {
+                pv = 1e-28 * dmax + 1e-300;
+                ++bad;
+            }
+            const double piv = sqrt(pv);
+            if (tid < a) {
+                const double v = tid == k ? 1.0 : tid < k ? P[k * (k + 1) / 2 + tid] : P[tid * (tid + 1) / 2 + k];
+                double q = v / piv;
+                if (drop && tid > k) q = 0.0;
+                res[tid] = q;
+                const double x = tid <= k ? q : 0.0;
+                if (transposed) X[tid * a + k] = x;
+                else X[k * a + tid] = x;
+                if (tid == k && dropped) dropped[k] = drop ? 1 : 0;
+            }
+        }
+        __syncthreads();
+        for (int i = k + 1 + warp; i < a; i += 32) {
+            const double li = -res[i];
+            double* row = P + i * (i + 1) / 2;
+            for (int j = lane; j <= i; j += 32) row[j] = fma(li, res[j], j == k ? 0.0 : row[j]);
+        }
+        __syncthreads();
+    }
+    if (tid == 0 && status) status[0] = bad;
+}
+
 // LU with partial pivoting in smem; returns 0 if an exactly zero pivot was met.
 __device__ bool lu_smem(double* S, int* piv, int a) {
     __shared__ int p_sh;
@@ -703,89 +864,123 @@ __global__ void k_inverse(const double* __restrict__ A, int a, double* __restric
     }
 }
 
-// safe_inv by Gauss-Jordan elimination on [A + eps I | I] in shared memory
-// (a <= kMaxGaussJordan), every thread of the CTA on each pivot step.  The
-// pivot search (first largest |value| in the column, from the diagonal down)
-// and the updates of the rows below the pivot are those of lu_smem, so the
-// pivots, and the exact-zero test that triggers the eps retry, are the same
-// as the LU's; the rows above the pivot are eliminated in the same sweep, so
-// the inverse needs no triangular solves.
-constexpr int kMaxGaussJordan = 112;  // 16 a^2 bytes of shared memory
-__global__ void __launch_bounds__(1024) k_inverse_gj(const double* __restrict__ A, int a, double* __restrict__ X,
-                                                     int* __restrict__ status, double* __restrict__ eps_used) {
-    extern __shared__ double S[];  // a rows x 2a columns
-    __shared__ double f[kMaxGaussJordan];
+__global__ void k_add_diag(double* __restrict__ A, int a, double v) {
+    for (int i = threadIdx.x; i < a; i += blockDim.x) A[i * a + i] += v;
+}
+
+// safe_inv of up to kMaxInverseJobs matrices, one CTA each, by Gauss-Jordan
+// elimination of A + shift I (+ eps I) in shared memory, in place: column k,
+// done with at step k, holds the inverse's column of the original row that
+// the k-th pivot came from (its entries before step k are that identity
+// column's, zeros and a one, so they need no storage).  The pivot search (first
+// largest |value| in the column, from the diagonal down) and the updates of the
+// rows below the pivot are those of lu_smem, so the pivots, and the exact-zero
+// test that triggers the eps retry, are the LU's.  A job without X wants
+// only that outcome: the rows above the pivot are left alone, a third of the
+// work.
+//
+// Per step: the search on one warp (magnitudes compared as integers, not on the
+// FP64 pipe), then every division of the step side by side (the factors of the
+// rows, the scaled pivot row), then a x a FMAs, a warp per row.  Bound by one
+// SM's FP64 pipe (two FMAs per cycle).
+constexpr int kMaxGaussJordan = 160;  // 8 a^2 bytes of shared memory
+struct InverseJobs {
+    InverseJob job[kMaxInverseJobs];
+};
+
+__global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant__ InverseJobs jobs) {
+    extern __shared__ double S[];  // a x a
+    __shared__ double f[kMaxGaussJordan], prow[kMaxGaussJordan];
+    __shared__ int rowid[kMaxGaussJordan], from[kMaxGaussJordan];
     __shared__ double eps;
     __shared__ int p_sh, ok;
-    const int ld = 2 * a, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const InverseJob& jb = jobs.job[blockIdx.x];
+    const double* A = jb.A;
+    const int a = jb.a, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    const bool inv = jb.X != nullptr;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
             double dmax = 0.0;
-            for (int k = 0; k < a; ++k) dmax = fmax(dmax, fabs(A[k * a + k]));
+            for (int k = 0; k < a; ++k) dmax = fmax(dmax, fabs(A[k * a + k] + jb.shift));
             dmax = fmax(dmax, 1e-300);
             eps = attempt == 0 ? 0.0 : 1e-8 * dmax;
             ok = 1;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < a * ld; e += blockDim.x) {
-            const int i = e / ld, j = e % ld;
-            S[e] = j < a ? A[i * a + j] + (i == j ? eps : 0.0) : (j - a == i ? 1.0 : 0.0);
-        }
+        for (int i = warp; i < a; i += nwarps)
+            for (int j = lane; j < a; j += 32) S[i * a + j] = i == j ? (A[i * a + j] + jb.shift) + eps : A[i * a + j];
+        for (int i = tid; i < a; i += blockDim.x) rowid[i] = i;
         __syncthreads();
         for (int k = 0; k < a; ++k) {
             if (warp == 0) {
-                int p = -1;
-                double best = -1.0;
+                unsigned long long best = 0ull;  // |value| bits + 1 (0: none; NaN never wins)
+                int p = k;
                 for (int i = k + lane; i < a; i += 32) {
-                    const double v = fabs(S[i * ld + k]);
-                    if (v > best) { best = v; p = i; }
+                    const unsigned long long u =
+                        (unsigned long long)__double_as_longlong(S[i * a + k]) & 0x7fffffffffffffffull;
+                    const unsigned long long key = u > 0x7ff0000000000000ull ? 0ull : u + 1ull;
+                    if (key > best) { best = key; p = i; }
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                    const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
                     const int op = __shfl_xor_sync(0xffffffffu, p, o);
-                    if (ob > best || (ob == best && op >= 0 && (p < 0 || op < p))) { best = ob; p = op; }
+                    if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
                 }
                 if (lane == 0) {
                     p_sh = p;
-                    if (best == 0.0) ok = 0;
+                    if (best <= 1ull) ok = 0;
+                    from[k] = rowid[p];
+                    rowid[p] = rowid[k];
                 }
             }
             __syncthreads();
             if (!ok) break;
             const int p = p_sh;
-            if (p != k)
-                for (int j = k + threadIdx.x; j < ld; j += blockDim.x) {
-                    const double t = S[k * ld + j];
-                    S[k * ld + j] = S[p * ld + j];
-                    S[p * ld + j] = t;
-                }
-            __syncthreads();
-            const double d = S[k * ld + k];
-            for (int i = threadIdx.x; i < a; i += blockDim.x) f[i] = i == k ? 0.0 : S[i * ld + k] / d;
-            __syncthreads();
-            const int span = ld - k - 1;
-            for (int e = threadIdx.x; e < a * span; e += blockDim.x) {
-                const int i = e / span, j = k + 1 + e % span;
-                if (i != k) S[i * ld + j] -= f[i] * S[k * ld + j];
+            const double d = S[p * a + k];
+            // the row factors on the first threads, the pivot row on the last
+            // ones: row k takes the scaled pivot row, row p what was in row k
+            if (tid < a) {
+                const int i = tid;
+                if (i != k) f[i] = S[(i == p ? k : i) * a + k] / d;
+            }
+            const int jt = (int)blockDim.x - 1 - tid;
+            double scaled = 0.0;
+            if (jt < a && jt != k) {
+                const double pj = S[p * a + jt], kj = S[k * a + jt];
+                prow[jt] = pj;
+                if (inv) scaled = pj / d;
+                if (p != k) S[p * a + jt] = kj;
+                S[k * a + jt] = inv ? scaled : pj;
             }
             __syncthreads();
-            for (int j = k + 1 + threadIdx.x; j < ld; j += blockDim.x) S[k * ld + j] /= d;
+            const int i0 = inv ? 0 : k + 1, j0 = inv ? 0 : k + 1;
+            for (int i = i0 + warp; i < a; i += nwarps) {
+                double* row = S + i * a;
+                if (i == k) {
+                    if (lane == 0) row[k] = 1.0 / d;
+                    continue;
+                }
+                const double fi = -f[i];
+                for (int j = j0 + lane; j < a; j += 32) row[j] = j == k ? fi : fma(fi, prow[j], row[j]);
+            }
             __syncthreads();
         }
         if (ok) {
-            for (int e = threadIdx.x; e < a * a; e += blockDim.x) X[e] = S[(e / a) * ld + a + e % a];
-            if (threadIdx.x == 0) {
-                if (status) status[0] = attempt;
-                if (eps_used) eps_used[0] = eps;
+            if (inv)
+                for (int i = warp; i < a; i += nwarps)
+                    for (int j = lane; j < a; j += 32) jb.X[i * a + from[j]] = S[i * a + j];
+            if (tid == 0) {
+                jb.status[0] = attempt;
+                jb.eps[0] = eps;
             }
             return;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        if (status) status[0] = 2;
-        if (eps_used) eps_used[0] = eps;
+    if (tid == 0) {
+        jb.status[0] = 2;
+        jb.eps[0] = eps;
     }
 }
 
@@ -1391,14 +1586,7 @@ void launch_trmul_f32(Ctx& c, float* A, int lda, uint64_t m, int a, const double
     if (m == 0) return;
     if (a <= 32) {
         if (narrow_tiled(A, lda)) {
-            // the factor travels in the launch (a x a doubles on the device)
-            std::vector<double> L((size_t)a * a);
-            SLFMM_CUDA(cudaMemcpyAsync(L.data(), Linv, L.size() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-            SLFMM_CUDA(cudaStreamSynchronize(c.stream));
-            Mat32 R{};
-            for (int i = 0; i < a; ++i)
-                for (int k = 0; k <= i; ++k) R.v[i][k] = (float)L[(size_t)i * a + k];
-            k_trmul_rows<<<grid_for(c, m, 256), 256, 0, c.stream>>>(A, lda, m, a, R);
+            k_trmul_rows<<<grid_for(c, ceil_div(m, (uint64_t)kTrmulRows), 256), 256, 0, c.stream>>>(A, lda, m, a, Linv);
             SLFMM_LAUNCHED(c, "k_trmul_rows");
             return;
         }
@@ -1424,6 +1612,36 @@ void launch_cholesky(Ctx& c, double* A, int a, int* status, double drop_tol, int
     SLFMM_LAUNCHED(c, "k_cholesky");
 }
 
+// X = L^-1 (or its transpose) of the Cholesky factor of G.  The fused kernel
+// keeps the packed triangle in registers up to 127 columns and in shared memory
+// up to 236; wider designs take the two separate kernels, on a copy of G.
+void launch_chol_inv(Ctx& c, const double* G, int a, double* X, bool transposed, int* status, double drop_tol,
+                     int* dropped) {
+    SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the small Cholesky");
+    if (a < 1) return;
+    const int ne = a * (a + 1) / 2, tr = transposed ? 1 : 0;
+#define SLFMM_CHOL_INV(T, R) k_chol_inv<T, R><<<1, T, 0, c.stream>>>(G, a, X, tr, status, drop_tol, dropped)
+    if (ne <= 256) SLFMM_CHOL_INV(256, 1);
+    else if (ne <= 256 * 2) SLFMM_CHOL_INV(256, 2);
+    else if (ne <= 256 * 4) SLFMM_CHOL_INV(256, 4);
+    else if (ne <= 256 * 9) SLFMM_CHOL_INV(256, 9);
+    else if (ne <= 512 * 16) SLFMM_CHOL_INV(512, 16);
+    else if (ne * sizeof(double) <= 220 * 1024) {
+        const size_t sm = ne * sizeof(double);
+        set_smem((const void*)k_chol_inv_wide, sm);
+        k_chol_inv_wide<<<1, 1024, sm, c.stream>>>(G, a, X, tr, status, drop_tol, dropped);
+    } else {
+        DBuf<double> L((size_t)a * a, c.stream), lower((size_t)a * a, c.stream);
+        SLFMM_CUDA(cudaMemcpyAsync(L.get(), G, (size_t)a * a * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+        launch_cholesky(c, L.get(), a, status, drop_tol, dropped);
+        launch_tri_inv_lower(c, L.get(), a, transposed ? lower.get() : X);
+        if (transposed) launch_transpose(c, lower.get(), a, a, X);
+        return;
+    }
+#undef SLFMM_CHOL_INV
+    SLFMM_LAUNCHED(c, "k_chol_inv");
+}
+
 void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv) {
     SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the triangular inverse");
     const bool sm = a <= kMaxSmall;
@@ -1432,20 +1650,61 @@ void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv) {
     SLFMM_LAUNCHED(c, "k_tri_inv_lower");
 }
 
-void launch_inverse(Ctx& c, const double* A, int a, double* Ainv, int* status, double* eps_used) {
-    SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the small inverse");
-    ProfScope ps(c, "small_inverse", 16.0 * a * a, 2.0 * a * a * a);
-    if (a <= kMaxGaussJordan) {
-        set_smem((const void*)k_inverse_gj, 2 * smem_sq(a));
-        k_inverse_gj<<<1, 1024, 2 * smem_sq(a), c.stream>>>(A, a, Ainv, status, eps_used);
-    } else if (a <= kMaxSmall) {
-        set_smem((const void*)k_inverse, smem_sq(a));
-        k_inverse<<<1, 256, smem_sq(a), c.stream>>>(A, a, Ainv, status, eps_used, nullptr);
-    } else {
-        DBuf<double> work((size_t)a * a + (size_t)(a + 1) / 2, c.stream);  // matrix, then a pivot ints
-        k_inverse<<<1, 1024, 0, c.stream>>>(A, a, Ainv, status, eps_used, work.get());
+// The elimination in shared memory takes status-only jobs up to its size, and
+// inverses up to 112 columns (wider ones keep the LU's solves and their bits).
+static bool inverse_in_shared(const InverseJob& j) { return j.a <= (j.X ? 112 : kMaxGaussJordan); }
+
+void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
+    SLFMM_REQUIRE(n <= kMaxInverseJobs, SLFMM_ERR_BAD_ARG, "too many matrices for one inversion launch");
+    double work = 0.0;
+    for (int i = 0; i < n; ++i) {
+        SLFMM_REQUIRE(jobs[i].a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the small inverse");
+        work += 2.0 * jobs[i].a * jobs[i].a * jobs[i].a;
     }
-    SLFMM_LAUNCHED(c, "k_inverse");
+    ProfScope ps(c, "small_inverse", 0.0, work);
+    InverseJobs js{};
+    int m = 0, amax = 0;
+    for (int i = 0; i < n; ++i)
+        if (inverse_in_shared(jobs[i])) {
+            js.job[m++] = jobs[i];
+            amax = std::max(amax, jobs[i].a);
+        }
+    if (m) {
+        set_smem((const void*)k_inverse_jobs, smem_sq(amax));
+        k_inverse_jobs<<<m, 1024, smem_sq(amax), c.stream>>>(js);
+        SLFMM_LAUNCHED(c, "k_inverse_jobs");
+    }
+    for (int i = 0; i < n; ++i) {
+        const InverseJob& j = jobs[i];
+        if (inverse_in_shared(j)) continue;
+        DBuf<double> A, X;
+        const double* src = j.A;
+        if (j.shift != 0.0) {
+            A.alloc((size_t)j.a * j.a, c.stream);
+            SLFMM_CUDA(cudaMemcpyAsync(A.get(), j.A, A.bytes(), cudaMemcpyDeviceToDevice, c.stream));
+            k_add_diag<<<1, 256, 0, c.stream>>>(A.get(), j.a, j.shift);
+            SLFMM_LAUNCHED(c, "k_add_diag");
+            src = A.get();
+        }
+        double* x = j.X;
+        if (!x) {
+            X.alloc((size_t)j.a * j.a, c.stream);
+            x = X.get();
+        }
+        if (j.a <= kMaxSmall) {
+            set_smem((const void*)k_inverse, smem_sq(j.a));
+            k_inverse<<<1, 256, smem_sq(j.a), c.stream>>>(src, j.a, x, j.status, j.eps, nullptr);
+        } else {
+            DBuf<double> work((size_t)j.a * j.a + (size_t)(j.a + 1) / 2, c.stream);  // matrix, then a pivot ints
+            k_inverse<<<1, 1024, 0, c.stream>>>(src, j.a, x, j.status, j.eps, work.get());
+        }
+        SLFMM_LAUNCHED(c, "k_inverse");
+    }
+}
+
+void launch_inverse(Ctx& c, const double* A, int a, double* Ainv, int* status, double* eps_used) {
+    const InverseJob j{A, a, 0.0, Ainv, status, eps_used};
+    launch_inverses(c, &j, 1);
 }
 
 void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {

@@ -382,12 +382,28 @@ void launch_trmul_f32(Ctx& c, float* A, int lda, uint64_t m, int a, const double
 // tiny value; drop_tol >= 0: drop (L_kk = 1, column zero) dependent columns
 void launch_cholesky(Ctx& c, double* A, int a, int* status, double drop_tol = -1.0,
                      int* dropped = nullptr);
+// X = L^-1 (lower triangular; or its transpose) of the Cholesky factor of G
+// (not changed), pivots as launch_cholesky
+void launch_chol_inv(Ctx& c, const double* G, int a, double* X, bool transposed, int* status,
+                     double drop_tol = -1.0, int* dropped = nullptr);
 void launch_transpose(Ctx& c, const double* A, int rows, int cols, double* At);
 void launch_scale_cols(Ctx& c, double* A, uint64_t m, int a, int lda, const double* f);
 void launch_build_design(Ctx& c, const double* X, int d, const double* U, int K, uint64_t n,
                          double* C);
 void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv);
 void launch_inverse(Ctx& c, const double* A, int a, double* Ainv, int* status, double* eps_used);
+// safe_inv of A + shift I (a x a) into X; X null: only the status and eps
+struct InverseJob {
+    const double* A;
+    int a;
+    double shift;
+    double* X;
+    int* status;
+    double* eps;
+};
+constexpr int kMaxInverseJobs = 3;
+// several at once, a CTA each
+void launch_inverses(Ctx& c, const InverseJob* jobs, int n);
 // one-sided Jacobi SVD (a <= 64): A is overwritten with U, V and sig
 // (descending) written
 void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig);
