@@ -1138,8 +1138,14 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     // stream while later chunks compute (only the p-values wait for the GIF).
     DBuf<float> U;
     int wp = 0;
-    const uint64_t chunk = round_up(ceil_div(p, 8), 128);
-    const bool chunked = c.precision == SLFMM_PREC_SPLIT_FP8 && st.fill.k == 0 && p >= 2 * chunk &&
+    // Chunks: up to eight, each with at least 8 MB to copy (42 us of the host
+    // link: a chunk costs about eight launches) and whole waves of one 128-row
+    // tile per SM (a tenth of a last wave costs as much as a full one).
+    const uint64_t wave = 128ull * (uint64_t)std::max(c.sm_count, 1), waves = ceil_div(std::max<uint64_t>(p, 1), wave);
+    const uint64_t copy_bytes = p * (2 * (uint64_t)d + 3) * sizeof(double);
+    const uint64_t nchunks = std::max<uint64_t>(1, std::min<uint64_t>({copy_bytes >> 23, 8, waves}));
+    const uint64_t chunk = ceil_div(waves, nchunks) * wave;
+    const bool chunked = c.precision == SLFMM_PREC_SPLIT_FP8 && st.fill.k == 0 && p > chunk &&
                          (out.beta || out.r2 || out.tstat) && (!out.beta || is_pinned(out.beta)) &&
                          (!out.r2 || is_pinned(out.r2)) && (!out.tstat || is_pinned(out.tstat));
     bool copied = false;

@@ -22,12 +22,15 @@
 namespace slfmm {
 namespace {
 
-// Tiles of 64 SNPs; each of 256 threads owns 4 SNPs x 4 traits of theta and
+// Tiles of SNPs; each of 256 threads owns 4 SNPs x 4 traits of theta and
 // beta.  The coefficient rows stay in shared memory (transposed, traits
-// padded to 64) for the whole persistent CTA; the tile's u values are staged
+// padded to TP) for the whole persistent CTA; the tile's u values are staged
 // k-major, so one k step is three 16-byte loads and 32 FMAs per thread.
-constexpr int kTileSnps = 64;
-constexpr int kTraitPad = 64;
+constexpr int kTraitPad = 64;   // traits of one launch
+constexpr __host__ __device__ int tile_snps(int tp) { return 4096 / tp; }
+constexpr size_t epilogue_smem(int tp, int w) {
+    return (size_t)(2 * w * tp + w * (tile_snps(tp) + 4) + 4 * tile_snps(tp)) * sizeof(float);
+}
 
 // Histogram bin of one FP32 t statistic by the reference's rule applied to
 // that value: t_sq = t * t in FP64, skipped when not finite, bin =
@@ -47,14 +50,44 @@ __device__ __forceinline__ int tsq_bin(float t) {
     const double q = floor(((double)t * (double)t) / kHistWidth);
     return q >= (double)(kHistBins - 1) ? kHistBins - 1 : (int)q;
 }
-constexpr int kUsStride = kTileSnps + 4;  // 16-byte rows, staggered banks
 
+// The per-SNP FP64 part: sigma^2 from ||u||^2 (ss) and TSS, and r2 from its
+// covariate part (sc).
+__device__ __forceinline__ float snp_sigma2(float ss, float sc, double T, bool zv, double df, double* r2) {
+    double rss = T - (double)ss;
+    if (rss < 0.0 || zv) rss = 0.0;
+    if (r2) {
+        double a = 0.0, b = 0.0, c = 0.0;
+        if (T > 1e-300 && !zv) {                        // src/testing.rs:394-404
+            const double ssc = (double)sc;
+            a = ssc / T;
+            b = fmax(T - rss - ssc, 0.0) / T;
+            c = rss / T;
+        }
+        r2[0] = a;
+        r2[1] = b;
+        r2[2] = c;
+    }
+    return (float)(rss / df);
+}
 
-// One block of up to 64 traits per launch: traits [t0, t0 + d) of a model
+__device__ __forceinline__ float t_stat(float th, float s2f, float cjj, bool usable) {
+    float t = 0.f;
+    const float var = s2f * cjj;
+    if (usable && var > 0.f && isfinite(var)) {  // t_test guards
+        t = th * rsqrtf(var);
+        if (!isfinite(t)) t = 0.f;
+    }
+    return t;
+}
+
+// One block of up to TP traits per launch: traits [t0, t0 + d) of a model
 // with d_model covariates (the first d_model coordinates of u are the
 // covariate ones, so SS_cov always sums over d_model); beta and t32 rows
 // have d_model entries and point at trait t0; r2 may be null (written by the
-// launch of the first block).
+// launch of the first block).  A tile is 4096 / TP SNPs: 64 for blocks of up
+// to 64 traits, 256 for up to 16.
+template <int TP>
 __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
     uint64_t p, const float* __restrict__ u, int ldu, const double* __restrict__ tss,
     const uint8_t* __restrict__ zero_var, int d, int d_model, int w, double df,
@@ -62,42 +95,43 @@ __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
     const double* __restrict__ cjj, const uint8_t* __restrict__ dropped,
     double* __restrict__ beta, float* __restrict__ t32, double* __restrict__ r2,
     uint32_t* __restrict__ hist) {
+    constexpr int kTile = tile_snps(TP), kStride = kTile + 4;  // 16-byte rows, staggered banks
     extern __shared__ __align__(16) float sm[];
-    float* thT = sm;                          // [w][64]
-    float* btT = thT + w * kTraitPad;         // [w][64]
-    float* us = btT + w * kTraitPad;          // [w][68]
-    float* s2s = us + w * kUsStride;          // [64] sigma^2 per SNP of the tile
-    int* zvs = reinterpret_cast<int*>(s2s + kTileSnps);
-    float* sss = s2s + 2 * kTileSnps;         // [64] ||u||^2 per SNP of the tile
-    float* scs = sss + kTileSnps;             // [64] its covariate part
-    __shared__ float cj[kTraitPad];
-    __shared__ int dr[kTraitPad];
+    float* thT = sm;                          // [w][TP]
+    float* btT = thT + w * TP;                // [w][TP]
+    float* us = btT + w * TP;                 // [w][kStride]
+    float* s2s = us + w * kStride;            // [kTile] sigma^2 per SNP of the tile
+    int* zvs = reinterpret_cast<int*>(s2s + kTile);
+    float* sss = s2s + 2 * kTile;             // [kTile] ||u||^2 per SNP of the tile
+    float* scs = sss + kTile;                 // [kTile] its covariate part
+    __shared__ float cj[TP];
+    __shared__ int dr[TP];
     const int tid = threadIdx.x;
-    for (int e = tid; e < w * kTraitPad; e += blockDim.x) {
-        const int k = e / kTraitPad, jj = e % kTraitPad;
+    for (int e = tid; e < w * TP; e += blockDim.x) {
+        const int k = e / TP, jj = e % TP;
         thT[e] = jj < d ? theta_rows[jj * w + k] : 0.f;
         btT[e] = jj < d ? beta_rows[jj * w + k] : 0.f;
     }
-    for (int jj = tid; jj < kTraitPad; jj += blockDim.x) {
+    for (int jj = tid; jj < TP; jj += blockDim.x) {
         cj[jj] = jj < d ? (float)cjj[jj] : 0.f;
         dr[jj] = jj < d ? (int)dropped[jj] : 1;
     }
-    const int sg = tid >> 4, tg = tid & 15;
-    const uint64_t ntiles = (p + kTileSnps - 1) / kTileSnps;
+    const int sg = tid / (TP / 4), tg = tid % (TP / 4);
+    const uint64_t ntiles = (p + kTile - 1) / kTile;
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t j0 = tile * kTileSnps;
+        const uint64_t j0 = tile * kTile;
         __syncthreads();  // the previous tile's values are consumed (and the tables are in place)
-        for (int e = tid; e < w * kTileSnps; e += blockDim.x) {
-            const int k = e / kTileSnps, sn = e % kTileSnps;
-            us[k * kUsStride + sn] = j0 + sn < p ? u[(j0 + sn) * ldu + k] : 0.f;
+        for (int e = tid; e < w * kTile; e += blockDim.x) {
+            const int k = e / kTile, sn = e % kTile;
+            us[k * kStride + sn] = j0 + sn < p ? u[(j0 + sn) * ldu + k] : 0.f;
         }
         __syncthreads();
-        // per-SNP sums, 8 lanes per SNP with stride-8 partials, two rounds of 32
-        for (int half = 0; half < 2; ++half) {
-            const int sn = half * 32 + (tid >> 3), l8 = tid & 7;
+        // per-SNP sums, 8 lanes per SNP with stride-8 partials, rounds of 32
+        for (int part = 0; part < kTile / 32; ++part) {
+            const int sn = part * 32 + (tid >> 3), l8 = tid & 7;
             float ss = 0.f, sc = 0.f;
             for (int k = l8; k < w; k += 8) {
-                const float v = us[k * kUsStride + sn];
+                const float v = us[k * kStride + sn];
                 ss = fmaf(v, v, ss);
                 if (k < d_model) sc = fmaf(v, v, sc);
             }
@@ -112,31 +146,16 @@ __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
             }
         }
         __syncthreads();
-        // the FP64 part per SNP on one lane each (two full warps): this part's
-        // FP64 pipe is a small fraction of the FP32 one
-        if (tid < kTileSnps) {
+        // the FP64 part per SNP on one lane each (full warps): this part's FP64
+        // pipe is a small fraction of the FP32 one
+        if (tid < kTile) {
             const int sn = tid;
             const uint64_t j = j0 + sn;
             float s2f = 0.f;
             int zv = 1;
             if (j < p) {
                 zv = zero_var && zero_var[j];
-                const double T = tss[j];
-                double rss = T - (double)sss[sn];
-                if (rss < 0.0 || zv) rss = 0.0;
-                s2f = (float)(rss / df);
-                double a = 0.0, b = 0.0, c = 0.0;
-                if (T > 1e-300 && !zv) {                        // src/testing.rs:394-404
-                    const double ssc = (double)scs[sn];
-                    a = ssc / T;
-                    b = fmax(T - rss - ssc, 0.0) / T;
-                    c = rss / T;
-                }
-                if (r2) {
-                    r2[j * 3 + 0] = a;
-                    r2[j * 3 + 1] = b;
-                    r2[j * 3 + 2] = c;
-                }
+                s2f = snp_sigma2(sss[sn], scs[sn], tss[j], zv != 0, df, r2 ? r2 + j * 3 : nullptr);
             }
             s2s[sn] = s2f;
             zvs[sn] = zv;
@@ -154,9 +173,9 @@ __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
         for (int k = 0; k < w; ++k) {
             const float4 uv = un, tv = tn, bv = bn;
             if (k + 1 < w) {
-                un = *reinterpret_cast<const float4*>(us + (k + 1) * kUsStride + 4 * sg);
-                tn = *reinterpret_cast<const float4*>(thT + (k + 1) * kTraitPad + 4 * tg);
-                bn = *reinterpret_cast<const float4*>(btT + (k + 1) * kTraitPad + 4 * tg);
+                un = *reinterpret_cast<const float4*>(us + (k + 1) * kStride + 4 * sg);
+                tn = *reinterpret_cast<const float4*>(thT + (k + 1) * TP + 4 * tg);
+                bn = *reinterpret_cast<const float4*>(btT + (k + 1) * TP + 4 * tg);
             }
             const float ua[4] = {uv.x, uv.y, uv.z, uv.w};
             const float ta[4] = {tv.x, tv.y, tv.z, tv.w};
@@ -180,17 +199,84 @@ __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
             for (int b = 0; b < 4; ++b) {
                 const int jj = 4 * tg + b;
                 if (jj >= d) continue;
-                float t = 0.f;
-                const float var = s2f * cj[jj];
-                if (!zv && !dr[jj] && var > 0.f && isfinite(var)) {  // t_test guards
-                    t = th[a][b] * rsqrtf(var);
-                    if (!isfinite(t)) t = 0.f;
-                }
+                const float t = t_stat(th[a][b], s2f, cj[jj], !zv && !dr[jj]);
                 beta[j * d_model + jj] = zv ? 0.0 : f64_of_f32(bb[a][b]);
                 t32[j * d_model + jj] = t;
                 const int bin = tsq_bin(t);
                 if (bin >= 0) atomicAdd(&hist[(uint64_t)jj * kHistBins + bin], 1u);
             }
+        }
+    }
+}
+
+// The same statistics for models of at most four covariates, one SNP per
+// thread: its u row comes as 16-byte loads (rows are 16-byte aligned, ldu a
+// multiple of 16) and the coefficients as broadcast shared-memory loads.  The
+// tiled kernel pads the traits to 16 or 64 and stages every u value.  The sums
+// run over the tiled kernel's eight strided partials and are added in its
+// order, so both give the same bits.
+constexpr int kFewTraits = 4;
+__global__ void __launch_bounds__(256) k_assoc_few(
+    uint64_t p, const float* __restrict__ u, int ldu, const double* __restrict__ tss,
+    const uint8_t* __restrict__ zero_var, int d, int w, double df, const float* __restrict__ theta_rows,
+    const float* __restrict__ beta_rows, const double* __restrict__ cjj, const uint8_t* __restrict__ dropped,
+    double* __restrict__ beta, float* __restrict__ t32, double* __restrict__ r2, uint32_t* __restrict__ hist) {
+    extern __shared__ __align__(16) float sm[];
+    float4* th4 = reinterpret_cast<float4*>(sm);  // [8 * ceil(w / 8)] theta, then beta, of the four traits
+    const int wq = (w + 7) & ~7;
+    float4* bt4 = th4 + wq;
+    for (int e = threadIdx.x; e < wq * kFewTraits; e += blockDim.x) {
+        const int k = e / kFewTraits, jj = e % kFewTraits;
+        const bool in = jj < d && k < w;
+        reinterpret_cast<float*>(th4)[e] = in ? theta_rows[jj * w + k] : 0.f;
+        reinterpret_cast<float*>(bt4)[e] = in ? beta_rows[jj * w + k] : 0.f;
+    }
+    __shared__ float cj[kFewTraits];
+    __shared__ int dr[kFewTraits];
+    if (threadIdx.x < kFewTraits) {
+        cj[threadIdx.x] = threadIdx.x < d ? (float)cjj[threadIdx.x] : 0.f;
+        dr[threadIdx.x] = threadIdx.x < d ? (int)dropped[threadIdx.x] : 1;
+    }
+    __syncthreads();
+    for (uint64_t j = (uint64_t)blockIdx.x * 256 + threadIdx.x; j < p; j += (uint64_t)gridDim.x * 256) {
+        const float4* row = reinterpret_cast<const float4*>(u + j * ldu);
+        float ss[8], sc[8], th[4], bb[4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss[i] = sc[i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) th[i] = bb[i] = 0.f;
+        for (int k0 = 0; k0 < w; k0 += 8) {
+            const float4 a = row[k0 / 4], b = row[k0 / 4 + 1];
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (k0 + i < w) {  // the row's padding may hold anything finite or not
+                    const float4 t4 = th4[k0 + i], b4 = bt4[k0 + i];
+                    ss[i] = fmaf(v[i], v[i], ss[i]);
+                    if (k0 + i < d) sc[i] = fmaf(v[i], v[i], sc[i]);
+                    th[0] = fmaf(t4.x, v[i], th[0]);
+                    th[1] = fmaf(t4.y, v[i], th[1]);
+                    th[2] = fmaf(t4.z, v[i], th[2]);
+                    th[3] = fmaf(t4.w, v[i], th[3]);
+                    bb[0] = fmaf(b4.x, v[i], bb[0]);
+                    bb[1] = fmaf(b4.y, v[i], bb[1]);
+                    bb[2] = fmaf(b4.z, v[i], bb[2]);
+                    bb[3] = fmaf(b4.w, v[i], bb[3]);
+                }
+            }
+        }
+        const float sst = ((ss[0] + ss[4]) + (ss[2] + ss[6])) + ((ss[1] + ss[5]) + (ss[3] + ss[7]));
+        const float sct = ((sc[0] + sc[4]) + (sc[2] + sc[6])) + ((sc[1] + sc[5]) + (sc[3] + sc[7]));
+        const bool zv = zero_var && zero_var[j];
+        const float s2f = snp_sigma2(sst, sct, tss[j], zv, df, r2 + j * 3);
+#pragma unroll
+        for (int jj = 0; jj < kFewTraits; ++jj) {
+            if (jj >= d) break;
+            const float t = t_stat(th[jj], s2f, cj[jj], !zv && !dr[jj]);
+            beta[j * d + jj] = zv ? 0.0 : f64_of_f32(bb[jj]);
+            t32[j * d + jj] = t;
+            const int bin = tsq_bin(t);
+            if (bin >= 0) atomicAdd(&hist[(uint64_t)jj * kHistBins + bin], 1u);
         }
     }
 }
@@ -354,28 +440,48 @@ void launch_gif_noalloc(Ctx& c, const float* t, uint64_t p, int d, double* gif_r
     SLFMM_LAUNCHED(c, "k_gif");
 }
 
-void launch_assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const double* tss,
-                           const AssocConsts& k, double* beta, float* t32, double* r2,
-                           uint32_t* hist) {
-    if (p == 0) return;
-    const size_t smem = (size_t)(2 * k.w * kTraitPad + k.w * kUsStride + 4 * kTileSnps) * sizeof(float);
+template <int TP>
+static void assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const double* tss, const AssocConsts& k,
+                           double* beta, float* t32, double* r2, uint32_t* hist) {
+    const size_t smem = epilogue_smem(TP, k.w);
     SLFMM_REQUIRE(smem <= 227 * 1024, SLFMM_ERR_BAD_ARG, "association design too wide for the epilogue");
-    raise_dynamic_smem((const void*)k_assoc_epilogue, smem);
-    const uint64_t tiles = ceil_div(p, (uint64_t)kTileSnps);
+    raise_dynamic_smem((const void*)k_assoc_epilogue<TP>, smem);
+    const uint64_t tiles = ceil_div(p, (uint64_t)tile_snps(TP));
     // one wave of persistent CTAs: as many per SM as fit (registers and
     // shared memory), so no CTA starts its share of tiles after the others
     int per_sm = 0;
-    SLFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_assoc_epilogue, 256, smem));
+    SLFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_assoc_epilogue<TP>, 256, smem));
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)c.sm_count * std::max(per_sm, 1));
-    // traits in blocks of 64 (the coefficient tables of one block stay in
+    // traits in blocks of TP (the coefficient tables of one block stay in
     // shared memory); every block reads the same u rows
-    for (int t0 = 0; t0 < k.d; t0 += kTraitPad) {
-        const int db = std::min(kTraitPad, k.d - t0);
-        k_assoc_epilogue<<<grid, 256, smem, c.stream>>>(
+    for (int t0 = 0; t0 < k.d; t0 += TP) {
+        const int db = std::min(TP, k.d - t0);
+        k_assoc_epilogue<TP><<<grid, 256, smem, c.stream>>>(
             p, u, ldu, tss, k.zero_var, db, k.d, k.w, k.df, k.theta_rows + (size_t)t0 * k.w,
             k.beta_rows + (size_t)t0 * k.w, k.cjj + t0, k.dropped + t0, beta + t0, t32 + t0, t0 == 0 ? r2 : nullptr,
             hist + (size_t)t0 * kHistBins);
         SLFMM_LAUNCHED(c, "k_assoc_epilogue");
+    }
+}
+
+// Up to four covariates take the thread-per-SNP form (1.8 M SNPs, 1 covariate,
+// 13 columns, eight launches: 0.58 ms in the 64-trait tiles), up to 16 the
+// tiles padded to 16 traits while two CTAs' tables and tiles fit an SM.
+void launch_assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const double* tss,
+                           const AssocConsts& k, double* beta, float* t32, double* r2,
+                           uint32_t* hist) {
+    if (p == 0) return;
+    if (k.d <= kFewTraits && ldu % 8 == 0 && ldu >= ((k.w + 7) & ~7) && r2 &&
+        reinterpret_cast<uintptr_t>(u) % 16 == 0) {
+        const size_t smem = (size_t)2 * ((k.w + 7) & ~7) * sizeof(float4);
+        k_assoc_few<<<grid_for(c, p, 256), 256, smem, c.stream>>>(p, u, ldu, tss, k.zero_var, k.d, k.w, k.df,
+                                                                  k.theta_rows, k.beta_rows, k.cjj, k.dropped, beta,
+                                                                  t32, r2, hist);
+        SLFMM_LAUNCHED(c, "k_assoc_few");
+    } else if (k.d <= 16 && epilogue_smem(16, k.w) <= 110 * 1024) {
+        assoc_epilogue<16>(c, p, u, ldu, tss, k, beta, t32, r2, hist);
+    } else {
+        assoc_epilogue<kTraitPad>(c, p, u, ldu, tss, k, beta, t32, r2, hist);
     }
 }
 
