@@ -747,12 +747,10 @@ void std_raw(Ctx& c, const Geno& g, const double* mean_src, SnpStd& s) {
     s.lut.alloc(p * 4, c.stream);
     if (mean_src) SLFMM_CUDA(cudaMemcpyAsync(s.mean.get(), mean_src, g.p * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
     else s.mean.zero();
-    std::vector<double> ones(p, 1.0);
-    h2d(c, s.scale.get(), ones.data(), p);
+    launch_fill(c, s.scale.get(), p, 1.0);
     s.tss.zero();
     s.zero_var.zero();
     launch_lut_std(c, g.p, s.mean.get(), s.scale.get(), s.lut.get());
-    sync(c);
 }
 
 struct Step0 {
@@ -827,7 +825,6 @@ void step0(Ctx& c, const double* x_host, uint64_t n, int d, double lambda, bool 
         launch_gemm_small(c, s.xs.get(), d, n, d, a.get(), s.r, s.r, 1.0, 0.0, s.qd.get(), s.r);
         launch_gemm_small(c, s.xs.get(), d, n, d, b.get(), s.r, s.r, 1.0, 0.0, s.qd_omd.get(), s.r);
         launch_gemm_small(c, s.xs.get(), d, n, d, e.get(), s.r, s.r, 1.0, 0.0, s.qd_omdinv.get(), s.r);
-        sync(c);
     }
 }
 
@@ -898,6 +895,7 @@ void rsvd(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, int K, int l
           uint64_t seed, const double* omega_host, DBuf<double>& u_hat, DBuf<float>* Z_pre = nullptr) {
     const uint64_t n = g.n;
     rsvd_checks(n, g.p, l);
+    Tc8Errors errors(c);
     DBuf<float> Z;
     int wp = 0;
     if (Z_pre) {
@@ -926,8 +924,10 @@ void rsvd(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, int K, int l
     DBuf<double> G(l * l, c.stream), V(l * l, c.stream), sig(l, c.stream);
     launch_atb(c, B.get(), wp, B.get(), wp, n, l, l, G.get());
     launch_jacobi_svd(c, G.get(), l, V.get(), sig.get());
-    std::vector<double> Vh = fetch(c, V.get(), (size_t)l * l);
-    std::vector<double> ev = fetch(c, sig.get(), (size_t)l);
+    std::vector<double> Vh((size_t)l * l), ev(l);
+    d2h(c, Vh.data(), V.get(), Vh.size());
+    d2h(c, ev.data(), sig.get(), ev.size());
+    errors.check();
     std::vector<double> Vk((size_t)l * K);
     for (int k = 0; k < K; ++k) {
         const double sg = std::sqrt(std::max(ev[k], 0.0));
@@ -937,7 +937,6 @@ void rsvd(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, int K, int l
     u_hat.alloc(n * K, c.stream);
     launch_gemm_small(c, B.get(), wp, n, l, Vkd.get(), K, K, 1.0, 0.0, u_hat.get(), K);
     apply_p(c, s0, u_hat.get(), K, K, true);                 // U_hat = Q D^-1 U_small
-    sync(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -1009,8 +1008,11 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     DBuf<int> st1(1, c.stream), dropped(w, c.stream);
     DBuf<double> Linv(w * w, c.stream);
     launch_chol_inv(c, L.get(), w, Linv.get(), false, st1.get(), 1e-10, dropped.get());
-    std::vector<double> Li = fetch(c, Linv.get(), (size_t)w * w);
-    std::vector<int> dr = fetch(c, dropped.get(), (size_t)w);
+    std::vector<double> Li((size_t)w * w);
+    std::vector<int> dr(w);
+    d2h(c, Li.data(), Linv.get(), Li.size());
+    d2h(c, dr.data(), dropped.get(), dr.size());
+    sync(c);
     for (int k = 0; k < w; ++k)
         if (dr[k])
             for (int m = 0; m < w; ++m) Li[k * w + m] = 0.0;
@@ -1138,6 +1140,7 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     // stream while later chunks compute (only the p-values wait for the GIF).
     DBuf<float> U;
     int wp = 0;
+    Tc8Errors errors(c);
     // Chunks: up to eight, each with at least 8 MB to copy (42 us of the host
     // link: a chunk costs about eight launches) and whole waves of one 128-row
     // tile per SM (a tenth of a last wave costs as much as a full one).
@@ -1154,8 +1157,6 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
         fp8_row_prepare(c, g, QC.get() + 1, wu, w, rp);
         wp = rp.wp;
         U.alloc(pp * wp, c.stream);
-        DBuf<int> err(1, c.stream);
-        err.zero();
         cudaEvent_t ev;
         SLFMM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         struct EvGuard {
@@ -1164,7 +1165,7 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
         } evg{ev};
         for (uint64_t r0 = 0; r0 < p; r0 += chunk) {
             const uint64_t rows = std::min(chunk, p - r0);
-            fp8_row_run(c, g, st, rp, r0, rows, U.get(), err.get());
+            fp8_row_run(c, g, st, rp, r0, rows, U.get(), nullptr);
             AssocConsts kc = k;
             kc.zero_var = k.zero_var ? k.zero_var + r0 : nullptr;
             {
@@ -1187,11 +1188,6 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
                 SLFMM_CUDA(cudaMemcpyAsync(out.r2 + r0 * 3, r2.get() + r0 * 3, rows * 3 * sizeof(double),
                                            cudaMemcpyDeviceToHost, c.copy_stream));
         }
-        const int e = fetch(c, err.get(), 1)[0];
-        if (e) {
-            SLFMM_CUDA(cudaStreamSynchronize(c.copy_stream));
-            throw_tc8_timeout(e);
-        }
         copied = true;
         phase(c, "association row pass and statistics");
     } else {
@@ -1202,7 +1198,12 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     }
     DBuf<double> graw(d, c.stream);
     launch_gif(c, hist.get(), d, graw.get());
-    std::vector<double> gr = fetch(c, graw.get(), (size_t)d);
+    std::vector<double> gr(d);
+    d2h(c, gr.data(), graw.get(), gr.size());
+    if (const int e = errors.read()) {
+        SLFMM_CUDA(cudaStreamSynchronize(c.copy_stream));  // no copy outlives a failed call
+        throw_tc8_timeout(e);
+    }
     std::vector<double> gpt(d);
     double gsum = 0.0;
     for (int jj = 0; jj < d; ++jj) {
@@ -1292,6 +1293,7 @@ void nmf_estimate(Ctx& c, const Geno& g, const slfmm_config* cfg, NmfModel& m) {
     const int l = k + 10;
     SLFMM_REQUIRE(p >= (uint64_t)l && n >= (uint64_t)l, SLFMM_ERR_BAD_ARG, "too few SNPs or samples for the NMF probe");
     m.k = k;
+    Tc8Errors errors(c);
     SnpStd sm, raw0, rawm;
     std_mean(c, g, SLFMM_NORM_EIGENSTRAT, sm);
     std_raw(c, g, nullptr, raw0);
@@ -1370,6 +1372,7 @@ void nmf_estimate(Ctx& c, const Geno& g, const slfmm_config* cfg, NmfModel& m) {
             fprintf(stderr, "NMF iteration %d: CV MAE %.6f (mean imputation %.6f, %llu held out)\n", it + 1,
                     m.cv.back(), m.cv_mean, (unsigned long long)cnt);
     }
+    errors.check();
 }
 
 void check_cfg(const slfmm_config* cfg) {
@@ -1477,6 +1480,7 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
         to_f32(c, nmf.Ht.get(), ge.p, k, He32, k);
         to_f32(c, Wpt.get(), gf.n, k, Wpt32, k);
         std_fill(c, ge, cfg->norm, NmfFill{k, W32.get(), He32.get()}, se);
+        Tc8Errors errors(c);
         SnpStd sm, rawm;
         std_mean(c, gf, SLFMM_NORM_EIGENSTRAT, sm);
         std_raw(c, gf, sm.mean.get(), rawm);
@@ -1488,6 +1492,7 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
         launch_nmf_gwas_cv(c, gf, cfg->chunk_size ? cfg->chunk_size : 10000, cfg->seed, cfg->nmf_cv_rate, W32.get(),
                            Wpt32.get(), k, part.get());
         const std::vector<double> t = sum3(c, part, gf.p);
+        errors.check();
         const uint64_t cnt = (uint64_t)(t[2] + 0.5);
         if (res) {
             if (res->nmf_cv)
@@ -1724,6 +1729,7 @@ void ctx_open(Ctx& c, int device, int precision, int verbose, cudaStream_t strea
 void ctx_close(Ctx& c) {
     cudaSetDevice(c.device);
     clear_phase_marks(c);
+    release_draws(c);
     c.dev_flags.release();
     if (c.stream) cudaStreamSynchronize(c.stream);
     if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
@@ -1902,6 +1908,7 @@ int slfmm_estimate_factors(slfmm_ctx* c, const slfmm_geno* y_est, const double* 
     SLFMM_CUDA(cudaSetDevice(c->device));
     check_cfg(cfg);
     SLFMM_REQUIRE(cfg->impute == SLFMM_IMPUTE_MEAN, SLFMM_ERR_BAD_ARG, "estimate_factors uses mean imputation");
+    if (!omega) prefetch_normal(*c, cfg->seed, y_est->n, (int)(cfg->k + cfg->oversampling));
     Step0 s0;
     step0(*c, x, y_est->n, (int)d, cfg->lambda, cfg->scale_cov != 0, s0);
     SnpStd st;
@@ -2050,6 +2057,8 @@ void fit_problem(Ctx& c, const slfmm_problem& pr) {
     SLFMM_REQUIRE(pr.packed && pr.x && pr.cfg, SLFMM_ERR_BAD_ARG, "null problem input");
     Geno full;
     Presketch ps;
+    if (!pr.omega && pr.cfg->impute == SLFMM_IMPUTE_MEAN)
+        prefetch_normal(c, pr.cfg->seed, pr.n_physical, (int)(pr.cfg->k + pr.cfg->oversampling));
     const bool pre = presketch_eligible(c, pr.n_physical, pr.n_snps, pr.x, (int)pr.d, pr.cfg, pr.omega, ps);
     upload_geno(c, full, pr.packed, pr.n_physical, pr.n_snps, nullptr, 0, nullptr,
                 pre ? &ps : nullptr);

@@ -309,23 +309,61 @@ void reference_normal(uint64_t seed, uint64_t rows, uint64_t cols, double* out) 
 struct Ctx::PendingNormal {
     uint64_t seed, rows;
     int cols;
-    std::future<std::vector<double>> draws;
+    double* out;              // the context's page-locked buffer, or `own`
+    std::vector<double> own;
+    std::future<void> done;
 };
+
+namespace {
+// Draws of a megabyte and more are made in page-locked memory: copied from
+// pageable memory, a 20 000 x 30 sketch holds the stream for half a
+// millisecond.
+constexpr size_t kPinnedDrawBytes = 1u << 20;
+
+// where a draw of `count` doubles goes; null: pageable memory of its own
+double* draw_target(Ctx& c, size_t count) {
+    if (count * sizeof(double) < kPinnedDrawBytes) return nullptr;
+    if (!c.draw_copied) SLFMM_CUDA(cudaEventCreateWithFlags(&c.draw_copied, cudaEventDisableTiming));
+    SLFMM_CUDA(cudaEventSynchronize(c.draw_copied));  // the buffer's last copy (none: at once)
+    if (count > c.draw_cap) {
+        if (c.draw_buf) cudaFreeHost(c.draw_buf);
+        c.draw_buf = nullptr;
+        c.draw_cap = 0;
+        if (cudaMallocHost(&c.draw_buf, count * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            c.draw_buf = nullptr;
+            return nullptr;
+        }
+        c.draw_cap = count;
+    }
+    return c.draw_buf;
+}
+
+std::shared_ptr<Ctx::PendingNormal> start_draw(Ctx& c, uint64_t seed, uint64_t rows, int cols) {
+    c.pending_normal.reset();  // waits for a draw that nobody took, before its buffer is used again
+    auto p = std::make_shared<Ctx::PendingNormal>();
+    p->seed = seed;
+    p->rows = rows;
+    p->cols = cols;
+    const size_t count = rows * (uint64_t)cols;
+    p->out = draw_target(c, count);
+    if (!p->out) {
+        p->own.resize(count);
+        p->out = p->own.data();
+    }
+    return p;
+}
+}  // namespace
 
 void prefetch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols) {
     if (c.rng != SLFMM_RNG_CHACHA8 || rows == 0 || cols <= 0 || cols > 64) return;  // the fit checks the shape
     if (c.pending_normal && c.pending_normal->seed == seed && c.pending_normal->rows == rows &&
         c.pending_normal->cols == cols)
         return;
-    auto p = std::make_shared<Ctx::PendingNormal>();
-    p->seed = seed;
-    p->rows = rows;
-    p->cols = cols;
-    p->draws = std::async(std::launch::async, [seed, rows, cols] {
-        std::vector<double> h(rows * (uint64_t)cols);
-        reference_normal(seed, rows, (uint64_t)cols, h.data());
-        return h;
-    });
+    auto p = start_draw(c, seed, rows, cols);
+    double* out = p->out;
+    p->done = std::async(std::launch::async,
+                         [seed, rows, cols, out] { reference_normal(seed, rows, (uint64_t)cols, out); });
     c.pending_normal = std::move(p);
 }
 
@@ -334,19 +372,33 @@ void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
         launch_normal(c, seed, rows, cols, out);
         return;
     }
-    std::vector<double> h;
-    auto& p = c.pending_normal;
-    if (p && p->seed == seed && p->rows == rows && p->cols == cols) {
-        auto mine = std::move(p);
-        h = mine->draws.get();
+    const size_t count = rows * (uint64_t)cols;
+    if (!count) return;
+    std::shared_ptr<Ctx::PendingNormal> p;
+    if (c.pending_normal && c.pending_normal->seed == seed && c.pending_normal->rows == rows &&
+        c.pending_normal->cols == cols) {
+        p = std::move(c.pending_normal);
+        c.pending_normal.reset();
+        p->done.get();
     } else {
-        h.resize(rows * (uint64_t)cols);
-        reference_normal(seed, rows, (uint64_t)cols, h.data());
+        p = start_draw(c, seed, rows, cols);
+        reference_normal(seed, rows, (uint64_t)cols, p->out);
     }
-    if (!h.empty()) {
-        SLFMM_CUDA(cudaMemcpyAsync(out, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        SLFMM_CUDA(cudaStreamSynchronize(c.stream));
+    SLFMM_CUDA(cudaMemcpyAsync(out, p->out, count * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    if (p->own.empty()) SLFMM_CUDA(cudaEventRecord(c.draw_copied, c.stream));
+    else SLFMM_CUDA(cudaStreamSynchronize(c.stream));
+}
+
+void release_draws(Ctx& c) {
+    c.pending_normal.reset();
+    if (c.draw_copied) {
+        cudaEventSynchronize(c.draw_copied);
+        cudaEventDestroy(c.draw_copied);
     }
+    if (c.draw_buf) cudaFreeHost(c.draw_buf);
+    c.draw_copied = nullptr;
+    c.draw_buf = nullptr;
+    c.draw_cap = 0;
 }
 
 }  // namespace slfmm

@@ -1351,6 +1351,11 @@ __global__ void k_f32_to_f64(const float* __restrict__ A, uint64_t m, int a, int
     }
 }
 
+__global__ void k_fill(double* __restrict__ x, uint64_t n, double v) {
+    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x)
+        x[t] = v;
+}
+
 __global__ void k_transpose(const double* __restrict__ A, int rows, int cols, double* __restrict__ At) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * cols; e += gridDim.x * blockDim.x) {
         const int i = e / cols, j = e % cols;
@@ -1721,6 +1726,12 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
         k_jacobi_svd<<<1, 1024, 0, c.stream>>>(const_cast<double*>(A), a, V, sig, ws.get());
     }
     SLFMM_LAUNCHED(c, "k_jacobi_svd");
+}
+
+void launch_fill(Ctx& c, double* x, uint64_t n, double v) {
+    if (!n) return;
+    k_fill<<<grid_for(c, n, 256), 256, 0, c.stream>>>(x, n, v);
+    SLFMM_LAUNCHED(c, "k_fill");
 }
 
 void launch_transpose(Ctx& c, const double* A, int rows, int cols, double* At) {

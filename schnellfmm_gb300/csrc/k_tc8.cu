@@ -1285,6 +1285,13 @@ void launch_fp8_terms_f32_pair(Ctx& c, const float* src, int ld, uint64_t K, int
     SLFMM_LAUNCHED(c, "k_fp8_terms_pair");
 }
 
+int Tc8Errors::read() {
+    int h = 0;
+    SLFMM_CUDA(cudaMemcpyAsync(&h, flag.get(), sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    SLFMM_CUDA(cudaStreamSynchronize(c.stream));
+    return h;
+}
+
 void throw_tc8_timeout(int site) {
     throw Error(SLFMM_ERR_DEVICE_TIMEOUT,
                 "split-FP8 contraction: a bounded device wait expired (site " + std::to_string(site) + ")");
@@ -1387,6 +1394,7 @@ static int tc8_launch(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t ro
                   "W operand not 16-byte aligned");
     raise_dynamic_smem((const void*)k_tc8_rows, pl.smem);
     DBuf<int> err;
+    if (!err_dev) err_dev = c.tc8_err;
     if (!err_dev) {
         err.alloc(1, c.stream);
         err.zero();

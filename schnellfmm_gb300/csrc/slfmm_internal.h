@@ -170,10 +170,16 @@ struct Ctx {
     };
     std::vector<PhaseMark> phase_marks;
     int rng = SLFMM_RNG_CHACHA8;  // stream of the Gaussian sketches
+    int* tc8_err = nullptr;  // a Tc8Errors scope's flag: contraction launches leave their check to it
     long long expire_next_wait = 0;  // test hook: next split-FP8 launch's wait limit (SM cycles)
     // a host draw of the reference's sketch stream started ahead of its use
     struct PendingNormal;
     std::shared_ptr<PendingNormal> pending_normal;
+    // page-locked buffer of large draws, kept for the context's life (the
+    // largest sketch drawn); its last copy to the device ends at draw_copied
+    double* draw_buf = nullptr;
+    size_t draw_cap = 0;
+    cudaEvent_t draw_copied = nullptr;
     bool autotune = false;   // time the tensor-core ring depths per shape once
     std::map<std::string, std::pair<int, int>> tuned;  // shape -> (packed ring cap, W ring cap)
 };
@@ -334,13 +340,33 @@ void launch_fp8_terms_f32_pair(Ctx& c, const float* src, int ld, uint64_t K, int
                                const double* ks_main, const double* ks_ind, int ind_row_off, int n_rows, uint8_t* B,
                                float* inv_scale);
 // mode 0: out = P (+ M); mode 1: out = s_r (P - mu_r (cs_c - M)) (needs the indicator).
-// err_dev null: the launch waits and throws when a bounded device wait expired;
-// non-null: the kernel records the site there and the caller checks it later.
+// err_dev null: the launch waits and throws when a bounded device wait expired,
+// or leaves the check to the Tc8Errors scope it runs in; non-null: the kernel
+// records the site there and the caller checks it later.
 int launch_tc8_rows(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t rows, uint64_t K,
                      const uint8_t* B, const float* inv_scale, uint64_t K_pad, int mode, const double* row_mean,
                      const double* row_scale, const double* cs, float* out, int ldo, int splits,
                      uint64_t split_stride, int* err_dev = nullptr);
 void throw_tc8_timeout(int site);
+// A scope whose contraction launches record an expired device wait in one
+// flag, which check() reads (a call of several passes waits once, not per
+// pass).
+struct Tc8Errors {
+    Ctx& c;
+    DBuf<int> flag;
+    int* outer;
+    explicit Tc8Errors(Ctx& ctx) : c(ctx), flag(1, ctx.stream), outer(ctx.tc8_err) {
+        flag.zero();
+        c.tc8_err = flag.get();
+    }
+    ~Tc8Errors() { c.tc8_err = outer; }
+    Tc8Errors(const Tc8Errors&) = delete;
+    Tc8Errors& operator=(const Tc8Errors&) = delete;
+    int read();  // the site of an expired wait, or 0 (synchronises the stream)
+    void check() {
+        if (const int e = read()) throw_tc8_timeout(e);
+    }
+};
 void launch_sub_colterm(Ctx& c, double* S, int lds, uint64_t n, int w, const double* colterm);
 
 // k_nmf.cu : NMF imputation -- fill-aware statistics, sparse corrections of
@@ -387,6 +413,7 @@ void launch_cholesky(Ctx& c, double* A, int a, int* status, double drop_tol = -1
 void launch_chol_inv(Ctx& c, const double* G, int a, double* X, bool transposed, int* status,
                      double drop_tol = -1.0, int* dropped = nullptr);
 void launch_transpose(Ctx& c, const double* A, int rows, int cols, double* At);
+void launch_fill(Ctx& c, double* x, uint64_t n, double v);
 void launch_scale_cols(Ctx& c, double* A, uint64_t m, int a, int lda, const double* f);
 void launch_build_design(Ctx& c, const double* X, int d, const double* U, int K, uint64_t n,
                          double* C);
@@ -415,6 +442,8 @@ void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out);
 // start the host draw of draw_normal(c, seed, rows, cols, .) on host threads
 // now (no-op for the device counter stream); draw_normal then waits for it
 void prefetch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols);
+// wait for a draw under way and free the draw buffer
+void release_draws(Ctx& c);
 void reference_normal(uint64_t seed, uint64_t rows, uint64_t cols, double* out);
 void launch_f64_to_f32_pad(Ctx& c, const double* A, uint64_t m, int a, int lda, float* out,
                            uint64_t m_pad, int ldo);
