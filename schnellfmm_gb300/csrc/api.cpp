@@ -1456,9 +1456,10 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
     if (!pre) phase(c, "", true);
     check_cfg(cfg);
     SLFMM_REQUIRE(ge.n == gf.n, SLFMM_ERR_BAD_ARG, "estimation and testing genotypes have different sample counts");
-    // the reference's sketch stream is drawn on host threads while Step 0 and
-    // the SNP statistics run on the device
-    if (!omega && cfg->impute == SLFMM_IMPUTE_MEAN)
+    // the reference's sketch stream is launched ahead of Step 0, whose reads
+    // back wait for it too (a sketch made under the upload has drawn it)
+    const DrawScope draw(c);
+    if (!pre && !omega && cfg->impute == SLFMM_IMPUTE_MEAN)
         prefetch_normal(c, cfg->seed, gf.n, (int)(cfg->k + cfg->oversampling));
     Step0 s0_own;
     Step0& s0 = pre ? pre->s0 : s0_own;
@@ -1908,6 +1909,7 @@ int slfmm_estimate_factors(slfmm_ctx* c, const slfmm_geno* y_est, const double* 
     SLFMM_CUDA(cudaSetDevice(c->device));
     check_cfg(cfg);
     SLFMM_REQUIRE(cfg->impute == SLFMM_IMPUTE_MEAN, SLFMM_ERR_BAD_ARG, "estimate_factors uses mean imputation");
+    const DrawScope draw(*c);
     if (!omega) prefetch_normal(*c, cfg->seed, y_est->n, (int)(cfg->k + cfg->oversampling));
     Step0 s0;
     step0(*c, x, y_est->n, (int)d, cfg->lambda, cfg->scale_cov != 0, s0);
@@ -1961,6 +1963,7 @@ int slfmm_fit_host(slfmm_ctx* c, const uint8_t* packed, uint64_t n_physical, uin
     // with every SNP in the estimation, the sketch pass runs under the upload
     Presketch ps;
     phase(*c, "", true);
+    const DrawScope draw(*c);
     if (cfg && !omega && cfg->impute == SLFMM_IMPUTE_MEAN)
         prefetch_normal(*c, cfg->seed, sample_keep ? n_keep : n_physical, (int)(cfg->k + cfg->oversampling));
     const bool pre = all && cfg && presketch_eligible(*c, sample_keep ? n_keep : n_physical, n_snps, x, (int)d,
@@ -2057,6 +2060,7 @@ void fit_problem(Ctx& c, const slfmm_problem& pr) {
     SLFMM_REQUIRE(pr.packed && pr.x && pr.cfg, SLFMM_ERR_BAD_ARG, "null problem input");
     Geno full;
     Presketch ps;
+    const DrawScope draw(c);
     if (!pr.omega && pr.cfg->impute == SLFMM_IMPUTE_MEAN)
         prefetch_normal(c, pr.cfg->seed, pr.n_physical, (int)(pr.cfg->k + pr.cfg->oversampling));
     const bool pre = presketch_eligible(c, pr.n_physical, pr.n_snps, pr.x, (int)pr.d, pr.cfg, pr.omega, ps);

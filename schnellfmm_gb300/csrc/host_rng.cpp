@@ -1,4 +1,5 @@
-// The reference's Gaussian sketch stream, drawn on the host.
+// The reference's Gaussian sketch stream on the host: the definition, and what
+// k_draw.cu falls back on.
 //
 // src/rsvd.rs:44-46 draws Omega (n x l) as
 //   Array2::from_shape_fn((n, l), |_| Normal::new(0, 1).sample(&mut ChaCha8Rng::seed_from_u64(seed)))
@@ -33,7 +34,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <future>
 #include <memory>
 #include <thread>
 #include <vector>
@@ -306,99 +306,18 @@ void reference_normal(uint64_t seed, uint64_t rows, uint64_t cols, double* out) 
 }
 
 
-struct Ctx::PendingNormal {
-    uint64_t seed, rows;
-    int cols;
-    double* out;              // the context's page-locked buffer, or `own`
-    std::vector<double> own;
-    std::future<void> done;
-};
-
-namespace {
-// Draws of a megabyte and more are made in page-locked memory: copied from
-// pageable memory, a 20 000 x 30 sketch holds the stream for half a
-// millisecond.
-constexpr size_t kPinnedDrawBytes = 1u << 20;
-
-// where a draw of `count` doubles goes; null: pageable memory of its own
-double* draw_target(Ctx& c, size_t count) {
-    if (count * sizeof(double) < kPinnedDrawBytes) return nullptr;
-    if (!c.draw_copied) SLFMM_CUDA(cudaEventCreateWithFlags(&c.draw_copied, cudaEventDisableTiming));
-    SLFMM_CUDA(cudaEventSynchronize(c.draw_copied));  // the buffer's last copy (none: at once)
-    if (count > c.draw_cap) {
-        if (c.draw_buf) cudaFreeHost(c.draw_buf);
-        c.draw_buf = nullptr;
-        c.draw_cap = 0;
-        if (cudaMallocHost(&c.draw_buf, count * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            c.draw_buf = nullptr;
-            return nullptr;
-        }
-        c.draw_cap = count;
-    }
-    return c.draw_buf;
+// The sampler's tables, x_0 .. x_256 then f_0 .. f_256, and the value of a tail
+// draw whose accepted pair began with the uniform `a`: the host's exp, log and
+// sqrt make both, so the draws made on the device equal reference_normal's.
+const double* normal_tables() {
+    const ZigTables& t = zig_tables();
+    static_assert(sizeof(ZigTables) == 2 * 257 * sizeof(double), "x then f, no padding");
+    return t.x;
 }
 
-std::shared_ptr<Ctx::PendingNormal> start_draw(Ctx& c, uint64_t seed, uint64_t rows, int cols) {
-    c.pending_normal.reset();  // waits for a draw that nobody took, before its buffer is used again
-    auto p = std::make_shared<Ctx::PendingNormal>();
-    p->seed = seed;
-    p->rows = rows;
-    p->cols = cols;
-    const size_t count = rows * (uint64_t)cols;
-    p->out = draw_target(c, count);
-    if (!p->out) {
-        p->own.resize(count);
-        p->out = p->own.data();
-    }
-    return p;
-}
-}  // namespace
-
-void prefetch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols) {
-    if (c.rng != SLFMM_RNG_CHACHA8 || rows == 0 || cols <= 0 || cols > 64) return;  // the fit checks the shape
-    if (c.pending_normal && c.pending_normal->seed == seed && c.pending_normal->rows == rows &&
-        c.pending_normal->cols == cols)
-        return;
-    auto p = start_draw(c, seed, rows, cols);
-    double* out = p->out;
-    p->done = std::async(std::launch::async,
-                         [seed, rows, cols, out] { reference_normal(seed, rows, (uint64_t)cols, out); });
-    c.pending_normal = std::move(p);
-}
-
-void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
-    if (c.rng != SLFMM_RNG_CHACHA8) {
-        launch_normal(c, seed, rows, cols, out);
-        return;
-    }
-    const size_t count = rows * (uint64_t)cols;
-    if (!count) return;
-    std::shared_ptr<Ctx::PendingNormal> p;
-    if (c.pending_normal && c.pending_normal->seed == seed && c.pending_normal->rows == rows &&
-        c.pending_normal->cols == cols) {
-        p = std::move(c.pending_normal);
-        c.pending_normal.reset();
-        p->done.get();
-    } else {
-        p = start_draw(c, seed, rows, cols);
-        reference_normal(seed, rows, (uint64_t)cols, p->out);
-    }
-    SLFMM_CUDA(cudaMemcpyAsync(out, p->out, count * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    if (p->own.empty()) SLFMM_CUDA(cudaEventRecord(c.draw_copied, c.stream));
-    else SLFMM_CUDA(cudaStreamSynchronize(c.stream));
-}
-
-void release_draws(Ctx& c) {
-    c.pending_normal.reset();
-    if (c.draw_copied) {
-        cudaEventSynchronize(c.draw_copied);
-        cudaEventDestroy(c.draw_copied);
-    }
-    if (c.draw_buf) cudaFreeHost(c.draw_buf);
-    c.draw_copied = nullptr;
-    c.draw_buf = nullptr;
-    c.draw_cap = 0;
+double normal_tail_value(double a, bool negative) {
+    const double ex = std::log(a) / kZigR;
+    return 0.0 + 1.0 * (negative ? ex - kZigR : kZigR - ex);
 }
 
 }  // namespace slfmm

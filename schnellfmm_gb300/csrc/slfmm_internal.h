@@ -172,14 +172,15 @@ struct Ctx {
     int rng = SLFMM_RNG_CHACHA8;  // stream of the Gaussian sketches
     int* tc8_err = nullptr;  // a Tc8Errors scope's flag: contraction launches leave their check to it
     long long expire_next_wait = 0;  // test hook: next split-FP8 launch's wait limit (SM cycles)
-    // a host draw of the reference's sketch stream started ahead of its use
+    // a draw of the reference's sketch stream started ahead of its use
     struct PendingNormal;
     std::shared_ptr<PendingNormal> pending_normal;
-    // page-locked buffer of large draws, kept for the context's life (the
-    // largest sketch drawn); its last copy to the device ends at draw_copied
-    double* draw_buf = nullptr;
-    size_t draw_cap = 0;
-    cudaEvent_t draw_copied = nullptr;
+    // page-locked block that a draw's tail list is read back to, kept for the
+    // context's life (the longest list); the last copy into it ends at draw_done
+    struct NormalTails;
+    NormalTails* draw_tails = nullptr;
+    size_t draw_tails_bytes = 0;
+    cudaEvent_t draw_done = nullptr;
     bool autotune = false;   // time the tensor-core ring depths per shape once
     std::map<std::string, std::pair<int, int>> tuned;  // shape -> (packed ring cap, W ring cap)
 };
@@ -437,13 +438,23 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig);
 void launch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out);
 // rows x cols Normal(0, 1) sketch into device memory from the context's
 // stream: the device counter stream (launch_normal) or the reference's ChaCha8
-// stream drawn on the host (reference_normal) and copied
+// stream (k_draw.cu)
 void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out);
-// start the host draw of draw_normal(c, seed, rows, cols, .) on host threads
-// now (no-op for the device counter stream); draw_normal then waits for it
+// launch the ChaCha8 draw of draw_normal(c, seed, rows, cols, .) now (no-op for
+// the device counter stream), so that its short read-back is done when
+// draw_normal wants it
 void prefetch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols);
-// wait for a draw under way and free the draw buffer
+// a draw started inside the scope and taken by nobody ends with it
+struct DrawScope {
+    Ctx& c;
+    explicit DrawScope(Ctx& ctx) : c(ctx) {}
+    DrawScope(const DrawScope&) = delete;
+    ~DrawScope() { c.pending_normal.reset(); }
+};
+// free the draw's buffers
 void release_draws(Ctx& c);
+const double* normal_tables();
+double normal_tail_value(double a, bool negative);
 void reference_normal(uint64_t seed, uint64_t rows, uint64_t cols, double* out);
 void launch_f64_to_f32_pad(Ctx& c, const double* A, uint64_t m, int a, int lda, float* out,
                            uint64_t m_pad, int ldo);
