@@ -1275,11 +1275,11 @@ void to_f32(Ctx& c, const double* A, uint64_t m, int a, DBuf<float>& out, int ld
     launch_f64_to_f32_pad(c, A, m, a, a, out.get(), m, ld);
 }
 
-// (sum |g - pred|, sum |g - mean|, count) over a p x 3 partials array
-std::vector<double> sum3(Ctx& c, const DBuf<double>& part, uint64_t p) {
+// (sum |g - pred|, sum |g - mean|, count) over an m x 3 partials array
+std::vector<double> sum3(Ctx& c, const DBuf<double>& part, uint64_t m) {
     DBuf<double> tot(3, c.stream);
     tot.zero();
-    launch_colsums(c, part.get(), p, 3, 3, tot.get());
+    launch_colsums(c, part.get(), m, 3, 3, tot.get());
     return fetch(c, tot.get(), 3);
 }
 
@@ -1330,7 +1330,7 @@ void nmf_estimate(Ctx& c, const Geno& g, const slfmm_config* cfg, NmfModel& m) {
     nmf_normalize(c, m, n, p, eps);
     const int kp = pad16(k);
     DBuf<double> hh(k * k, c.stream), wtw(k * k, c.stream), denW(n * k, c.stream), denH(p * k, c.stream);
-    DBuf<double> part(std::max<uint64_t>(p, 1) * 3, c.stream);
+    DBuf<double> part;
     m.cv.clear();
     m.total = 0;
     for (int it = 0; it < (int)cfg->nmf_iter; ++it) {
@@ -1362,8 +1362,9 @@ void nmf_estimate(Ctx& c, const Geno& g, const slfmm_config* cfg, NmfModel& m) {
         // CV on held-out calls (src/nmf.rs:379-455), mask stream seed + it
         to_f32(c, m.W.get(), n, k, W32, k);
         to_f32(c, m.Ht.get(), p, k, H32, k);
-        launch_nmf_cv(c, g, chunk, cfg->seed + (uint64_t)it, cfg->nmf_cv_rate, W32.get(), H32.get(), k, part.get());
-        const std::vector<double> t = sum3(c, part, p);
+        const uint64_t rows = launch_nmf_cv(c, g, chunk, cfg->seed + (uint64_t)it, cfg->nmf_cv_rate, W32.get(),
+                                            H32.get(), k, part);
+        const std::vector<double> t = sum3(c, part, rows);
         const uint64_t cnt = (uint64_t)(t[2] + 0.5);
         m.cv.push_back(cnt ? t[0] / (double)cnt : 0.0);
         m.cv_mean = cnt ? t[1] / (double)cnt : 0.0;
@@ -1489,10 +1490,10 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
         to_f32(c, Hf.get(), gf.p, k, Hf32, k);
         std_fill(c, gf, cfg->norm, NmfFill{k, W32.get(), Hf32.get()}, sf);
         sfp = &sf;
-        DBuf<double> part(std::max<uint64_t>(gf.p, 1) * 3, c.stream);
-        launch_nmf_gwas_cv(c, gf, cfg->chunk_size ? cfg->chunk_size : 10000, cfg->seed, cfg->nmf_cv_rate, W32.get(),
-                           Wpt32.get(), k, part.get());
-        const std::vector<double> t = sum3(c, part, gf.p);
+        DBuf<double> part;
+        const uint64_t rows = launch_nmf_gwas_cv(c, gf, cfg->chunk_size ? cfg->chunk_size : 10000, cfg->seed,
+                                                 cfg->nmf_cv_rate, W32.get(), Wpt32.get(), k, part);
+        const std::vector<double> t = sum3(c, part, rows);
         errors.check();
         const uint64_t cnt = (uint64_t)(t[2] + 0.5);
         if (res) {

@@ -327,250 +327,388 @@ __global__ void k_nmf_sign(const TS* __restrict__ src, int ldsrc, double* __rest
     }
 }
 
+// Hold-out draws, eight consecutive counters of a stream at a time: bit j of
+// mask8(blk) is set iff draw 8 blk + j is below the rate.  The counter stream
+// (draw_below), or with kChaCha one ChaCha8 block, its comparison
+// (u64 >> 12) < thresh made on the whole u64.
+template <bool kChaCha>
+struct HoldDraws {
+    ChaCha8Draws cc;
+    uint64_t key, thresh;
+    bool all;
+    __device__ HoldDraws(uint64_t seed, uint64_t t)
+        : cc(seed), key(mix64(seed + kGamma)), thresh(kChaCha ? t << 12 : t), all(kChaCha && (t >> 52) != 0) {}
+    __device__ __forceinline__ uint32_t mask8(uint64_t blk) {
+        uint32_t m = 0;
+        if constexpr (kChaCha) {
+            cc.blk = blk;
+            cc.refill();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) m |= cc.word(j) < thresh ? 1u << j : 0u;
+            if (all) m = 0xffu;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) m |= draw_below(key, 8 * blk + j, thresh) ? 1u << j : 0u;
+        }
+        return m;
+    }
+};
+
+// the even bits 0, 2 .. 14 of x as bits 0 .. 7
+__device__ __forceinline__ uint32_t even_bits8(uint32_t x) {
+    x &= 0x5555u;
+    x = (x | (x >> 1)) & 0x3333u;
+    x = (x | (x >> 2)) & 0x0f0fu;
+    return (x | (x >> 4)) & 0xffu;
+}
+// bit b: code b of the eight is 01, a missing call
+__device__ __forceinline__ uint32_t missing8(uint32_t codes) { return even_bits8(codes & ~(codes >> 1)); }
+
+// Held-out calls are few (1 % by default) and uneven over the lanes, and their
+// absolute errors are FP64: warps queue them and take 32 at a time.
+struct HeldCounts {
+    uint32_t g0 = 0, g1 = 0, g2 = 0;  // held-out calls by genotype
+    __device__ __forceinline__ void add(uint32_t code, bool on) {
+        g0 += __popc(__ballot_sync(0xffffffffu, on && code == 0u));
+        g1 += __popc(__ballot_sync(0xffffffffu, on && code == 2u));
+        g2 += __popc(__ballot_sync(0xffffffffu, on && code == 3u));
+    }
+    __device__ __forceinline__ uint32_t total() const { return g0 + g1 + g2; }
+};
+
 // Estimation-phase CV (compute_cv_error_masked, src/nmf.rs:379-455).  Chunk
 // `seq` of `chunk` SNPs uses the stream of mask_seed + seq (the counter
 // stream, or ChaCha8 with kChaCha); entry (i, r) draws counter
 // (r - chunk start) n + i (column-major, missing calls included) and is held
-// out iff the draw is below `rate` and the call is observed.  Per SNP:
-// sum |g - W_i.H_r|, sum |g - mean_r|, count.
+// out iff the draw is below `rate` and the call is observed.  Sums of
+// |g - W_i.H_r|, |g - mean_r| and the count, one row of `part` per warp.
+//
+// Bound by the integer pipe: a ChaCha8 block is 384 additions, exclusive-ors
+// and rotations for eight calls.  A lane takes one whole block, whatever the
+// alignment of the SNP's first counter to the blocks.  100 000 SNPs x 3 000
+// samples, rate 1 %: 1.10 ms with the calls laid out by code words, 0.71 ms so.
 template <bool kChaCha, int KM>
 __global__ void __launch_bounds__(256) k_nmf_cv(const uint8_t* __restrict__ packed, uint64_t stride, uint64_t n,
                                                 uint64_t p, uint64_t chunk, uint64_t mask_seed, uint64_t thresh,
                                                 const float* __restrict__ W, const float* __restrict__ H, int k,
                                                 const int32_t* __restrict__ counts, double* __restrict__ part) {
     __shared__ float hs[8][KM];
+    __shared__ uint32_t queue[8][64];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint64_t nw = (uint64_t)gridDim.x * 8;
-    for (uint64_t r = (uint64_t)blockIdx.x * 8 + wl; r < p; r += nw) {
+    const uint64_t nw = (uint64_t)gridDim.x * 8, first = (uint64_t)blockIdx.x * 8 + wl;
+    uint32_t* q = queue[wl];
+    const uint64_t nwords = (n + 15) / 16;
+    double e1 = 0.0, e2 = 0.0;
+    unsigned long long cnt = 0;
+    // SNP number j of the warp leaves its held-out counts with lane j mod 32;
+    // the means they are compared with are divided out 32 SNPs at a time
+    HeldCounts mine;
+    uint64_t mine_r = 0;
+    auto mean_errors = [&]() {
+        if (mine.total()) {
+            const int4 cs = *reinterpret_cast<const int4*>(counts + mine_r * 4);
+            const int64_t nobs = (int64_t)cs.x + cs.y + cs.z;
+            const double cm = (double)((int64_t)cs.y + 2 * (int64_t)cs.z) / (double)nobs;
+            e2 += (double)mine.g0 * fabs(0.0 - cm) + (double)mine.g1 * fabs(1.0 - cm) + (double)mine.g2 * fabs(2.0 - cm);
+        }
+        mine = HeldCounts();
+    };
+    int turn = 0;
+    for (uint64_t r = first; r < p; r += nw, turn = (turn + 1) & 31) {
         __syncwarp();
         if (lane < k) hs[wl][lane] = H[r * k + lane];
         __syncwarp();
-        const uint64_t seq = r / chunk, col = r - seq * chunk;
-        const uint64_t key = mix64(mask_seed + seq + kGamma);
-        ChaCha8Draws cc(mask_seed + seq);
-        const int64_t c0 = counts[r * 4], c1 = counts[r * 4 + 1], c2 = counts[r * 4 + 2];
-        const int64_t nobs = c0 + c1 + c2;
-        const double cm = nobs > 0 ? (double)(c1 + 2 * c2) / (double)nobs : 0.0;
-        // a lane takes the 16 codes of one 32-bit word at a time; the draw
-        // input key + (ctr + 1) gamma of consecutive samples differs by gamma
-        const uint32_t* row = reinterpret_cast<const uint32_t*>(packed + r * stride);
-        const uint64_t nwords = (n + 15) / 16;
-        double e1 = 0.0, e2 = 0.0, cnt = 0.0;
-        auto held_out = [&](uint64_t i, uint32_t code) {
-            const double g = code == 0 ? 0.0 : (double)(code - 1);
-            e1 += fabs(g - (double)fill_dot<KM>(W + i * k, hs[wl], k));
-            e2 += fabs(g - cm);
-            cnt += 1.0;
+        const uint64_t seq = r / chunk, e0 = (r - seq * chunk) * n;
+        HoldDraws<kChaCha> draws(mask_seed + seq, thresh);
+        const uint8_t* rowb = packed + r * stride;
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(rowb);
+        HeldCounts held_here;
+        int queued = 0;
+        auto take = [&](int m) {
+            uint32_t code = 0;
+            if (lane < m) {
+                const uint64_t i = q[lane];
+                code = code_at(rowb, i);
+                const double g = code == 0 ? 0.0 : (double)(code - 1);
+                e1 += fabs(g - (double)fill_dot<KM>(W + i * k, hs[wl], k));
+            }
+            held_here.add(code, lane < m);
         };
-        for (uint64_t wd = lane; wd < nwords; wd += 32) {
-            const uint32_t v = row[wd];
-            const uint64_t i0 = wd * 16;
-            const int nb = n - i0 < 16 ? (int)(n - i0) : 16;
-            if constexpr (kChaCha) {
-                // the word's entries use the blocks e0 / 8 .. (e0 + nb - 1) / 8;
-                // every lane refills at the same points (e0 is the same modulo
-                // 8 for all lanes of the SNP), so the refills do not diverge
-                const uint64_t e0 = col * n + i0, last = (e0 + nb - 1) >> 3;
-                for (uint64_t bk = e0 >> 3; bk <= last; ++bk) {
-                    cc.blk = bk;
-                    cc.refill();
-                    const int lo = bk * 8 > e0 ? (int)(bk * 8 - e0) : 0;
-                    const int hi = min(nb, (int)((bk + 1) * 8 - e0));
-                    for (int b = lo; b < hi; ++b) {
-                        const uint32_t code = (v >> (2 * b)) & 3u;
-                        if (code == 1u || (cc.word((int)((e0 + b) & 7)) >> 12) >= thresh) continue;
-                        held_out(i0 + b, code);
-                    }
+        const uint64_t b1 = (e0 + n + 7) >> 3;
+        for (uint64_t bb = e0 >> 3; bb < b1; bb += 32) {
+            // the block's calls i0 .. i0 + 7 of the SNP (i0 may be below 0)
+            const int64_t i0 = (int64_t)(8 * (bb + lane)) - (int64_t)e0;
+            const int64_t wd = i0 >> 4;
+            uint32_t w0 = 0, w1 = 0;
+            if (wd >= 0 && wd < (int64_t)nwords) w0 = row[wd];
+            if (wd + 1 < (int64_t)nwords) w1 = row[wd + 1];
+            const uint32_t codes = __funnelshift_r(w0, w1, 2 * (uint32_t)(i0 & 15));
+            const int lo = i0 < 0 ? (int)-i0 : 0;
+            const int hi = i0 + 8 <= (int64_t)n ? 8 : i0 < (int64_t)n ? (int)((int64_t)n - i0) : 0;
+            uint32_t held = draws.mask8(bb + lane) & ~missing8(codes);
+            held &= hi > lo ? (1u << hi) - (1u << lo) : 0u;
+            while (const uint32_t any = __ballot_sync(0xffffffffu, held != 0)) {
+                if (held) {
+                    q[queued + __popc(any & ((1u << lane) - 1))] = (uint32_t)(i0 + __ffs(held) - 1);
+                    held &= held - 1;
                 }
-            } else {
-                uint64_t z = key + (col * n + i0 + 1) * kGamma;
-                for (int b = 0; b < nb; ++b, z += kGamma) {
-                    const uint32_t code = (v >> (2 * b)) & 3u;
-                    if (code == 1u || (mix64(z) >> 11) >= thresh) continue;
-                    held_out(i0 + b, code);
+                queued += __popc(any);
+                __syncwarp();
+                if (queued >= 32) {
+                    take(32);
+                    queued -= 32;
+                    const uint32_t v = q[32 + lane];
+                    __syncwarp();
+                    q[lane] = v;
+                    __syncwarp();
                 }
             }
         }
-        e1 = warp_sum_d(e1);
-        e2 = warp_sum_d(e2);
-        cnt = warp_sum_d(cnt);
-        if (lane == 0) {
-            part[r * 3] = e1;
-            part[r * 3 + 1] = e2;
-            part[r * 3 + 2] = cnt;
+        take(queued);
+        if (lane == turn) {
+            mine = held_here;
+            mine_r = r;
         }
+        cnt += held_here.total();
+        if (turn == 31) mean_errors();
+    }
+    mean_errors();
+    e1 = warp_sum_d(e1);
+    e2 = warp_sum_d(e2);
+    if (lane == 0) {
+        part[first * 3] = e1;
+        part[first * 3 + 1] = e2;
+        part[first * 3 + 2] = (double)cnt;
     }
 }
 
 // Observed calls before each SNP within its chunk (the GWAS-phase CV numbers
-// its draws by the rank of the observed call in column-major order)
-__global__ void k_obs_base(const int32_t* __restrict__ counts, uint64_t p, uint64_t chunk, uint64_t* __restrict__ base) {
+// its draws by the rank of the observed call in column-major order).  A block
+// per chunk, 1 024 SNPs at a time; a thread walking each chunk of 10 000 took
+// 1.2 ms.
+__global__ void __launch_bounds__(1024) k_obs_base(const int32_t* __restrict__ counts, uint64_t p, uint64_t chunk,
+                                                   uint64_t* __restrict__ base) {
+    __shared__ uint64_t wsum[32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint64_t nchunks = (p + chunk - 1) / chunk;
-    for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b < nchunks;
-         b += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t acc = 0;
-        const uint64_t r1 = min(p, (b + 1) * chunk);
-        for (uint64_t r = b * chunk; r < r1; ++r) {
-            base[r] = acc;
-            acc += (uint64_t)(counts[r * 4] + counts[r * 4 + 1] + counts[r * 4 + 2]);
+    for (uint64_t b = blockIdx.x; b < nchunks; b += gridDim.x) {
+        uint64_t carry = 0;
+        const uint64_t r0 = b * chunk, r1 = chunk < p - r0 ? r0 + chunk : p;
+        for (uint64_t s = r0; s < r1; s += 1024) {
+            const uint64_t r = s + threadIdx.x;
+            uint64_t v = 0;
+            if (r < r1) v = (uint64_t)(counts[r * 4] + counts[r * 4 + 1] + counts[r * 4 + 2]);
+            uint64_t incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            if (lane == 31) wsum[wl] = incl;
+            __syncthreads();
+            uint64_t before = carry;
+            for (int w = 0; w < 32; ++w) {
+                if (w < wl) before += wsum[w];
+                carry += wsum[w];
+            }
+            if (r < r1) base[r] = before + incl - v;
+            __syncthreads();
         }
     }
 }
 
-// Hold-out draws of the warp's 256 samples i0 .. i0 + 255 with the draws
-// laid out so that one ChaCha8 block (eight outputs) serves up to eight of
-// them: lane l takes samples i0 + 8 l .. i0 + 8 l + 7, whose observed calls
-// (code != 01) have consecutive counters -- `before` (observed calls of the
-// SNP's chunk before i0) plus those of the lower lanes, by a warp scan.
-// Returns the lane's held-out bits (bit b: sample i0 + 8 l + b) and its 16
-// code bits in `codes`; `before` advances past the 256 samples.  The callers
-// move the bits back to one sample per lane with shuffles, so their W-row
-// loads stay coalesced.
+// The hold-out draws of consecutive counters from `before` on, for a warp that
+// takes them up to 256 at a time: two runs of 32 blocks, a block per lane, so
+// that every block is computed once.
 template <bool kChaCha>
-__device__ __forceinline__ uint32_t lane_held8(const uint8_t* row, uint64_t n, uint64_t i0, uint64_t& before,
-                                               uint64_t key, ChaCha8Draws& cc, uint64_t thresh, uint32_t& codes) {
-    const uint64_t ib = i0 + 8 * (uint64_t)(threadIdx.x & 31);
-    uint32_t obs = 0;
-    codes = 0x5555u;  // past n: "missing", neither observed nor drawn
-    if (ib < n) {
-        codes = *reinterpret_cast<const uint16_t*>(row + ib / 4);
+struct HeldStream {
+    HoldDraws<kChaCha> draws;
+    uint64_t before, base;  // next counter; first block of `cur`
+    uint32_t cur = 0, nxt = 0;
+    int filled = 0;
+    __device__ HeldStream(uint64_t seed, uint64_t thresh, uint64_t c0)
+        : draws(seed, thresh), before(c0), base(c0 >> 3) {}
+    // Bits of the lane's eight calls that are held out: `obs` marks those that
+    // draw, lane 0's first, each lane's in order; `before` moves past them.
+    __device__ __forceinline__ uint32_t held8(uint32_t obs) {
+        const int lane = threadIdx.x & 31;
+        const int cnt = __popc(obs);
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const uint32_t rel = (uint32_t)(before - 8 * base);  // below 256
+        const uint32_t total = (uint32_t)__shfl_sync(0xffffffffu, incl, 31);
+        const int need = rel + total > 256u ? 2 : 1;
+        for (; filled < need; ++filled) {
+            const uint32_t m = draws.mask8(base + 32 * (uint64_t)filled + lane);
+            if (filled == 0) cur = m;
+            else nxt = m;
+        }
+        const uint32_t both = cur | nxt << 8;
+        const uint32_t c = rel + (uint32_t)(incl - cnt), o = c >> 3;
+        const uint32_t v0 = __shfl_sync(0xffffffffu, both, o & 31), v1 = __shfl_sync(0xffffffffu, both, (o + 1) & 31);
+        const uint32_t lo8 = o < 32 ? v0 & 0xffu : v0 >> 8, hi8 = o + 1 < 32 ? v1 & 0xffu : v1 >> 8;
+        uint32_t bits = (lo8 | hi8 << 8) >> (c & 7), held = 0;
 #pragma unroll
         for (int b = 0; b < 8; ++b)
-            if (ib + b < n && ((codes >> (2 * b)) & 3u) != 1u) obs |= 1u << b;
-    }
-    const int cnt = __popc(obs);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)(threadIdx.x & 31) >= o) incl += v;
-    }
-    const uint64_t c0 = before + (uint64_t)(incl - cnt);
-    before += (uint64_t)__shfl_sync(0xffffffffu, incl, 31);
-    uint32_t held = 0;
-    if constexpr (kChaCha) {
-        // at most eight consecutive counters: blocks c0 / 8 and c0 / 8 + 1,
-        // computed by every lane together (no divergent refills)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            cc.blk = (c0 >> 3) + (uint64_t)half;
-            cc.refill();
-            uint64_t ctr = c0;
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                if (!((obs >> b) & 1u)) continue;
-                if ((ctr >> 3) == cc.blk && (cc.word((int)(ctr & 7)) >> 12) < thresh) held |= 1u << b;
-                ++ctr;
+            if ((obs >> b) & 1u) {
+                held |= (bits & 1u) << b;
+                bits >>= 1;
             }
+        before += total;
+        if (rel + total >= 256u) {
+            cur = nxt;
+            base += 32;
+            --filled;
         }
-    } else {
-        uint64_t ctr = c0;
-        for (int b = 0; b < 8; ++b) {
-            if (!((obs >> b) & 1u)) continue;
-            if (draw_below(key, ctr, thresh)) held |= 1u << b;
-            ++ctr;
-        }
+        return held;
     }
-    return held;
+};
+
+// acc[c] += row[c] * g, or += row[c], for c < k
+template <bool W4, int KM>
+__device__ __forceinline__ void load_row(const float* __restrict__ wp, int k, float (&w)[KM]) {
+    if constexpr (W4) {
+#pragma unroll
+        for (int c = 0; c < KM; c += 4)
+            if (c < k) {
+                const float4 v = *reinterpret_cast<const float4*>(wp + c);
+                w[c] = v.x, w[c + 1] = v.y, w[c + 2] = v.z, w[c + 3] = v.w;
+            }
+    } else {
+#pragma unroll
+        for (int c = 0; c < KM; ++c)
+            if (c < k) w[c] = wp[c];
+    }
 }
+
+constexpr int kHeldList = 512;
 
 // GWAS-phase CV (src/testing.rs:423-487): per chunk the stream seed + seq,
 // one draw per OBSERVED call (counter = its column-major rank in the chunk),
 // held out iff the draw is below `rate`; the held-out column is refilled with
 // its leave-out mean mu', H = max(0, W+ y~) and the MAE of W_i.H and of mu'
-// over the held-out calls accumulate.  W+ y~ = A + mu' B with A = sum over
-// kept observed calls of W+_i g, B = sum over missing and held-out calls of
-// W+_i.  One warp per SNP, two passes over its codes; the hold-out draws of
-// each 256 samples come from lane_held8.  kChaCha draws from the reference's
-// ChaCha8 stream instead of the counter stream.
-template <bool kChaCha, int KM>
+// over the held-out calls accumulate, one row of `part` per warp.  W+ y~ = A +
+// mu' B with A = sum over kept observed calls of W+_i g, B = sum over missing
+// and held-out calls of W+_i.  One warp per SNP: lane l draws for samples
+// i0 + 8 l .. i0 + 8 l + 7 of each 256, and takes i0 + l, i0 + l + 32 .. of
+// A and B, so that its W+ rows are read in order.  The held-out calls are
+// listed for the errors (kHeldList of them; a SNP with more goes over its
+// codes and draws a second time).
+//
+// Bound by the draws, as k_nmf_cv.  100 000 SNPs x 3 000 samples, rate 1 %:
+// 6.96 ms with each block computed four times (for two lanes, in two
+// passes) and FP64 counts, 1.97 ms so.
+template <bool kChaCha, bool W4, int KM>
 __global__ void __launch_bounds__(256) k_nmf_gwas_cv(const uint8_t* __restrict__ packed, uint64_t stride, uint64_t n,
                                                      uint64_t p, uint64_t chunk, uint64_t seed, uint64_t thresh,
                                                      const float* __restrict__ W, const float* __restrict__ Wpt, int k,
+                                                     const int32_t* __restrict__ counts,
                                                      const uint64_t* __restrict__ base, double* __restrict__ part) {
     __shared__ float hh[8][KM];
+    __shared__ uint32_t list[8][kHeldList];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint64_t nw = (uint64_t)gridDim.x * 8;
-    for (uint64_t r = (uint64_t)blockIdx.x * 8 + wl; r < p; r += nw) {
+    const uint64_t nw = (uint64_t)gridDim.x * 8, first = (uint64_t)blockIdx.x * 8 + wl;
+    uint32_t* q = list[wl];
+    double e1 = 0.0, e2 = 0.0;
+    unsigned long long cnt = 0;
+    for (uint64_t r = first; r < p; r += nw) {
         const uint64_t seq = r / chunk;
-        const uint64_t key = mix64(seed + seq + kGamma);
-        ChaCha8Draws cc(seed + seq);
         const uint8_t* row = packed + r * stride;
         float A[KM], B[KM];
 #pragma unroll
         for (int c = 0; c < KM; ++c) A[c] = B[c] = 0.f;
-        double s1 = 0.0, nk = 0.0;
-        int nmask = 0;
-        uint64_t before = base[r];
-        for (uint64_t i0 = 0; i0 < n; i0 += 256) {
-            uint32_t codes;
-            const uint32_t held8 = lane_held8<kChaCha>(row, n, i0, before, key, cc, thresh, codes);
-            // the warp's 256 samples in the coalesced layout: sample i0 + 32 j + lane
-            for (int j = 0; j < 8; ++j) {
-                const uint64_t i = i0 + 32 * (uint64_t)j + lane;
-                const int src = 4 * j + (lane >> 3), bit = lane & 7;
-                const uint32_t hm = __shfl_sync(0xffffffffu, held8, src);
-                const uint32_t cw = __shfl_sync(0xffffffffu, codes, src);
-                if (i >= n) continue;
-                const uint32_t code = (cw >> (2 * bit)) & 3u;
-                const bool held = (hm >> bit) & 1u;
-                const float* wp = Wpt + i * k;
-                if (code != 1u && !held) {
-                    const float g = code == 0 ? 0.f : (float)(code - 1);
-                    s1 += (double)g;
-                    nk += 1.0;
-#pragma unroll
-                    for (int c = 0; c < KM; ++c)
-                        if (c < k) A[c] = fmaf(wp[c], g, A[c]);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < KM; ++c)
-                        if (c < k) B[c] += wp[c];
+        HeldCounts held_here;
+        // pass 0 fills A, B and the list; pass 1, only when the list did not
+        // hold every held-out call, takes their errors from the draws again
+        for (int pass = 0; pass < 2; ++pass) {
+            HeldStream<kChaCha> draws(seed + seq, thresh, base[r]);
+            uint32_t listed = 0;
+            for (uint64_t i0 = 0; i0 < n; i0 += 256) {
+                const uint64_t ib = i0 + 8 * (uint64_t)lane;
+                uint32_t codes = 0x5555u, obs = 0;  // past n: neither observed nor drawn
+                if (ib < n) {
+                    codes = *reinterpret_cast<const uint16_t*>(row + ib / 4);
+                    obs = 0xffu & ~missing8(codes);
+                    if (n - ib < 8) obs &= (1u << (n - ib)) - 1;
                 }
-                nmask += held ? 1 : 0;
-            }
-        }
-        nmask = __reduce_add_sync(0xffffffffu, nmask);
-        if (nmask == 0) {
-            if (lane == 0) part[r * 3] = part[r * 3 + 1] = part[r * 3 + 2] = 0.0;
-            continue;
-        }
-        s1 = warp_sum_d(s1);
-        nk = warp_sum_d(nk);
-        const double mu = nk > 0.0 ? s1 / nk : 0.0;
+                uint32_t held = draws.held8(obs);
+                if (pass == 0) {
+                    const uint32_t both = codes | held << 16;
+#pragma unroll 2
+                    for (int j = 0; j < 8; ++j) {
+                        const uint64_t i = i0 + 32 * (uint64_t)j + lane;
+                        const uint32_t v = __shfl_sync(0xffffffffu, both, 4 * j + (lane >> 3));
+                        if (i >= n) continue;
+                        const uint32_t code = (v >> (2 * (lane & 7))) & 3u;
+                        const bool kept = code != 1u && !((v >> (16 + (lane & 7))) & 1u);
+                        float w[KM];
+                        load_row<W4, KM>(Wpt + i * k, k, w);
+                        const float g = code == 0 ? 0.f : (float)(code - 1);
+                        if (kept) {
 #pragma unroll
-        for (int c = 0; c < KM; ++c) {
-            if (c < k) {
-                const float a = warp_sum_f(A[c]), b = warp_sum_f(B[c]);
-                if (lane == 0) hh[wl][c] = fmaxf(a + (float)mu * b, 0.f);
+                            for (int c = 0; c < KM; ++c)
+                                if (c < k) A[c] = fmaf(w[c], g, A[c]);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < KM; ++c)
+                                if (c < k) B[c] += w[c];
+                        }
+                    }
+                }
+                while (const uint32_t any = __ballot_sync(0xffffffffu, held != 0)) {
+                    const int b = held ? __ffs(held) - 1 : 0;
+                    const uint32_t code = (codes >> (2 * b)) & 3u;
+                    const uint32_t at = listed + __popc(any & ((1u << lane) - 1));
+                    if (pass == 0) {
+                        if (held && at < kHeldList) q[at] = (uint32_t)(ib + b);
+                        held_here.add(code, held != 0);
+                    } else if (held) {
+                        const double g = code == 0 ? 0.0 : (double)(code - 1);
+                        e1 += fabs(g - (double)fill_dot<KM>(W + (ib + b) * k, hh[wl], k));
+                    }
+                    held &= held - 1;
+                    listed += __popc(any);
+                }
             }
-        }
-        __syncwarp();
-        double e1 = 0.0, e2 = 0.0;
-        before = base[r];
-        for (uint64_t i0 = 0; i0 < n; i0 += 256) {
-            uint32_t codes;
-            const uint32_t held8 = lane_held8<kChaCha>(row, n, i0, before, key, cc, thresh, codes);
-            for (int j = 0; j < 8; ++j) {
-                const uint64_t i = i0 + 32 * (uint64_t)j + lane;
-                const int src = 4 * j + (lane >> 3), bit = lane & 7;
-                const uint32_t hm = __shfl_sync(0xffffffffu, held8, src);
-                const uint32_t cw = __shfl_sync(0xffffffffu, codes, src);
-                if (i >= n || !((hm >> bit) & 1u)) continue;
-                const uint32_t code = (cw >> (2 * bit)) & 3u;
+            if (pass == 1 || listed == 0) break;
+            const int4 cs = *reinterpret_cast<const int4*>(counts + r * 4);
+            const int64_t s1 = (int64_t)cs.y + 2 * (int64_t)cs.z - held_here.g1 - 2 * (int64_t)held_here.g2;
+            const int64_t nk = (int64_t)cs.x + cs.y + cs.z - held_here.total();
+            const double mu = nk > 0 ? (double)s1 / (double)nk : 0.0;
+            __syncwarp();  // the last SNP's errors are done with hh
+#pragma unroll
+            for (int c = 0; c < KM; ++c) {
+                if (c < k) {
+                    const float a = warp_sum_f(A[c]), b = warp_sum_f(B[c]);
+                    if (lane == 0) hh[wl][c] = fmaxf(a + (float)mu * b, 0.f);
+                }
+            }
+            __syncwarp();
+            if (lane < 3)
+                e2 += (double)(lane == 0 ? held_here.g0 : lane == 1 ? held_here.g1 : held_here.g2) *
+                      fabs((double)lane - mu);
+            cnt += listed;
+            if (listed > kHeldList) continue;
+            for (uint32_t t = lane; t < listed; t += 32) {
+                const uint64_t i = q[t];
+                const uint32_t code = code_at(row, i);
                 const double g = code == 0 ? 0.0 : (double)(code - 1);
                 e1 += fabs(g - (double)fill_dot<KM>(W + i * k, hh[wl], k));
-                e2 += fabs(g - mu);
             }
-        }
-        e1 = warp_sum_d(e1);
-        e2 = warp_sum_d(e2);
-        if (lane == 0) {
-            part[r * 3] = e1;
-            part[r * 3 + 1] = e2;
-            part[r * 3 + 2] = (double)nmask;
+            break;
         }
         __syncwarp();
+    }
+    e1 = warp_sum_d(e1);
+    e2 = warp_sum_d(e2);
+    if (lane == 0) {
+        part[first * 3] = e1;
+        part[first * 3 + 1] = e2;
+        part[first * 3 + 2] = (double)cnt;
     }
 }
 
@@ -728,15 +866,21 @@ void launch_nmf_clamp0_f32(Ctx& c, const float* src, int ld, double* X, uint64_t
     SLFMM_LAUNCHED(c, "k_nmf_sign");
 }
 
-void launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed, double rate, const float* W,
-                   const float* H, int k, double* part) {
-    if (!g.p) return;
+// a warp per SNP at a time, as many as are resident
+static unsigned cv_grid(const Ctx& c, uint64_t p) {
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(p, 8), (uint64_t)c.sm_count * 8));
+}
+
+uint64_t launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed, double rate, const float* W,
+                       const float* H, int k, DBuf<double>& part) {
     const bool cc = c.rng == SLFMM_RNG_CHACHA8;
     const uint64_t th = cc ? rate_threshold(rate, 52) : rate_threshold(rate);
-    const unsigned grid = (unsigned)grid_for(c, g.p, 8);
+    const unsigned grid = cv_grid(c, g.p);
+    const uint64_t rows = (uint64_t)grid * 8;
+    if (part.n < rows * 3) part.alloc(rows * 3, c.stream);
     auto go = [&](auto kern) {
         kern<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.stride, g.n, g.p, chunk, mask_seed, th, W, H, k,
-                                         g.counts.get(), part);
+                                         g.counts.get(), part.get());
     };
     if (k <= 16) {
         if (cc) go(k_nmf_cv<true, 16>);
@@ -746,30 +890,35 @@ void launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed, do
         else go(k_nmf_cv<false, 32>);
     }
     SLFMM_LAUNCHED(c, "k_nmf_cv");
+    return rows;
 }
 
-void launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed, double rate, const float* W,
-                        const float* Wpt, int k, double* part) {
-    if (!g.p) return;
-    DBuf<uint64_t> base(g.p, c.stream);
+uint64_t launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed, double rate, const float* W,
+                            const float* Wpt, int k, DBuf<double>& part) {
+    DBuf<uint64_t> base(std::max<uint64_t>(g.p, 1), c.stream);
     const uint64_t nchunks = ceil_div(g.p, chunk);
-    k_obs_base<<<grid_for(c, nchunks, 64), 64, 0, c.stream>>>(g.counts.get(), g.p, chunk, base.get());
+    k_obs_base<<<grid_for(c, nchunks, 1), 1024, 0, c.stream>>>(g.counts.get(), g.p, chunk, base.get());
     SLFMM_LAUNCHED(c, "k_obs_base");
     const bool cc = c.rng == SLFMM_RNG_CHACHA8;
     const uint64_t th = cc ? rate_threshold(rate, 52) : rate_threshold(rate);
-    const unsigned grid = (unsigned)grid_for(c, g.p, 8);
+    const unsigned grid = cv_grid(c, g.p);
+    const uint64_t rows = (uint64_t)grid * 8;
+    if (part.n < rows * 3) part.alloc(rows * 3, c.stream);
+    // rows of W+ as 16-byte vectors
+    const bool w4 = k % 4 == 0 && reinterpret_cast<uintptr_t>(Wpt) % 16 == 0;
     auto go = [&](auto kern) {
-        kern<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.stride, g.n, g.p, chunk, seed, th, W, Wpt, k, base.get(),
-                                         part);
+        kern<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.stride, g.n, g.p, chunk, seed, th, W, Wpt, k,
+                                         g.counts.get(), base.get(), part.get());
     };
     if (k <= 16) {
-        if (cc) go(k_nmf_gwas_cv<true, 16>);
-        else go(k_nmf_gwas_cv<false, 16>);
+        if (cc) w4 ? go(k_nmf_gwas_cv<true, true, 16>) : go(k_nmf_gwas_cv<true, false, 16>);
+        else w4 ? go(k_nmf_gwas_cv<false, true, 16>) : go(k_nmf_gwas_cv<false, false, 16>);
     } else {
-        if (cc) go(k_nmf_gwas_cv<true, 32>);
-        else go(k_nmf_gwas_cv<false, 32>);
+        if (cc) w4 ? go(k_nmf_gwas_cv<true, true, 32>) : go(k_nmf_gwas_cv<true, false, 32>);
+        else w4 ? go(k_nmf_gwas_cv<false, true, 32>) : go(k_nmf_gwas_cv<false, false, 32>);
     }
     SLFMM_LAUNCHED(c, "k_nmf_gwas_cv");
+    return rows;
 }
 
 }  // namespace slfmm

@@ -387,10 +387,12 @@ void launch_nmf_normalize(Ctx& c, double* W, uint64_t n, double* H, uint64_t p, 
                           double eps);
 void launch_nmf_abs_f64(Ctx& c, const double* src, int ld, double* X, uint64_t m, int k);
 void launch_nmf_clamp0_f32(Ctx& c, const float* src, int ld, double* X, uint64_t m, int k);
-void launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed, double rate, const float* W,
-                   const float* H, int k, double* part);
-void launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed, double rate, const float* W,
-                        const float* Wpt, int k, double* part);
+// both leave one row of three sums per warp in `part` (grown as needed) and
+// return the number of rows
+uint64_t launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed, double rate, const float* W,
+                       const float* H, int k, DBuf<double>& part);
+uint64_t launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed, double rate, const float* W,
+                            const float* Wpt, int k, DBuf<double>& part);
 
 // k_small.cu : FP64 dense helpers (row-major)
 void launch_colmeans(Ctx& c, const double* A, uint64_t m, int a, int lda, double* out);
