@@ -4,6 +4,8 @@
 // src/rsvd.rs:75,105,131), the small SVD (src/rsvd.rs:162, src/nmf.rs:321)
 // and safe_inv (src/testing.rs:996-1024).  GB300's FP64 rate is low, so
 // these only ever touch n x w, w x w or p x w objects with tiny w.
+#include <cooperative_groups.h>
+
 #include "slfmm_internal.h"
 
 namespace slfmm {
@@ -984,197 +986,378 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant_
     }
 }
 
-// One-sided (Hestenes) Jacobi SVD of a square a x a matrix in one
-// CTA: A V = U diag(sig).  Outputs V (a x a), sig (descending) and U = A V
-// / sig in place of A.  Pairs are rotated in parallel with a round-robin
-// ordering, one warp per pair.
-//
-// GB300 runs FP64 at a small fraction of its FP32 rate, so the sweeps run in
-// FP32 first (to ~1e-5 relative orthogonality, at most 12 sweeps); V is then
-// re-orthonormalised in FP64 (classical Gram-Schmidt, twice), M = A V formed
-// in FP64, and FP64 sweeps polish to the FP64 tolerance -- typically two or
-// three, against the ~10 a cold FP64 start needs.
+// Columns that k_jacobi_svd gives one CTA; wider ones go to a cluster.  A solve
+// with its copies, one CTA against eight: 30 columns 601 and 651 us, 33 columns 848
+// and 837, 40 columns 1107 and 984.
+constexpr int kEighOneCta = 32;
+constexpr int kEighCluster = 8;
+constexpr size_t kEighClusterSmem = 208 << 10;  // beside 17 KB of static arrays
+// with those arrays a launch passes 48 KB before its dynamic part does
+constexpr size_t kEighLimit = (48 << 10) + 1;
+
 __device__ __forceinline__ float warp_sumf(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// one Jacobi sweep-set on column-major M (ap x ap, rows a used) with
-// accumulated V; returns after convergence or max_sweeps
-template <typename F>
-__device__ void jacobi_sweeps(F* M, F* Vs, int a, int ap, F tol, int max_sweeps, int* rotated, F abs_tol = 0) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+// x, unknown to the compiler: a sum that starts from plain(0) of one product
+// stays a fused multiply-add with zero, whatever the trip count
+__device__ __forceinline__ float plain(float x) { asm("" : "+f"(x)); return x; }
+__device__ __forceinline__ double plain(double x) { asm("" : "+d"(x)); return x; }
+
+// warp_sum of four values at once, in the same order of additions: the lanes
+// split over the values in the first two steps, so that the sums take six FP64
+// additions of the warp instead of twenty.  The lane's result is value
+// 2 (lane >= 16) + (lane / 8 odd).
+__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, odd = lane & 8;
+    double a = up ? v[2] : v[0], b = up ? v[3] : v[1];
+    a += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+    double t = odd ? b : a;
+    t += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// slot of the round-robin tournament of m (even) players: player 0 fixed, the
+// others rotate
+__device__ __forceinline__ int tournament_slot(int idx, int round, int m) {
+    if (idx == 0) return 0;
+    int s = idx - 1 + round;
+    if (s >= m - 1) s -= m - 1;
+    return 1 + s;
+}
+
+// FP32 one-sided Jacobi sweeps with accumulated V, until a sweep rotates nothing
+// or max_sweeps.  column(c) is column c of M (ap long) and `to_v` floats behind
+// it that of V; the NC CTAs share the pairs of a round, a warp per pair, NR
+// elements of a column per lane (two at least: a lone product would be fused into
+// the sum over the lanes).  A round is a chain of five divisions and square
+// roots: the angle is computed beside the test of whether it is needed, and the
+// columns are read once.  rotated: a flag in each CTA for even and for odd sweeps.
+template <int NC, int NR, class Column, class Sync>
+__device__ void jacobi_sweeps32(Column column, int to_v, int ap, int rank, float tol, int max_sweeps, int* rotated,
+                                float abs_tol, Sync sync_all) {
+    const int lane = threadIdx.x & 31, nwarps = NC * (blockDim.x >> 5);
+    const int warp = rank + NC * (threadIdx.x >> 5);
     const int npairs = ap / 2;
     for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-        if (threadIdx.x == 0) *rotated = 0;
-        __syncthreads();
+        int* flag = rotated + (sweep & 1);
         for (int round = 0; round < ap - 1; ++round) {
             for (int pr = warp; pr < npairs; pr += nwarps) {
-                // round-robin tournament: player 0 fixed, the others rotate
-                auto pos = [&](int idx) { return idx == 0 ? 0 : 1 + ((idx - 1 + round) % (ap - 1)); };
-                int pcol = pos(pr), qcol = pos(ap - 1 - pr);
-                if (pcol > qcol) { const int t = pcol; pcol = qcol; qcol = t; }
-                F* mp = M + pcol * ap;
-                F* mq = M + qcol * ap;
-                F al = 0, be = 0, ga = 0;
-                for (int r = lane; r < a; r += 32) {
-                    al += mp[r] * mp[r];
-                    be += mq[r] * mq[r];
-                    ga += mp[r] * mq[r];
-                }
-                if constexpr (sizeof(F) == 8) {
-                    al = warp_sum(al); be = warp_sum(be); ga = warp_sum(ga);
-                } else {
-                    al = warp_sumf(al); be = warp_sumf(be); ga = warp_sumf(ga);
-                }
-                const F tiny = sizeof(F) == 8 ? (F)1e-300 : (F)1e-37;
-                if (fabs(ga) > tol * sqrt(al * be) && fabs(ga) > tiny && fabs(ga) > abs_tol) {
-                    const F zeta = (be - al) / (2 * ga);
-                    const F t = (zeta >= 0 ? (F)1 : (F)-1) / (fabs(zeta) + sqrt((F)1 + zeta * zeta));
-                    const F cs = (F)1 / sqrt((F)1 + t * t), sn = cs * t;
-                    for (int r = lane; r < ap; r += 32) {
-                        const F x = mp[r], y = mq[r];
-                        mp[r] = cs * x - sn * y;
-                        mq[r] = sn * x + cs * y;
-                        F* vp = Vs + pcol * ap;
-                        F* vq = Vs + qcol * ap;
-                        const F vx = vp[r], vy = vq[r];
-                        vp[r] = cs * vx - sn * vy;
-                        vq[r] = sn * vx + cs * vy;
+                const int s0 = tournament_slot(pr, round, ap), s1 = tournament_slot(ap - 1 - pr, round, ap);
+                float* mp = column(min(s0, s1));
+                float* mq = column(max(s0, s1));
+                float x[NR], y[NR], vx[NR], vy[NR];
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    const int r = lane + 32 * q;
+                    x[q] = r < ap ? mp[r] : 0.f;
+                    y[q] = r < ap ? mq[r] : 0.f;
+                    if constexpr (NC > 1) {  // another CTA's memory is far: V's columns come along
+                        vx[q] = r < ap ? mp[to_v + r] : 0.f;
+                        vy[q] = r < ap ? mq[to_v + r] : 0.f;
                     }
-                    if (lane == 0) *rotated = 1;
                 }
+                float al = 0.f, be = 0.f, ga = 0.f;
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    al += x[q] * x[q];
+                    be += y[q] * y[q];
+                    ga += x[q] * y[q];
+                }
+                al = warp_sumf(al);
+                be = warp_sumf(be);
+                ga = warp_sumf(ga);
+                const float zeta = (be - al) / (2 * ga);
+                const float bound = tol * sqrtf(al * be);
+                const float t = (zeta >= 0 ? 1.f : -1.f) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
+                const float cs = 1.f / sqrtf(1.f + t * t), sn = cs * t;
+                const float g = fabsf(ga);
+                if (!(g > bound && g > 1e-37f && g > abs_tol)) continue;
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    const int r = lane + 32 * q;
+                    if (r >= ap) continue;
+                    if constexpr (NC == 1) {
+                        vx[q] = mp[to_v + r];
+                        vy[q] = mq[to_v + r];
+                    }
+                    mp[r] = cs * x[q] - sn * y[q];
+                    mq[r] = sn * x[q] + cs * y[q];
+                    mp[to_v + r] = cs * vx[q] - sn * vy[q];
+                    mq[to_v + r] = sn * vx[q] + cs * vy[q];
+                }
+                if (lane == 0) *flag = 1;
             }
-            __syncthreads();
+            // the next sweep's flag: every CTA has read it (a round has ended since)
+            if (round == ap - 2 && threadIdx.x == 0) rotated[(sweep & 1) ^ 1] = 0;
+            sync_all();
         }
-        if (!*rotated) break;
-        __syncthreads();
+        if constexpr (NC == 1) {
+            const int any = *flag;
+            __syncthreads();
+            if (!any) break;
+        } else {
+            const int* f = lane < NC ? cooperative_groups::this_cluster().map_shared_rank(flag, lane) : flag;
+            if (!__any_sync(0xffffffffu, *f)) break;
+        }
     }
 }
 
-// classical Gram-Schmidt, twice, of the ap columns of column-major Vs (FP64)
-__device__ void gs_columns(double* Vs, int ap, double* dots) {
+// Classical Gram-Schmidt, twice, of the ap columns of column-major Vs (FP64);
+// acc: ap x ap scratch.  Column j's first pass takes its products with the
+// column as it came in, so it runs ahead: as soon as column i is final, its
+// part leaves every later column, the next one first and the others (warps
+// from kTrail on) while the next one's second pass sums its chain and its norm.
+// FP64 instructions hold a scheduler for 64 cycles whatever the lanes active,
+// so the dot products are summed four to a warp.
+constexpr int kTrail = 4;
+template <int NR>
+__device__ void gs_columns(double* Vs, double* acc, int ap, double* dots) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    constexpr int kChainWarps = NR < kTrail ? NR : kTrail;
+    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) acc[e] = Vs[e];
+    __syncthreads();
+    // the products of NR elements a lane with four columns from col on (cols past `end` as zero)
+    auto dot4 = [&](const double* cols, int col, int end, const double (&v)[NR], double (&t)[4]) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            t[m] = plain(0.0);
+            if (col + m < end) {
+                const double* c = cols + (col + m) * ap;
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t[m] += c[lane + 32 * q] * v[q];
+            }
+        }
+    };
+    auto load = [&](const double* c, double (&v)[NR]) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) v[q] = lane + 32 * q < ap ? c[lane + 32 * q] : 0.0;
+    };
     for (int j = 0; j < ap; ++j) {
         double* vj = Vs + j * ap;
-        for (int pass = 0; pass < 2; ++pass) {
-            for (int i = warp; i < j; i += nwarps) {
-                const double* vi = Vs + i * ap;
-                double t = 0.0;
-                for (int r = lane; r < ap; r += 32) t += vi[r] * vj[r];
+        double* aj = acc + j * ap;
+        if (j > 0) {
+            if (warp == 0) {  // the last term of the column's first pass
+                const double* vi = vj - ap;
+                double t = plain(0.0);
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t += vi[lane + 32 * q] * vj[lane + 32 * q];
                 t = warp_sum(t);
-                if (lane == 0) dots[i] = t;
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) aj[lane + 32 * q] -= t * vi[lane + 32 * q];
             }
             __syncthreads();
-            for (int r = threadIdx.x; r < ap; r += blockDim.x) {
-                double t = vj[r];
-                for (int i = 0; i < j; ++i) t -= dots[i] * Vs[i * ap + r];
-                vj[r] = t;
+            // the second pass's products
+            for (int i = 4 * warp; i < j; i += 4 * nwarps) {
+                double v[NR], t[4];
+                load(aj, v);
+                dot4(Vs, i, j, v, t);
+                const double s = warp_sum4(t);
+                if ((lane & 7) == 0 && i + (lane >> 3) < j) dots[i + (lane >> 3)] = s;
             }
             __syncthreads();
         }
-        if (warp == 0) {
-            double t = 0.0;
-            for (int r = lane; r < ap; r += 32) t += vj[r] * vj[r];
-            t = warp_sum(t);
-            const double inv = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
-            for (int r = lane; r < ap; r += 32) vj[r] *= inv;
+        if (warp < kChainWarps) {
+            double s[NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) s[q] = 0.0;
+#pragma unroll
+            for (int q = 0; q < (NR + kChainWarps - 1) / kChainWarps; ++q) {
+                const int r = lane + 32 * (warp + q * kChainWarps);
+                if (r < ap) {
+                    double t = aj[r];
+#pragma unroll 4
+                    for (int i = 0; i < j; ++i) t -= dots[i] * Vs[i * ap + r];
+                    if (kChainWarps == 1) s[q] = t;
+                    else vj[r] = t;
+                }
+            }
+            if (kChainWarps > 1) asm volatile("bar.sync 1, %0;" ::"n"(32 * kChainWarps) : "memory");
+            if (warp == 0) {
+                if (kChainWarps > 1) load(vj, s);
+                double t = plain(0.0);
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t += s[q] * s[q];
+                t = warp_sum(t);
+                const double inv = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) vj[lane + 32 * q] = s[q] * inv;
+            }
+        } else if (warp >= kTrail && j > 0) {
+            // column j - 1 leaves the columns behind j
+            const double* vi = vj - ap;
+            double v[NR], t[4];
+            load(vi, v);
+            for (int k = j + 1 + 4 * (warp - kTrail); k < ap; k += 4 * (nwarps - kTrail)) {
+                dot4(Vs, k, ap, v, t);
+                const double s = warp_sum4(t);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double d = __shfl_sync(0xffffffffu, s, 8 * m);
+                    if (k + m < ap) {
+                        double* ak = acc + (k + m) * ap;
+#pragma unroll
+                        for (int q = 0; q < NR; ++q)
+                            if (lane + 32 * q < ap) ak[lane + 32 * q] -= d * v[q];
+                    }
+                }
+            }
         }
         __syncthreads();
     }
 }
 
 // Eigen-decomposition of a symmetric positive semi-definite a x a matrix
-// (a <= kMaxDesign; the Gram matrices of Step 0, the RSVD and the NMF probe) in one
-// CTA: A V = V diag(sig), sig descending, V orthonormal; A is overwritten by V
-// (its left singular vectors).
+// (a <= kMaxDesign; the Gram matrices of Step 0, the RSVD and the NMF probe) in
+// NC CTAs: A V = V diag(sig), sig descending, V orthonormal; A is overwritten by
+// V (its left singular vectors).
 //
 // GB300 runs FP64 at a small fraction of its FP32 rate, so the bulk of the
 // rotation work runs as FP32 one-sided Jacobi sweeps (pairs in parallel,
-// round-robin order, one warp per pair) to ~1e-5 (at most 12 sweeps: with
-// Gram matrices of condition 1e6 and more, FP32 rounding keeps rotating the
-// small columns, and the FP64 phase converges quadratically from there
-// anyway); V is re-orthonormalised in FP64 (Gram-Schmidt, twice) and
-// B = V^T A V formed in FP64.  B is then diagonal up to ~1e-5 of its norm,
-// and two-sided cyclic Jacobi sweeps in
-// FP64 (Golub & Van Loan, Algorithm 8.5.2 with the parallel round-robin
-// ordering) finish it -- quadratic convergence, typically two sweeps --
-// accumulating their rotations into R; V <- V R and a final Gram-Schmidt.
+// round-robin order) to ~1e-5 (at most 12 sweeps: with Gram matrices of
+// condition 1e6 and more, FP32 rounding keeps rotating the small columns, and
+// the FP64 phase converges quadratically from there anyway); V is
+// re-orthonormalised in FP64 (Gram-Schmidt, twice) and B = V^T A V formed in
+// FP64.  B is then diagonal up to ~1e-5 of its norm, and two-sided cyclic Jacobi
+// sweeps in FP64 (Golub & Van Loan, Algorithm 8.5.2 with the parallel
+// round-robin ordering) finish it -- quadratic convergence, typically two sweeps
+// -- accumulating their rotations into R; V <- V R and a final Gram-Schmidt.
 // Jacobi rotations are bounded (|tan| <= 1), so clusters of equal or nearly
 // equal eigenvalues need no special case.  Eigenvalues are v_j^T A v_j of the
 // final vectors.
-// Matrices wider than 64 columns work in `ws` (global memory, L2-resident:
-// 2 ap^2 doubles + 2 ap^2 floats) instead of shared memory.
-__global__ void __launch_bounds__(1024) k_jacobi_svd(double* __restrict__ A, int a,
-                                                     double* __restrict__ V, double* __restrict__ sig,
-                                                     double* __restrict__ ws) {
+//
+// Every round of the FP64 sweeps is the latency of an angle (five divisions and
+// square roots) plus the rotations of ap^2 elements at a sixteenth of the FP32
+// rate.  One CTA holds it all in shared memory up to kEighOneCta columns.  Wider
+// ones run as a cluster of eight: the FP32 matrices' and B's columns and R's rows
+// are spread over the CTAs' shared memory, a round's pairs and 2 x 2 blocks are
+// shared out and read and written there, and the products take a share of the
+// columns each; Gram-Schmidt stays with the first CTA.  A solve with its copies
+// (45 us), before and so: 13 columns 275 and 243 us, 20 463 and 351, 50 2464 and
+// 1402, 100 14.1 and 4.8 ms, 256 222 and 57 ms.
+template <int NC, int NR>
+__global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, int a, double* __restrict__ V,
+                                                        double* __restrict__ sig, double* ws) {
     extern __shared__ double sm_dyn[];
-    double* sm = ws ? ws : sm_dyn;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = NC > 1 ? (int)cluster.block_rank() : 0;
+    // all CTAs' writes before it are seen by all after it
+    auto sync_all = [&]() {
+        if (NC > 1) cluster.sync();
+        else __syncthreads();
+    };
     const int ap = a + (a & 1);     // even number of columns (padded column is zero)
-    double* M = sm;                 // column-major ap x ap scratch
-    double* Vs = sm + ap * ap;      // column-major eigenvectors
-    float* M32 = reinterpret_cast<float*>(Vs + ap * ap);
-    float* V32 = M32 + ap * ap;
-    double* B = reinterpret_cast<double*>(M32);  // reuses the FP32 area after phase 1
-    __shared__ int rotated;
+    const int share = (ap + NC - 1) / NC;  // columns (rows of R) of one CTA
+    const int c0 = min(ap, rank * share), c1 = min(ap, c0 + share), nc = c1 - c0;
+    const int sq = ap * ap;
+    // One CTA: three squares of shared memory -- Gram-Schmidt's scratch, T and R;
+    // the vectors; the FP32 matrices, B and V R.  A cluster: three squares of
+    // global memory for what the CTAs pass on, the first CTA's own two in shared
+    // memory where they fit, and in each a share of the FP32 matrices, later of T
+    // or R, and of B.
+    double *vec, *scratch, *fp32, *T, *Bs, *R, *VR;
+    if (NC == 1) {
+        scratch = T = R = sm_dyn;
+        vec = sm_dyn + sq;
+        fp32 = Bs = VR = sm_dyn + 2 * sq;
+    } else {
+        const bool fits = 2 * (size_t)sq * sizeof(double) <= kEighClusterSmem;
+        scratch = fits ? sm_dyn : ws;
+        vec = fits ? sm_dyn + sq : ws + sq;
+        fp32 = T = R = sm_dyn;
+        Bs = sm_dyn + share * ap;
+        VR = ws;
+    }
+    double* vecs = NC == 1 ? vec : ws + sq;  // the vectors where every CTA reads them
+    float* M32 = reinterpret_cast<float*>(fp32);  // the share's columns of M, then of V
+    const int to_v = share * ap;
+    __shared__ int rotated, rotated32[2], nact;
     __shared__ double sg[kMaxDesign];
     __shared__ double dots[kMaxDesign];
     __shared__ double bmax;
     __shared__ int order[kMaxDesign];
-    __shared__ int jp[kMaxDesign / 2], jq[kMaxDesign / 2];
-    __shared__ double jc[kMaxDesign / 2], js[kMaxDesign / 2];
+    __shared__ int jp[2][kMaxDesign / 2], jq[2][kMaxDesign / 2];
+    __shared__ double jc[2][kMaxDesign / 2], js[2][kMaxDesign / 2];
+    __shared__ double* bcol[kMaxDesign];  // columns of B, wherever they are
+    __shared__ float* mcol[kMaxDesign];   // and of the FP32 matrix
+    __shared__ int act[kMaxDesign], rest[kMaxDesign], actflag[kMaxDesign];
+    __shared__ float colmax2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     // phase 1: FP32 sweeps
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) {
-        const int col = e / ap, row = e % ap;
+    for (int e = threadIdx.x; e < nc * ap; e += blockDim.x) {
+        const int col = c0 + e / ap, row = e % ap;
         M32[e] = (row < a && col < a) ? (float)A[row * a + col] : 0.f;
-        V32[e] = (row == col) ? 1.f : 0.f;
+        M32[to_v + e] = (row == col) ? 1.f : 0.f;
+    }
+    for (int cc = threadIdx.x; cc < ap; cc += blockDim.x) {
+        bcol[cc] = NC == 1 ? Bs + cc * ap : cluster.map_shared_rank(Bs, cc / share) + (cc % share) * ap;
+        mcol[cc] = NC == 1 ? M32 + cc * ap : cluster.map_shared_rank(M32, cc / share) + (cc % share) * ap;
     }
     // FP32 resolution of the whole matrix: couplings below 1e-7 of the largest
     // squared column norm are left to the FP64 sweeps (columns of a rank-deficient
     // Gram that are zero up to FP32 rounding would otherwise keep rotating
     // until the sweep limit)
-    __shared__ float colmax2;
-    if (threadIdx.x == 0) colmax2 = 0.f;
-    __syncthreads();
-    if (warp < ap) {
-        for (int cc = warp; cc < ap; cc += nwarps) {
-            float t = 0.f;
-            for (int r = lane; r < a; r += 32) t += M32[cc * ap + r] * M32[cc * ap + r];
-            t = warp_sumf(t);
-            if (lane == 0) atomicMax(reinterpret_cast<int*>(&colmax2), __float_as_int(t));
-        }
+    if (threadIdx.x == 0) {
+        colmax2 = 0.f;
+        rotated32[0] = rotated32[1] = 0;
     }
-    __syncthreads();
-    jacobi_sweeps<float>(M32, V32, a, ap, 1.0e-5f, 12, &rotated, 1e-7f * colmax2);
-    // phase 2: FP64 orthonormal V
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) Vs[e] = (double)V32[e];
-    __syncthreads();
-    gs_columns(Vs, ap, dots);
-    // phase 3: T = A V (in M), B = V^T T (over the FP32 area)
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) {
-        const int col = e / ap, row = e % ap;
+    sync_all();
+    for (int cc = warp; cc < ap; cc += nwarps) {
+        float t = 0.f;
+        for (int r = lane; r < a; r += 32) t += mcol[cc][r] * mcol[cc][r];
+        t = warp_sumf(t);
+        if (lane == 0) atomicMax(reinterpret_cast<int*>(&colmax2), __float_as_int(t));
+    }
+    sync_all();
+    jacobi_sweeps32<NC, (NR > 2 ? NR : 2)>([&](int cc) { return NC == 1 ? M32 + cc * ap : mcol[cc]; }, to_v, ap,
+                                          rank, 1.0e-5f, 12, rotated32, 1e-7f * colmax2, sync_all);
+    sync_all();
+    if (rank == 0) {
+        // phase 2: FP64 orthonormal V
+        for (int e = threadIdx.x; e < sq; e += blockDim.x) vec[e] = (double)mcol[e / ap][to_v + e % ap];
+        __syncthreads();
+        gs_columns<NR>(vec, scratch, ap, dots);
+        if (vecs != vec)
+            for (int e = threadIdx.x; e < sq; e += blockDim.x) vecs[e] = vec[e];
+    }
+    sync_all();
+    // phase 3: the share's columns of T = A V and of B = V^T T
+    for (int e = threadIdx.x; e < nc * ap; e += blockDim.x) {
+        const int col = c0 + e / ap, row = e % ap;
         double t = 0.0;
         if (row < a)
-            for (int k = 0; k < a; ++k) t += A[row * a + k] * Vs[col * ap + k];
-        M[e] = t;
+            for (int k = 0; k < a; ++k) t += A[row * a + k] * vecs[col * ap + k];
+        T[e] = t;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) {
+    for (int e = threadIdx.x; e < nc * ap; e += blockDim.x) {
         const int col = e / ap, row = e % ap;
         double t = 0.0;
-        for (int k = 0; k < ap; ++k) t += Vs[row * ap + k] * M[col * ap + k];
-        B[e] = t;  // B[col * ap + row] = v_row^T A v_col
+        for (int k = 0; k < ap; ++k) t += vecs[row * ap + k] * T[col * ap + k];
+        Bs[e] = t;  // B[col * ap + row] = v_row^T A v_col
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    sync_all();
+    if (warp == 0) {
         double m = 0.0;
-        for (int j = 0; j < ap; ++j) m = fmax(m, fabs(B[j * ap + j]));
-        bmax = m;
+        for (int j = lane; j < ap; j += 32) m = fmax(m, fabs(bcol[j][j]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) bmax = m;
     }
-    __syncthreads();
-    // phase 4: FP64 two-sided Jacobi on B, rotations accumulated in R (in M).
+    // phase 4: FP64 two-sided Jacobi on B, rotations accumulated in R (the
+    // share's rows, column-major).
     // Each sweep pairs only the active columns, those with an off-diagonal
     // entry above the skip level, in the round-robin order over them: a
     // column whose couplings are all at that level stays there while the
@@ -1183,129 +1366,206 @@ __global__ void __launch_bounds__(1024) k_jacobi_svd(double* __restrict__ A, int
     // columns left, the ones of the small eigenvalues the FP32 phase could
     // not resolve -- a sweep over all columns costs ap - 1 rounds of block
     // barriers and FP64 rotation angles whatever the number rotated.
-    double* R = M;
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) R[e] = (e / ap == e % ap) ? 1.0 : 0.0;
+    for (int e = threadIdx.x; e < ap * nc; e += blockDim.x) R[e] = (e / nc == c0 + e % nc) ? 1.0 : 0.0;
+    __syncthreads();
     const double skip = 4e-16 * bmax;  // off-diagonals at the rounding level of B
-    __shared__ int act[kMaxDesign];
-    __shared__ int actflag[kMaxDesign];
-    __shared__ int nact;
+    const int np2 = ap / 2;            // pairs, those of columns at rest among them
+    const int kshare = (np2 + NC - 1) / NC, k0 = min(np2, rank * kshare), nk = min(np2, k0 + kshare) - k0;
+    // warps 0 .. angle_warps - 1 compute a round's angles; R's rotations run beside
+    // them on the schedulers (warp mod 4) that no angle's chain is on
+    const int angle_warps = (np2 + 31) / 32, free_sched = 4 - angle_warps;
+    const int r_warps = free_sched ? nwarps / 4 * free_sched : nwarps - 4;
+    const int r_warp = free_sched ? (warp & 3) < angle_warps ? -1 : (warp >> 2) * free_sched + (warp & 3) - angle_warps
+                                  : warp - 4;
+    int buf = 0;
+    bool pending = false;  // the last round's rotations are not in R yet
+    // R <- R J of the rotations in buffer b, by thread `t` of `step`
+    auto rotate_r = [&](int b, int t, int step) {
+        for (int e = t; e < np2 * nc; e += step) {
+            const int k = e / nc, i = e - k * nc;
+            const double cs = jc[b][k], sn = js[b][k];
+            if (sn == 0.0) continue;
+            double* rp = R + jp[b][k] * nc;
+            double* rq = R + jq[b][k] * nc;
+            const double x = rp[i], y = rq[i];
+            rp[i] = cs * x - sn * y;
+            rq[i] = sn * x + cs * y;
+        }
+    };
     for (int sweep = 0; sweep < 12; ++sweep) {
         if (threadIdx.x == 0) rotated = 0;
-        __syncthreads();
-        for (int cc = warp; cc < ap; cc += nwarps) {
+        for (int cc = c0 + warp; cc < c1; cc += nwarps) {
             bool any = false;
-            for (int r = lane; r < ap; r += 32) any |= r != cc && fabs(B[cc * ap + r]) > skip;
+            for (int r = lane; r < ap; r += 32) any |= r != cc && fabs(bcol[cc][r]) > skip;
             any = __any_sync(0xffffffffu, any);
-            if (lane == 0) actflag[cc] = any ? 1 : 0;
+            if (lane < NC) {
+                int* f = NC == 1 ? actflag : cluster.map_shared_rank(actflag, lane);
+                f[cc] = any ? 1 : 0;
+            }
         }
-        __syncthreads();
-        if (warp == 0) {  // the active columns in ascending order
-            int run = 0;
+        sync_all();
+        if (warp == 0) {  // the active columns in ascending order, and the others
+            int run = 0, idle = 0;
             for (int base = 0; base < ap; base += 32) {
-                const bool f = base + lane < ap && actflag[base + lane];
-                const unsigned m = __ballot_sync(0xffffffffu, f);
+                const bool in = base + lane < ap, f = in && actflag[base + lane];
+                const unsigned m = __ballot_sync(0xffffffffu, f), z = __ballot_sync(0xffffffffu, in && !f);
                 if (f) act[run + __popc(m & ((1u << lane) - 1u))] = base + lane;
+                else if (in) rest[idle + __popc(z & ((1u << lane) - 1u))] = base + lane;
                 run += __popc(m);
+                idle += __popc(z);
             }
             if (lane == 0) nact = run;
         }
         __syncthreads();
         const int na = nact;
         if (na < 2) break;
-        const int nap = na + (na & 1);  // even; position na (odd na) pairs with no column
+        const int nap = na + (na & 1);  // even; position na (odd na) pairs with a column at rest
         const int npairs = nap / 2;
         for (int round = 0; round < nap - 1; ++round) {
-            auto pos = [&](int idx) { return idx == 0 ? 0 : 1 + ((idx - 1 + round) % (nap - 1)); };
-            for (int k = threadIdx.x; k < npairs; k += blockDim.x) {
-                const int x = pos(k), y = pos(nap - 1 - k);
+            if (warp < angle_warps) {
+                const int k = threadIdx.x;
                 double cs = 1.0, sn = 0.0;
                 int pc = 0, qc = 0;
-                if (x < na && y < na) {
-                    pc = act[x];
-                    qc = act[y];
-                    if (pc > qc) { const int t = pc; pc = qc; qc = t; }
-                    const double app = B[pc * ap + pc], aqq = B[qc * ap + qc], apq = B[qc * ap + pc];
-                    if (fabs(apq) > skip && apq != 0.0) {
-                        const double tau = (aqq - app) / (2.0 * apq);
-                        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-                        cs = 1.0 / sqrt(1.0 + t * t);
-                        sn = t * cs;
-                        rotated = 1;
+                if (k < npairs) {
+                    const int x = tournament_slot(k, round, nap), y = tournament_slot(nap - 1 - k, round, nap);
+                    if (x < na && y < na) {
+                        pc = act[x];
+                        qc = act[y];
+                        if (pc > qc) { const int t = pc; pc = qc; qc = t; }
+                        const double app = bcol[pc][pc], aqq = bcol[qc][qc], apq = bcol[qc][pc];
+                        if (fabs(apq) > skip && apq != 0.0) {
+                            const double tau = (aqq - app) / (2.0 * apq);
+                            const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+                            cs = 1.0 / sqrt(1.0 + t * t);
+                            sn = t * cs;
+                            rotated = 1;
+                        }
+                    } else {
+                        pc = act[x < na ? x : y];
+                        qc = rest[0];
                     }
+                } else if (k < np2) {
+                    pc = rest[(na & 1) + 2 * (k - npairs)];
+                    qc = rest[(na & 1) + 2 * (k - npairs) + 1];
                 }
-                jp[k] = pc; jq[k] = qc; jc[k] = cs; js[k] = sn;
+                if (k < np2) {
+                    jp[buf][k] = pc; jq[buf][k] = qc; jc[buf][k] = cs; js[buf][k] = sn;
+                }
+            } else if (pending && r_warp >= 0) {
+                rotate_r(buf ^ 1, 32 * r_warp + lane, 32 * r_warps);
             }
             __syncthreads();
-            // B <- B J and R <- R J (columns p, q of each pair)
-            for (int e = threadIdx.x; e < npairs * ap; e += blockDim.x) {
-                const int k = e / ap, i = e % ap;
-                if (js[k] == 0.0) continue;
-                const double cs = jc[k], sn = js[k];
-                double* bp = B + jp[k] * ap;
-                double* bq = B + jq[k] * ap;
-                double x = bp[i], y = bq[i];
-                bp[i] = cs * x - sn * y;
-                bq[i] = sn * x + cs * y;
-                double* rp = R + jp[k] * ap;
-                double* rq = R + jq[k] * ap;
-                x = rp[i]; y = rq[i];
-                rp[i] = cs * x - sn * y;
-                rq[i] = sn * x + cs * y;
+            // B <- J^T (B J), the 2 x 2 blocks of the share's pairs of columns
+            // with every pair of rows
+            for (int e = threadIdx.x; e < nk * np2; e += blockDim.x) {
+                const int k = k0 + e / np2, l = e % np2;
+                const double sk = js[buf][k], sl = js[buf][l];
+                if (sk == 0.0 && sl == 0.0) continue;
+                double* bp = bcol[jp[buf][k]];
+                double* bq = bcol[jq[buf][k]];
+                const int pr = jp[buf][l], qr = jq[buf][l];
+                double pp = bp[pr], pq = bp[qr], qp = bq[pr], qq = bq[qr];
+                if (sk != 0.0) {
+                    const double cs = jc[buf][k], sn = sk;
+                    double x = pp, y = qp;
+                    pp = cs * x - sn * y;
+                    qp = sn * x + cs * y;
+                    x = pq; y = qq;
+                    pq = cs * x - sn * y;
+                    qq = sn * x + cs * y;
+                }
+                if (sl != 0.0) {
+                    const double cs = jc[buf][l], sn = sl;
+                    double x = pp, y = pq;
+                    pp = cs * x - sn * y;
+                    pq = sn * x + cs * y;
+                    x = qp; y = qq;
+                    qp = cs * x - sn * y;
+                    qq = sn * x + cs * y;
+                }
+                bp[pr] = pp; bp[qr] = pq; bq[pr] = qp; bq[qr] = qq;
             }
-            __syncthreads();
-            // B <- J^T B (rows p, q of each pair)
-            for (int e = threadIdx.x; e < npairs * ap; e += blockDim.x) {
-                const int k = e / ap, j = e % ap;
-                if (js[k] == 0.0) continue;
-                const double cs = jc[k], sn = js[k];
-                const int pr = jp[k], qr = jq[k];
-                const double x = B[j * ap + pr], y = B[j * ap + qr];
-                B[j * ap + pr] = cs * x - sn * y;
-                B[j * ap + qr] = sn * x + cs * y;
-            }
+            sync_all();
+            buf ^= 1;
+            pending = true;
+        }
+        const int any = rotated;
+        __syncthreads();
+        if (!any) break;
+    }
+    if (pending) rotate_r(buf ^ 1, threadIdx.x, blockDim.x);
+    // V <- V R
+    double* Rall = R;
+    if (NC > 1) {
+        Rall = ws + 2 * sq;
+        __syncthreads();
+        for (int e = threadIdx.x; e < ap * nc; e += blockDim.x) Rall[(e / nc) * ap + c0 + e % nc] = R[e];
+    }
+    sync_all();
+    for (int e = threadIdx.x; e < nc * ap; e += blockDim.x) {
+        const int col = c0 + e / ap, row = e % ap;
+        double t = 0.0;
+        for (int i = 0; i < ap; ++i) t += vecs[i * ap + row] * Rall[col * ap + i];
+        VR[col * ap + row] = t;
+    }
+    sync_all();
+    double* fin = VR;
+    if (rank == 0) {
+        if (NC > 1) {
+            for (int e = threadIdx.x; e < sq; e += blockDim.x) vec[e] = VR[e];
+            fin = vec;
             __syncthreads();
         }
-        if (!rotated) break;
+        gs_columns<NR>(fin, scratch, ap, dots);
+        if (vecs != vec)
+            for (int e = threadIdx.x; e < sq; e += blockDim.x) vecs[e] = fin[e];
     }
-    // V <- V R (into B's area, no longer needed)
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) {
-        const int col = e / ap, row = e % ap;
-        double t = 0.0;
-        for (int i = 0; i < ap; ++i) t += Vs[i * ap + row] * R[col * ap + i];
-        B[e] = t;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < ap * ap; e += blockDim.x) Vs[e] = B[e];
-    __syncthreads();
-    gs_columns(Vs, ap, dots);
+    if (NC > 1) fin = vecs;
+    sync_all();
     // phase 5: eigenvalues v_j^T A v_j, descending order
-    for (int cc = warp; cc < ap; cc += nwarps) {
+    for (int cc = c0 + warp; cc < c1; cc += nwarps) {
         double s = 0.0;
         for (int r = lane; r < a; r += 32) {
             double t = 0.0;
-            for (int k = 0; k < a; ++k) t += A[r * a + k] * Vs[cc * ap + k];
-            s += Vs[cc * ap + r] * t;
+            for (int k = 0; k < a; ++k) t += A[r * a + k] * fin[cc * ap + k];
+            s += fin[cc * ap + r] * t;
         }
         s = warp_sum(s);
-        if (lane == 0) sg[cc] = fabs(s);
+        if (lane == 0) *(NC == 1 ? sg + cc : cluster.map_shared_rank(sg, 0) + cc) = fabs(s);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < a; ++i) order[i] = i;
-        for (int i = 0; i < a; ++i) {
-            int best = i;
-            for (int j = i + 1; j < a; ++j)
-                if (sg[order[j]] > sg[order[best]]) best = j;
-            const int t = order[i]; order[i] = order[best]; order[best] = t;
+    sync_all();
+    if (rank != 0) return;
+    // a column's place is the number of larger ones (compared as integers: no
+    // value is negative); equal values, and NaN, are put where a selection sort
+    // does, the first largest of the rest swapped to the front
+    bool plain_order = true;
+    for (int i = threadIdx.x; i < a; i += blockDim.x) {
+        const long long key = __double_as_longlong(sg[i]);
+        int place = 0;
+        for (int j = 0; j < a; ++j) {
+            const long long other = __double_as_longlong(sg[j]);
+            place += other > key;
+            plain_order = plain_order && (other != key || j == i);
         }
+        plain_order = plain_order && !isnan(sg[i]);
+        order[place] = i;
     }
-    __syncthreads();
+    if (!__syncthreads_and(plain_order)) {
+        if (threadIdx.x == 0) {
+            for (int i = 0; i < a; ++i) order[i] = i;
+            for (int i = 0; i < a; ++i) {
+                int best = i;
+                for (int j = i + 1; j < a; ++j)
+                    if (sg[order[j]] > sg[order[best]]) best = j;
+                const int t = order[i]; order[i] = order[best]; order[best] = t;
+            }
+        }
+        __syncthreads();
+    }
     for (int e = threadIdx.x; e < a * a; e += blockDim.x) {
         const int row = e / a, cc = e % a;
-        V[row * a + cc] = Vs[order[cc] * ap + row];
+        V[e] = A[e] = fin[order[cc] * ap + row];
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < a * a; e += blockDim.x) A[e] = V[e];
     for (int cc = threadIdx.x; cc < a; cc += blockDim.x) sig[cc] = sg[order[cc]];
 }
 
@@ -1716,14 +1976,35 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
     SLFMM_REQUIRE(a >= 1 && a <= kMaxDesign, SLFMM_ERR_BAD_ARG,
                   "small eigen-solve limited to " + std::to_string(kMaxDesign) + " x " + std::to_string(kMaxDesign));
     const int ap = a + (a & 1);
-    const size_t sm = 2 * (size_t)ap * ap * (sizeof(double) + sizeof(float));
     ProfScope ps(c, "small_eigh", 16.0 * a * a, 0.0);
-    if (a <= 64) {
-        set_smem((const void*)k_jacobi_svd, sm);
-        k_jacobi_svd<<<1, 1024, sm, c.stream>>>(const_cast<double*>(A), a, V, sig, nullptr);
+    const size_t square = (size_t)ap * ap * sizeof(double);
+    if (a <= kEighOneCta) {
+        // a warp per pair of columns, in fours, and those of Gram-Schmidt
+        const int threads = std::max(256, (int)round_up(32 * (uint64_t)(ap / 2), 128));
+        static_assert(kEighOneCta <= 32 && 3 * 32 * 32 * sizeof(double) + (20 << 10) <= (48 << 10), "");
+        k_jacobi_svd<1, 1><<<1, threads, 3 * square, c.stream>>>(const_cast<double*>(A), a, V, sig, nullptr);
     } else {
-        DBuf<double> ws((sm + sizeof(double) - 1) / sizeof(double), c.stream);
-        k_jacobi_svd<<<1, 1024, 0, c.stream>>>(const_cast<double*>(A), a, V, sig, ws.get());
+        DBuf<double> ws(3 * (size_t)ap * ap, c.stream);
+        const size_t share = 2 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
+        const size_t sm = 2 * square <= kEighClusterSmem ? std::max(2 * square, share) : share;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kEighCluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3(kEighCluster);
+        lc.blockDim = dim3(1024);
+        lc.dynamicSmemBytes = sm;
+        lc.stream = c.stream;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        auto go = [&](auto kern) {
+            set_smem((const void*)kern, std::max(sm, kEighLimit));
+            SLFMM_CUDA(cudaLaunchKernelEx(&lc, kern, const_cast<double*>(A), a, V, sig, ws.get()));
+        };
+        if (ap <= 64) go(k_jacobi_svd<kEighCluster, 2>);
+        else if (ap <= 128) go(k_jacobi_svd<kEighCluster, 4>);
+        else go(k_jacobi_svd<kEighCluster, 8>);
     }
     SLFMM_LAUNCHED(c, "k_jacobi_svd");
 }
