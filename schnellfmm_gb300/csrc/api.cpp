@@ -417,10 +417,8 @@ bool fp8_row_operand(Ctx& c, uint64_t n, uint64_t tiles, const double* W, int w,
     op.B.alloc((uint64_t)op.pl.n_total * op.n_pad, c.stream);
     op.isc.alloc(op.pl.n_total, c.stream);
     const int nr = (int)op.pl.n_total;
-    launch_fp8_terms_f64(c, W, ldw, n, w, op.wp, op.n_pad, nullptr, 4, 0, nr, op.B.get(), op.isc.get());
-    if (!op.pl.ind_shared)
-        launch_fp8_terms_f64(c, W, ldw, n, w, op.wp, op.n_pad, nullptr, 3, (int)op.pl.n_main, nr, op.B.get(),
-                             op.isc.get());
+    launch_fp8_terms_f64(c, W, ldw, n, w, op.wp, op.n_pad, op.pl.ind_shared ? 0 : (int)op.pl.n_main, nr, op.B.get(),
+                         op.isc.get());
     op.ok = true;
     return true;
 }
@@ -518,8 +516,7 @@ void fp8_row_operand_prepare(Ctx& c, uint64_t n, uint64_t tiles, const double* W
         const Fp8Plan pb = bp == rp.wp ? pl : fp8_plan(bp, false, tiles);
         DBuf<uint8_t> B((uint64_t)pb.n_total * rp.n_pad, c.stream);
         DBuf<float> isc(pb.n_total, c.stream);
-        launch_fp8_terms_f64(c, W + c0, ldw, n, wb, bp, rp.n_pad, nullptr, 4, 0, (int)pb.n_total, B.get(),
-                             isc.get());
+        launch_fp8_terms_f64(c, W + c0, ldw, n, wb, bp, rp.n_pad, 0, (int)pb.n_total, B.get(), isc.get());
         rp.plans.push_back(pb);
         rp.Bs.push_back(std::move(B));
         rp.iscs.push_back(std::move(isc));
@@ -655,7 +652,7 @@ void col_contract_base(Ctx& c, const Geno& g, const SnpStd& s, const float* Q, i
             used = launch_tc8_rows(c, pl, tv, g.n, g.p, B.get(), isc.get(), p_pad, 0, nullptr,
                                    nullptr, nullptr, part.get(), wp, splits, g.n * wp);
         }
-        launch_reduce_splits(c, part.get(), used, g.n, wp, g.n, S.get());
+        launch_reduce_splits(c, part.get(), used, g.n, w, wp, g.n, S.get());
         launch_weighted_colsum(c, Q, wp, g.p, w, coef.get(), colterm.get());
         if (ind) {
             launch_sub_colterm(c, S.get(), wp, g.n, w, colterm.get());
@@ -682,7 +679,7 @@ void col_contract_base(Ctx& c, const Geno& g, const SnpStd& s, const float* Q, i
             used = launch_tc_rows(c, g.packedT.get(), g.strideT, g.n, g.p, bs.get(), p_pad, wp, part.get(), wp, splits,
                                   g.n * wp);
         }
-        launch_reduce_splits(c, part.get(), used, g.n, wp, g.n, S.get());
+        launch_reduce_splits(c, part.get(), used, g.n, w, wp, g.n, S.get());
         DBuf<double> coef(std::max<uint64_t>(g.p, 1), c.stream), colterm(wp, c.stream);
         launch_scale_product(c, s.mean.get(), s.scale.get(), g.p, coef.get());
         launch_weighted_colsum(c, Q, wp, g.p, w, coef.get(), colterm.get());
@@ -2271,11 +2268,8 @@ int slfmm_contract_raw(slfmm_ctx* c, const slfmm_geno* g, int flags, const doubl
             const Fp8Plan pb = bp == wp ? pl : fp8_plan(bp, false, tiles);
             DBuf<uint8_t> B((uint64_t)pb.n_total * K_pad, c->stream);
             DBuf<float> isc(pb.n_total, c->stream);
-            launch_fp8_terms_f64(*c, Wd.get() + c0, (int)w, K, wb, bp, K_pad, nullptr, 4, 0, (int)pb.n_total,
-                                 B.get(), isc.get());
-            if (with_ind && !pb.ind_shared)
-                launch_fp8_terms_f64(*c, Wd.get() + c0, (int)w, K, wb, bp, K_pad, nullptr, 3, (int)pb.n_main,
-                                     (int)pb.n_total, B.get(), isc.get());
+            launch_fp8_terms_f64(*c, Wd.get() + c0, (int)w, K, wb, bp, K_pad,
+                                 with_ind && !pb.ind_shared ? (int)pb.n_main : 0, (int)pb.n_total, B.get(), isc.get());
             launch_tc8_rows(*c, pb, tv, rows, K, B.get(), isc.get(), K_pad, 0, nullptr, nullptr, nullptr,
                             o.get() + c0, wp, 1, 0);
         }

@@ -31,6 +31,7 @@
 
 #include <cstdlib>
 
+#include "fp_convert.cuh"
 #include "slfmm_internal.h"
 #include "tc_common.cuh"
 
@@ -604,20 +605,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
 }
 
 // per-column max |x * kscale| as float bits (non-negative floats order as
-// ints); one warp per row, lanes over columns (w <= 128), the per-row scale
-// converted once per row
+// ints); one warp per row, lanes over columns (w <= 128), four rows in flight.
+// A block's warps are combined before the atomics: with a block per eight rows
+// and a warp's own atomics, 20 000 x 72 took 60 us, all of it on 72 addresses.
 template <typename T>
 __global__ void __launch_bounds__(256) k_colmax_abs(const T* __restrict__ src, int ld, uint64_t K, int w,
                                                     const double* __restrict__ kscale, unsigned* __restrict__ colmax) {
+    __shared__ unsigned red[128];
     const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 128) red[threadIdx.x] = 0u;
+    __syncthreads();
     float m[4] = {0.f, 0.f, 0.f, 0.f};
     const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
+#pragma unroll 4
     for (uint64_t k = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < K; k += nw) {
-        float ks = 1.f;
-        if (kscale) {
-            if (lane == 0) ks = (float)kscale[k];
-            ks = __shfl_sync(0xffffffffu, ks, 0);
-        }
+        const float ks = kscale ? (float)kscale[k] : 1.f;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const int c = lane + 32 * t;
@@ -627,8 +629,10 @@ __global__ void __launch_bounds__(256) k_colmax_abs(const T* __restrict__ src, i
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
         const int c = lane + 32 * t;
-        if (c < w) atomicMax(colmax + c, __float_as_uint(m[t]));
+        if (c < w) atomicMax(red + c, __float_as_uint(m[t]));
     }
+    __syncthreads();
+    if ((int)threadIdx.x < w) atomicMax(colmax + threadIdx.x, red[threadIdx.x]);
 }
 
 __device__ __forceinline__ int term_e0(unsigned bits) {
@@ -657,72 +661,9 @@ __device__ __forceinline__ uint64_t wop_offset(uint32_t row, uint64_t k, uint32_
            ((((kk >> 4) ^ (row & 7u)) << 4) | (kk & 15u));
 }
 
-// W (K x w) -> `terms` E4M3 rows per column at B rows row_off + t * wpad + c
-// of a stage-major operand with n_rows rows (wop_offset), zero padded to
-// K_pad; inv_scale[row] = 2^-(e0 + 4t).
-// Term t is round_e4m3((r - terms_<t) * 2^(e0 + 4t)); the power-of-two scales
-// are exact, so each step's residual is rounded once.
-template <typename T>
-__global__ void __launch_bounds__(256) k_fp8_terms(const T* __restrict__ src, int ld, uint64_t K, int w, int wpad,
-                                                   uint64_t K_pad, const double* __restrict__ kscale, int terms,
-                                                   int row_off, int n_rows, const unsigned* __restrict__ colmax,
-                                                   uint8_t* __restrict__ B, float* __restrict__ inv_scale) {
-    __shared__ __align__(16) uint8_t tile[kMainTerms][32][132];
-    __shared__ float ks[128];
-    __shared__ int e0s[32];
-    const uint64_t k0 = (uint64_t)blockIdx.x * 128;
-    const int c0 = blockIdx.y * 32;
-    for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-        const uint64_t k = k0 + i;
-        ks[i] = (kscale && k < K) ? (float)kscale[k] : 1.f;
-    }
-    for (int i = threadIdx.x; i < 32; i += blockDim.x) {
-        const int c = c0 + i;
-        e0s[i] = c < w ? term_e0(colmax[c]) : 0;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 128 * 32; e += blockDim.x) {
-        const int kk = e / 32, cc = e % 32;
-        const uint64_t k = k0 + kk;
-        const int c = c0 + cc;
-        float r = 0.f;
-        if (k < K && c < w) r = (float)src[k * ld + c] * ks[kk];
-        const int e0 = e0s[cc];
-        for (int t = 0; t < terms; ++t) {
-            const int ex = e0 + 4 * t;
-            const __nv_fp8_storage_t qv = __nv_cvt_float_to_fp8(r * pow2f(ex), __NV_SATFINITE, __NV_E4M3);
-            const __half_raw hr = __nv_cvt_fp8_to_halfraw(qv, __NV_E4M3);
-            r = fmaf(-__half2float(__half(hr)), pow2f(-ex), r);
-            tile[t][cc][kk] = (uint8_t)qv;
-        }
-    }
-    __syncthreads();
-    if (blockIdx.x == 0)
-        for (int e = threadIdx.x; e < terms * 32; e += blockDim.x) {
-            const int t = e / 32, cc = e % 32, c = c0 + cc;
-            if (c < wpad) inv_scale[row_off + t * wpad + c] = c < w ? pow2f(-(e0s[cc] + 4 * t)) : 1.f;
-        }
-    // B position kp within each 16-group holds K index kk = perm(kp): the even
-    // K indices of the group, then the odd ones (the order the unpackers emit
-    // the genotypes of a 32-bit code word in); written as 32-bit words
-    for (int e = threadIdx.x; e < terms * 32 * 32; e += blockDim.x) {
-        const int t = e / (32 * 32), rem = e % (32 * 32), cc = rem / 32, kp0 = (rem % 32) * 4;
-        const int c = c0 + cc;
-        if (c >= wpad) continue;
-        uint32_t word = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int kp = kp0 + b;
-            const int kk = (kp & ~15) | ((kp & 7) << 1) | ((kp >> 3) & 1);
-            word |= (uint32_t)tile[t][cc][kk] << (8 * b);
-        }
-        *reinterpret_cast<uint32_t*>(B + wop_offset((uint32_t)(row_off + t * wpad + c), k0 + kp0, (uint32_t)n_rows)) =
-            word;
-    }
-}
-
-// The two scalings of one narrow FP32 operand that a transposed pass splits
-// (diag(s) Q for the genotypes, diag(mu s) Q for the missing-call indicator).
+// The E4M3 terms of one scaling of an operand: a transposed pass splits two of
+// them (diag(s) Q for the genotypes, diag(mu s) Q for the missing-call
+// indicator), a row pass W and, for the indicator, its leading terms again.
 struct TermSet {
     const double* kscale;    // per-K-row scale (null: 1)
     int terms;               // E4M3 terms (0: set absent)
@@ -746,22 +687,23 @@ __global__ void __launch_bounds__(256) k_colmax_pair(const float* __restrict__ s
     float ma[4] = {0.f, 0.f, 0.f, 0.f}, mb[4] = {0.f, 0.f, 0.f, 0.f};
     for (uint64_t j0 = tid / q; j0 < K; j0 += 4 * step) {
         float4 v[4];
-        float fa[4], fb[4];
+        double da[4], db[4];  // all loads before the first conversion's branch
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const uint64_t j = j0 + u * step;
             const bool ok = j < K;
             v[u] = ok ? s4[j * q + qp] : make_float4(0.f, 0.f, 0.f, 0.f);
-            fa[u] = ok && ksa ? (float)ksa[j] : 1.f;
-            fb[u] = ok && ksb ? (float)ksb[j] : 1.f;
+            da[u] = ok && ksa ? ksa[j] : 1.0;
+            db[u] = ok && ksb ? ksb[j] : 1.0;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            const float fa = f32_of_f64(da[u]), fb = f32_of_f64(db[u]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                ma[i] = fmaxf(ma[i], fabsf(x[i] * fa[u]));
-                mb[i] = fmaxf(mb[i], fabsf(x[i] * fb[u]));
+                ma[i] = fmaxf(ma[i], fabsf(x[i] * fa));
+                mb[i] = fmaxf(mb[i], fabsf(x[i] * fb));
             }
         }
     }
@@ -798,79 +740,88 @@ __global__ void __launch_bounds__(256) k_colmax_pair(const float* __restrict__ s
     }
 }
 
-// Split-FP8 terms of both sets in one pass (the loads of the operand are
-// shared): as k_fp8_terms, with two K rows per E4M3 conversion (the paired
-// conversion rounds each value as the scalar one does, so the terms are the
-// same) and the power-of-two scales taken from per-column tables.
-__global__ void __launch_bounds__(256) k_fp8_terms_pair(const float* __restrict__ src, int ld, uint64_t K, int w,
-                                                        int wpad, uint64_t K_pad, TermSet sa, TermSet sb, int n_rows,
-                                                        uint8_t* __restrict__ B, float* __restrict__ inv_scale) {
+// W (K x w) -> the E4M3 rows of both sets, row_off + t * wpad + c for term t of
+// column c, of a stage-major operand with n_rows rows (wop_offset), zero padded
+// to whole stages; inv_scale[row] = 2^-(e0 + 4t).  Term t is
+// round_e4m3((r - terms_<t) * 2^(e0 + 4t)); the power-of-two scales are exact, so
+// each step's residual is rounded once.
+//
+// A block makes one stage (256 K rows) of 16 columns, a thread 16 K rows of a
+// column: those are one 16-byte chunk of every term, the even K indices of its
+// halves, then the odd ones (the order the unpackers emit the genotypes of a
+// 32-bit code word in), converted in the pairs that the words take.  The chunks
+// pass through shared memory so that every term's 16 rows leave as 2 KB in a row.
+// With a thread per K pair and the terms through shared memory byte by byte,
+// 400 000 x 20 (seven terms) took 87 us and 8 500 x 20 (four) 18 us; so 37
+// and 6.
+constexpr int kTermCols = 16;
+template <typename T>
+__global__ void __launch_bounds__(256) k_fp8_terms(const T* __restrict__ src, int ld, uint64_t K, int w, int wpad,
+                                                   TermSet sa, TermSet sb, int n_rows, uint8_t* __restrict__ B,
+                                                   float* __restrict__ inv_scale) {
     constexpr int kT = kMainTerms + kIndTerms;
-    __shared__ __align__(16) uint8_t tile[kT][32][132];
-    __shared__ float ksa[128], ksb[128];
-    __shared__ float up[kT][32], dn[kT][32];
-    const uint64_t k0 = (uint64_t)blockIdx.x * 128;
-    const int c0 = blockIdx.y * 32;
+    __shared__ uint4 tile[kT][2][kTermCols][8];
+    __shared__ float ks[2][kStageK];
+    __shared__ float up[kT][kTermCols], dn[kT][kTermCols];
+    const uint64_t k0 = (uint64_t)blockIdx.x * kStageK;
+    const int c0 = blockIdx.y * kTermCols;
     const int nt = sa.terms + sb.terms;
-    for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-        const uint64_t k = k0 + i;
-        ksa[i] = (sa.kscale && k < K) ? (float)sa.kscale[k] : 1.f;
-        ksb[i] = (sb.kscale && k < K) ? (float)sb.kscale[k] : 1.f;
+    const int cc = threadIdx.x % kTermCols, g = threadIdx.x / kTermCols;
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const uint64_t k = k0 + 16 * g + i;
+        x[i] = k < K && c0 + cc < w ? (float)src[k * ld + c0 + cc] : 0.f;
     }
-    for (int e = threadIdx.x; e < nt * 32; e += blockDim.x) {
-        const int t = e / 32, cc = e % 32, c = c0 + cc;
+    {
+        const uint64_t k = k0 + threadIdx.x;
+        ks[0][threadIdx.x] = sa.kscale && k < K ? f32_of_f64(sa.kscale[k]) : 1.f;
+        ks[1][threadIdx.x] = sb.kscale && k < K ? f32_of_f64(sb.kscale[k]) : 1.f;
+    }
+    for (int e = threadIdx.x; e < nt * kTermCols; e += blockDim.x) {
+        const int t = e / kTermCols, c = c0 + e % kTermCols;
         const bool first = t < sa.terms;
         const int tt = first ? t : t - sa.terms;
         const int e0 = c < w ? term_e0((first ? sa.colmax : sb.colmax)[c]) : 0;
-        up[t][cc] = pow2f(e0 + 4 * tt);
-        dn[t][cc] = pow2f(-(e0 + 4 * tt));
-        if (blockIdx.x == 0 && c < wpad)
+        up[t][e % kTermCols] = pow2f(e0 + 4 * tt);
+        dn[t][e % kTermCols] = pow2f(-(e0 + 4 * tt));
+        if (blockIdx.x == 0)
             inv_scale[(first ? sa.row_off : sb.row_off) + tt * wpad + c] = c < w ? pow2f(-(e0 + 4 * tt)) : 1.f;
     }
     __syncthreads();
-    for (int pr = threadIdx.x; pr < 64 * 32; pr += blockDim.x) {
-        const int kk = 2 * (pr / 32), cc = pr % 32;
-        const uint64_t k = k0 + kk;
-        const int c = c0 + cc;
-        float x0 = 0.f, x1 = 0.f;
-        if (c < w) {
-            if (k < K) x0 = (float)src[k * ld + c];
-            if (k + 1 < K) x1 = (float)src[(k + 1) * ld + c];
-        }
 #pragma unroll
-        for (int set = 0; set < 2; ++set) {
-            const int terms = set ? sb.terms : sa.terms, base = set ? sa.terms : 0;
-            const float* ks = set ? ksb : ksa;
-            float r0 = x0 * ks[kk], r1 = x1 * ks[kk + 1];
+    for (int set = 0; set < 2; ++set) {
+        const int terms = set ? sb.terms : sa.terms, base = set ? sa.terms : 0;
+        if (!terms) break;
+        float r[16];
 #pragma unroll
-            for (int t = 0; t < kMainTerms; ++t) {
-                if (t < terms) {
-                    const float u = up[base + t][cc], d = dn[base + t][cc];
-                    const __nv_fp8x2_storage_t q2 =
-                        __nv_cvt_float2_to_fp8x2(make_float2(r0 * u, r1 * u), __NV_SATFINITE, __NV_E4M3);
-                    const float2 f = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(q2, __NV_E4M3)));
-                    r0 = fmaf(-f.x, d, r0);
-                    r1 = fmaf(-f.y, d, r1);
-                    tile[base + t][cc][kk] = (uint8_t)(q2 & 0xffu);
-                    tile[base + t][cc][kk + 1] = (uint8_t)(q2 >> 8);
-                }
+        for (int i = 0; i < 16; ++i) r[i] = x[i] * ks[set][16 * g + i];
+#pragma unroll
+        for (int t = 0; t < kMainTerms; ++t) {
+            if (t >= terms) break;
+            const float u = up[base + t][cc], d = dn[base + t][cc];
+            uint32_t word[4];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                // pairs (0, 2), (4, 6), (8, 10), (12, 14), (1, 3) ..: two to a word
+                const int i = (q & 3) * 4 + (q >> 2);
+                const __nv_fp8x2_storage_t q2 =
+                    __nv_cvt_float2_to_fp8x2(make_float2(r[i] * u, r[i + 2] * u), __NV_SATFINITE, __NV_E4M3);
+                const float2 f = __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(q2, __NV_E4M3)));
+                r[i] = fmaf(-f.x, d, r[i]);
+                r[i + 2] = fmaf(-f.y, d, r[i + 2]);
+                if (q & 1) word[q >> 1] |= (uint32_t)q2 << 16;
+                else word[q >> 1] = q2;
             }
+            tile[base + t][g >> 3][cc][(g & 7) ^ (cc & 7)] = make_uint4(word[0], word[1], word[2], word[3]);
         }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < nt * 32 * 32; e += blockDim.x) {
-        const int t = e / (32 * 32), rem = e % (32 * 32), cc = rem / 32, kp0 = (rem % 32) * 4;
-        const int c = c0 + cc;
-        if (c >= wpad) continue;
-        const int row = t < sa.terms ? sa.row_off + t * wpad + c : sb.row_off + (t - sa.terms) * wpad + c;
-        uint32_t word = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int kp = kp0 + b;
-            const int kk = (kp & ~15) | ((kp & 7) << 1) | ((kp >> 3) & 1);
-            word |= (uint32_t)tile[t][cc][kk] << (8 * b);
-        }
-        *reinterpret_cast<uint32_t*>(B + wop_offset((uint32_t)row, k0 + kp0, (uint32_t)n_rows)) = word;
+    uint8_t* stage = B + (uint64_t)blockIdx.x * n_rows * kStageK;
+    for (int e = threadIdx.x; e < nt * 2 * kTermCols * 8; e += blockDim.x) {
+        const int t = e / (2 * kTermCols * 8), h = e / (kTermCols * 8) % 2, at = e % (kTermCols * 8);
+        const int row = (t < sa.terms ? sa.row_off + t * wpad : sb.row_off + (t - sa.terms) * wpad) + c0;
+        reinterpret_cast<uint4*>(stage + (uint64_t)(h * n_rows + row) * 128)[at] = tile[t][h][0][at];
     }
 }
 
@@ -1238,18 +1189,27 @@ TileView build_tiles(Ctx& c, const Geno& g, bool transposed) {
     return TileView{g.tilesT.get(), g.kbtT, g.ntilesT};
 }
 
+// blocks of k_colmax_abs: few enough for their atomics, eight warps with four
+// rows in flight each
+static unsigned colmax_blocks(const Ctx& c, uint64_t K) {
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(K, 32), (uint64_t)c.sm_count * 4));
+}
+
 void launch_fp8_terms_f64(Ctx& c, const double* src, int ld, uint64_t K, int w, int wpad, uint64_t K_pad,
-                          const double* kscale, int terms, int row_off, int n_rows, uint8_t* B, float* inv_scale) {
+                          int ind_row_off, int n_rows, uint8_t* B, float* inv_scale) {
     DBuf<unsigned> cm(wpad, c.stream);
     cm.zero();
     SLFMM_REQUIRE(w >= 1 && w <= 128 && wpad <= 128, SLFMM_ERR_BAD_ARG, "operand wider than 128 columns");
-    SLFMM_REQUIRE(n_rows % 8 == 0 && row_off + terms * wpad <= n_rows && K_pad % kStageK == 0, SLFMM_ERR_BAD_ARG,
-                  "bad stage-major operand shape");
-    k_colmax_abs<double><<<grid_for(c, K, 8), 256, 0, c.stream>>>(src, ld, K, w, kscale, cm.get());
+    SLFMM_REQUIRE(n_rows % 8 == 0 && kMainTerms * wpad <= n_rows && ind_row_off % 8 == 0 &&
+                      (!ind_row_off || ind_row_off + kIndTerms * wpad <= n_rows) && wpad % kTermCols == 0 &&
+                      K_pad % kStageK == 0,
+                  SLFMM_ERR_BAD_ARG, "bad stage-major operand shape");
+    k_colmax_abs<double><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, nullptr, cm.get());
     SLFMM_LAUNCHED(c, "k_colmax_abs");
-    dim3 grid((unsigned)ceil_div(K_pad, 128), (unsigned)ceil_div(wpad, 32));
-    k_fp8_terms<double><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, K_pad, kscale, terms, row_off, n_rows,
-                                                    cm.get(), B, inv_scale);
+    const TermSet sa{nullptr, kMainTerms, 0, cm.get()};
+    const TermSet sb{nullptr, ind_row_off ? kIndTerms : 0, ind_row_off, cm.get()};
+    dim3 grid((unsigned)(K_pad / kStageK), (unsigned)(wpad / kTermCols));
+    k_fp8_terms<double><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
     SLFMM_LAUNCHED(c, "k_fp8_terms");
 }
 
@@ -1258,7 +1218,8 @@ void launch_fp8_terms_f32_pair(Ctx& c, const float* src, int ld, uint64_t K, int
                                float* inv_scale) {
     SLFMM_REQUIRE(w >= 1 && w <= 128 && wpad <= 128, SLFMM_ERR_BAD_ARG, "operand wider than 128 columns");
     SLFMM_REQUIRE(n_rows % 8 == 0 && kMainTerms * wpad <= n_rows &&
-                      (!ks_ind || ind_row_off + kIndTerms * wpad <= n_rows) && K_pad % kStageK == 0,
+                      (!ks_ind || (ind_row_off % 8 == 0 && ind_row_off + kIndTerms * wpad <= n_rows)) &&
+                      wpad % kTermCols == 0 && K_pad % kStageK == 0,
                   SLFMM_ERR_BAD_ARG, "bad stage-major operand shape");
     DBuf<unsigned> cm(2 * (uint64_t)wpad, c.stream);
     cm.zero();
@@ -1271,18 +1232,18 @@ void launch_fp8_terms_f32_pair(Ctx& c, const float* src, int ld, uint64_t K, int
         k_colmax_pair<<<blocks, 256, 0, c.stream>>>(src, ld, K, w, ks_main, ks_ind, cma, cmb);
         SLFMM_LAUNCHED(c, "k_colmax_pair");
     } else {
-        k_colmax_abs<float><<<grid_for(c, K, 8), 256, 0, c.stream>>>(src, ld, K, w, ks_main, cma);
+        k_colmax_abs<float><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, ks_main, cma);
         SLFMM_LAUNCHED(c, "k_colmax_abs");
         if (ks_ind) {
-            k_colmax_abs<float><<<grid_for(c, K, 8), 256, 0, c.stream>>>(src, ld, K, w, ks_ind, cmb);
+            k_colmax_abs<float><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, ks_ind, cmb);
             SLFMM_LAUNCHED(c, "k_colmax_abs");
         }
     }
     const TermSet sa{ks_main, kMainTerms, 0, cma};
     const TermSet sb{ks_ind, ks_ind ? kIndTerms : 0, ind_row_off, cmb};
-    dim3 grid((unsigned)ceil_div(K_pad, 128), (unsigned)ceil_div(wpad, 32));
-    k_fp8_terms_pair<<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, K_pad, sa, sb, n_rows, B, inv_scale);
-    SLFMM_LAUNCHED(c, "k_fp8_terms_pair");
+    dim3 grid((unsigned)(K_pad / kStageK), (unsigned)(wpad / kTermCols));
+    k_fp8_terms<float><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
+    SLFMM_LAUNCHED(c, "k_fp8_terms");
 }
 
 int Tc8Errors::read() {

@@ -268,7 +268,7 @@ void launch_row_lut(Ctx& c, const Geno& g, const float* lut, const float* W, int
 // S[i, c] = sum_j lut_j[code_ij] * Q[j, c]        (FP64 result, n x wp)
 void launch_col_lut(Ctx& c, const Geno& g, const float* lut, const float* Q, int wp, double* S);
 
-void launch_reduce_splits(Ctx& c, const float* part, int splits, uint64_t n, int wp, uint64_t n_pad,
+void launch_reduce_splits(Ctx& c, const float* part, int splits, uint64_t n, int w, int wp, uint64_t n_pad,
                           double* S);
 
 // k_tc.cu : tcgen05 split-BF16 contractions
@@ -328,11 +328,11 @@ TileView build_tiles(Ctx& c, const Geno& g, bool transposed);
 // the sample-major tiles, their 2-bit transpose, counts from the tiles.
 void tiles_subset_samples(Ctx& c, const Geno& full, const uint32_t* keep_dev, uint64_t n_keep, Geno& sub);
 void tile_chunk(Ctx& c, const Geno& g, uint64_t r0, uint64_t r1, bool last);
-// `terms` E4M3 terms of diag(kscale) src at rows row_off + t * wpad + c of a
-// stage-major W operand of n_rows rows (every 256-sample stage one contiguous,
-// pre-swizzled blob: one bulk copy per stage in k_tc8_rows)
+// 4 E4M3 terms of src at rows t * wpad + c of a stage-major W operand of n_rows
+// rows (every 256-sample stage one contiguous, pre-swizzled blob: one bulk copy
+// per stage in k_tc8_rows), and with ind_row_off the leading 3 again from there on
 void launch_fp8_terms_f64(Ctx& c, const double* src, int ld, uint64_t K, int w, int wpad, uint64_t K_pad,
-                          const double* kscale, int terms, int row_off, int n_rows, uint8_t* B, float* inv_scale);
+                          int ind_row_off, int n_rows, uint8_t* B, float* inv_scale);
 // both operands of a transposed pass in one pass over src: 4 terms of
 // diag(ks_main) src at B rows 0.., and (ks_ind non-null) 3 terms of
 // diag(ks_ind) src at B rows ind_row_off..; the same terms as two separate
