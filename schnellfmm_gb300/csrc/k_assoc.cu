@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(256, 3) k_assoc_epilogue(
     const double* __restrict__ cjj, const uint8_t* __restrict__ dropped,
     double* __restrict__ beta, float* __restrict__ t32, double* __restrict__ r2,
     uint32_t* __restrict__ hist) {
+    dependent_wait();
     constexpr int kTile = tile_snps(TP), kStride = kTile + 4;  // 16-byte rows, staggered banks
     extern __shared__ __align__(16) float sm[];
     float* thT = sm;                          // [w][TP]
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(256) k_assoc_few(
     const uint8_t* __restrict__ zero_var, int d, int w, double df, const float* __restrict__ theta_rows,
     const float* __restrict__ beta_rows, const double* __restrict__ cjj, const uint8_t* __restrict__ dropped,
     double* __restrict__ beta, float* __restrict__ t32, double* __restrict__ r2, uint32_t* __restrict__ hist) {
+    dependent_wait();
     extern __shared__ __align__(16) float sm[];
     float4* th4 = reinterpret_cast<float4*>(sm);  // [8 * ceil(w / 8)] theta, then beta, of the four traits
     const int wq = (w + 7) & ~7;
@@ -291,6 +293,7 @@ __global__ void __launch_bounds__(256) k_assoc_few(
 constexpr int kHistGroup = 128, kHistGroups = (kHistBins + kHistGroup - 1) / kHistGroup;
 __global__ void __launch_bounds__(1024) k_gif(const uint32_t* __restrict__ hist,
                                               double* __restrict__ gif_raw) {
+    dependent_start();
     constexpr int kPer = (kHistGroups + 1023) / 1024;  // groups of a thread
     __shared__ unsigned group[kPer * 1024];
     __shared__ unsigned long long wsum[32], before[2];
@@ -385,6 +388,7 @@ constexpr int kMaxCalibTraits = 1024;
 __global__ void k_calibrate(uint64_t p, int d, const float* __restrict__ t32,
                             const double* __restrict__ gif, double* __restrict__ t64,
                             double* __restrict__ pval) {
+    dependent_wait();
     __shared__ float zs[kMaxCalibTraits];
     __shared__ double rs[kMaxCalibTraits];
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
@@ -419,6 +423,7 @@ static __device__ __align__(256) uint32_t g_noalloc_hist[kGifNoAllocMaxTraits * 
 
 // Same binning as the association epilogue (tsq_bin) for every t of trait j.
 __global__ void k_tsq_hist(const float* __restrict__ t, uint64_t p, int d, uint32_t* __restrict__ hist) {
+    dependent_wait();
     const uint64_t total = p * (uint64_t)d;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -494,7 +499,7 @@ static void assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const do
     // shared memory); every block reads the same u rows
     for (int t0 = 0; t0 < k.d; t0 += TP) {
         const int db = std::min(TP, k.d - t0);
-        k_assoc_epilogue<TP><<<grid, 256, smem, c.stream>>>(
+        launch_next(c, k_assoc_epilogue<TP>, grid, 256, smem, 
             p, u, ldu, tss, k.zero_var, db, k.d, k.w, k.df, k.theta_rows + (size_t)t0 * k.w,
             k.beta_rows + (size_t)t0 * k.w, k.cjj + t0, k.dropped + t0, beta + t0, t32 + t0, t0 == 0 ? r2 : nullptr,
             hist + (size_t)t0 * kHistBins);
@@ -512,7 +517,7 @@ void launch_assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const do
     if (k.d <= kFewTraits && ldu % 8 == 0 && ldu >= ((k.w + 7) & ~7) && r2 &&
         reinterpret_cast<uintptr_t>(u) % 16 == 0) {
         const size_t smem = (size_t)2 * ((k.w + 7) & ~7) * sizeof(float4);
-        k_assoc_few<<<grid_for(c, p, 256), 256, smem, c.stream>>>(p, u, ldu, tss, k.zero_var, k.d, k.w, k.df,
+        launch_next(c, k_assoc_few, grid_for(c, p, 256), 256, smem, p, u, ldu, tss, k.zero_var, k.d, k.w, k.df,
                                                                   k.theta_rows, k.beta_rows, k.cjj, k.dropped, beta,
                                                                   t32, r2, hist);
         SLFMM_LAUNCHED(c, "k_assoc_few");
@@ -525,7 +530,7 @@ void launch_assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const do
 
 void launch_gif(Ctx& c, const uint32_t* hist, int d, double* gif_raw) {
     if (d == 0) return;
-    k_gif<<<d, 1024, 0, c.stream>>>(hist, gif_raw);
+    launch_next(c, k_gif, d, 1024, 0, hist, gif_raw);
     SLFMM_LAUNCHED(c, "k_gif");
 }
 
@@ -535,7 +540,7 @@ void launch_calibrate(Ctx& c, uint64_t p, int d, const float* t32, const double*
     SLFMM_REQUIRE(d <= kMaxCalibTraits, SLFMM_ERR_BAD_ARG, "too many traits for the calibration kernel");
     // few blocks: each forms the d per-trait factors in FP64 before its loop
     const unsigned grid = (unsigned)std::min<int>(grid_for(c, p * d, 256), c.sm_count * 8);
-    k_calibrate<<<grid, 256, 0, c.stream>>>(p, d, t32, gif, t64, pval);
+    launch_next(c, k_calibrate, grid, 256, 0, p, d, t32, gif, t64, pval);
     SLFMM_LAUNCHED(c, "k_calibrate");
 }
 

@@ -26,6 +26,7 @@ __device__ __forceinline__ uint32_t code_at(const uint8_t* row, uint64_t s) {
 __global__ void k_repack(const uint8_t* __restrict__ in, uint64_t rows, uint64_t in_bps,
                          const uint32_t* __restrict__ keep, uint64_t n_out,
                          uint8_t* __restrict__ out, uint64_t stride) {
+    dependent_wait();
     const uint64_t words_per_row = stride / 4;
     const uint64_t total = rows * words_per_row;
     const uint64_t out_bps = (n_out + 3) / 4;
@@ -65,6 +66,7 @@ __global__ void k_repack(const uint8_t* __restrict__ in, uint64_t rows, uint64_t
 __global__ void __launch_bounds__(256) k_repack_keep(const uint8_t* __restrict__ in, uint64_t rows, uint64_t in_bps,
                                                      const uint32_t* __restrict__ keep, uint64_t n_out,
                                                      uint8_t* __restrict__ out, uint64_t stride) {
+    dependent_wait();
     extern __shared__ __align__(16) uint8_t sm_keep[];
     const uint64_t words = (n_out + 15) / 16;           // output words holding kept samples
     uint32_t* ks = reinterpret_cast<uint32_t*>(sm_keep);  // 16 x words indices
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(256) k_repack_keep(const uint8_t* __restrict__
 template <typename V>
 __global__ void k_repack_vec(const uint8_t* __restrict__ in, uint64_t rows, uint64_t in_bps, uint64_t n_out,
                              uint8_t* __restrict__ out, uint64_t stride) {
+    dependent_wait();
     constexpr int kw = sizeof(V) / 4;
     const uint64_t in_vecs = in_bps / sizeof(V), out_vecs = stride / sizeof(V);
     const uint64_t last_word = in_bps / 4 - 1;
@@ -134,6 +137,7 @@ __global__ void k_repack_vec(const uint8_t* __restrict__ in, uint64_t rows, uint
 __global__ void k_snp_counts(const uint8_t* __restrict__ packed, uint64_t p, uint64_t stride,
                              uint64_t n, int32_t* __restrict__ counts,
                              uint64_t* __restrict__ miss_count) {
+    dependent_wait();
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (warp >= p) return;
@@ -174,6 +178,7 @@ __global__ void k_snp_counts(const uint8_t* __restrict__ packed, uint64_t p, uin
 __global__ void k_miss_fill(const uint8_t* __restrict__ packed, uint64_t p, uint64_t stride,
                             uint64_t n, const uint64_t* __restrict__ ptr,
                             uint32_t* __restrict__ idx, uint32_t* __restrict__ rowid, uint64_t cap) {
+    dependent_wait();
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (warp >= p) return;
@@ -223,6 +228,7 @@ __global__ void k_miss_fill(const uint8_t* __restrict__ packed, uint64_t p, uint
 // threads walks the chunk in tiles of 4096 rows with a running carry.
 __global__ void __launch_bounds__(1024) k_miss_ptr_chunk(const int32_t* __restrict__ counts, uint64_t rows,
                                                          uint64_t* __restrict__ ptr) {
+    dependent_wait();
     __shared__ uint64_t warp_sum[32];
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
     uint64_t carry = ptr[0];
@@ -266,12 +272,14 @@ __global__ void __launch_bounds__(1024) k_miss_ptr_chunk(const int32_t* __restri
 
 __global__ void k_count_keys(const uint32_t* __restrict__ keys, uint64_t nnz,
                              uint32_t* __restrict__ cnt) {
+    dependent_wait();
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < nnz;
          t += (uint64_t)gridDim.x * blockDim.x)
         atomicAdd(&cnt[keys[t]], 1u);
 }
 
 __global__ void k_u32_to_u64(const uint32_t* __restrict__ a, uint64_t m, uint64_t* __restrict__ b) {
+    dependent_wait();
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < m;
          t += (uint64_t)gridDim.x * blockDim.x)
         b[t] = a[t];
@@ -283,6 +291,7 @@ __global__ void k_u32_to_u64(const uint32_t* __restrict__ a, uint64_t m, uint64_
 __global__ void k_stats_mean(const int32_t* __restrict__ counts, uint64_t p, int norm,
                              double* __restrict__ mean, double* __restrict__ scale,
                              double* __restrict__ tss, uint8_t* __restrict__ zero_var) {
+    dependent_wait();
     for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < p;
          j += (uint64_t)gridDim.x * blockDim.x) {
         const int64_t c0 = counts[j * 4 + 0], c1 = counts[j * 4 + 1], c2 = counts[j * 4 + 2];
@@ -301,6 +310,7 @@ __global__ void k_stats_mean(const int32_t* __restrict__ counts, uint64_t p, int
 __global__ void k_decode_chunk(const uint8_t* __restrict__ packed, uint64_t stride, uint64_t n,
                                uint64_t snp0, uint64_t ncols, const double* __restrict__ mean,
                                const double* __restrict__ scale, double* __restrict__ out) {
+    dependent_wait();
     const uint64_t total = n * ncols;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -318,6 +328,7 @@ __global__ void k_decode_chunk(const uint8_t* __restrict__ packed, uint64_t stri
 
 __global__ void k_lut_std(uint64_t p, const double* __restrict__ mean,
                           const double* __restrict__ scale, float* __restrict__ lut) {
+    dependent_wait();
     for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < p;
          j += (uint64_t)gridDim.x * blockDim.x) {
         const double mu = mean[j], sc = scale[j];

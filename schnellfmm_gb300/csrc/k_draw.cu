@@ -66,6 +66,7 @@ __device__ __forceinline__ bool less_or_near(double a, double b, bool& near) {
 __global__ void __launch_bounds__(kDrawThreads) k_draw(uint64_t seed, const double* __restrict__ tables, unsigned cap,
                                                        double* __restrict__ vals, unsigned* __restrict__ counts,
                                                        Tails* __restrict__ tails) {
+    dependent_start();
     __shared__ uint64_t bits[kDrawWindow];
     __shared__ double x[257], f[257];
     __shared__ uint8_t cons[kDrawWindow];
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(kDrawThreads) k_draw(uint64_t seed, const doub
 // the tail values, computed by the host, into the scratch
 __global__ void k_draw_tails(const Tails* __restrict__ tails, const double* __restrict__ tail_vals, unsigned n,
                              double* __restrict__ vals) {
+    dependent_start();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) vals[tails->e[i].slot >> 1] = tail_vals[i];
 }
@@ -198,6 +200,7 @@ __global__ void k_draw_tails(const Tails* __restrict__ tails, const double* __re
 __global__ void __launch_bounds__(kDrawThreads) k_draw_place(const double* __restrict__ vals,
                                                              const unsigned* __restrict__ counts, uint64_t count,
                                                              double* __restrict__ out) {
+    dependent_start();
     __shared__ unsigned long long part[kDrawThreads / 32];
     unsigned long long before = 0;
     for (unsigned b = threadIdx.x; b < blockIdx.x; b += kDrawThreads) before += counts[b];
@@ -267,8 +270,8 @@ std::shared_ptr<Ctx::PendingNormal> start_draw(Ctx& c, uint64_t seed, uint64_t r
     SLFMM_CUDA(cudaMemcpyAsync(p->tables.get(), normal_tables(), p->tables.bytes(), cudaMemcpyHostToDevice, c.stream));
     SLFMM_CUDA(cudaMemsetAsync(p->tails.get(), 0, sizeof(Tails), c.stream));
     Tails* tails = reinterpret_cast<Tails*>(p->tails.get());
-    k_draw<<<p->blocks, kDrawThreads, 0, c.stream>>>(seed, p->tables.get(), p->cap, p->vals.get(), p->counts.get(),
-                                                     tails);
+    launch_next(c, k_draw, p->blocks, kDrawThreads, 0, seed, p->tables.get(), p->cap, p->vals.get(), p->counts.get(),
+                tails);
     SLFMM_LAUNCHED(c, "k_draw");
     SLFMM_CUDA(cudaMemcpyAsync(c.draw_tails, tails, bytes, cudaMemcpyDeviceToHost, c.stream));
     SLFMM_CUDA(cudaEventRecord(c.draw_done, c.stream));
@@ -305,11 +308,11 @@ void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
                 for (unsigned i = 0; i < t.n; ++i) tv[i] = normal_tail_value(t.e[i].a, t.e[i].slot & 1);
                 DBuf<double> tvd(tv.size(), c.stream);
                 SLFMM_CUDA(cudaMemcpyAsync(tvd.get(), tv.data(), tvd.bytes(), cudaMemcpyHostToDevice, c.stream));
-                k_draw_tails<<<(unsigned)ceil_div(t.n, 128), 128, 0, c.stream>>>(
+                launch_next(c, k_draw_tails, (unsigned)ceil_div(t.n, 128), 128, 0, 
                     reinterpret_cast<const Tails*>(p->tails.get()), tvd.get(), t.n, p->vals.get());
                 SLFMM_LAUNCHED(c, "k_draw_tails");
             }
-            k_draw_place<<<p->blocks, kDrawThreads, 0, c.stream>>>(p->vals.get(), p->counts.get(), count, out);
+            launch_next(c, k_draw_place, p->blocks, kDrawThreads, 0, p->vals.get(), p->counts.get(), count, out);
             SLFMM_LAUNCHED(c, "k_draw_place");
         }
     }

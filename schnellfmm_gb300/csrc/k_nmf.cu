@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(256) k_fill_stats(uint64_t p, uint64_t n, int 
                                                     const float* __restrict__ W, const float* __restrict__ H, int k,
                                                     double* __restrict__ mean, double* __restrict__ scale,
                                                     double* __restrict__ tss, uint8_t* __restrict__ zero_var) {
+    dependent_wait();
     __shared__ float hs[8][KM];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint64_t nw = (uint64_t)gridDim.x * 8;
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(256) k_fill_row_correct(float* __restrict__ ou
                                                           const float* __restrict__ H, int k,
                                                           const double* __restrict__ mean,
                                                           const double* __restrict__ scale) {
+    dependent_wait();
     __shared__ float hs[8][KM];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint64_t nw = (uint64_t)gridDim.x * 8;
@@ -232,6 +234,7 @@ __global__ void __launch_bounds__(256) k_fill_col_correct(double* __restrict__ S
                                                           const float* __restrict__ Qop, int ldq,
                                                           const float* __restrict__ Wn, const float* __restrict__ H,
                                                           int k, const float2* __restrict__ sm) {
+    dependent_wait();
     __shared__ float ws[8][KM];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint64_t nw = (uint64_t)gridDim.x * 8;
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(256) k_fill_col_correct(double* __restrict__ S
 // raw mean-filled product (MeanRaw, src/parallel.rs:53-71)
 __global__ void k_add_mean_colsum(float* __restrict__ out, int ldo, uint64_t p, int w,
                                   const double* __restrict__ mean, const double* __restrict__ cs) {
+    dependent_start();
     const uint64_t total = p * (uint64_t)w;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -284,6 +288,7 @@ __global__ void k_add_mean_colsum(float* __restrict__ out, int ldo, uint64_t p, 
 template <typename TN>
 __global__ void k_nmf_update(double* __restrict__ X, uint64_t m, int k, const TN* __restrict__ num, int ldn,
                              const double* __restrict__ denom, double eps) {
+    dependent_start();
     const uint64_t total = m * (uint64_t)k;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -300,6 +305,7 @@ __global__ void k_nmf_update(double* __restrict__ X, uint64_t m, int k, const TN
 // H[:, j] *= ||W[:, j]||_1 for columns whose L1 norm (W >= 0) exceeds eps
 __global__ void k_nmf_normalize(double* __restrict__ W, uint64_t n, double* __restrict__ H, uint64_t p, int k,
                                 const double* __restrict__ colsum, double eps) {
+    dependent_start();
     const uint64_t total = (n + p) * (uint64_t)k;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -316,6 +322,7 @@ __global__ void k_nmf_normalize(double* __restrict__ W, uint64_t n, double* __re
 template <typename TS>
 __global__ void k_nmf_sign(const TS* __restrict__ src, int ldsrc, double* __restrict__ X, uint64_t m, int k,
                            int mode) {
+    dependent_start();
     const uint64_t total = m * (uint64_t)k;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -391,6 +398,7 @@ __global__ void __launch_bounds__(256) k_nmf_cv(const uint8_t* __restrict__ pack
                                                 uint64_t p, uint64_t chunk, uint64_t mask_seed, uint64_t thresh,
                                                 const float* __restrict__ W, const float* __restrict__ H, int k,
                                                 const int32_t* __restrict__ counts, double* __restrict__ part) {
+    dependent_wait();
     __shared__ float hs[8][KM];
     __shared__ uint32_t queue[8][64];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -487,6 +495,7 @@ __global__ void __launch_bounds__(256) k_nmf_cv(const uint8_t* __restrict__ pack
 // 1.2 ms.
 __global__ void __launch_bounds__(1024) k_obs_base(const int32_t* __restrict__ counts, uint64_t p, uint64_t chunk,
                                                    uint64_t* __restrict__ base) {
+    dependent_start();
     __shared__ uint64_t wsum[32];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint64_t nchunks = (p + chunk - 1) / chunk;
@@ -607,6 +616,7 @@ __global__ void __launch_bounds__(256) k_nmf_gwas_cv(const uint8_t* __restrict__
                                                      const float* __restrict__ W, const float* __restrict__ Wpt, int k,
                                                      const int32_t* __restrict__ counts,
                                                      const uint64_t* __restrict__ base, double* __restrict__ part) {
+    dependent_wait();
     __shared__ float hh[8][KM];
     __shared__ uint32_t list[8][kHeldList];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -726,11 +736,11 @@ void launch_fill_stats(Ctx& c, const Geno& g, int norm, const float* W, const fl
     if (!g.p) return;
     SLFMM_REQUIRE(k >= 1 && k <= kMaxNmfK, SLFMM_ERR_BAD_ARG, "NMF rank must be in 1.." + std::to_string(kMaxNmfK));
     if (k <= 16)
-        k_fill_stats<16><<<grid_for(c, g.p, 8), 256, 0, c.stream>>>(g.p, g.n, norm, g.counts.get(), g.miss_ptr.get(),
+        launch_next(c, k_fill_stats<16>, grid_for(c, g.p, 8), 256, 0, g.p, g.n, norm, g.counts.get(), g.miss_ptr.get(),
                                                                      g.miss_idx.get(), W, H, k, mean, scale, tss,
                                                                      zero_var);
     else
-        k_fill_stats<32><<<grid_for(c, g.p, 8), 256, 0, c.stream>>>(g.p, g.n, norm, g.counts.get(), g.miss_ptr.get(),
+        launch_next(c, k_fill_stats<32>, grid_for(c, g.p, 8), 256, 0, g.p, g.n, norm, g.counts.get(), g.miss_ptr.get(),
                                                                      g.miss_idx.get(), W, H, k, mean, scale, tss,
                                                                      zero_var);
     SLFMM_LAUNCHED(c, "k_fill_stats");
@@ -761,19 +771,23 @@ static void fill_row_correct_launch(Ctx& c, const Geno& g, unsigned grid, float*
     const uint32_t* mi = g.miss_idx.get();
     switch (narrow_group(w)) {
         case 8:
-            k_fill_row_correct<8, VW, KM><<<grid, 256, 0, c.stream>>>(out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k, mean,
+            launch_next(c, k_fill_row_correct<8, VW, KM>, grid, 256, 0, out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k,
+                        mean,
                                                                   scale);
             break;
         case 16:
-            k_fill_row_correct<16, VW, KM><<<grid, 256, 0, c.stream>>>(out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k, mean,
+            launch_next(c, k_fill_row_correct<16, VW, KM>, grid, 256, 0, out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k,
+                        mean,
                                                                    scale);
             break;
         case 32:
-            k_fill_row_correct<32, VW, KM><<<grid, 256, 0, c.stream>>>(out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k, mean,
+            launch_next(c, k_fill_row_correct<32, VW, KM>, grid, 256, 0, out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k,
+                        mean,
                                                                    scale);
             break;
         default:
-            k_fill_row_correct<0, VW, KM><<<grid, 256, 0, c.stream>>>(out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k, mean,
+            launch_next(c, k_fill_row_correct<0, VW, KM>, grid, 256, 0, out, ldo, g.p, w, mp, mi, Wop, ldw, Wn, H, k,
+                        mean,
                                                                   scale);
     }
 }
@@ -792,6 +806,7 @@ void launch_fill_row_correct(Ctx& c, const Geno& g, float* out, int ldo, int w, 
 
 __global__ void k_scale_mean_f32(const double* __restrict__ mean, const double* __restrict__ scale, uint64_t p,
                                  float2* __restrict__ out) {
+    dependent_start();
     for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < p; r += (uint64_t)gridDim.x * blockDim.x)
         out[r] = make_float2((float)scale[r], (float)mean[r]);
 }
@@ -804,16 +819,20 @@ static void fill_col_correct_launch(Ctx& c, const Geno& g, unsigned grid, uint64
     const uint32_t* ci = g.missT_idx.get();
     switch (narrow_group(w)) {
         case 8:
-            k_fill_col_correct<8, VW, KM><<<grid, 256, 0, c.stream>>>(S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H, k, sm);
+            launch_next(c, k_fill_col_correct<8, VW, KM>, grid, 256, 0, S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H,
+                        k, sm);
             break;
         case 16:
-            k_fill_col_correct<16, VW, KM><<<grid, 256, 0, c.stream>>>(S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H, k, sm);
+            launch_next(c, k_fill_col_correct<16, VW, KM>, grid, 256, 0, S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn,
+                        H, k, sm);
             break;
         case 32:
-            k_fill_col_correct<32, VW, KM><<<grid, 256, 0, c.stream>>>(S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H, k, sm);
+            launch_next(c, k_fill_col_correct<32, VW, KM>, grid, 256, 0, S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn,
+                        H, k, sm);
             break;
         default:
-            k_fill_col_correct<0, VW, KM><<<grid, 256, 0, c.stream>>>(S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H, k, sm);
+            launch_next(c, k_fill_col_correct<0, VW, KM>, grid, 256, 0, S, lds, g.n, w, nseg, cp, ci, Qop, ldq, Wn, H,
+                        k, sm);
     }
 }
 
@@ -824,7 +843,7 @@ void launch_fill_col_correct(Ctx& c, const Geno& g, double* S, int lds, int w, c
     const uint64_t nseg = std::max<uint64_t>(1, ceil_div(g.missT_max, kColSeg));
     const unsigned grid = (unsigned)grid_for(c, g.n * nseg, 8);
     DBuf<float2> sm(std::max<uint64_t>(g.p, 1), c.stream);
-    k_scale_mean_f32<<<grid_for(c, g.p, 256), 256, 0, c.stream>>>(mean, scale, g.p, sm.get());
+    launch_next(c, k_scale_mean_f32, grid_for(c, g.p, 256), 256, 0, mean, scale, g.p, sm.get());
     SLFMM_LAUNCHED(c, "k_scale_mean_f32");
     // 3 000 samples x 7 000 missing calls, rank 8, with 16 and 32 bytes at a time: 8
     // columns 317 and 265 us, 18 (a lane each) 588 and 720
@@ -837,39 +856,39 @@ void launch_fill_col_correct(Ctx& c, const Geno& g, double* S, int lds, int w, c
 
 void launch_add_mean_colsum(Ctx& c, float* out, int ldo, uint64_t p, int w, const double* mean, const double* cs) {
     if (!p || !w) return;
-    k_add_mean_colsum<<<grid_for(c, p * w, 256), 256, 0, c.stream>>>(out, ldo, p, w, mean, cs);
+    launch_next(c, k_add_mean_colsum, grid_for(c, p * w, 256), 256, 0, out, ldo, p, w, mean, cs);
     SLFMM_LAUNCHED(c, "k_add_mean_colsum");
 }
 
 void launch_nmf_update_f64(Ctx& c, double* X, uint64_t m, int k, const double* num, int ldn, const double* denom,
                            double eps) {
     if (!m) return;
-    k_nmf_update<double><<<grid_for(c, m * k, 256), 256, 0, c.stream>>>(X, m, k, num, ldn, denom, eps);
+    launch_next(c, k_nmf_update<double>, grid_for(c, m * k, 256), 256, 0, X, m, k, num, ldn, denom, eps);
     SLFMM_LAUNCHED(c, "k_nmf_update");
 }
 
 void launch_nmf_update_f32(Ctx& c, double* X, uint64_t m, int k, const float* num, int ldn, const double* denom,
                            double eps) {
     if (!m) return;
-    k_nmf_update<float><<<grid_for(c, m * k, 256), 256, 0, c.stream>>>(X, m, k, num, ldn, denom, eps);
+    launch_next(c, k_nmf_update<float>, grid_for(c, m * k, 256), 256, 0, X, m, k, num, ldn, denom, eps);
     SLFMM_LAUNCHED(c, "k_nmf_update");
 }
 
 void launch_nmf_normalize(Ctx& c, double* W, uint64_t n, double* H, uint64_t p, int k, const double* colsum,
                           double eps) {
-    k_nmf_normalize<<<grid_for(c, (n + p) * k, 256), 256, 0, c.stream>>>(W, n, H, p, k, colsum, eps);
+    launch_next(c, k_nmf_normalize, grid_for(c, (n + p) * k, 256), 256, 0, W, n, H, p, k, colsum, eps);
     SLFMM_LAUNCHED(c, "k_nmf_normalize");
 }
 
 void launch_nmf_abs_f64(Ctx& c, const double* src, int ld, double* X, uint64_t m, int k) {
     if (!m) return;
-    k_nmf_sign<double><<<grid_for(c, m * k, 256), 256, 0, c.stream>>>(src, ld, X, m, k, 0);
+    launch_next(c, k_nmf_sign<double>, grid_for(c, m * k, 256), 256, 0, src, ld, X, m, k, 0);
     SLFMM_LAUNCHED(c, "k_nmf_sign");
 }
 
 void launch_nmf_clamp0_f32(Ctx& c, const float* src, int ld, double* X, uint64_t m, int k) {
     if (!m) return;
-    k_nmf_sign<float><<<grid_for(c, m * k, 256), 256, 0, c.stream>>>(src, ld, X, m, k, 1);
+    launch_next(c, k_nmf_sign<float>, grid_for(c, m * k, 256), 256, 0, src, ld, X, m, k, 1);
     SLFMM_LAUNCHED(c, "k_nmf_sign");
 }
 
@@ -886,7 +905,7 @@ uint64_t launch_nmf_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t mask_seed
     const uint64_t rows = (uint64_t)grid * 8;
     if (part.n < rows * 3) part.alloc(rows * 3, c.stream);
     auto go = [&](auto kern) {
-        kern<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.stride, g.n, g.p, chunk, mask_seed, th, W, H, k,
+        launch_next(c, kern, grid, 256, 0, packed_rows(g), g.stride, g.n, g.p, chunk, mask_seed, th, W, H, k,
                                          g.counts.get(), part.get());
     };
     if (k <= 16) {
@@ -904,7 +923,7 @@ uint64_t launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed
                             const float* Wpt, int k, DBuf<double>& part) {
     DBuf<uint64_t> base(std::max<uint64_t>(g.p, 1), c.stream);
     const uint64_t nchunks = ceil_div(g.p, chunk);
-    k_obs_base<<<grid_for(c, nchunks, 1), 1024, 0, c.stream>>>(g.counts.get(), g.p, chunk, base.get());
+    launch_next(c, k_obs_base, grid_for(c, nchunks, 1), 1024, 0, g.counts.get(), g.p, chunk, base.get());
     SLFMM_LAUNCHED(c, "k_obs_base");
     const bool cc = c.rng == SLFMM_RNG_CHACHA8;
     const uint64_t th = cc ? rate_threshold(rate, 52) : rate_threshold(rate);
@@ -914,7 +933,7 @@ uint64_t launch_nmf_gwas_cv(Ctx& c, const Geno& g, uint64_t chunk, uint64_t seed
     // rows of W+ as 16-byte vectors
     const bool w4 = k % 4 == 0 && reinterpret_cast<uintptr_t>(Wpt) % 16 == 0;
     auto go = [&](auto kern) {
-        kern<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.stride, g.n, g.p, chunk, seed, th, W, Wpt, k,
+        launch_next(c, kern, grid, 256, 0, packed_rows(g), g.stride, g.n, g.p, chunk, seed, th, W, Wpt, k,
                                          g.counts.get(), base.get(), part.get());
     };
     if (k <= 16) {

@@ -25,6 +25,7 @@ __device__ __forceinline__ double u53(uint64_t key, uint64_t ctr) {
 // f[j * n_pop + k]: drifted population frequencies
 __global__ void k_sim_freq(uint64_t p, int n_pop, double fst, double f_lo, double f_hi, uint64_t key,
                            float* __restrict__ f) {
+    dependent_wait();
     for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < p;
          j += (uint64_t)gridDim.x * blockDim.x) {
         const double fa = f_lo + (f_hi - f_lo) * u53(key, j * 64);
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(256) k_sim_geno(uint64_t n, uint64_t p, int n_
                                                   const float* __restrict__ f, double miss,
                                                   double inbreeding, uint64_t key, uint64_t snps_per_cta,
                                                   uint8_t* __restrict__ out, uint64_t stride) {
+    dependent_wait();
     extern __shared__ float sm[];
     float* q = sm;                              // kSimSamples x n_pop
     float* fs = sm + kSimSamples * n_pop;       // kSimSnps x n_pop
@@ -104,7 +106,7 @@ void launch_simulate(Ctx& c, uint64_t n, uint64_t p, int n_pop, const float* adm
     SLFMM_REQUIRE(n_pop >= 1 && n_pop <= 32, SLFMM_ERR_BAD_ARG, "1..32 populations");
     const uint64_t key = mix64(seed + 0x9E3779B97F4A7C15ull);
     DBuf<float> f(std::max<uint64_t>(p, 1) * n_pop, c.stream);
-    k_sim_freq<<<grid_for(c, p, 256), 256, 0, c.stream>>>(p, n_pop, fst, f_lo, f_hi, key, f.get());
+    launch_next(c, k_sim_freq, grid_for(c, p, 256), 256, 0, p, n_pop, fst, f_lo, f_hi, key, f.get());
     SLFMM_LAUNCHED(c, "k_sim_freq");
     SLFMM_CUDA(cudaMemsetAsync(out, 0, p * stride, c.stream));
     const uint64_t sblocks = ceil_div(n, kSimSamples);
@@ -113,7 +115,7 @@ void launch_simulate(Ctx& c, uint64_t n, uint64_t p, int n_pop, const float* adm
     dim3 grid((unsigned)sblocks, (unsigned)ceil_div(p, per));
     const size_t smem = (size_t)(kSimSamples + kSimSnps) * n_pop * sizeof(float);
     raise_dynamic_smem((const void*)k_sim_geno, smem);
-    k_sim_geno<<<grid, 256, smem, c.stream>>>(n, p, n_pop, admix_dev, f.get(), miss, inbreeding, key ^ 0x5bd1e995ull,
+    launch_next(c, k_sim_geno, grid, 256, smem, n, p, n_pop, admix_dev, f.get(), miss, inbreeding, key ^ 0x5bd1e995ull,
                                               per, out, stride);
     SLFMM_LAUNCHED(c, "k_sim_geno");
 }

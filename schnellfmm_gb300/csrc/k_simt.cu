@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kLutThreads) k_row_lut(const uint8_t* __restri
                                                          uint64_t p, uint64_t n, const float4* __restrict__ lut,
                                                          const float* __restrict__ W, int wp,
                                                          float* __restrict__ out) {
+    dependent_wait();
     __shared__ __align__(16) float ws[2][kRowSamples][kLutCols];
     __shared__ float luts[R][4][kLutThreads];
     const int tid = threadIdx.x;
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kLutThreads) k_col_lut(const uint8_t* __restri
                                                          uint64_t p, uint64_t n_pad, const float4* __restrict__ lut,
                                                          const float* __restrict__ Q, int wp, uint64_t per_split,
                                                          float* __restrict__ part) {
+    dependent_wait();
     __shared__ __align__(16) float qs[2][kColStage][kLutCols];
     __shared__ __align__(16) float luts[2][kColStage][4];
     __shared__ __align__(16) uint8_t codes[2][kColStage][kColSamples / 4];
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(kLutThreads) k_col_lut(const uint8_t* __restri
 // with a load per addition, 30 us so.
 __global__ void __launch_bounds__(256) k_reduce_splits(const float* __restrict__ part, int splits, uint64_t n, int w,
                                                        int wp, uint64_t n_pad, double* __restrict__ S) {
+    dependent_start();
     const uint64_t total = n * (uint64_t)w, stride = n_pad * wp;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(256) k_reduce_splits(const float* __restrict__
 void launch_reduce_splits(Ctx& c, const float* part, int splits, uint64_t n, int w, int wp, uint64_t n_pad,
                           double* S) {
     if (!n) return;
-    k_reduce_splits<<<grid_for(c, n * w, 256), 256, 0, c.stream>>>(part, splits, n, w, wp, n_pad, S);
+    launch_next(c, k_reduce_splits, grid_for(c, n * w, 256), 256, 0, part, splits, n, w, wp, n_pad, S);
     SLFMM_LAUNCHED(c, "k_reduce_splits");
 }
 
@@ -222,6 +225,8 @@ void launch_row_lut(Ctx& c, const Geno& g, const float* lut, const float* W, int
     // than a block per SM on (2 504 samples x 16, one and two to a thread: 18 000 SNPs
     // 74 and 101 us, 25 000 107 and 109, 32 000 126 and 110, 60 000 222 and 165)
     auto go = [&](auto kern, int r) {
+        // not launch_next: under a kernel that still runs the three blocks per SM
+        // would take unequal places, and the pass lasts as long as the fullest SM
         kern<<<dim3((unsigned)ceil_div(g.p, (uint64_t)kLutThreads * r), (unsigned)(wp / kLutCols)), kLutThreads, 0,
                c.stream>>>(packed_rows(g), g.stride, g.p, g.n, reinterpret_cast<const float4*>(lut), W, wp, out);
     };

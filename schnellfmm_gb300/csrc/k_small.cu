@@ -40,6 +40,7 @@ __device__ double block_sum(double v, double* red) {
 
 __global__ void k_colmeans(const double* __restrict__ A, uint64_t m, int lda, double* __restrict__ out,
                            int divide) {
+    dependent_start();
     __shared__ double red[32];
     const int col = blockIdx.x;
     double s = 0.0;
@@ -50,6 +51,7 @@ __global__ void k_colmeans(const double* __restrict__ A, uint64_t m, int lda, do
 
 __global__ void k_center_cols(double* __restrict__ A, uint64_t m, int a, int lda,
                               const double* __restrict__ means) {
+    dependent_start();
     const uint64_t total = m * a;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -61,6 +63,7 @@ __global__ void k_center_cols(double* __restrict__ A, uint64_t m, int a, int lda
 
 // divide a column by its sample sd (n-1 denominator) unless sd <= 1e-14
 __global__ void k_scale_cols_sd(double* __restrict__ A, uint64_t m, int lda) {
+    dependent_start();
     __shared__ double red[32];
     const int col = blockIdx.x;
     double s = 0.0;
@@ -80,6 +83,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_atb(const T* __restrict__ A, int lda, const T* __restrict__ B,
                                              int ldb, uint64_t m, int a, int b, uint64_t rows_per_split,
                                              double* __restrict__ part) {
+    dependent_start();
     __shared__ double As[32][33];
     __shared__ double Bs[32][33];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -126,6 +130,7 @@ template <typename T, int R>
 __global__ void __launch_bounds__(256) k_atb_flat(const T* __restrict__ A, int lda, const T* __restrict__ B,
                                                   int ldb, uint64_t m, int a, int b, uint64_t rows_per_split,
                                                   double* __restrict__ part) {
+    dependent_start();
     extern __shared__ double stage[];
     double* As = stage;             // [32][a]
     double* Bs = stage + 32 * a;    // [32][b]
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(256) k_atb_flat(const T* __restrict__ A, int l
 // tiles (used for the p x l sketches, whose FP64 Gram would dominate).
 __global__ void __launch_bounds__(256) k_gram_f32(const float* __restrict__ A, int lda, uint64_t m, int a,
                                                   uint64_t rows_per_split, double* __restrict__ part) {
+    dependent_start();
     __shared__ float As[32][33];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -240,6 +246,7 @@ constexpr int kGramRun = 256;
 constexpr size_t kGramNarrowSmem = 8 * 32 * 33 * sizeof(double);
 __global__ void __launch_bounds__(256, 2) k_gram_narrow(const float* __restrict__ A, int lda, uint64_t m, int a,
                                                         double* __restrict__ part) {
+    dependent_start();
     extern __shared__ double gsm[];  // [8 warps][32][33] FP64 sums
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* mine = gsm + warp * 32 * 33;
@@ -279,6 +286,7 @@ __global__ void __launch_bounds__(256, 2) k_gram_narrow(const float* __restrict_
 // from the broadcast row elements; loads and stores are whole rows.
 __global__ void __launch_bounds__(256) k_trmul_narrow(float* __restrict__ A, int lda, uint64_t m, int a,
                                                       const double* __restrict__ Linv) {
+    dependent_start();
     const int lane = threadIdx.x & 31;
     float R[32];
 #pragma unroll
@@ -344,6 +352,7 @@ __device__ __forceinline__ void pipe_wait() {
 // memory; the warps are added in a fixed order into one partial per block.
 __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __restrict__ A, int lda, uint64_t m, int a,
                                                             double* __restrict__ part) {
+    dependent_start();
     extern __shared__ __align__(16) float ring[];  // [kPipe][128 rows][lda], then [16 warps][32][32] FP64
     double* dsum = reinterpret_cast<double*>(reinterpret_cast<uint8_t*>(ring) + kPipeRing);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -416,6 +425,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __re
 constexpr int kTrmulRows = 2;
 __global__ void __launch_bounds__(256) k_trmul_rows(float* __restrict__ A, int lda, uint64_t m, int a,
                                                     const double* __restrict__ Linv) {
+    dependent_start();
     __shared__ __align__(16) float Rt[32][32];  // Rt[k][c] = Linv[c][k], zero padded
     for (int e = threadIdx.x; e < 32 * 32; e += 256) {
         const int k = e >> 5, c = e & 31;
@@ -482,6 +492,7 @@ __global__ void __launch_bounds__(256) k_trmul_rows(float* __restrict__ A, int l
 // a fixed-shape tree (warp shuffles, then the four warps in order)
 __global__ void __launch_bounds__(128) k_sum_partials_wide(const double* __restrict__ part, int splits,
                                                            uint64_t count, double* __restrict__ out) {
+    dependent_start();
     __shared__ double ws[4];
     for (uint64_t e = blockIdx.x; e < count; e += gridDim.x) {
         double s = 0.0;
@@ -497,6 +508,7 @@ __global__ void __launch_bounds__(128) k_sum_partials_wide(const double* __restr
 
 __global__ void k_sum_partials(const double* __restrict__ part, int splits, uint64_t count,
                                double* __restrict__ out) {
+    dependent_start();
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < count;
          t += (uint64_t)gridDim.x * blockDim.x) {
         double s = 0.0;
@@ -510,6 +522,7 @@ template <typename TO>
 __global__ void k_gemm_small(const double* __restrict__ A, int lda, uint64_t m, int a,
                              const double* __restrict__ B, int ldb, int b, double alpha, double beta,
                              TO* __restrict__ C, int ldc) {
+    dependent_start();
     extern __shared__ double Bsm[];  // a x b
     for (int e = threadIdx.x; e < a * b; e += blockDim.x) Bsm[e] = B[(e / b) * ldb + (e % b)];
     __syncthreads();
@@ -532,6 +545,7 @@ __global__ void k_gemm_small(const double* __restrict__ A, int lda, uint64_t m, 
 template <int AMAX>
 __global__ void __launch_bounds__(128) k_trmul_f32(float* __restrict__ A, int lda, uint64_t m, int a,
                                                    const double* __restrict__ Linv) {
+    dependent_start();
     __shared__ float R[AMAX * AMAX];  // R[k][c] = Linv[c][k], zero padded
     for (int e = threadIdx.x; e < AMAX * AMAX; e += blockDim.x) {
         const int k = e / AMAX, cc = e % AMAX;
@@ -564,6 +578,7 @@ __global__ void __launch_bounds__(128) k_trmul_f32(float* __restrict__ A, int ld
 // (rank-deficient design columns).  status[0] counts replaced/dropped pivots.
 __global__ void k_cholesky(double* __restrict__ G, int a, int* __restrict__ status,
                            double drop_tol, int* __restrict__ dropped, double* __restrict__ work) {
+    dependent_start();
     extern __shared__ double S_sm[];
     double* S = work ? work : S_sm;   // global scratch for matrices wider than kMaxSmall
     __shared__ double piv;
@@ -607,6 +622,7 @@ __global__ void k_cholesky(double* __restrict__ G, int a, int* __restrict__ stat
 
 // Inverse of a lower-triangular matrix: one thread per column.
 __global__ void k_tri_inv_lower(const double* __restrict__ L, int a, double* __restrict__ X, int in_smem) {
+    dependent_start();
     extern __shared__ double S_sm[];
     const double* S = in_smem ? S_sm : L;   // matrices wider than kMaxSmall are read in place
     if (in_smem) {
@@ -644,6 +660,7 @@ template <int T, int R>
 __global__ void __launch_bounds__(T, 1) k_chol_inv(const double* __restrict__ G, int a, double* __restrict__ X,
                                                 int transposed, int* __restrict__ status, double drop_tol,
                                                 int* __restrict__ dropped) {
+    dependent_start();
     __shared__ double vec[2][kMaxDesign];  // step k's column below the diagonal, row up to it
     __shared__ double res[kMaxDesign];     // L_ik (i > k) and X_kj (j <= k)
     __shared__ double diag[kMaxDesign];
@@ -719,6 +736,7 @@ __global__ void __launch_bounds__(1024, 1) k_chol_inv_wide(const double* __restr
                                                            double* __restrict__ X, int transposed,
                                                            int* __restrict__ status, double drop_tol,
                                                            int* __restrict__ dropped) {
+    dependent_start();
     extern __shared__ double P[];          // packed lower triangle
     __shared__ double res[kMaxDesign];
     __shared__ double diag[kMaxDesign];
@@ -811,6 +829,7 @@ __device__ bool lu_smem(double* S, int* piv, int a) {
 // global memory) instead of shared memory.
 __global__ void k_inverse(const double* __restrict__ A, int a, double* __restrict__ X,
                           int* __restrict__ status, double* __restrict__ eps_used, double* __restrict__ work) {
+    dependent_start();
     extern __shared__ double S_sm[];
     __shared__ int piv_sm[kMaxSmall];
     double* S = work ? work : S_sm;
@@ -867,6 +886,7 @@ __global__ void k_inverse(const double* __restrict__ A, int a, double* __restric
 }
 
 __global__ void k_add_diag(double* __restrict__ A, int a, double v) {
+    dependent_start();
     for (int i = threadIdx.x; i < a; i += blockDim.x) A[i * a + i] += v;
 }
 
@@ -891,6 +911,7 @@ struct InverseJobs {
 };
 
 __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant__ InverseJobs jobs) {
+    dependent_start();
     extern __shared__ double S[];  // a x a
     __shared__ double f[kMaxGaussJordan], prow[kMaxGaussJordan];
     __shared__ int rowid[kMaxGaussJordan], from[kMaxGaussJordan];
@@ -1249,6 +1270,7 @@ __device__ void gs_columns(double* Vs, double* acc, int ap, double* dots) {
 template <int NC, int NR>
 __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, int a, double* __restrict__ V,
                                                         double* __restrict__ sig, double* ws) {
+    dependent_start();
     extern __shared__ double sm_dyn[];
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -1578,6 +1600,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
 }
 
 __global__ void k_normal(uint64_t seed, uint64_t total, double* __restrict__ out) {
+    dependent_start();
     const uint64_t key = mix64(seed + 0x9E3779B97F4A7C15ull);
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1591,6 +1614,7 @@ __global__ void k_normal(uint64_t seed, uint64_t total, double* __restrict__ out
 
 __global__ void k_f64_to_f32_pad(const double* __restrict__ A, uint64_t m, int a, int lda,
                                  float* __restrict__ out, uint64_t m_pad, int ldo) {
+    dependent_start();
     const uint64_t total = m_pad * ldo;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1602,6 +1626,7 @@ __global__ void k_f64_to_f32_pad(const double* __restrict__ A, uint64_t m, int a
 
 __global__ void k_f32_to_f64(const float* __restrict__ A, uint64_t m, int a, int lda,
                              double* __restrict__ out, int ldo) {
+    dependent_start();
     const uint64_t total = m * a;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1612,11 +1637,13 @@ __global__ void k_f32_to_f64(const float* __restrict__ A, uint64_t m, int a, int
 }
 
 __global__ void k_fill(double* __restrict__ x, uint64_t n, double v) {
+    dependent_start();
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x)
         x[t] = v;
 }
 
 __global__ void k_transpose(const double* __restrict__ A, int rows, int cols, double* __restrict__ At) {
+    dependent_start();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * cols; e += gridDim.x * blockDim.x) {
         const int i = e / cols, j = e % cols;
         At[j * rows + i] = A[e];
@@ -1625,6 +1652,7 @@ __global__ void k_transpose(const double* __restrict__ A, int rows, int cols, do
 
 __global__ void k_scale_cols(double* __restrict__ A, uint64_t m, int a, int lda,
                              const double* __restrict__ f) {
+    dependent_start();
     const uint64_t total = m * a;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -1637,6 +1665,7 @@ __global__ void k_scale_cols(double* __restrict__ A, uint64_t m, int a, int lda,
 // C = [1 | X | U] (n x (1+d+K))
 __global__ void k_build_design(const double* __restrict__ X, int d, const double* __restrict__ U, int K,
                                uint64_t n, double* __restrict__ C) {
+    dependent_start();
     const int w = 1 + d + K;
     const uint64_t total = n * w;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
@@ -1668,6 +1697,7 @@ __global__ void k_colsum_split(const double* __restrict__ A, uint64_t m, int a, 
 
 __global__ void k_mean_partials(const double* __restrict__ part, int splits, int a, uint64_t m,
                                 double* __restrict__ out) {
+    dependent_start();
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= a) return;
     double s = 0.0;
@@ -1678,16 +1708,16 @@ __global__ void k_mean_partials(const double* __restrict__ part, int splits, int
 void launch_colmeans(Ctx& c, const double* A, uint64_t m, int a, int lda, double* out) {
     if (a == 0) return;
     if (m <= 2 * kColRows) {
-        k_colmeans<<<a, 256, 0, c.stream>>>(A, m, lda, out, 1);
+        launch_next(c, k_colmeans, a, 256, 0, A, m, lda, out, 1);
         SLFMM_LAUNCHED(c, "k_colmeans");
         return;
     }
     const uint64_t splits = std::min<uint64_t>(ceil_div(m, kColRows), 512);
     const uint64_t per = ceil_div(m, splits);
     DBuf<double> part(splits * a, c.stream);
-    k_colsum_split<<<dim3(a, (unsigned)splits), 256, 0, c.stream>>>(A, m, a, lda, per, part.get());
+    launch_next(c, k_colsum_split, dim3(a, (unsigned)splits), 256, 0, A, m, a, lda, per, part.get());
     SLFMM_LAUNCHED(c, "k_colsum_split");
-    k_mean_partials<<<(unsigned)ceil_div((uint64_t)a, 128), 128, 0, c.stream>>>(part.get(), (int)splits, a, m,
+    launch_next(c, k_mean_partials, (unsigned)ceil_div((uint64_t)a, 128), 128, 0, part.get(), (int)splits, a, m,
                                                                                  out);
     SLFMM_LAUNCHED(c, "k_mean_partials");
 }
@@ -1696,6 +1726,7 @@ void launch_colmeans(Ctx& c, const double* A, uint64_t m, int a, int lda, double
 // the partials summed in order
 __global__ void k_colsum_split(const double* __restrict__ A, uint64_t m, int a, int lda, uint64_t per,
                                double* __restrict__ part) {
+    dependent_start();
     __shared__ double red[32];
     const int col = blockIdx.x;
     const uint64_t r0 = (uint64_t)blockIdx.y * per, r1 = min(m, r0 + per);
@@ -1708,14 +1739,14 @@ __global__ void k_colsum_split(const double* __restrict__ A, uint64_t m, int a, 
 void launch_colsums(Ctx& c, const double* A, uint64_t m, int a, int lda, double* out) {
     if (a == 0) return;
     if (m <= 2 * kColRows) {
-        k_colmeans<<<a, 256, 0, c.stream>>>(A, m, lda, out, 0);
+        launch_next(c, k_colmeans, a, 256, 0, A, m, lda, out, 0);
         SLFMM_LAUNCHED(c, "k_colsums");
         return;
     }
     const uint64_t splits = std::min<uint64_t>(ceil_div(m, m <= 65536 ? kColRows : 16384), 512);
     const uint64_t per = ceil_div(m, splits);
     DBuf<double> part(splits * a, c.stream);
-    k_colsum_split<<<dim3(a, (unsigned)splits), 256, 0, c.stream>>>(A, m, a, lda, per, part.get());
+    launch_next(c, k_colsum_split, dim3(a, (unsigned)splits), 256, 0, A, m, a, lda, per, part.get());
     SLFMM_LAUNCHED(c, "k_colsum_split");
     launch_sum_partials(c, part.get(), (int)splits, (uint64_t)a, out);
 }
@@ -1723,24 +1754,24 @@ void launch_colsums(Ctx& c, const double* A, uint64_t m, int a, int lda, double*
 void launch_sum_partials(Ctx& c, const double* part, int splits, uint64_t count, double* out) {
     if (!count) return;
     if (splits >= 32) {
-        k_sum_partials_wide<<<(unsigned)std::min<uint64_t>(count, 65535), 128, 0, c.stream>>>(part, splits, count,
+        launch_next(c, k_sum_partials_wide, (unsigned)std::min<uint64_t>(count, 65535), 128, 0, part, splits, count,
                                                                                              out);
         SLFMM_LAUNCHED(c, "k_sum_partials_wide");
         return;
     }
-    k_sum_partials<<<grid_for(c, count, 256), 256, 0, c.stream>>>(part, splits, count, out);
+    launch_next(c, k_sum_partials, grid_for(c, count, 256), 256, 0, part, splits, count, out);
     SLFMM_LAUNCHED(c, "k_sum_partials");
 }
 
 void launch_center_cols(Ctx& c, double* A, uint64_t m, int a, int lda, const double* means) {
     if (a == 0 || m == 0) return;
-    k_center_cols<<<grid_for(c, m * a, 256), 256, 0, c.stream>>>(A, m, a, lda, means);
+    launch_next(c, k_center_cols, grid_for(c, m * a, 256), 256, 0, A, m, a, lda, means);
     SLFMM_LAUNCHED(c, "k_center_cols");
 }
 
 void launch_scale_cols_sd(Ctx& c, double* A, uint64_t m, int a, int lda) {
     if (a == 0) return;
-    k_scale_cols_sd<<<a, 256, 0, c.stream>>>(A, m, lda);
+    launch_next(c, k_scale_cols_sd, a, 256, 0, A, m, lda);
     SLFMM_LAUNCHED(c, "k_scale_cols_sd");
 }
 
@@ -1764,7 +1795,7 @@ static void atb_impl(Ctx& c, const T* A, int lda, const T* B, int ldb, uint64_t 
 #define SLFMM_ATB_FLAT(RR)                                                                        \
     do {                                                                                          \
         raise_dynamic_smem((const void*)k_atb_flat<T, RR>, smem);                                 \
-        k_atb_flat<T, RR><<<grid, 256, smem, c.stream>>>(A, lda, B, ldb, m, a, b, per, part.get()); \
+        launch_next(c, k_atb_flat<T, RR>, grid, 256, smem, A, lda, B, ldb, m, a, b, per, part.get()); \
     } while (0)
         switch (R) {
             case 1: SLFMM_ATB_FLAT(1); break;
@@ -1786,7 +1817,7 @@ static void atb_impl(Ctx& c, const T* A, int lda, const T* B, int ldb, uint64_t 
     splits = std::max<uint64_t>(1, ceil_div(m, per));
     DBuf<double> part(splits * a * b, c.stream);
     dim3 grid(ta, tb, (unsigned)splits);
-    k_atb<T><<<grid, 256, 0, c.stream>>>(A, lda, B, ldb, m, a, b, per, part.get());
+    launch_next(c, k_atb<T>, grid, 256, 0, A, lda, B, ldb, m, a, b, per, part.get());
     SLFMM_LAUNCHED(c, "k_atb");
     launch_sum_partials(c, part.get(), (int)splits, (uint64_t)a * b, out);
 }
@@ -1804,7 +1835,7 @@ void launch_gram_f32(Ctx& c, const float* A, int lda, uint64_t m, int a, double*
             const size_t sm = kPipeRing + (size_t)(kPipeThreads / 32) * 32 * 32 * sizeof(double);
             DBuf<double> tpart(tb * a * a, c.stream);
             set_smem((const void*)k_gram_tile, sm);
-            k_gram_tile<<<(unsigned)tb, kPipeThreads, sm, c.stream>>>(A, lda, m, a, tpart.get());
+            launch_next(c, k_gram_tile, (unsigned)tb, kPipeThreads, sm, A, lda, m, a, tpart.get());
             SLFMM_LAUNCHED(c, "k_gram_tile");
             launch_sum_partials(c, tpart.get(), (int)tb, (uint64_t)a * a, out);
             return;
@@ -1813,7 +1844,7 @@ void launch_gram_f32(Ctx& c, const float* A, int lda, uint64_t m, int a, double*
         const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(runs, 8), (uint64_t)c.sm_count * 4));
         DBuf<double> part(blocks * a * a, c.stream);
         set_smem((const void*)k_gram_narrow, kGramNarrowSmem);
-        k_gram_narrow<<<(unsigned)blocks, 256, kGramNarrowSmem, c.stream>>>(A, lda, m, a, part.get());
+        launch_next(c, k_gram_narrow, (unsigned)blocks, 256, kGramNarrowSmem, A, lda, m, a, part.get());
         SLFMM_LAUNCHED(c, "k_gram_narrow");
         launch_sum_partials(c, part.get(), (int)blocks, (uint64_t)a * a, out);
         return;
@@ -1826,7 +1857,7 @@ void launch_gram_f32(Ctx& c, const float* A, int lda, uint64_t m, int a, double*
     splits = std::max<uint64_t>(1, ceil_div(m, per));
     DBuf<double> part(splits * a * a, c.stream);
     dim3 grid(ta, ta, (unsigned)splits);
-    k_gram_f32<<<grid, 256, 0, c.stream>>>(A, lda, m, a, per, part.get());
+    launch_next(c, k_gram_f32, grid, 256, 0, A, lda, m, a, per, part.get());
     SLFMM_LAUNCHED(c, "k_gram_f32");
     launch_sum_partials(c, part.get(), (int)splits, (uint64_t)a * a, out);
 }
@@ -1840,7 +1871,7 @@ void launch_gemm_small(Ctx& c, const double* A, int lda, uint64_t m, int a, cons
         const int nb = std::min(bb, b - c0);
         const size_t sm = (size_t)a * nb * sizeof(double);
         set_smem((const void*)k_gemm_small<double>, sm);
-        k_gemm_small<double><<<grid_for(c, m * nb, 256), 256, sm, c.stream>>>(A, lda, m, a, B + c0, ldb, nb, alpha,
+        launch_next(c, k_gemm_small<double>, grid_for(c, m * nb, 256), 256, sm, A, lda, m, a, B + c0, ldb, nb, alpha,
                                                                               beta, C + c0, ldc);
         SLFMM_LAUNCHED(c, "k_gemm_small");
     }
@@ -1851,15 +1882,16 @@ void launch_trmul_f32(Ctx& c, float* A, int lda, uint64_t m, int a, const double
     if (m == 0) return;
     if (a <= 32) {
         if (narrow_tiled(A, lda)) {
-            k_trmul_rows<<<grid_for(c, ceil_div(m, (uint64_t)kTrmulRows), 256), 256, 0, c.stream>>>(A, lda, m, a, Linv);
+            launch_next(c, k_trmul_rows, grid_for(c, ceil_div(m, (uint64_t)kTrmulRows), 256), 256, 0, A, lda, m, a,
+                        Linv);
             SLFMM_LAUNCHED(c, "k_trmul_rows");
             return;
         }
-        k_trmul_narrow<<<grid_for(c, m, 32), 256, 0, c.stream>>>(A, lda, m, a, Linv);
+        launch_next(c, k_trmul_narrow, grid_for(c, m, 32), 256, 0, A, lda, m, a, Linv);
         SLFMM_LAUNCHED(c, "k_trmul_narrow");
         return;
     }
-    k_trmul_f32<64><<<grid_for(c, m, 128), 128, 0, c.stream>>>(A, lda, m, a, Linv);
+    launch_next(c, k_trmul_f32<64>, grid_for(c, m, 128), 128, 0, A, lda, m, a, Linv);
     SLFMM_LAUNCHED(c, "k_trmul_f32");
 }
 
@@ -1869,10 +1901,10 @@ void launch_cholesky(Ctx& c, double* A, int a, int* status, double drop_tol, int
     SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the small Cholesky");
     if (a <= kMaxSmall) {
         set_smem((const void*)k_cholesky, smem_sq(a));
-        k_cholesky<<<1, 512, smem_sq(a), c.stream>>>(A, a, status, drop_tol, dropped, nullptr);
+        launch_next(c, k_cholesky, 1, 512, smem_sq(a), A, a, status, drop_tol, dropped, nullptr);
     } else {
         DBuf<double> work((size_t)a * a, c.stream);
-        k_cholesky<<<1, 1024, 0, c.stream>>>(A, a, status, drop_tol, dropped, work.get());
+        launch_next(c, k_cholesky, 1, 1024, 0, A, a, status, drop_tol, dropped, work.get());
     }
     SLFMM_LAUNCHED(c, "k_cholesky");
 }
@@ -1885,7 +1917,7 @@ void launch_chol_inv(Ctx& c, const double* G, int a, double* X, bool transposed,
     SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the small Cholesky");
     if (a < 1) return;
     const int ne = a * (a + 1) / 2, tr = transposed ? 1 : 0;
-#define SLFMM_CHOL_INV(T, R) k_chol_inv<T, R><<<1, T, 0, c.stream>>>(G, a, X, tr, status, drop_tol, dropped)
+#define SLFMM_CHOL_INV(T, R) launch_next(c, k_chol_inv<T, R>, 1, T, 0, G, a, X, tr, status, drop_tol, dropped)
     if (ne <= 256) SLFMM_CHOL_INV(256, 1);
     else if (ne <= 256 * 2) SLFMM_CHOL_INV(256, 2);
     else if (ne <= 256 * 4) SLFMM_CHOL_INV(256, 4);
@@ -1894,7 +1926,7 @@ void launch_chol_inv(Ctx& c, const double* G, int a, double* X, bool transposed,
     else if (ne * sizeof(double) <= 220 * 1024) {
         const size_t sm = ne * sizeof(double);
         set_smem((const void*)k_chol_inv_wide, sm);
-        k_chol_inv_wide<<<1, 1024, sm, c.stream>>>(G, a, X, tr, status, drop_tol, dropped);
+        launch_next(c, k_chol_inv_wide, 1, 1024, sm, G, a, X, tr, status, drop_tol, dropped);
     } else {
         DBuf<double> L((size_t)a * a, c.stream), lower((size_t)a * a, c.stream);
         SLFMM_CUDA(cudaMemcpyAsync(L.get(), G, (size_t)a * a * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
@@ -1911,7 +1943,7 @@ void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv) {
     SLFMM_REQUIRE(a <= kMaxDesign, SLFMM_ERR_BAD_ARG, "matrix too large for the triangular inverse");
     const bool sm = a <= kMaxSmall;
     if (sm) set_smem((const void*)k_tri_inv_lower, smem_sq(a));
-    k_tri_inv_lower<<<1, sm ? 128 : 256, sm ? smem_sq(a) : 0, c.stream>>>(L, a, Linv, sm ? 1 : 0);
+    launch_next(c, k_tri_inv_lower, 1, sm ? 128 : 256, sm ? smem_sq(a) : 0, L, a, Linv, sm ? 1 : 0);
     SLFMM_LAUNCHED(c, "k_tri_inv_lower");
 }
 
@@ -1936,7 +1968,7 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
         }
     if (m) {
         set_smem((const void*)k_inverse_jobs, smem_sq(amax));
-        k_inverse_jobs<<<m, 1024, smem_sq(amax), c.stream>>>(js);
+        launch_next(c, k_inverse_jobs, m, 1024, smem_sq(amax), js);
         SLFMM_LAUNCHED(c, "k_inverse_jobs");
     }
     for (int i = 0; i < n; ++i) {
@@ -1947,7 +1979,7 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
         if (j.shift != 0.0) {
             A.alloc((size_t)j.a * j.a, c.stream);
             SLFMM_CUDA(cudaMemcpyAsync(A.get(), j.A, A.bytes(), cudaMemcpyDeviceToDevice, c.stream));
-            k_add_diag<<<1, 256, 0, c.stream>>>(A.get(), j.a, j.shift);
+            launch_next(c, k_add_diag, 1, 256, 0, A.get(), j.a, j.shift);
             SLFMM_LAUNCHED(c, "k_add_diag");
             src = A.get();
         }
@@ -1958,10 +1990,10 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
         }
         if (j.a <= kMaxSmall) {
             set_smem((const void*)k_inverse, smem_sq(j.a));
-            k_inverse<<<1, 256, smem_sq(j.a), c.stream>>>(src, j.a, x, j.status, j.eps, nullptr);
+            launch_next(c, k_inverse, 1, 256, smem_sq(j.a), src, j.a, x, j.status, j.eps, nullptr);
         } else {
             DBuf<double> work((size_t)j.a * j.a + (size_t)(j.a + 1) / 2, c.stream);  // matrix, then a pivot ints
-            k_inverse<<<1, 1024, 0, c.stream>>>(src, j.a, x, j.status, j.eps, work.get());
+            launch_next(c, k_inverse, 1, 1024, 0, src, j.a, x, j.status, j.eps, work.get());
         }
         SLFMM_LAUNCHED(c, "k_inverse");
     }
@@ -1982,22 +2014,24 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
         // a warp per pair of columns, in fours, and those of Gram-Schmidt
         const int threads = std::max(256, (int)round_up(32 * (uint64_t)(ap / 2), 128));
         static_assert(kEighOneCta <= 32 && 3 * 32 * 32 * sizeof(double) + (20 << 10) <= (48 << 10), "");
-        k_jacobi_svd<1, 1><<<1, threads, 3 * square, c.stream>>>(const_cast<double*>(A), a, V, sig, nullptr);
+        launch_next(c, k_jacobi_svd<1, 1>, 1, threads, 3 * square, const_cast<double*>(A), a, V, sig, nullptr);
     } else {
         DBuf<double> ws(3 * (size_t)ap * ap, c.stream);
         const size_t share = 2 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
         const size_t sm = 2 * square <= kEighClusterSmem ? std::max(2 * square, share) : share;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = kEighCluster;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchAttribute at[2] = {};
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kEighCluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3(kEighCluster);
         lc.blockDim = dim3(1024);
         lc.dynamicSmemBytes = sm;
         lc.stream = c.stream;
-        lc.attrs = &at;
-        lc.numAttrs = 1;
+        lc.attrs = at;
+        lc.numAttrs = 2;
         auto go = [&](auto kern) {
             set_smem((const void*)kern, std::max(sm, kEighLimit));
             SLFMM_CUDA(cudaLaunchKernelEx(&lc, kern, const_cast<double*>(A), a, V, sig, ws.get()));
@@ -2011,45 +2045,45 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
 
 void launch_fill(Ctx& c, double* x, uint64_t n, double v) {
     if (!n) return;
-    k_fill<<<grid_for(c, n, 256), 256, 0, c.stream>>>(x, n, v);
+    launch_next(c, k_fill, grid_for(c, n, 256), 256, 0, x, n, v);
     SLFMM_LAUNCHED(c, "k_fill");
 }
 
 void launch_transpose(Ctx& c, const double* A, int rows, int cols, double* At) {
     if (!rows || !cols) return;
-    k_transpose<<<grid_for(c, (uint64_t)rows * cols, 256), 256, 0, c.stream>>>(A, rows, cols, At);
+    launch_next(c, k_transpose, grid_for(c, (uint64_t)rows * cols, 256), 256, 0, A, rows, cols, At);
     SLFMM_LAUNCHED(c, "k_transpose");
 }
 
 void launch_scale_cols(Ctx& c, double* A, uint64_t m, int a, int lda, const double* f) {
     if (!m || !a) return;
-    k_scale_cols<<<grid_for(c, m * a, 256), 256, 0, c.stream>>>(A, m, a, lda, f);
+    launch_next(c, k_scale_cols, grid_for(c, m * a, 256), 256, 0, A, m, a, lda, f);
     SLFMM_LAUNCHED(c, "k_scale_cols");
 }
 
 void launch_build_design(Ctx& c, const double* X, int d, const double* U, int K, uint64_t n, double* C) {
     if (!n) return;
-    k_build_design<<<grid_for(c, n * (1 + d + K), 256), 256, 0, c.stream>>>(X, d, U, K, n, C);
+    launch_next(c, k_build_design, grid_for(c, n * (1 + d + K), 256), 256, 0, X, d, U, K, n, C);
     SLFMM_LAUNCHED(c, "k_build_design");
 }
 
 void launch_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
     const uint64_t total = rows * cols;
     if (!total) return;
-    k_normal<<<grid_for(c, total, 256), 256, 0, c.stream>>>(seed, total, out);
+    launch_next(c, k_normal, grid_for(c, total, 256), 256, 0, seed, total, out);
     SLFMM_LAUNCHED(c, "k_normal");
 }
 
 void launch_f64_to_f32_pad(Ctx& c, const double* A, uint64_t m, int a, int lda, float* out,
                            uint64_t m_pad, int ldo) {
     if (!m_pad || !ldo) return;
-    k_f64_to_f32_pad<<<grid_for(c, m_pad * ldo, 256), 256, 0, c.stream>>>(A, m, a, lda, out, m_pad, ldo);
+    launch_next(c, k_f64_to_f32_pad, grid_for(c, m_pad * ldo, 256), 256, 0, A, m, a, lda, out, m_pad, ldo);
     SLFMM_LAUNCHED(c, "k_f64_to_f32_pad");
 }
 
 void launch_f32_to_f64(Ctx& c, const float* A, uint64_t m, int a, int lda, double* out, int ldo) {
     if (!m || !a) return;
-    k_f32_to_f64<<<grid_for(c, m * a, 256), 256, 0, c.stream>>>(A, m, a, lda, out, ldo);
+    launch_next(c, k_f32_to_f64, grid_for(c, m * a, 256), 256, 0, A, m, a, lda, out, ldo);
     SLFMM_LAUNCHED(c, "k_f32_to_f64");
 }
 

@@ -57,6 +57,7 @@ __device__ __forceinline__ uint32_t bf16_of_code(uint32_t c) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_tc_rows(const __grid_constant__ CUtensorMap tm_packed, const __grid_constant__ CUtensorMap tm_b, TcArgs a) {
+    dependent_wait();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t S = a.stages, N = 2 * a.wpad;
@@ -195,6 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 template <typename T>
 __global__ void k_split_bf16(const T* __restrict__ src, int ld, uint64_t K, int w, int wpad, uint64_t K_pad,
                              const double* __restrict__ kscale, __nv_bfloat16* __restrict__ dst) {
+    dependent_wait();
     __shared__ float tile[64][33];
     const uint64_t k0 = (uint64_t)blockIdx.x * 64;
     const int c0 = blockIdx.y * 32;
@@ -228,6 +230,7 @@ __global__ void k_split_bf16(const T* __restrict__ src, int ld, uint64_t K, int 
 // Transposed 2-bit matrix: row i (sample) holds the codes of every SNP.
 __global__ void k_transpose_packed(const uint8_t* __restrict__ in, uint64_t p, uint64_t stride, uint64_t n,
                                    uint8_t* __restrict__ out, uint64_t strideT) {
+    dependent_wait();
     __shared__ uint8_t tile[128][33];
     const uint64_t j0 = (uint64_t)blockIdx.x * 128;  // SNPs
     const uint64_t i0 = (uint64_t)blockIdx.y * 128;  // samples
@@ -259,6 +262,7 @@ __global__ void k_rowfix_mean(float* __restrict__ P, int ldp, uint64_t rows, int
                               const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ idx,
                               const float* __restrict__ W, int ldw, const double* __restrict__ cs,
                               const double* __restrict__ mean, const double* __restrict__ scale) {
+    dependent_wait();
     const uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (j >= rows) return;
@@ -303,6 +307,7 @@ __global__ void __launch_bounds__(256, 8) k_rowfix_mean4(float* __restrict__ P, 
                                const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ idx,
                                const float* __restrict__ W, int ldw, const double* __restrict__ cs,
                                const double* __restrict__ mean, const double* __restrict__ scale) {
+    dependent_wait();
     constexpr int G = 32 / L;  // missing calls per warp step
     const uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31, q = lane % L, grp = lane / L;
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(256) k_colfix_mean(double* __restrict__ S, int
                                                      const uint32_t* __restrict__ idx, const float* __restrict__ Q,
                                                      int ldq, const double* __restrict__ coef,
                                                      const double* __restrict__ colterm) {
+    dependent_wait();
     constexpr int kRows = 32 / NQ;
     const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
@@ -426,6 +432,7 @@ __global__ void __launch_bounds__(256) k_colfix_mean(double* __restrict__ S, int
 template <int T>
 __global__ void __launch_bounds__(256) k_weighted_colsum(const float* __restrict__ Q, int ldq, uint64_t p, int w,
                                                          const double* __restrict__ coef, double* __restrict__ part) {
+    dependent_start();
     __shared__ double red[8][32 * T];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc[T];
@@ -468,6 +475,7 @@ __global__ void __launch_bounds__(256) k_weighted_colsum(const float* __restrict
 __global__ void __launch_bounds__(256) k_weighted_colsum_quads(const float* __restrict__ Q, int ldq, uint64_t p,
                                                                int w, const double* __restrict__ coef,
                                                                double* __restrict__ part) {
+    dependent_start();
     const int q = ldq >> 2;  // 1, 2, 4 or 8 quads per row
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x / q;
@@ -522,6 +530,7 @@ __global__ void __launch_bounds__(256) k_weighted_colsum_quads(const float* __re
 
 __global__ void k_scale_product(const double* __restrict__ a, const double* __restrict__ b, uint64_t n,
                                 double* __restrict__ out) {
+    dependent_wait();
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x)
         out[t] = a[t] * b[t];
 }
@@ -610,14 +619,14 @@ bool tc_available(Ctx& c) { return c.precision == SLFMM_PREC_SPLIT_BF16; }
 void launch_split_bf16_f64(Ctx& c, const double* src, int ld, uint64_t K, int w, int wpad, uint64_t K_pad,
                            const double* kscale, __nv_bfloat16* dst) {
     dim3 grid((unsigned)ceil_div(K_pad, 64), (unsigned)ceil_div(wpad, 32));
-    k_split_bf16<double><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, K_pad, kscale, dst);
+    launch_next(c, k_split_bf16<double>, grid, 256, 0, src, ld, K, w, wpad, K_pad, kscale, dst);
     SLFMM_LAUNCHED(c, "k_split_bf16");
 }
 
 void launch_split_bf16_f32(Ctx& c, const float* src, int ld, uint64_t K, int w, int wpad, uint64_t K_pad,
                            const double* kscale, __nv_bfloat16* dst) {
     dim3 grid((unsigned)ceil_div(K_pad, 64), (unsigned)ceil_div(wpad, 32));
-    k_split_bf16<float><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, K_pad, kscale, dst);
+    launch_next(c, k_split_bf16<float>, grid, 256, 0, src, ld, K, w, wpad, K_pad, kscale, dst);
     SLFMM_LAUNCHED(c, "k_split_bf16");
 }
 
@@ -627,7 +636,7 @@ void build_transposed(Ctx& c, const Geno& g) {
     g.packedT.alloc(g.n * g.strideT, c.stream);
     SLFMM_CUDA(cudaMemsetAsync(g.packedT.get(), 0, g.n * g.strideT, c.stream));
     dim3 grid((unsigned)ceil_div(g.p, 128), (unsigned)ceil_div(g.n, 128));
-    k_transpose_packed<<<grid, 256, 0, c.stream>>>(packed_rows(g), g.p, g.stride, g.n, g.packedT.get(), g.strideT);
+    launch_next(c, k_transpose_packed, grid, 256, 0, packed_rows(g), g.p, g.stride, g.n, g.packedT.get(), g.strideT);
     SLFMM_LAUNCHED(c, "k_transpose_packed");
     g.have_T = true;
 }
@@ -663,7 +672,7 @@ int launch_tc_rows(Ctx& c, const uint8_t* packed, uint64_t stride, uint64_t rows
     a.err = err.get();
     const unsigned gy = (unsigned)ceil_div(a.kb_total, a.kb_per_split);
     dim3 grid((unsigned)ceil_div(rows, kM), gy);
-    k_tc_rows<<<grid, kThreads, pl.smem, c.stream>>>(tp, tb, a);
+    launch_next(c, k_tc_rows, grid, kThreads, pl.smem, tp, tb, a);
     SLFMM_LAUNCHED(c, "k_tc_rows");
     check_err(c, err);
     return (int)gy;
@@ -698,7 +707,7 @@ void launch_rowfix_mean(Ctx& c, float* P, int ldp, uint64_t rows, int w, const u
             const int nq = (wb + 3) / 4;
             const unsigned grid = (unsigned)ceil_div(rows * 32, 256);
 #define SLFMM_ROWFIX4(LL)                                                                                     \
-    k_rowfix_mean4<LL><<<grid, 256, 0, c.stream>>>(P + c0, ldp, rows, wb, ptr, idx, W + c0, ldw, cs + c0, mean, \
+    launch_next(c, k_rowfix_mean4<LL>, grid, 256, 0, P + c0, ldp, rows, wb, ptr, idx, W + c0, ldw, cs + c0, mean, \
                                                    scale)
             if (nq <= 1) SLFMM_ROWFIX4(1);
             else if (nq <= 2) SLFMM_ROWFIX4(2);
@@ -711,7 +720,7 @@ void launch_rowfix_mean(Ctx& c, float* P, int ldp, uint64_t rows, int w, const u
             continue;
         }
         // a warp covers 128 columns (4 per lane): wider operands in column blocks
-        k_rowfix_mean<<<(unsigned)ceil_div(rows * 32, 256), 256, 0, c.stream>>>(
+        launch_next(c, k_rowfix_mean, (unsigned)ceil_div(rows * 32, 256), 256, 0, 
             P + c0, ldp, rows, std::min(128, w - c0), ptr, idx, W + c0, ldw, cs + c0, mean, scale);
         SLFMM_LAUNCHED(c, "k_rowfix_mean");
         c0 += 128;
@@ -722,7 +731,7 @@ void launch_colfix_mean(Ctx& c, double* S, int lds, uint64_t n, int w, const uin
                         const float* Q, int ldq, const double* coef, const double* colterm) {
     if (!n) return;
     auto go = [&](auto kern) {
-        kern<<<(unsigned)ceil_div(n * 32, 256), 256, 0, c.stream>>>(S, lds, n, w, ptr, idx, Q, ldq, coef, colterm);
+        launch_next(c, kern, (unsigned)ceil_div(n * 32, 256), 256, 0, S, lds, n, w, ptr, idx, Q, ldq, coef, colterm);
     };
     SLFMM_REQUIRE(w <= 64, SLFMM_ERR_BAD_ARG, "width");  // a sketch's
     if (w <= 32) go(k_colfix_mean<1>);
@@ -736,23 +745,23 @@ void launch_weighted_colsum(Ctx& c, const float* Q, int ldq, uint64_t p, int w, 
         const uint64_t qb = std::max<uint64_t>(
             1, std::min<uint64_t>(ceil_div(p * (uint64_t)(ldq / 4), 1024), (uint64_t)c.sm_count * 4));
         DBuf<double> qpart(qb * w, c.stream);
-        k_weighted_colsum_quads<<<(unsigned)qb, 256, 0, c.stream>>>(Q, ldq, p, w, coef, qpart.get());
+        launch_next(c, k_weighted_colsum_quads, (unsigned)qb, 256, 0, Q, ldq, p, w, coef, qpart.get());
         SLFMM_LAUNCHED(c, "k_weighted_colsum_quads");
         launch_sum_partials(c, qpart.get(), (int)qb, (uint64_t)w, out);
         return;
     }
     const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(p, 256), (uint64_t)c.sm_count * 4));
     DBuf<double> part(blocks * w, c.stream);
-    if (w <= 32) k_weighted_colsum<1><<<(unsigned)blocks, 256, 0, c.stream>>>(Q, ldq, p, w, coef, part.get());
-    else if (w <= 64) k_weighted_colsum<2><<<(unsigned)blocks, 256, 0, c.stream>>>(Q, ldq, p, w, coef, part.get());
-    else k_weighted_colsum<4><<<(unsigned)blocks, 256, 0, c.stream>>>(Q, ldq, p, w, coef, part.get());
+    if (w <= 32) launch_next(c, k_weighted_colsum<1>, (unsigned)blocks, 256, 0, Q, ldq, p, w, coef, part.get());
+    else if (w <= 64) launch_next(c, k_weighted_colsum<2>, (unsigned)blocks, 256, 0, Q, ldq, p, w, coef, part.get());
+    else launch_next(c, k_weighted_colsum<4>, (unsigned)blocks, 256, 0, Q, ldq, p, w, coef, part.get());
     SLFMM_LAUNCHED(c, "k_weighted_colsum");
     launch_sum_partials(c, part.get(), (int)blocks, (uint64_t)w, out);
 }
 
 void launch_scale_product(Ctx& c, const double* a, const double* b, uint64_t n, double* out) {
     if (!n) return;
-    k_scale_product<<<grid_for(c, n, 256), 256, 0, c.stream>>>(a, b, n, out);
+    launch_next(c, k_scale_product, grid_for(c, n, 256), 256, 0, a, b, n, out);
     SLFMM_LAUNCHED(c, "k_scale_product");
 }
 

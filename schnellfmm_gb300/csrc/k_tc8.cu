@@ -381,6 +381,7 @@ __device__ __forceinline__ void read_terms(const Tc8Args& a, uint32_t d0, const 
 // (d_empty).  A unit's accumulation order depends only on its tile and
 // split, so every grid gives the same bits.
 __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant__ Tc8Args a) {
+    dependent_wait();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t S = a.slots, SW = a.wstages, P = a.pstages;
@@ -611,6 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc8_rows(const __grid_constant_
 template <typename T>
 __global__ void __launch_bounds__(256) k_colmax_abs(const T* __restrict__ src, int ld, uint64_t K, int w,
                                                     const double* __restrict__ kscale, unsigned* __restrict__ colmax) {
+    dependent_start();
     __shared__ unsigned red[128];
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 128) red[threadIdx.x] = 0u;
@@ -678,6 +680,7 @@ struct TermSet {
 __global__ void __launch_bounds__(256) k_colmax_pair(const float* __restrict__ src, int ld, uint64_t K, int w,
                                                      const double* __restrict__ ksa, const double* __restrict__ ksb,
                                                      unsigned* __restrict__ cma, unsigned* __restrict__ cmb) {
+    dependent_start();
     const int q = ld >> 2;  // quads per row: 1, 2, 4 or 8 (divides the thread count)
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
@@ -759,6 +762,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_fp8_terms(const T* __restrict__ src, int ld, uint64_t K, int w, int wpad,
                                                    TermSet sa, TermSet sb, int n_rows, uint8_t* __restrict__ B,
                                                    float* __restrict__ inv_scale) {
+    dependent_start();
     constexpr int kT = kMainTerms + kIndTerms;
     __shared__ uint4 tile[kT][2][kTermCols][8];
     __shared__ float ks[2][kStageK];
@@ -826,6 +830,7 @@ __global__ void __launch_bounds__(256) k_fp8_terms(const T* __restrict__ src, in
 }
 
 __global__ void k_sub_colterm(double* __restrict__ S, int lds, uint64_t n, int w, const double* __restrict__ colterm) {
+    dependent_start();
     const uint64_t total = n * w;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t i = t / w;
@@ -917,6 +922,7 @@ Fp8Plan fp8_plan(int wpad, bool ind, uint64_t tiles, bool ind_shared) {
 // 32-byte sector
 __global__ void k_tile_rows(const uint8_t* __restrict__ in, uint64_t rows, uint64_t stride, uint64_t kbt,
                             uint64_t chunks, uint8_t* __restrict__ out) {
+    dependent_wait();
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < chunks;
          e += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t h = e & 1u, r = (e >> 1) & 127u, rest = e >> 8;
@@ -938,6 +944,7 @@ __global__ void __launch_bounds__(256) k_transpose_tiles(const uint8_t* __restri
                                                          uint64_t ntiles_src, uint8_t* __restrict__ dst,
                                                          uint64_t kbt_dst, uint64_t ntiles_dst, uint64_t kb_lo,
                                                          uint64_t kb_hi) {
+    dependent_wait();
     __shared__ __align__(16) uint8_t in[128 * 32];
     const uint64_t nk = kb_hi - kb_lo;  // output K blocks [kb_lo, kb_hi) of every sample tile
     const uint64_t nblocks = ntiles_dst * nk;
@@ -973,6 +980,7 @@ __global__ void __launch_bounds__(256) k_transpose_tiles(const uint8_t* __restri
 // per 16 bytes (two per 32-byte tile row).
 __global__ void k_gather_tile_rows(const uint8_t* __restrict__ src, uint64_t kbt, const uint32_t* __restrict__ keep,
                                    uint64_t n_keep, uint64_t ntiles_dst, uint8_t* __restrict__ dst) {
+    dependent_wait();
     const uint64_t total = ntiles_dst * kbt * 256;
     const uint4* s4 = reinterpret_cast<const uint4*>(src);
     uint4* d4 = reinterpret_cast<uint4*>(dst);
@@ -994,6 +1002,7 @@ __global__ void k_gather_tile_rows(const uint8_t* __restrict__ src, uint64_t kbt
 // K blocks of its tile row; counts as k_snp_counts (c0 = n - c1 - c2 - cm).
 __global__ void k_snp_counts_tiles(const uint8_t* __restrict__ tiles, uint64_t kbt, uint64_t p, uint64_t n,
                                    int32_t* __restrict__ counts) {
+    dependent_wait();
     constexpr uint32_t kLo2 = 0x55555555u;
     const uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
@@ -1032,6 +1041,7 @@ __global__ void k_snp_counts_tiles(const uint8_t* __restrict__ tiles, uint64_t k
 // lanes by a warp scan of the per-lane counts.
 __global__ void k_miss_fill_tiles(const uint8_t* __restrict__ tiles, uint64_t kbt, uint64_t p,
                                   const uint64_t* __restrict__ ptr, uint32_t* __restrict__ idx) {
+    dependent_wait();
     constexpr uint32_t kLo2 = 0x55555555u;
     const uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
@@ -1075,20 +1085,21 @@ __global__ void k_miss_fill_tiles(const uint8_t* __restrict__ tiles, uint64_t kb
 }
 
 __global__ void k_miss_counts_of(const int32_t* __restrict__ counts, uint64_t p, uint64_t* __restrict__ mc) {
+    dependent_wait();
     for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < p; j += (uint64_t)gridDim.x * blockDim.x)
         mc[j] = (uint64_t)counts[j * 4 + 3];
 }
 
 void launch_miss_counts_of(Ctx& c, const Geno& g, uint64_t* mc) {
     if (!g.p) return;
-    k_miss_counts_of<<<grid_for(c, g.p, 256), 256, 0, c.stream>>>(g.counts.get(), g.p, mc);
+    launch_next(c, k_miss_counts_of, grid_for(c, g.p, 256), 256, 0, g.counts.get(), g.p, mc);
     SLFMM_LAUNCHED(c, "k_miss_counts_of");
 }
 
 void launch_miss_fill_tiles(Ctx& c, const Geno& g) {
     SLFMM_REQUIRE(g.have_tiles, SLFMM_ERR_BAD_ARG, "this matrix has neither a row-major copy nor SNP-major tiles");
     if (!g.p) return;
-    k_miss_fill_tiles<<<(unsigned)ceil_div(g.p * 32, 256), 256, 0, c.stream>>>(g.tiles.get(), g.kbt, g.p,
+    launch_next(c, k_miss_fill_tiles, (unsigned)ceil_div(g.p * 32, 256), 256, 0, g.tiles.get(), g.kbt, g.p,
                                                                                g.miss_ptr.get(), g.miss_idx.get());
     SLFMM_LAUNCHED(c, "k_miss_fill_tiles");
 }
@@ -1101,7 +1112,7 @@ static void tile_rows(Ctx& c, const uint8_t* in, uint64_t rows, uint64_t stride,
     const uint64_t bytes = ntiles * kbt * kTileBytes;
     out.alloc(bytes, c.stream);
     const uint64_t chunks = bytes / 16;
-    k_tile_rows<<<grid_for(c, chunks, 256), 256, 0, c.stream>>>(in, rows, stride, kbt, chunks, out.get());
+    launch_next(c, k_tile_rows, grid_for(c, chunks, 256), 256, 0, in, rows, stride, kbt, chunks, out.get());
     SLFMM_LAUNCHED(c, "k_tile_rows");
 }
 
@@ -1121,14 +1132,14 @@ void tile_chunk(Ctx& c, const Geno& g, uint64_t r0, uint64_t r1, bool last) {
     }
     const uint64_t t0 = r0 / kM, t1 = last ? g.ntiles : ceil_div(r1, kM);
     const uint64_t chunks = (t1 - t0) * g.kbt * (kTileBytes / 16);
-    k_tile_rows<<<grid_for(c, chunks, 256), 256, 0, c.stream>>>(packed_rows(g) + r0 * g.stride, r1 - r0, g.stride,
+    launch_next(c, k_tile_rows, grid_for(c, chunks, 256), 256, 0, packed_rows(g) + r0 * g.stride, r1 - r0, g.stride,
                                                                  g.kbt, chunks,
                                                                  g.tiles.get() + t0 * g.kbt * kTileBytes);
     SLFMM_LAUNCHED(c, "k_tile_rows");
     const uint64_t k1 = last ? g.kbtT : std::min(g.kbtT, ceil_div(r1, kM));
     if (k1 > t0) {
         const uint64_t blocks = std::min<uint64_t>(g.ntilesT * (k1 - t0), (uint64_t)c.sm_count * 16);
-        k_transpose_tiles<<<(unsigned)blocks, 256, 0, c.stream>>>(g.tiles.get(), g.kbt, g.ntiles, g.tilesT.get(),
+        launch_next(c, k_transpose_tiles, (unsigned)blocks, 256, 0, g.tiles.get(), g.kbt, g.ntiles, g.tilesT.get(),
                                                                    g.kbtT, g.ntilesT, t0, k1);
         SLFMM_LAUNCHED(c, "k_transpose_tiles");
     }
@@ -1146,7 +1157,7 @@ void tiles_subset_samples(Ctx& c, const Geno& full, const uint32_t* keep_dev, ui
     sub.ntilesT = round_up(std::max<uint64_t>(ceil_div(n_keep, kM), 1), 8);
     sub.tilesT.alloc(sub.ntilesT * sub.kbtT * kTileBytes, c.stream);
     const uint64_t rows16 = sub.ntilesT * sub.kbtT * 256;
-    k_gather_tile_rows<<<grid_for(c, rows16, 256), 256, 0, c.stream>>>(full.tilesT.get(), full.kbtT, keep_dev, n_keep,
+    launch_next(c, k_gather_tile_rows, grid_for(c, rows16, 256), 256, 0, full.tilesT.get(), full.kbtT, keep_dev, n_keep,
                                                                        sub.ntilesT, sub.tilesT.get());
     SLFMM_LAUNCHED(c, "k_gather_tile_rows");
     // SNP-major: the 2-bit transpose of those blocks
@@ -1154,13 +1165,14 @@ void tiles_subset_samples(Ctx& c, const Geno& full, const uint32_t* keep_dev, ui
     sub.ntiles = round_up(std::max<uint64_t>(ceil_div(sub.p, kM), 1), 8);
     sub.tiles.alloc(sub.ntiles * sub.kbt * kTileBytes, c.stream);
     const uint64_t blocks = std::min<uint64_t>(sub.ntiles * sub.kbt, (uint64_t)c.sm_count * 16);
-    k_transpose_tiles<<<(unsigned)blocks, 256, 0, c.stream>>>(sub.tilesT.get(), sub.kbtT, sub.ntilesT, sub.tiles.get(),
+    launch_next(c, k_transpose_tiles, (unsigned)blocks, 256, 0, sub.tilesT.get(), sub.kbtT, sub.ntilesT,
+                sub.tiles.get(),
                                                                sub.kbt, sub.ntiles, 0, sub.kbt);
     SLFMM_LAUNCHED(c, "k_transpose_tiles");
     sub.have_tiles = sub.have_tilesT = true;
     sub.counts.alloc(std::max<uint64_t>(sub.p, 1) * 4, c.stream);
     if (sub.p) {
-        k_snp_counts_tiles<<<(unsigned)ceil_div(sub.p * 32, 256), 256, 0, c.stream>>>(sub.tiles.get(), sub.kbt, sub.p,
+        launch_next(c, k_snp_counts_tiles, (unsigned)ceil_div(sub.p * 32, 256), 256, 0, sub.tiles.get(), sub.kbt, sub.p,
                                                                                       sub.n, sub.counts.get());
         SLFMM_LAUNCHED(c, "k_snp_counts_tiles");
     }
@@ -1181,7 +1193,7 @@ TileView build_tiles(Ctx& c, const Geno& g, bool transposed) {
         g.ntilesT = round_up(std::max<uint64_t>(ceil_div(g.n, kM), 1), 8);
         g.tilesT.alloc(g.ntilesT * g.kbtT * kTileBytes, c.stream);
         const uint64_t blocks = std::min<uint64_t>(g.ntilesT * g.kbtT, (uint64_t)c.sm_count * 16);
-        k_transpose_tiles<<<(unsigned)blocks, 256, 0, c.stream>>>(g.tiles.get(), g.kbt, g.ntiles, g.tilesT.get(),
+        launch_next(c, k_transpose_tiles, (unsigned)blocks, 256, 0, g.tiles.get(), g.kbt, g.ntiles, g.tilesT.get(),
                                                                    g.kbtT, g.ntilesT, 0, g.kbtT);
         SLFMM_LAUNCHED(c, "k_transpose_tiles");
         g.have_tilesT = true;
@@ -1204,12 +1216,12 @@ void launch_fp8_terms_f64(Ctx& c, const double* src, int ld, uint64_t K, int w, 
                       (!ind_row_off || ind_row_off + kIndTerms * wpad <= n_rows) && wpad % kTermCols == 0 &&
                       K_pad % kStageK == 0,
                   SLFMM_ERR_BAD_ARG, "bad stage-major operand shape");
-    k_colmax_abs<double><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, nullptr, cm.get());
+    launch_next(c, k_colmax_abs<double>, colmax_blocks(c, K), 256, 0, src, ld, K, w, nullptr, cm.get());
     SLFMM_LAUNCHED(c, "k_colmax_abs");
     const TermSet sa{nullptr, kMainTerms, 0, cm.get()};
     const TermSet sb{nullptr, ind_row_off ? kIndTerms : 0, ind_row_off, cm.get()};
     dim3 grid((unsigned)(K_pad / kStageK), (unsigned)(wpad / kTermCols));
-    k_fp8_terms<double><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
+    launch_next(c, k_fp8_terms<double>, grid, 256, 0, src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
     SLFMM_LAUNCHED(c, "k_fp8_terms");
 }
 
@@ -1229,20 +1241,20 @@ void launch_fp8_terms_f32_pair(Ctx& c, const float* src, int ld, uint64_t K, int
     if (quads) {
         const unsigned blocks = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>(ceil_div(K * (uint64_t)(ld / 4), 1024), (uint64_t)c.sm_count * 4));
-        k_colmax_pair<<<blocks, 256, 0, c.stream>>>(src, ld, K, w, ks_main, ks_ind, cma, cmb);
+        launch_next(c, k_colmax_pair, blocks, 256, 0, src, ld, K, w, ks_main, ks_ind, cma, cmb);
         SLFMM_LAUNCHED(c, "k_colmax_pair");
     } else {
-        k_colmax_abs<float><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, ks_main, cma);
+        launch_next(c, k_colmax_abs<float>, colmax_blocks(c, K), 256, 0, src, ld, K, w, ks_main, cma);
         SLFMM_LAUNCHED(c, "k_colmax_abs");
         if (ks_ind) {
-            k_colmax_abs<float><<<colmax_blocks(c, K), 256, 0, c.stream>>>(src, ld, K, w, ks_ind, cmb);
+            launch_next(c, k_colmax_abs<float>, colmax_blocks(c, K), 256, 0, src, ld, K, w, ks_ind, cmb);
             SLFMM_LAUNCHED(c, "k_colmax_abs");
         }
     }
     const TermSet sa{ks_main, kMainTerms, 0, cma};
     const TermSet sb{ks_ind, ks_ind ? kIndTerms : 0, ind_row_off, cmb};
     dim3 grid((unsigned)(K_pad / kStageK), (unsigned)(wpad / kTermCols));
-    k_fp8_terms<float><<<grid, 256, 0, c.stream>>>(src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
+    launch_next(c, k_fp8_terms<float>, grid, 256, 0, src, ld, K, w, wpad, sa, sb, n_rows, B, inv_scale);
     SLFMM_LAUNCHED(c, "k_fp8_terms");
 }
 
@@ -1434,7 +1446,7 @@ static int tc8_launch(Ctx& c, const Fp8Plan& pl, const TileView& tv, uint64_t ro
 
 void launch_sub_colterm(Ctx& c, double* S, int lds, uint64_t n, int w, const double* colterm) {
     if (!n || !w) return;
-    k_sub_colterm<<<grid_for(c, n * w, 256), 256, 0, c.stream>>>(S, lds, n, w, colterm);
+    launch_next(c, k_sub_colterm, grid_for(c, n * w, 256), 256, 0, S, lds, n, w, colterm);
     SLFMM_LAUNCHED(c, "k_sub_colterm");
 }
 

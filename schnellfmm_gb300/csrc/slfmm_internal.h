@@ -219,6 +219,42 @@ inline int grid_for(const Ctx& c, uint64_t work, int block) {
     return (int)(g > 0 ? g : 1);
 }
 
+#ifdef __CUDACC__
+// First statement of every kernel: wait until the kernels before it in the stream
+// are complete and their writes visible (at once for a kernel launched without
+// launch_next).
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The same in a short kernel, which also lets the next one be launched under it.
+// Not in one that runs long: blocks waiting beside it take from its SM's resources
+// (with it in every kernel a biobank fit took 33.9 ms instead of 32.5, an NMF fit
+// 26.4 instead of 24.8).
+__device__ __forceinline__ void dependent_start() {
+    dependent_wait();
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+// Launch on the context's stream with the launch itself, but not the kernel,
+// overlapping the kernel before it: its blocks take their places as that one's last
+// ones leave and wait in dependent_start.  A chain of 6 us kernels with an
+// allocation each runs at 4.0 us a step instead of 6.5 us, and a fit is a chain of
+// 130 to 170.  Errors surface in SLFMM_LAUNCHED, as with <<<>>>.
+template <class... P, class... A>
+void launch_next(Ctx& c, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = c.stream;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&lc, kernel, std::forward<A>(args)...);
+}
+#endif
+
 // Raise a kernel's dynamic shared-memory limit to at least `bytes` (no-op up
 // to 48 KiB).  The limit is a process-wide attribute of the function, and
 // contexts may launch from several host threads, so it only ever grows:
