@@ -5,8 +5,8 @@
 // IEEE-754 fields (sign, exponent rebiased between 127 and 1023, mantissa
 // shifted between 23 and 52 bits, rounded to nearest even when narrowing)
 // and give the conversion instruction's result bit for bit; the values they
-// do not handle (zeros, subnormals, infinities, NaNs, and narrowing results
-// outside the normal FP32 range) take the instruction.
+// do not handle (subnormals, infinities, NaNs, and narrowing results outside
+// the normal FP32 range, zero among them) take the instruction.
 #pragma once
 #include <cstdint>
 
@@ -15,8 +15,9 @@ namespace slfmm {
 __device__ __forceinline__ double f64_of_f32(float x) {
     const uint32_t b = __float_as_uint(x);
     const uint32_t e = (b >> 23) & 0xffu;
-    if (e == 0u || e == 0xffu) return (double)x;
-    const uint64_t r = ((uint64_t)(b >> 31) << 63) | ((uint64_t)(e + 896u) << 52) | ((uint64_t)(b & 0x7fffffu) << 29);
+    const uint32_t m = b & 0x7fffffu;
+    if (e == 0xffu || (e == 0u && m)) return (double)x;
+    const uint64_t r = ((uint64_t)(b >> 31) << 63) | (e ? ((uint64_t)(e + 896u) << 52) | ((uint64_t)m << 29) : 0ull);
     return __longlong_as_double((long long)r);
 }
 

@@ -6,6 +6,7 @@
 // these only ever touch n x w, w x w or p x w objects with tiny w.
 #include <cooperative_groups.h>
 
+#include "fp_convert.cuh"
 #include "slfmm_internal.h"
 
 namespace slfmm {
@@ -358,13 +359,26 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __re
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ky = lane >> 3, cx = lane & 7;
     double* mine = dsum + warp * 32 * 32;  // [entry][lane]
-#pragma unroll
-    for (int k = 0; k < 32; ++k) mine[k * 32 + lane] = 0.0;
-    const uint64_t ntiles = (m + kNarrowTile - 1) / kNarrowTile;
-    const int tsz = kNarrowTile * lda;
     float acc[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+    bool first = true;
+    // The first sums are only widened, by integer operations: 32 conversions and 32
+    // additions to zero by every warp held the FP64 pipe for half of a small Gram.
+    auto flush = [&]() {
+        if (first) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) mine[k * 32 + lane] = f64_of_f32(acc[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) mine[k * 32 + lane] += (double)acc[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+        first = false;
+    };
+    const uint64_t ntiles = (m + kNarrowTile - 1) / kNarrowTile;
+    const int tsz = kNarrowTile * lda;
     for (int k = 0; k < kPipe - 1; ++k) {
         const uint64_t t = blockIdx.x + (uint64_t)k * gridDim.x;
         if (t < ntiles) pipe_issue(A, lda, m, t, ring + k * tsz);
@@ -396,14 +410,12 @@ __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __re
             }
         }
         if (++since == 32) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) mine[k * 32 + lane] += (double)acc[k], acc[k] = 0.f;
+            flush();
             since = 0;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < 32; ++k) mine[k * 32 + lane] += (double)acc[k];
+    flush();
     __syncthreads();
     // entry (k, c) of the block partial: lane 8 (k / 8) + c / 4, slot (k % 8) 4 + c % 4
     for (int e = threadIdx.x; e < a * a; e += kPipeThreads) {
