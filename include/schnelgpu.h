@@ -59,9 +59,8 @@ extern "C" {
 #define SLFMM_RNG_CHACHA8      0      /* the reference's streams (default):
                                          ChaCha8Rng::seed_from_u64(seed) sampled
                                          by Normal(0, 1) in row-major order for
-                                         the sketches (on the host threads) and by
-                                         Uniform(0, 1) for the masks (on the
-                                         device)                                 */
+                                         the sketches and by Uniform(0, 1) for
+                                         the masks, drawn on the device          */
 #define SLFMM_RNG_COUNTER      1      /* SplitMix64 counter streams, drawn on the
                                          device                                  */
 

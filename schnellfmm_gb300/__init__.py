@@ -77,8 +77,8 @@ class SketchRng(enum.IntEnum):
     """Streams of the Gaussian sketches (src/rsvd.rs:44-46,
     src/nmf.rs:291-293) and the NMF CV hold-out masks (src/nmf.rs:433-448,
     src/testing.rs:437-452): the device counter streams, or the reference's
-    ChaCha8Rng::seed_from_u64 streams (Normal(0, 1) sketches drawn on the
-    host threads, Uniform(0, 1) masks drawn on the device), the default."""
+    ChaCha8Rng::seed_from_u64 streams (Normal(0, 1) sketches and
+    Uniform(0, 1) masks, drawn on the device), the default."""
     CHACHA8 = 0
     COUNTER = 1
 

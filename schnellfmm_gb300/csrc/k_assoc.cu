@@ -499,7 +499,7 @@ static void assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const do
     // shared memory); every block reads the same u rows
     for (int t0 = 0; t0 < k.d; t0 += TP) {
         const int db = std::min(TP, k.d - t0);
-        launch_next(c, k_assoc_epilogue<TP>, grid, 256, smem, 
+        launch_next(c, k_assoc_epilogue<TP>, grid, 256, smem,
             p, u, ldu, tss, k.zero_var, db, k.d, k.w, k.df, k.theta_rows + (size_t)t0 * k.w,
             k.beta_rows + (size_t)t0 * k.w, k.cjj + t0, k.dropped + t0, beta + t0, t32 + t0, t0 == 0 ? r2 : nullptr,
             hist + (size_t)t0 * kHistBins);
@@ -508,7 +508,7 @@ static void assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const do
 }
 
 // Up to four covariates take the thread-per-SNP form (1.8 M SNPs, 1 covariate,
-// 13 columns, eight launches: 0.58 ms in the 64-trait tiles), up to 16 the
+// 13 columns, eight launches: 0.58 ms in the 64-trait tiles, 0.28 ms so), up to 16 the
 // tiles padded to 16 traits while two CTAs' tables and tiles fit an SM.
 void launch_assoc_epilogue(Ctx& c, uint64_t p, const float* u, int ldu, const double* tss,
                            const AssocConsts& k, double* beta, float* t32, double* r2,

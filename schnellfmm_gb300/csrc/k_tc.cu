@@ -720,7 +720,7 @@ void launch_rowfix_mean(Ctx& c, float* P, int ldp, uint64_t rows, int w, const u
             continue;
         }
         // a warp covers 128 columns (4 per lane): wider operands in column blocks
-        launch_next(c, k_rowfix_mean, (unsigned)ceil_div(rows * 32, 256), 256, 0, 
+        launch_next(c, k_rowfix_mean, (unsigned)ceil_div(rows * 32, 256), 256, 0,
             P + c0, ldp, rows, std::min(128, w - c0), ptr, idx, W + c0, ldw, cs + c0, mean, scale);
         SLFMM_LAUNCHED(c, "k_rowfix_mean");
         c0 += 128;
