@@ -917,7 +917,9 @@ __global__ void k_add_diag(double* __restrict__ A, int a, double v) {
 // FP64 pipe), then every division of the step side by side (the factors of the
 // rows, the scaled pivot row), then a x a FMAs, a warp per row.  Bound by one
 // SM's FP64 pipe (two FMAs per cycle).
-constexpr int kMaxGaussJordan = 160;  // 8 a^2 bytes of shared memory
+// Widest that one CTA takes (8 a^2 bytes of shared memory); a cluster above.  The
+// inverses of 50 columns: 194 us in one CTA, 124 us in a cluster.
+constexpr int kInvOneCta = 40;
 struct InverseJobs {
     InverseJob job[kMaxInverseJobs];
 };
@@ -925,8 +927,8 @@ struct InverseJobs {
 __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant__ InverseJobs jobs) {
     dependent_start();
     extern __shared__ double S[];  // a x a
-    __shared__ double f[kMaxGaussJordan], prow[kMaxGaussJordan];
-    __shared__ int rowid[kMaxGaussJordan], from[kMaxGaussJordan];
+    __shared__ double f[kInvOneCta], prow[kInvOneCta];
+    __shared__ int rowid[kInvOneCta], from[kInvOneCta];
     __shared__ double eps;
     __shared__ int p_sh, ok;
     const InverseJob& jb = jobs.job[blockIdx.x];
@@ -1016,6 +1018,123 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant_
     if (tid == 0) {
         jb.status[0] = 2;
         jb.eps[0] = eps;
+    }
+}
+
+// The same elimination for wide matrices, a job to a cluster of kInvCluster CTAs:
+// column j lives column-major in the shared memory of CTA j mod kInvCluster.  Step
+// k's owner searches its column and divides it, and leaves the pivot, its row and
+// the row factors with every CTA (two sets of them, for even and odd steps: a step's
+// are read until the next one's barrier); then each CTA updates its columns, a warp
+// per column.  One SM spent a^2 FMAs of its FP64 pipe per step: two launches with
+// designs of 100 and 131 columns took 1.41 ms, 0.78 ms so.
+constexpr int kInvCluster = 8;
+__global__ void __launch_bounds__(1024, 1) k_inverse_cluster(const __grid_constant__ InverseJobs jobs) {
+    dependent_start();
+    extern __shared__ double S[];  // the CTA's columns, a long each
+    __shared__ double f[2][kMaxDesign], piv[2];
+    __shared__ int prow[2], found[2];
+    __shared__ int rowid[kMaxDesign], from[kMaxDesign];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const InverseJob& jb = jobs.job[blockIdx.x / kInvCluster];
+    const double* A = jb.A;
+    const int a = jb.a, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    const int ncol = (a - rank + kInvCluster - 1) / kInvCluster;  // columns rank, rank + 8 ..
+    const bool inv = jb.X != nullptr;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        double dmax = 0.0;
+        for (int k = lane; k < a; k += 32) dmax = fmax(dmax, fabs(A[k * a + k] + jb.shift));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        dmax = fmax(dmax, 1e-300);
+        const double eps = attempt == 0 ? 0.0 : 1e-8 * dmax;
+        for (int e = tid; e < ncol * a; e += blockDim.x) {
+            const int jl = e / a, i = e - jl * a, j = rank + kInvCluster * jl;
+            S[e] = i == j ? (A[i * a + j] + jb.shift) + eps : A[i * a + j];
+        }
+        for (int i = tid; i < a; i += blockDim.x) rowid[i] = i;
+        bool ok = true;
+        cluster.sync();  // every CTA runs, and is done with the last attempt's sets
+        for (int k = 0; k < a; ++k) {
+            const int b = k & 1;
+            if (rank == k % kInvCluster) {
+                const double* col = S + (k / kInvCluster) * a;
+                if (warp == 0) {
+                    unsigned long long best = 0ull;  // |value| bits + 1 (0: none; NaN never wins)
+                    int p = k;
+                    for (int i = k + lane; i < a; i += 32) {
+                        const unsigned long long u =
+                            (unsigned long long)__double_as_longlong(col[i]) & 0x7fffffffffffffffull;
+                        const unsigned long long key = u > 0x7ff0000000000000ull ? 0ull : u + 1ull;
+                        if (key > best) { best = key; p = i; }
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+                        const int op = __shfl_xor_sync(0xffffffffu, p, o);
+                        if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
+                    }
+                    if (lane < kInvCluster) {
+                        cluster.map_shared_rank(prow, lane)[b] = p;
+                        cluster.map_shared_rank(found, lane)[b] = best > 1ull;
+                        cluster.map_shared_rank(piv, lane)[b] = col[p];
+                    }
+                }
+                __syncthreads();
+                const int p = prow[b];
+                const double d = piv[b];
+                for (int i = tid; i < a; i += blockDim.x) {
+                    if (i == k) continue;
+                    const double fi = col[i == p ? k : i] / d;
+#pragma unroll
+                    for (int c = 0; c < kInvCluster; ++c) cluster.map_shared_rank(f[b], c)[i] = fi;
+                }
+            }
+            cluster.sync();
+            ok = found[b] != 0;
+            if (!ok) break;
+            const int p = prow[b];
+            const double d = piv[b];
+            if (tid == 0) {
+                from[k] = rowid[p];
+                rowid[p] = rowid[k];
+            }
+            for (int jl = warp; jl < ncol; jl += nwarps) {
+                const int j = rank + kInvCluster * jl;
+                double* col = S + jl * a;
+                if (j == k) {
+                    if (!inv) continue;
+                    for (int i = lane; i < a; i += 32) col[i] = i == k ? 1.0 / d : -f[b][i];
+                    continue;
+                }
+                if (!inv && j < k) continue;
+                const double pj = col[p], kj = col[k];
+                __syncwarp();
+                for (int i = (inv ? 0 : (k & ~31)) + lane; i < a; i += 32) {
+                    if (i == k) col[i] = inv ? pj / d : pj;
+                    else if (inv || i > k) col[i] = fma(-f[b][i], pj, i == p ? kj : col[i]);
+                }
+            }
+            __syncthreads();
+        }
+        if (ok) {
+            if (inv)
+                for (int e = tid; e < ncol * a; e += blockDim.x) {
+                    const int jl = e / a, i = e - jl * a;
+                    jb.X[i * a + from[rank + kInvCluster * jl]] = S[e];
+                }
+            if (tid == 0 && rank == 0) {
+                jb.status[0] = attempt;
+                jb.eps[0] = eps;
+            }
+            return;
+        }
+        if (attempt == 1 && tid == 0 && rank == 0) {
+            jb.status[0] = 2;
+            jb.eps[0] = eps;
+        }
     }
 }
 
@@ -1959,9 +2078,9 @@ void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv) {
     SLFMM_LAUNCHED(c, "k_tri_inv_lower");
 }
 
-// The elimination in shared memory takes status-only jobs up to its size, and
-// inverses up to 112 columns (wider ones keep the LU's solves and their bits).
-static bool inverse_in_shared(const InverseJob& j) { return j.a <= (j.X ? 112 : kMaxGaussJordan); }
+// The elimination in shared memory takes every status-only job, and inverses up
+// to 112 columns (wider ones keep the LU's solves and their bits).
+static bool inverse_in_shared(const InverseJob& j) { return j.a <= (j.X ? 112 : kMaxDesign); }
 
 void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
     SLFMM_REQUIRE(n <= kMaxInverseJobs, SLFMM_ERR_BAD_ARG, "too many matrices for one inversion launch");
@@ -1978,8 +2097,12 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
             js.job[m++] = jobs[i];
             amax = std::max(amax, jobs[i].a);
         }
-    if (m) {
-        set_smem((const void*)k_inverse_jobs, smem_sq(amax));
+    if (amax > kInvOneCta) {
+        const size_t sm = ceil_div(amax, kInvCluster) * amax * sizeof(double);
+        set_smem((const void*)k_inverse_cluster, std::max(sm, kEighLimit));
+        launch_next_clusters(c, k_inverse_cluster, m, kInvCluster, 1024, sm, js);
+        SLFMM_LAUNCHED(c, "k_inverse_cluster");
+    } else if (m) {
         launch_next(c, k_inverse_jobs, m, 1024, smem_sq(amax), js);
         SLFMM_LAUNCHED(c, "k_inverse_jobs");
     }
@@ -2031,22 +2154,9 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
         DBuf<double> ws(3 * (size_t)ap * ap, c.stream);
         const size_t share = 2 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
         const size_t sm = 2 * square <= kEighClusterSmem ? std::max(2 * square, share) : share;
-        cudaLaunchAttribute at[2] = {};
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kEighCluster;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t lc{};
-        lc.gridDim = dim3(kEighCluster);
-        lc.blockDim = dim3(1024);
-        lc.dynamicSmemBytes = sm;
-        lc.stream = c.stream;
-        lc.attrs = at;
-        lc.numAttrs = 2;
         auto go = [&](auto kern) {
             set_smem((const void*)kern, std::max(sm, kEighLimit));
-            SLFMM_CUDA(cudaLaunchKernelEx(&lc, kern, const_cast<double*>(A), a, V, sig, ws.get()));
+            launch_next_clusters(c, kern, 1, kEighCluster, 1024, sm, const_cast<double*>(A), a, V, sig, ws.get());
         };
         if (ap <= 64) go(k_jacobi_svd<kEighCluster, 2>);
         else if (ap <= 128) go(k_jacobi_svd<kEighCluster, 4>);

@@ -240,6 +240,24 @@ __device__ __forceinline__ void dependent_start() {
 // allocation each runs at 4.0 us a step instead of 6.5 us, and a fit is a chain of
 // 130 to 170.  Errors surface in SLFMM_LAUNCHED, as with <<<>>>.
 template <class... P, class... A>
+void launch_next_clusters(Ctx& c, void (*kernel)(P...), unsigned clusters, unsigned size, dim3 block, size_t smem,
+                          A&&... args) {
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = size;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(clusters * size);
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = c.stream;
+    lc.attrs = at;
+    lc.numAttrs = size > 1 ? 2 : 1;
+    (void)cudaLaunchKernelEx(&lc, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
 void launch_next(Ctx& c, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

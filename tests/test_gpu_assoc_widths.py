@@ -43,3 +43,24 @@ def test_chunks_equal_one_piece(engine, d):
     del a
     for v in pinned.values():
         v.free()
+
+
+@pytest.mark.parametrize("d", [38, 45, 130])
+def test_singular_wide_design(engine, capfd, d):
+    """A constant covariate: the elimination finds an exactly zero pivot, adds
+    eps and starts again, in one CTA (38) and in clusters, and the covariate
+    gets t = 0."""
+    import schnellfmm_gb300 as sg
+    c = simdata.simulate(500, 1200, k_pop=3, fst=0.1, miss=0.01, d=d, n_causal=20, seed=40 + d)
+    x = 0.5 * c.x
+    x[:, 7] = 2.5
+    omega = O.rng_normal_matrix(5, c.n, 13)
+    geno = engine.upload(c.packed, c.n)
+    capfd.readouterr()
+    res = sg.fit_lfmm2(geno, sg.SubsetSpec.all(), geno, x, sg.Lfmm2Config(k=3, norm=sg.SnpNorm.EIGENSTRAT),
+                       omega=omega, engine=engine)
+    assert "is singular, adding epsilon" in capfd.readouterr().err
+    ref = O.fit_oracle64(c.raw, c.raw, x, k=3, norm=O.NORM_EIGENSTRAT, omega=omega)
+    check_fit(res, ref.assoc, ref.u_hat)
+    assert (res.tstat[:, 7] == 0).all() and (ref.assoc.tstat[:, 7] == 0).all()
+    geno.free()
