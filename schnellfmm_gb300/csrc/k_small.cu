@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_cluster(const __grid_consta
 // and 837, 40 columns 1107 and 984.
 constexpr int kEighOneCta = 32;
 constexpr int kEighCluster = 8;
-constexpr size_t kEighClusterSmem = 208 << 10;  // beside 17 KB of static arrays
+constexpr size_t kEighClusterSmem = 200 << 10;  // beside 25 KB of static arrays
 // with those arrays a launch passes 48 KB before its dynamic part does
 constexpr size_t kEighLimit = (48 << 10) + 1;
 
@@ -1370,6 +1370,135 @@ __device__ void gs_columns(double* Vs, double* acc, int ap, double* dots) {
     }
 }
 
+// gs_columns over a cluster: column k and its running first pass belong to CTA k mod
+// kEighCluster (own: the first passes, the columns as they came in, the final
+// ones, `area` doubles each), which gives the second pass's products with its final
+// columns; the chain and the norm stay with the first CTA, where the columns are
+// put together (vec).  Per column the owner ends its first pass and hands it to all
+// (cur), all hand their products to the first, and that one the final column to
+// all (last, for even and odd columns): three barriers.
+template <int NR>
+__device__ void gs_cluster(double* own, int area, double* vec, int ap, double* dots, double* cur,
+                           double (*last)[kMaxDesign]) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int kN = kEighCluster;
+    const int rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    constexpr int kChainWarps = NR < kTrail ? NR : kTrail;
+    double *acc = own, *orig = own + area, *fin = own + 2 * area;
+    auto load = [&](const double* c, double (&v)[NR]) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) v[q] = lane + 32 * q < ap ? c[lane + 32 * q] : 0.0;
+    };
+    // products of v with four of the CTA's columns from slot s on (slots past `end` as zero)
+    auto dot4 = [&](const double* cols, int s, int end, const double (&v)[NR], double (&t)[4]) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            t[m] = plain(0.0);
+            if (s + m < end) {
+                const double* c = cols + (s + m) * ap;
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t[m] += c[lane + 32 * q] * v[q];
+            }
+        }
+    };
+    auto to_all = [&](double* dst, const double (&v)[NR]) {
+#pragma unroll
+        for (int c = 0; c < kN; ++c) {
+            double* d = cluster.map_shared_rank(dst, c);
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (lane + 32 * q < ap) d[lane + 32 * q] = v[q];
+        }
+    };
+    const int slots = (ap - rank + kN - 1) / kN;
+    for (int j = 0; j < ap; ++j) {
+        const double* prev = last[(j - 1) & 1];
+        if (j > 0 && rank == (j - 1) % kN)
+            for (int r = tid; r < ap; r += blockDim.x) fin[(j - 1) / kN * ap + r] = prev[r];
+        if (rank == j % kN && warp == 0) {
+            double x[NR];
+            load(acc + j / kN * ap, x);
+            if (j > 0) {  // the last term of the column's first pass
+                const double* vj = orig + j / kN * ap;
+                double t = plain(0.0);
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t += prev[lane + 32 * q] * vj[lane + 32 * q];
+                t = warp_sum(t);
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) x[q] -= t * prev[lane + 32 * q];
+            }
+            to_all(cur, x);
+        }
+        cluster.sync();
+        const int done = j > rank ? (j - rank + kN - 1) / kN : 0;  // the CTA's final columns
+        for (int s = 4 * warp; s < done; s += 4 * nwarps) {
+            double v[NR], t[4];
+            load(cur, v);
+            dot4(fin, s, done, v, t);
+            const double d = warp_sum4(t);
+            if ((lane & 7) == 0 && s + (lane >> 3) < done)
+                cluster.map_shared_rank(dots, 0)[rank + kN * (s + (lane >> 3))] = d;
+        }
+        cluster.sync();
+        const int w = rank == 0 ? warp - kTrail : warp, nw = rank == 0 ? nwarps - kTrail : nwarps;
+        if (rank == 0 && warp < kChainWarps) {
+            double* vj = vec + j * ap;
+#pragma unroll
+            for (int q = 0; q < (NR + kChainWarps - 1) / kChainWarps; ++q) {
+                const int r = lane + 32 * (warp + q * kChainWarps);
+                if (r < ap) {
+                    double t = cur[r];
+#pragma unroll 4
+                    for (int i = 0; i < j; ++i) t -= dots[i] * vec[i * ap + r];
+                    vj[r] = t;
+                }
+            }
+            if (kChainWarps > 1) asm volatile("bar.sync 1, %0;" ::"n"(32 * kChainWarps) : "memory");
+            if (warp == 0) {
+                double x[NR];
+                load(vj, x);
+                double t = plain(0.0);
+#pragma unroll
+                for (int q = 0; q < NR; ++q)
+                    if (lane + 32 * q < ap) t += x[q] * x[q];
+                t = warp_sum(t);
+                const double inv = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    x[q] *= inv;
+                    if (lane + 32 * q < ap) vj[lane + 32 * q] = x[q];
+                }
+                to_all(last[j & 1], x);
+            }
+        } else if (w >= 0 && j > 0) {
+            // column j - 1 leaves the columns behind j
+            double v[NR], t[4];
+            load(prev, v);
+            const int first = j >= rank ? (j - rank) / kN + 1 : 0;
+            for (int s = first + 4 * w; s < slots; s += 4 * nw) {
+                dot4(orig, s, slots, v, t);
+                const double d4 = warp_sum4(t);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const double d = __shfl_sync(0xffffffffu, d4, 8 * m);
+                    if (s + m < slots) {
+                        double* ak = acc + (s + m) * ap;
+#pragma unroll
+                        for (int q = 0; q < NR; ++q)
+                            if (lane + 32 * q < ap) ak[lane + 32 * q] -= d * v[q];
+                    }
+                }
+            }
+        }
+        cluster.sync();
+    }
+}
+
 // Eigen-decomposition of a symmetric positive semi-definite a x a matrix
 // (a <= kMaxDesign; the Gram matrices of Step 0, the RSVD and the NMF probe) in
 // NC CTAs: A V = V diag(sig), sig descending, V orthonormal; A is overwritten by
@@ -1395,9 +1524,9 @@ __device__ void gs_columns(double* Vs, double* acc, int ap, double* dots) {
 // ones run as a cluster of eight: the FP32 matrices' and B's columns and R's rows
 // are spread over the CTAs' shared memory, a round's pairs and 2 x 2 blocks are
 // shared out and read and written there, and the products take a share of the
-// columns each; Gram-Schmidt stays with the first CTA.  A solve with its copies
-// (45 us), before and so: 13 columns 275 and 243 us, 20 463 and 351, 50 2464 and
-// 1402, 100 14.1 and 4.8 ms, 256 222 and 57 ms.
+// columns each; of Gram-Schmidt the chains and norms stay with the first CTA.
+// A solve with its copies (45 us), before and so: 13 columns 275 and 235 us, 20 461 and 348, 50 2457 and
+// 1375, 100 14.1 and 4.1 ms, 256 221 and 52 ms.
 template <int NC, int NR>
 __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, int a, double* __restrict__ V,
                                                         double* __restrict__ sig, double* ws) {
@@ -1417,17 +1546,16 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
     const int sq = ap * ap;
     // One CTA: three squares of shared memory -- Gram-Schmidt's scratch, T and R;
     // the vectors; the FP32 matrices, B and V R.  A cluster: three squares of
-    // global memory for what the CTAs pass on, the first CTA's own two in shared
-    // memory where they fit, and in each a share of the FP32 matrices, later of T
-    // or R, and of B.
-    double *vec, *scratch, *fp32, *T, *Bs, *R, *VR;
+    // global memory for what the CTAs pass on, the first CTA's vectors in shared
+    // memory where they fit, and in each a share of the FP32 matrices, then of
+    // Gram-Schmidt's columns, then of T or R, and of B.
+    double *vec, *scratch = nullptr, *fp32, *T, *Bs, *R, *VR;
     if (NC == 1) {
         scratch = T = R = sm_dyn;
         vec = sm_dyn + sq;
         fp32 = Bs = VR = sm_dyn + 2 * sq;
     } else {
         const bool fits = 2 * (size_t)sq * sizeof(double) <= kEighClusterSmem;
-        scratch = fits ? sm_dyn : ws;
         vec = fits ? sm_dyn + sq : ws + sq;
         fp32 = T = R = sm_dyn;
         Bs = sm_dyn + share * ap;
@@ -1436,6 +1564,8 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
     double* vecs = NC == 1 ? vec : ws + sq;  // the vectors where every CTA reads them
     float* M32 = reinterpret_cast<float*>(fp32);  // the share's columns of M, then of V
     const int to_v = share * ap;
+    // Gram-Schmidt over the cluster: the columns rank, rank + NC .. , `area` doubles of them
+    const int area = share * ap, mine = (ap - rank + NC - 1) / NC * ap;
     __shared__ int rotated, rotated32[2], nact;
     __shared__ double sg[kMaxDesign];
     __shared__ double dots[kMaxDesign];
@@ -1447,6 +1577,7 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
     __shared__ float* mcol[kMaxDesign];   // and of the FP32 matrix
     __shared__ int act[kMaxDesign], rest[kMaxDesign], actflag[kMaxDesign];
     __shared__ float colmax2;
+    __shared__ double cur[NC > 1 ? kMaxDesign : 1], last[NC > 1 ? 2 : 1][kMaxDesign];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     // phase 1: FP32 sweeps
     for (int e = threadIdx.x; e < nc * ap; e += blockDim.x) {
@@ -1477,12 +1608,19 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
     jacobi_sweeps32<NC, (NR > 2 ? NR : 2)>([&](int cc) { return NC == 1 ? M32 + cc * ap : mcol[cc]; }, to_v, ap,
                                           rank, 1.0e-5f, 12, rotated32, 1e-7f * colmax2, sync_all);
     sync_all();
-    if (rank == 0) {
-        // phase 2: FP64 orthonormal V
+    // phase 2: FP64 orthonormal V
+    if constexpr (NC == 1) {
         for (int e = threadIdx.x; e < sq; e += blockDim.x) vec[e] = (double)mcol[e / ap][to_v + e % ap];
         __syncthreads();
         gs_columns<NR>(vec, scratch, ap, dots);
-        if (vecs != vec)
+    } else {
+        for (int e = threadIdx.x; e < mine; e += blockDim.x)
+            sm_dyn[area + e] = (double)mcol[rank + NC * (e / ap)][to_v + e % ap];
+        sync_all();  // the FP32 matrices are done with
+        for (int e = threadIdx.x; e < mine; e += blockDim.x) sm_dyn[e] = sm_dyn[area + e];
+        __syncthreads();
+        gs_cluster<NR>(sm_dyn, area, vec, ap, dots, cur, last);
+        if (rank == 0 && vecs != vec)
             for (int e = threadIdx.x; e < sq; e += blockDim.x) vecs[e] = vec[e];
     }
     sync_all();
@@ -1663,15 +1801,15 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
     }
     sync_all();
     double* fin = VR;
-    if (rank == 0) {
-        if (NC > 1) {
-            for (int e = threadIdx.x; e < sq; e += blockDim.x) vec[e] = VR[e];
-            fin = vec;
-            __syncthreads();
-        }
+    if constexpr (NC == 1) {
         gs_columns<NR>(fin, scratch, ap, dots);
-        if (vecs != vec)
-            for (int e = threadIdx.x; e < sq; e += blockDim.x) vecs[e] = fin[e];
+    } else {
+        for (int e = threadIdx.x; e < mine; e += blockDim.x)
+            sm_dyn[e] = sm_dyn[area + e] = VR[(rank + NC * (e / ap)) * ap + e % ap];
+        __syncthreads();
+        gs_cluster<NR>(sm_dyn, area, vec, ap, dots, cur, last);
+        if (rank == 0 && vecs != vec)
+            for (int e = threadIdx.x; e < sq; e += blockDim.x) vecs[e] = vec[e];
     }
     if (NC > 1) fin = vecs;
     sync_all();
@@ -2152,7 +2290,7 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
         launch_next(c, k_jacobi_svd<1, 1>, 1, threads, 3 * square, const_cast<double*>(A), a, V, sig, nullptr);
     } else {
         DBuf<double> ws(3 * (size_t)ap * ap, c.stream);
-        const size_t share = 2 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
+        const size_t share = 3 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
         const size_t sm = 2 * square <= kEighClusterSmem ? std::max(2 * square, share) : share;
         auto go = [&](auto kern) {
             set_smem((const void*)kern, std::max(sm, kEighLimit));
