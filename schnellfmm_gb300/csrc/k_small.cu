@@ -1525,8 +1525,8 @@ __device__ void gs_cluster(double* own, int area, double* vec, int ap, double* d
 // are spread over the CTAs' shared memory, a round's pairs and 2 x 2 blocks are
 // shared out and read and written there, and the products take a share of the
 // columns each; of Gram-Schmidt the chains and norms stay with the first CTA.
-// A solve with its copies (45 us), before and so: 13 columns 275 and 235 us, 20 461 and 348, 50 2457 and
-// 1375, 100 14.1 and 4.1 ms, 256 221 and 52 ms.
+// A solve with its copies (45 us), before and so: 13 columns 275 and 235 us, 20
+// 461 and 348, 50 2457 and 1375, 100 14.1 and 4.1 ms, 256 221 and 52 ms.
 template <int NC, int NR>
 __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, int a, double* __restrict__ V,
                                                         double* __restrict__ sig, double* ws) {
