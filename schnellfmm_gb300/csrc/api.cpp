@@ -363,9 +363,15 @@ struct NmfFill {
 struct SnpStd {
     DBuf<double> mean, scale, tss;
     DBuf<uint8_t> zero_var;
-    DBuf<float> lut;  // p x 4
+    DBuf<float> lut;  // p x 4, the FP32 contractions' values of the four codes (theirs alone)
     NmfFill fill;
 };
+
+void std_lut(Ctx& c, uint64_t p, SnpStd& s) {
+    if (c.precision != SLFMM_PREC_FP32) return;
+    s.lut.alloc(std::max<uint64_t>(p, 1) * 4, c.stream);
+    launch_lut_std(c, p, s.mean.get(), s.scale.get(), s.lut.get());
+}
 
 void std_mean(Ctx& c, const Geno& g, int norm, SnpStd& s) {
     const uint64_t p = std::max<uint64_t>(g.p, 1);
@@ -373,9 +379,8 @@ void std_mean(Ctx& c, const Geno& g, int norm, SnpStd& s) {
     s.scale.alloc(p, c.stream);
     s.tss.alloc(p, c.stream);
     s.zero_var.alloc(p, c.stream);
-    s.lut.alloc(p * 4, c.stream);
     launch_stats_mean(c, g, norm, s.mean.get(), s.scale.get(), s.tss.get(), s.zero_var.get());
-    launch_lut_std(c, g.p, s.mean.get(), s.scale.get(), s.lut.get());
+    std_lut(c, g.p, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -728,10 +733,9 @@ void std_fill(Ctx& c, const Geno& g, int norm, const NmfFill& f, SnpStd& s) {
     s.scale.alloc(p, c.stream);
     s.tss.alloc(p, c.stream);
     s.zero_var.alloc(p, c.stream);
-    s.lut.alloc(p * 4, c.stream);
     build_missing_lists(c, g);
     launch_fill_stats(c, g, norm, f.W, f.H, f.k, s.mean.get(), s.scale.get(), s.tss.get(), s.zero_var.get());
-    launch_lut_std(c, g.p, s.mean.get(), s.scale.get(), s.lut.get());
+    std_lut(c, g.p, s);
     s.fill = f;
 }
 
@@ -744,13 +748,12 @@ void std_raw(Ctx& c, const Geno& g, const double* mean_src, SnpStd& s) {
     s.scale.alloc(p, c.stream);
     s.tss.alloc(p, c.stream);
     s.zero_var.alloc(p, c.stream);
-    s.lut.alloc(p * 4, c.stream);
     if (mean_src) SLFMM_CUDA(cudaMemcpyAsync(s.mean.get(), mean_src, g.p * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
     else s.mean.zero();
     launch_fill(c, s.scale.get(), p, 1.0);
     s.tss.zero();
     s.zero_var.zero();
-    launch_lut_std(c, g.p, s.mean.get(), s.scale.get(), s.lut.get());
+    std_lut(c, g.p, s);
 }
 
 struct Step0 {
@@ -1545,12 +1548,7 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
             res->nmf_gwas_cv_count = cnt;
         }
     } else {
-        if (pre) {
-            se.lut.alloc(ge.p * 4, c.stream);
-            launch_lut_std(c, ge.p, se.mean.get(), se.scale.get(), se.lut.get());
-        } else {
-            std_mean(c, ge, cfg->norm, se);
-        }
+        if (!pre) std_mean(c, ge, cfg->norm, se);
         if (&ge != &gf) {
             std_mean(c, gf, cfg->norm, sf);
             sfp = &sf;
