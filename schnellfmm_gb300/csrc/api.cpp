@@ -18,6 +18,7 @@
 #include <fstream>
 #include <memory>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -1472,9 +1473,12 @@ public:
     void start() {
 #ifdef MADV_POPULATE_WRITE
         if (ranges_.empty()) return;
-        done_ = std::async(std::launch::async, [r = ranges_] {
-            for (const auto& x : r) (void)madvise(reinterpret_cast<void*>(x.first), x.second, MADV_POPULATE_WRITE);
-        });
+        try {
+            done_ = std::async(std::launch::async, [r = ranges_] {
+                for (const auto& x : r) (void)madvise(reinterpret_cast<void*>(x.first), x.second, MADV_POPULATE_WRITE);
+            });
+        } catch (const std::system_error&) {  // no thread to be had: the copies take the faults
+        }
 #endif
     }
 
