@@ -293,6 +293,11 @@ int slfmm_phase_read(slfmm_ctx* ctx, int i, char* name, size_t name_len, double*
  * bounded-wait path of the device pipeline (no counterpart in the
  * reference, whose CPU workers cannot stall on a device). */
 int slfmm_debug_expire_next_wait(slfmm_ctx* ctx, uint64_t cycles);
+/* In the context's next eigen-solve of more than 32 columns one of its eight
+ * CTAs starts each round of the FP64 sweeps `cycles` SM cycles (1 .. 1e6)
+ * late.  The result does not depend on it: a solve whose CTAs were ordered
+ * by their usual pace alone would give another. */
+int slfmm_debug_hold_next_solve(slfmm_ctx* ctx, uint64_t cycles);
 
 /* ---- allocation-free entry point ----------------------------------------- */
 /* Raw genomic inflation factor of each trait from device-resident t

@@ -126,7 +126,8 @@ EXPORTED_SYMBOLS = (
     "slfmm_fit_host", "slfmm_write_tsv", "slfmm_format_exp6", "slfmm_simulate", "slfmm_geno_download",
     "slfmm_profile_enable", "slfmm_profile_read", "slfmm_host_alloc", "slfmm_host_free", "slfmm_contract_raw",
     "slfmm_gif_noalloc", "slfmm_fit_traits", "slfmm_fit_many", "slfmm_reference_normal", "slfmm_write_parquet",
-    "slfmm_phase_count", "slfmm_phase_read", "slfmm_debug_expire_next_wait", "slfmm_small_eigh",
+    "slfmm_phase_count", "slfmm_phase_read", "slfmm_debug_expire_next_wait", "slfmm_debug_hold_next_solve",
+    "slfmm_small_eigh",
 )
 
 _lib_handle = None
@@ -173,6 +174,7 @@ def load_library(path: Optional[os.PathLike] = None) -> C.CDLL:
         "slfmm_phase_count": (i32, [vp]),
         "slfmm_small_eigh": (i32, [vp, vp, u32, vp, vp]),
         "slfmm_debug_expire_next_wait": (i32, [vp, u64]),
+        "slfmm_debug_hold_next_solve": (i32, [vp, u64]),
         "slfmm_phase_read": (i32, [vp, i32, C.c_char_p, C.c_size_t, _dp, _dp]),
         "slfmm_host_alloc": (i32, [C.c_size_t, C.POINTER(vp)]),
         "slfmm_host_free": (i32, [vp]),

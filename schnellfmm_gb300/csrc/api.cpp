@@ -2272,6 +2272,12 @@ int slfmm_debug_expire_next_wait(slfmm_ctx* c, uint64_t cycles) {
     return SLFMM_OK;
 }
 
+int slfmm_debug_hold_next_solve(slfmm_ctx* c, uint64_t cycles) {
+    if (!c || cycles == 0 || cycles > 1000000) return SLFMM_ERR_BAD_ARG;
+    c->hold_next_solve = (long long)cycles;
+    return SLFMM_OK;
+}
+
 int slfmm_phase_count(const slfmm_ctx* c) {
     return c && c->phase_marks.size() > 1 ? (int)c->phase_marks.size() - 1 : 0;
 }

@@ -1140,7 +1140,8 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_cluster(const __grid_consta
 
 // Columns that k_jacobi_svd gives one CTA; wider ones go to a cluster.  A solve
 // with its copies, one CTA against eight: 30 columns 601 and 651 us, 33 columns 848
-// and 837, 40 columns 1107 and 984.
+// and 870, 40 columns 1107 and 1018 (and one CTA holds a column in one element per
+// lane up to 32).
 constexpr int kEighOneCta = 32;
 constexpr int kEighCluster = 8;
 constexpr size_t kEighClusterSmem = 200 << 10;  // beside 25 KB of static arrays
@@ -1174,6 +1175,11 @@ __device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
     for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     return t;
 }
+
+// the two halves of a cluster barrier: what a thread reads or writes before its
+// arrival comes before what any thread does after its wait
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 // slot of the round-robin tournament of m (even) players: player 0 fixed, the
 // others rotate
@@ -1526,10 +1532,11 @@ __device__ void gs_cluster(double* own, int area, double* vec, int ap, double* d
 // shared out and read and written there, and the products take a share of the
 // columns each; of Gram-Schmidt the chains and norms stay with the first CTA.
 // A solve with its copies (45 us), before and so: 13 columns 275 and 235 us, 20
-// 461 and 348, 50 2457 and 1375, 100 14.1 and 4.1 ms, 256 221 and 52 ms.
+// 461 and 348, 50 2457 and 1413, 100 14.1 and 4.2 ms, 256 221 and 53 ms (the wait in
+// the middle of a round is 1 to 3 % of these).
 template <int NC, int NR>
 __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, int a, double* __restrict__ V,
-                                                        double* __restrict__ sig, double* ws) {
+                                                        double* __restrict__ sig, double* ws, long long hold) {
     dependent_start();
     extern __shared__ double sm_dyn[];
     namespace cg = cooperative_groups;
@@ -1713,24 +1720,24 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
         const int nap = na + (na & 1);  // even; position na (odd na) pairs with a column at rest
         const int npairs = nap / 2;
         for (int round = 0; round < nap - 1; ++round) {
+            // test hook: one CTA comes late to its reads
+            if (NC > 1 && hold > 0 && rank == 1)
+                for (const long long t0 = clock64(); clock64() - t0 < hold;) {}
+            const int k = threadIdx.x;
+            int pc = 0, qc = 0;
+            bool meet = false;  // a pair of active columns
+            double app = 0.0, aqq = 0.0, apq = 0.0;
             if (warp < angle_warps) {
-                const int k = threadIdx.x;
-                double cs = 1.0, sn = 0.0;
-                int pc = 0, qc = 0;
                 if (k < npairs) {
                     const int x = tournament_slot(k, round, nap), y = tournament_slot(nap - 1 - k, round, nap);
                     if (x < na && y < na) {
                         pc = act[x];
                         qc = act[y];
                         if (pc > qc) { const int t = pc; pc = qc; qc = t; }
-                        const double app = bcol[pc][pc], aqq = bcol[qc][qc], apq = bcol[qc][pc];
-                        if (fabs(apq) > skip && apq != 0.0) {
-                            const double tau = (aqq - app) / (2.0 * apq);
-                            const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-                            cs = 1.0 / sqrt(1.0 + t * t);
-                            sn = t * cs;
-                            rotated = 1;
-                        }
+                        meet = true;
+                        app = bcol[pc][pc];
+                        aqq = bcol[qc][qc];
+                        apq = bcol[qc][pc];
                     } else {
                         pc = act[x < na ? x : y];
                         qc = rest[0];
@@ -1739,6 +1746,20 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
                     pc = rest[(na & 1) + 2 * (k - npairs)];
                     qc = rest[(na & 1) + 2 * (k - npairs) + 1];
                 }
+            }
+            // Every CTA forms every angle, from elements that lie with the CTAs that
+            // rotate them below: no block is written before all have read.  The wait
+            // is behind the angles, which take longer than the barrier.
+            if (NC > 1) cluster_arrive();
+            if (warp < angle_warps) {
+                double cs = 1.0, sn = 0.0;
+                if (meet && fabs(apq) > skip && apq != 0.0) {
+                    const double tau = (aqq - app) / (2.0 * apq);
+                    const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+                    cs = 1.0 / sqrt(1.0 + t * t);
+                    sn = t * cs;
+                    rotated = 1;
+                }
                 if (k < np2) {
                     jp[buf][k] = pc; jq[buf][k] = qc; jc[buf][k] = cs; js[buf][k] = sn;
                 }
@@ -1746,6 +1767,7 @@ __global__ void __launch_bounds__(1024, 1) k_jacobi_svd(double* __restrict__ A, 
                 rotate_r(buf ^ 1, 32 * r_warp + lane, 32 * r_warps);
             }
             __syncthreads();
+            if (NC > 1) cluster_wait();
             // B <- J^T (B J), the 2 x 2 blocks of the share's pairs of columns
             // with every pair of rows
             for (int e = threadIdx.x; e < nk * np2; e += blockDim.x) {
@@ -2287,14 +2309,16 @@ void launch_jacobi_svd(Ctx& c, const double* A, int a, double* V, double* sig) {
         // a warp per pair of columns, in fours, and those of Gram-Schmidt
         const int threads = std::max(256, (int)round_up(32 * (uint64_t)(ap / 2), 128));
         static_assert(kEighOneCta <= 32 && 3 * 32 * 32 * sizeof(double) + (20 << 10) <= (48 << 10), "");
-        launch_next(c, k_jacobi_svd<1, 1>, 1, threads, 3 * square, const_cast<double*>(A), a, V, sig, nullptr);
+        launch_next(c, k_jacobi_svd<1, 1>, 1, threads, 3 * square, const_cast<double*>(A), a, V, sig, nullptr, 0ll);
     } else {
         DBuf<double> ws(3 * (size_t)ap * ap, c.stream);
         const size_t share = 3 * ceil_div(ap, kEighCluster) * ap * sizeof(double);
         const size_t sm = 2 * square <= kEighClusterSmem ? std::max(2 * square, share) : share;
         auto go = [&](auto kern) {
             set_smem((const void*)kern, std::max(sm, kEighLimit));
-            launch_next_clusters(c, kern, 1, kEighCluster, 1024, sm, const_cast<double*>(A), a, V, sig, ws.get());
+            launch_next_clusters(c, kern, 1, kEighCluster, 1024, sm, const_cast<double*>(A), a, V, sig, ws.get(),
+                                 c.hold_next_solve);
+            c.hold_next_solve = 0;
         };
         if (ap <= 64) go(k_jacobi_svd<kEighCluster, 2>);
         else if (ap <= 128) go(k_jacobi_svd<kEighCluster, 4>);

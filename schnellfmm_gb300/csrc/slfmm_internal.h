@@ -172,6 +172,7 @@ struct Ctx {
     int rng = SLFMM_RNG_CHACHA8;  // stream of the Gaussian sketches
     int* tc8_err = nullptr;  // a Tc8Errors scope's flag: contraction launches leave their check to it
     long long expire_next_wait = 0;  // test hook: next split-FP8 launch's wait limit (SM cycles)
+    long long hold_next_solve = 0;   // test hook: cycles that a CTA of the next clustered eigen-solve is late by
     // a draw of the reference's sketch stream started ahead of its use
     struct PendingNormal;
     std::shared_ptr<PendingNormal> pending_normal;
