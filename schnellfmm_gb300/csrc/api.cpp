@@ -75,7 +75,10 @@ template <typename T>
 void d2h(Ctx& c, T* dst, const T* src, size_t count) {
     if (count) SLFMM_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, c.stream));
 }
-void sync(Ctx& c) { SLFMM_CUDA(cudaStreamSynchronize(c.stream)); }
+void sync(Ctx& c) {
+    SLFMM_CUDA(cudaStreamSynchronize(c.stream));
+    c.in_copy.clear();
+}
 
 template <typename T>
 std::vector<T> fetch(Ctx& c, const T* src, size_t count) {
@@ -88,6 +91,13 @@ template <typename T>
 DBuf<T> upload(Ctx& c, const T* src, size_t count) {
     DBuf<T> b(count, c.stream);
     h2d(c, b.get(), src, count);
+    return b;
+}
+// of a buffer that goes out of scope before the next synchronisation
+template <typename T>
+DBuf<T> upload(Ctx& c, std::vector<T>&& v) {
+    DBuf<T> b(v.size(), c.stream);
+    h2d(c, b.get(), hold(c, std::move(v)), b.n);
     return b;
 }
 
@@ -824,8 +834,7 @@ void step0(Ctx& c, const double* x_host, uint64_t n, int d, double lambda, bool 
     s.qd_omd.alloc(n * std::max(s.r, 1), c.stream);
     s.qd_omdinv.alloc(n * std::max(s.r, 1), c.stream);
     if (s.r) {
-        DBuf<double> a = upload(c, Vs.data(), Vs.size()), b = upload(c, Vo.data(), Vo.size()),
-                     e = upload(c, Vi.data(), Vi.size());
+        DBuf<double> a = upload(c, std::move(Vs)), b = upload(c, std::move(Vo)), e = upload(c, std::move(Vi));
         launch_gemm_small(c, s.xs.get(), d, n, d, a.get(), s.r, s.r, 1.0, 0.0, s.qd.get(), s.r);
         launch_gemm_small(c, s.xs.get(), d, n, d, b.get(), s.r, s.r, 1.0, 0.0, s.qd_omd.get(), s.r);
         launch_gemm_small(c, s.xs.get(), d, n, d, e.get(), s.r, s.r, 1.0, 0.0, s.qd_omdinv.get(), s.r);
@@ -937,7 +946,7 @@ void rsvd(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, int K, int l
         const double sg = std::sqrt(std::max(ev[k], 0.0));
         for (int i = 0; i < l; ++i) Vk[i * K + k] = sg > 0 ? Vh[i * l + k] / sg : 0.0;
     }
-    DBuf<double> Vkd = upload(c, Vk.data(), Vk.size());
+    DBuf<double> Vkd = upload(c, std::move(Vk));
     u_hat.alloc(n * K, c.stream);
     launch_gemm_small(c, B.get(), wp, n, l, Vkd.get(), K, K, 1.0, 0.0, u_hat.get(), K);
     apply_p(c, s0, u_hat.get(), K, K, true);                 // U_hat = Q D^-1 U_small
@@ -1776,6 +1785,7 @@ void ctx_close(Ctx& c) {
     release_draws(c);
     c.dev_flags.release();
     if (c.stream) cudaStreamSynchronize(c.stream);
+    c.in_copy.clear();
     if (c.copy_stream) cudaStreamDestroy(c.copy_stream);
     if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
     c.copy_stream = nullptr;

@@ -307,7 +307,8 @@ void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
                 std::vector<double> tv(t.n);
                 for (unsigned i = 0; i < t.n; ++i) tv[i] = normal_tail_value(t.e[i].a, t.e[i].slot & 1);
                 DBuf<double> tvd(tv.size(), c.stream);
-                SLFMM_CUDA(cudaMemcpyAsync(tvd.get(), tv.data(), tvd.bytes(), cudaMemcpyHostToDevice, c.stream));
+                SLFMM_CUDA(cudaMemcpyAsync(tvd.get(), hold(c, std::move(tv)), tvd.bytes(), cudaMemcpyHostToDevice,
+                                           c.stream));
                 launch_next(c, k_draw_tails, (unsigned)ceil_div(t.n, 128), 128, 0,
                     reinterpret_cast<const Tails*>(p->tails.get()), tvd.get(), t.n, p->vals.get());
                 SLFMM_LAUNCHED(c, "k_draw_tails");

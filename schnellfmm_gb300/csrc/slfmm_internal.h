@@ -182,9 +182,21 @@ struct Ctx {
     NormalTails* draw_tails = nullptr;
     size_t draw_tails_bytes = 0;
     cudaEvent_t draw_done = nullptr;
+    // host buffers that copies in the stream still read (see hold)
+    std::vector<std::shared_ptr<const void>> in_copy;
     bool autotune = false;   // time the tensor-core ring depths per shape once
     std::map<std::string, std::pair<int, int>> tuned;  // shape -> (packed ring cap, W ring cap)
 };
+
+// Keeps a copy's pageable source past the scope that filled it: the runtime may
+// read it until the stream is synchronised, where the buffers held are let go
+// (sync and the end of the context).
+template <typename T>
+const T* hold(Ctx& c, std::vector<T>&& v) {
+    auto kept = std::make_shared<const std::vector<T>>(std::move(v));
+    c.in_copy.push_back(kept);
+    return kept->data();
+}
 
 // bracket a launch with CUDA events when profiling is on
 struct ProfScope {
