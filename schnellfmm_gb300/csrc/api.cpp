@@ -1497,8 +1497,18 @@ private:
     std::future<void> done_;  // waits in its destructor: no call outlives the arrays
 };
 
-void add_results(ResultPages& pages, const slfmm_results* res, uint64_t p, int d) {
-    if (!res) return;
+// Only for a call whose arguments its checks accept (those of the calls below,
+// with l columns in the randomized SVD over p_est SNPs, 0 without one): a refused
+// one leaves the arrays alone, whose sizes may not be those of a d it refuses.
+void populate_results(ResultPages& pages, const slfmm_results* res, const slfmm_config* cfg, uint64_t n, uint64_t p,
+                      int d, uint64_t p_est = 0, uint64_t l = 0) {
+    const uint64_t w = 1 + (uint64_t)std::max(d, 0) + cfg->k;
+    if (!res || !(cfg->lambda > 0.0) || d < 1 || w > (uint64_t)kMaxDesign || n <= w || l > 64 || p_est < l || n < l)
+        return;
+    if (l && cfg->impute == SLFMM_IMPUTE_NMF) {
+        const uint64_t k = cfg->nmf_k ? cfg->nmf_k : cfg->k;
+        if (k > (uint64_t)kMaxNmfK || p_est < k + 10 || n < k + 10) return;
+    }
     pages.add(res->beta, p * d);
     pages.add(res->tstat, p * d);
     pages.add(res->r2, p * 3);
@@ -1512,7 +1522,7 @@ void fit_impl(Ctx& c, const Geno& ge, const Geno& gf, const double* x, int d, co
     check_cfg(cfg);
     SLFMM_REQUIRE(ge.n == gf.n, SLFMM_ERR_BAD_ARG, "estimation and testing genotypes have different sample counts");
     ResultPages pages;
-    add_results(pages, res, gf.p, d);
+    populate_results(pages, res, cfg, gf.n, gf.p, d, ge.p, (uint64_t)cfg->k + cfg->oversampling);
     // the reference's sketch stream is launched ahead of Step 0, whose reads
     // back wait for it too (a sketch made under the upload has drawn it)
     const DrawScope draw(c);
@@ -1984,7 +1994,7 @@ int slfmm_test_associations(slfmm_ctx* c, const slfmm_geno* y_full, const double
     check_cfg(cfg);
     SLFMM_REQUIRE(cfg->impute == SLFMM_IMPUTE_MEAN, SLFMM_ERR_BAD_ARG, "test_associations uses mean imputation");
     ResultPages pages;
-    add_results(pages, res, y_full->p, (int)d);
+    populate_results(pages, res, cfg, y_full->n, y_full->p, (int)d);
     Step0 s0;
     step0(*c, x, y_full->n, (int)d, cfg->lambda, cfg->scale_cov != 0, s0);
     SnpStd st;

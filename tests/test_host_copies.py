@@ -74,3 +74,62 @@ def run_with(fake, script, *args):
 
 def test_sources_outlive_their_copies(fake):
     run_with(fake, CALLS)
+
+
+REFUSED = r'''
+import ctypes as C, mmap, sys
+import numpy as np
+import schnellfmm_gb300 as sg
+libc = C.CDLL(None, use_errno=True)
+rng = np.random.default_rng(3)
+p, size = 4000, 64 << 20
+
+def attempt(what, d, want, n=400, fit=True, tests=True, **cfg):
+    packed = rng.integers(0, 256, size=(p, n // 4), dtype=np.uint8)
+    args = dict(k=3, lambda_=1e-3, oversampling=5)
+    args.update(cfg)
+    c = sg.Lfmm2Config(**args)._c()
+    x, u = rng.standard_normal((n, max(d, 1))), rng.standard_normal((n, args["k"]))
+    g = eng.upload(packed, n)
+    calls = []
+    if fit:
+        calls.append(lambda r: eng.lib.slfmm_fit(eng.h, g.h, g.h, x.ctypes.data, d, C.byref(c), None, C.byref(r)))
+        calls.append(lambda r: eng.lib.slfmm_fit_host(eng.h, packed.ctypes.data, n, p, None, 0, None, x.ctypes.data, d,
+                                                      C.byref(c), None, C.byref(r)))
+    if tests:
+        calls.append(lambda r: eng.lib.slfmm_test_associations(eng.h, g.h, x.ctypes.data, d, u.ctypes.data, C.byref(c),
+                                                               C.byref(r)))
+    for i, call in enumerate(calls):
+        r, maps = sg._Results(), []
+        for f in ("beta", "tstat", "pvalue", "r2"):
+            m = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+            buf = (C.c_char * size).from_buffer(m)
+            setattr(r, f, C.cast(buf, C.POINTER(C.c_double)))
+            maps.append((f, m, buf))
+        rc = call(r)
+        assert rc == want, f"{what}, call {i}: {rc}"
+        for f, m, buf in maps:
+            there = (C.c_ubyte * (size // mmap.PAGESIZE))()
+            assert libc.mincore(C.c_void_p(C.addressof(buf)), C.c_size_t(size), there) == 0
+            touched = sum(b & 1 for b in there)
+            assert touched == 0 or rc == 0, f"{what}, call {i}: {touched} pages of {f} touched"
+    g.free()
+
+with sg.Engine() as eng:
+    attempt("accepted", 60, sg.OK)
+    attempt("too many covariates", 257, sg.ERR_BAD_ARG)
+    attempt("too wide a design", 253, sg.ERR_BAD_ARG)
+    attempt("no degrees of freedom", 238, sg.ERR_DF_NONPOSITIVE, n=240)
+    attempt("no penalty", 60, sg.ERR_BAD_ARG, lambda_=0.0)
+    attempt("too wide a sketch", 60, sg.ERR_BAD_ARG, tests=False, k=30, oversampling=35)
+    attempt("no covariates", 0, sg.ERR_BAD_ARG)
+    attempt("NMF rank", 60, sg.ERR_BAD_ARG, tests=False, impute=sg.ImputeStrategy.NMF, nmf=sg.NmfConfig(k=33, n_iter=2))
+print("ran")
+'''
+
+
+def test_refused_calls_leave_the_results_alone(fake):
+    """Result arrays that the process has not touched are made present while a
+    call runs: not by a call that is refused, whose arrays may be smaller than
+    its d says."""
+    run_with(fake, REFUSED)
