@@ -924,6 +924,15 @@ struct InverseJobs {
     InverseJob job[kMaxInverseJobs];
 };
 
+// Order of the pivot candidates, lu_smem's: 1 + the bits of |x|, and 0 for NaN,
+// which no comparison prefers; but a NaN on the diagonal, where the search starts,
+// is passed by no other.  1 is an exact zero.
+__device__ __forceinline__ unsigned long long pivot_key(double x, bool diagonal) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    if (u > 0x7ff0000000000000ull) return diagonal ? ~0ull : 0ull;
+    return u + 1ull;
+}
+
 __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant__ InverseJobs jobs) {
     dependent_start();
     extern __shared__ double S[];  // a x a
@@ -950,12 +959,10 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant_
         __syncthreads();
         for (int k = 0; k < a; ++k) {
             if (warp == 0) {
-                unsigned long long best = 0ull;  // |value| bits + 1 (0: none; NaN never wins)
+                unsigned long long best = 0ull;
                 int p = k;
                 for (int i = k + lane; i < a; i += 32) {
-                    const unsigned long long u =
-                        (unsigned long long)__double_as_longlong(S[i * a + k]) & 0x7fffffffffffffffull;
-                    const unsigned long long key = u > 0x7ff0000000000000ull ? 0ull : u + 1ull;
+                    const unsigned long long key = pivot_key(S[i * a + k], i == k);
                     if (key > best) { best = key; p = i; }
                 }
 #pragma unroll
@@ -1062,12 +1069,10 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_cluster(const __grid_consta
             if (rank == k % kInvCluster) {
                 const double* col = S + (k / kInvCluster) * a;
                 if (warp == 0) {
-                    unsigned long long best = 0ull;  // |value| bits + 1 (0: none; NaN never wins)
+                    unsigned long long best = 0ull;
                     int p = k;
                     for (int i = k + lane; i < a; i += 32) {
-                        const unsigned long long u =
-                            (unsigned long long)__double_as_longlong(col[i]) & 0x7fffffffffffffffull;
-                        const unsigned long long key = u > 0x7ff0000000000000ull ? 0ull : u + 1ull;
+                        const unsigned long long key = pivot_key(col[i], i == k);
                         if (key > best) { best = key; p = i; }
                     }
 #pragma unroll
