@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(1024) k_gif(const uint32_t* __restrict__ hist,
                                               double* __restrict__ gif_raw) {
     dependent_start();
     constexpr int kPer = (kHistGroups + 1023) / 1024;  // groups of a thread
-    __shared__ unsigned group[kPer * 1024];
+    __shared__ unsigned long long group[kPer * 1024];
     __shared__ unsigned long long wsum[32], before[2];
     __shared__ int found[2];
     __shared__ long long bin[2];
@@ -303,14 +303,17 @@ __global__ void __launch_bounds__(1024) k_gif(const uint32_t* __restrict__ hist,
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 #pragma unroll 8
     for (int g = warp; g < kPer * 1024; g += 32) {
-        unsigned s = 0;
+        unsigned low = 0, high = 0;  // of halves: the warp's sums stay below 2^23
 #pragma unroll
         for (int i = 0; i < kHistGroup / 32; ++i) {
             const int b = kHistGroup * g + 32 * i + lane;
-            s += b < kHistBins ? h[b] : 0u;
+            const unsigned v = b < kHistBins ? h[b] : 0u;
+            low += v & 0xffffu;
+            high += v >> 16;
         }
-        s = __reduce_add_sync(0xffffffffu, s);
-        if (lane == 0) group[g] = s;
+        low = __reduce_add_sync(0xffffffffu, low);
+        high = __reduce_add_sync(0xffffffffu, high);
+        if (lane == 0) group[g] = low + ((unsigned long long)high << 16);
     }
     __syncthreads();
     unsigned long long mine = 0;
@@ -338,7 +341,7 @@ __global__ void __launch_bounds__(1024) k_gif(const uint32_t* __restrict__ hist,
     // the groups where the cumulative count passes `target` and target + 1
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-        const unsigned s = group[kPer * t + i];
+        const unsigned long long s = group[kPer * t + i];
 #pragma unroll
         for (int which = 0; which < 2; ++which)
             if (target + which >= cum && target + which < cum + s) {
