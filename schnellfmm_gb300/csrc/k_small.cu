@@ -349,8 +349,9 @@ __device__ __forceinline__ void pipe_wait() {
 // G[8 ky + i][4 cx + j] (i < 8, j < 4) and reads its 12 row elements as three
 // 16-byte shared-memory loads per row.  Elements past column a (padding, or
 // the next row when lda < 32) only reach entries that are never written out.
-// FP32 sums over up to 16 tiles, then into per-warp FP64 sums in shared
-// memory; the warps are added in a fixed order into one partial per block.
+// FP32 sums over up to 32 tiles (256 rows of a warp), then into per-warp FP64
+// sums in shared memory; the warps are added in a fixed order into one partial
+// per block.
 __global__ void __launch_bounds__(kPipeThreads, 1) k_gram_tile(const float* __restrict__ A, int lda, uint64_t m, int a,
                                                             double* __restrict__ part) {
     dependent_start();
@@ -2274,7 +2275,7 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
     for (int i = 0; i < n; ++i) {
         const InverseJob& j = jobs[i];
         if (inverse_in_shared(j)) continue;
-        DBuf<double> A, X;
+        DBuf<double> A;
         const double* src = j.A;
         if (j.shift != 0.0) {
             A.alloc((size_t)j.a * j.a, c.stream);
@@ -2283,17 +2284,12 @@ void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
             SLFMM_LAUNCHED(c, "k_add_diag");
             src = A.get();
         }
-        double* x = j.X;
-        if (!x) {
-            X.alloc((size_t)j.a * j.a, c.stream);
-            x = X.get();
-        }
         if (j.a <= kMaxSmall) {
             set_smem((const void*)k_inverse, smem_sq(j.a));
-            launch_next(c, k_inverse, 1, 256, smem_sq(j.a), src, j.a, x, j.status, j.eps, nullptr);
+            launch_next(c, k_inverse, 1, 256, smem_sq(j.a), src, j.a, j.X, j.status, j.eps, nullptr);
         } else {
             DBuf<double> work((size_t)j.a * j.a + (size_t)(j.a + 1) / 2, c.stream);  // matrix, then a pivot ints
-            launch_next(c, k_inverse, 1, 1024, 0, src, j.a, x, j.status, j.eps, work.get());
+            launch_next(c, k_inverse, 1, 1024, 0, src, j.a, j.X, j.status, j.eps, work.get());
         }
         SLFMM_LAUNCHED(c, "k_inverse");
     }

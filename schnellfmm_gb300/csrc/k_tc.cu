@@ -730,10 +730,10 @@ void launch_rowfix_mean(Ctx& c, float* P, int ldp, uint64_t rows, int w, const u
 void launch_colfix_mean(Ctx& c, double* S, int lds, uint64_t n, int w, const uint64_t* ptr, const uint32_t* idx,
                         const float* Q, int ldq, const double* coef, const double* colterm) {
     if (!n) return;
+    SLFMM_REQUIRE(w <= 64, SLFMM_ERR_BAD_ARG, "sketch width must be <= 64");
     auto go = [&](auto kern) {
         launch_next(c, kern, (unsigned)ceil_div(n * 32, 256), 256, 0, S, lds, n, w, ptr, idx, Q, ldq, coef, colterm);
     };
-    SLFMM_REQUIRE(w <= 64, SLFMM_ERR_BAD_ARG, "width");  // a sketch's
     if (w <= 32) go(k_colfix_mean<1>);
     else go(k_colfix_mean<2>);
     SLFMM_LAUNCHED(c, "k_colfix_mean");

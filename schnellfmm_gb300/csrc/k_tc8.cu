@@ -79,7 +79,7 @@ struct Tc8Args {
     uint32_t none;          // 0 (see tc8_unpack)
     uint32_t b_stage_bytes; // n_total * 256: one stage of the stage-major W operand
     const float* inv_scale; // n_total: 2^-(e0 + 4t) per B row
-    const uint8_t* wop;     // stage-major, pre-swizzled W operand (wop_offset)
+    const uint8_t* wop;     // stage-major, pre-swizzled W operand
     int mode;               // 0: out = P + M; 1: out = s_r (P - mu_r (cs_c - M))
     long long expire_cycles;  // > 0: test hook, see below
     uint32_t tile0;           // matrix index of the tile of unit 0
@@ -650,18 +650,11 @@ __device__ __forceinline__ float pow2f(int ex) {
     return (ex >= -126 && ex <= 127) ? __int_as_float((127 + ex) << 23) : ldexpf(1.f, ex);
 }
 
-// Byte offset of element (row, k) of a stage-major W operand with n_rows rows:
-// stage kb = k / 256 is the contiguous blob [half][row][128 B] at
-// kb * n_rows * 256, and within each 128-byte row the 16-byte chunk j sits at
-// chunk j ^ (row & 7) -- the 128-byte swizzle the MMA descriptors expect of a
-// 1024-byte aligned shared-memory stage (n_rows % 8 == 0 keeps every half's
-// rows aligned to the 8-row swizzle period).
-__device__ __forceinline__ uint64_t wop_offset(uint32_t row, uint64_t k, uint32_t n_rows) {
-    const uint64_t kb = k >> 8;
-    const uint32_t h = (uint32_t)(k >> 7) & 1u, kk = (uint32_t)k & 127u;
-    return kb * (uint64_t)n_rows * 256 + (uint64_t)(h * n_rows + row) * 128 +
-           ((((kk >> 4) ^ (row & 7u)) << 4) | (kk & 15u));
-}
+// A stage-major W operand with n_rows rows: stage kb = k / 256 is the contiguous
+// blob [half][row][128 B] at kb * n_rows * 256, and within each 128-byte row the
+// 16-byte chunk j sits at chunk j ^ (row & 7) -- the 128-byte swizzle the MMA
+// descriptors expect of a 1024-byte aligned shared-memory stage (n_rows % 8 == 0
+// keeps every half's rows aligned to the 8-row swizzle period).
 
 // The E4M3 terms of one scaling of an operand: a transposed pass splits two of
 // them (diag(s) Q for the genotypes, diag(mu s) Q for the missing-call
@@ -744,7 +737,7 @@ __global__ void __launch_bounds__(256) k_colmax_pair(const float* __restrict__ s
 }
 
 // W (K x w) -> the E4M3 rows of both sets, row_off + t * wpad + c for term t of
-// column c, of a stage-major operand with n_rows rows (wop_offset), zero padded
+// column c, of a stage-major operand with n_rows rows, zero padded
 // to whole stages; inv_scale[row] = 2^-(e0 + 4t).  Term t is
 // round_e4m3((r - terms_<t) * 2^(e0 + 4t)); the power-of-two scales are exact, so
 // each step's residual is rounded once.
@@ -1159,14 +1152,14 @@ static void tile_rows(Ctx& c, const uint8_t* in, uint64_t rows, uint64_t stride,
     SLFMM_LAUNCHED(c, "k_tile_rows");
 }
 
-// Tile-major copies built chunk by chunk while a matrix is uploaded: rows
-// [r0, r1) of the SNP-major matrix (r0 a multiple of 128) are tiled and
-// transposed as soon as they land.  `last` also writes the padding tiles.
 // four 4 KiB blocks to a CTA, as many CTAs as are resident (34 KB each)
 static unsigned transpose_grid(const Ctx& c, uint64_t blocks) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(blocks, 4), (uint64_t)c.sm_count * 6));
 }
 
+// Tile-major copies built chunk by chunk while a matrix is uploaded: rows
+// [r0, r1) of the SNP-major matrix (r0 a multiple of 128) are tiled and
+// transposed as soon as they land.  `last` also writes the padding tiles.
 void tile_chunk(Ctx& c, const Geno& g, uint64_t r0, uint64_t r1, bool last) {
     SLFMM_REQUIRE(r0 % kM == 0, SLFMM_ERR_BAD_ARG, "upload chunks must start on a 128-row tile");
     if (r0 == 0) {

@@ -76,16 +76,8 @@ __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* tm, int x, 
         : "memory");
 }
 
-// contiguous global -> shared bulk copy (16-byte aligned addresses and size)
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// the same with the barrier's expected bytes announced first, by the elected
-// lane of a converged warp
+// contiguous global -> shared bulk copy (16-byte aligned addresses and size), the
+// barrier's expected bytes announced first, by the elected lane of a converged warp
 __device__ __forceinline__ void bulk_g2s_tx(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
                                             uint32_t elected) {
     asm volatile(
