@@ -1736,22 +1736,39 @@ bool write_tsv_body(FILE* f, uint64_t p, uint32_t d, const char* const* chrom, c
 // ===========================================================================
 using namespace slfmm;
 
+// A call that fails in its middle returns, as one that succeeds, with nothing in
+// flight: copies may still read or write the caller's arrays, or buffers that the
+// unwinding freed on the other stream.  (Under capture nothing was begun: the
+// calls that end here synchronise before they launch.)
+static Ctx& settle(Ctx& c) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c.stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        cudaStreamSynchronize(c.stream);
+        cudaStreamSynchronize(c.copy_stream);
+        c.in_copy.clear();
+    }
+    cudaGetLastError();  // the return code says it, not the next launch
+    return c;
+}
+
 #define API_TRY try {
-#define API_CATCH(ctxp)                                                        \
+#define API_FAILED(ctx)                                                        \
     }                                                                          \
     catch (const slfmm::Error& e) {                                            \
-        if (ctxp) (ctxp)->last_error = e.what();                               \
+        (ctx).last_error = e.what();                                           \
         return e.code;                                                         \
     }                                                                          \
     catch (const std::bad_alloc&) {                                            \
-        if (ctxp) (ctxp)->last_error = "host allocation failed";               \
+        (ctx).last_error = "host allocation failed";                           \
         return SLFMM_ERR_NOMEM;                                                \
     }                                                                          \
     catch (const std::exception& e) {                                          \
-        if (ctxp) (ctxp)->last_error = e.what();                               \
+        (ctx).last_error = e.what();                                           \
         return SLFMM_ERR_CUDA;                                                 \
     }                                                                          \
     return SLFMM_OK;
+#define API_CATCH(c) API_FAILED(settle(*(c)))
+#define API_CATCH_ASYNC(c) API_FAILED(*(c))  // of a call that does not wait for its work
 
 extern "C" {
 
@@ -2191,6 +2208,7 @@ int slfmm_fit_many(slfmm_ctx* c, const slfmm_problem* problems, uint32_t n_probl
                 st[i] = SLFMM_ERR_CUDA;
                 msg[i] = e.what();
             }
+            if (st[i] != SLFMM_OK) settle(w);
         }
         ctx_close(w);
     };
@@ -2370,7 +2388,7 @@ int slfmm_gif_noalloc(slfmm_ctx* c, const float* t_dev, uint64_t p, uint32_t d, 
                       " traits (its static histogram holds " + std::to_string(kGifNoAllocMaxTraits) +
                       " x 100000 counters); got " + std::to_string(d));
     launch_gif_noalloc(*c, t_dev, p, (int)d, gif_dev);
-    API_CATCH(c)
+    API_CATCH_ASYNC(c)
 }
 
 int slfmm_format_exp6(double v, char* buf, size_t len) { return format_exp6(v, buf, len); }

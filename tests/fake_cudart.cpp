@@ -198,6 +198,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStr
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { finish(false, s); return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { finish(true, nullptr); return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
+    *s = cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 // an event stands for the stream of its last record
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t) new cudaStream_t(nullptr); return cudaSuccess; }

@@ -80,6 +80,7 @@ REFUSED = r'''
 import ctypes as C, mmap, sys
 import numpy as np
 import schnellfmm_gb300 as sg
+fake = C.CDLL(sys.argv[1])
 libc = C.CDLL(None, use_errno=True)
 rng = np.random.default_rng(3)
 p, size = 4000, 64 << 20
@@ -108,6 +109,7 @@ def attempt(what, d, want, n=400, fit=True, tests=True, **cfg):
             maps.append((f, m, buf))
         rc = call(r)
         assert rc == want, f"{what}, call {i}: {rc}"
+        assert fake.fake_pending() == 0, f"{what}, call {i}: copies in flight when the call returned"
         for f, m, buf in maps:
             there = (C.c_ubyte * (size // mmap.PAGESIZE))()
             assert libc.mincore(C.c_void_p(C.addressof(buf)), C.c_size_t(size), there) == 0
