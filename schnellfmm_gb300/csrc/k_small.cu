@@ -925,12 +925,19 @@ struct InverseJobs {
     InverseJob job[kMaxInverseJobs];
 };
 
+// Inverses up to here are eliminated in shared memory; wider ones keep the LU's
+// solves and their bits.
+constexpr int kInvShared = 112;
+
 // Order of the pivot candidates, lu_smem's: 1 + the bits of |x|, and 0 for NaN,
 // which no comparison prefers; but a NaN on the diagonal, where the search starts,
-// is passed by no other.  1 is an exact zero.
-__device__ __forceinline__ unsigned long long pivot_key(double x, bool diagonal) {
+// is passed by no other, and goes on into the inverse.  1 is an exact zero.
+// Where it starts with the first of several columns nothing is left to invert:
+// the matrix counts as singular (the factors of a sketch that broke down are NaN
+// altogether), up to the widths that the LU does not take.
+__device__ __forceinline__ unsigned long long pivot_key(double x, int i, int k, int a) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
-    if (u > 0x7ff0000000000000ull) return diagonal ? ~0ull : 0ull;
+    if (u > 0x7ff0000000000000ull) return i == k && (k > 0 || a == 1 || a > kInvShared) ? ~0ull : 0ull;
     return u + 1ull;
 }
 
@@ -963,7 +970,7 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_jobs(const __grid_constant_
                 unsigned long long best = 0ull;
                 int p = k;
                 for (int i = k + lane; i < a; i += 32) {
-                    const unsigned long long key = pivot_key(S[i * a + k], i == k);
+                    const unsigned long long key = pivot_key(S[i * a + k], i, k, a);
                     if (key > best) { best = key; p = i; }
                 }
 #pragma unroll
@@ -1073,7 +1080,7 @@ __global__ void __launch_bounds__(1024, 1) k_inverse_cluster(const __grid_consta
                     unsigned long long best = 0ull;
                     int p = k;
                     for (int i = k + lane; i < a; i += 32) {
-                        const unsigned long long key = pivot_key(col[i], i == k);
+                        const unsigned long long key = pivot_key(col[i], i, k, a);
                         if (key > best) { best = key; p = i; }
                     }
 #pragma unroll
@@ -2245,8 +2252,8 @@ void launch_tri_inv_lower(Ctx& c, const double* L, int a, double* Linv) {
 }
 
 // The elimination in shared memory takes every status-only job, and inverses up
-// to 112 columns (wider ones keep the LU's solves and their bits).
-static bool inverse_in_shared(const InverseJob& j) { return j.a <= (j.X ? 112 : kMaxDesign); }
+// to kInvShared columns.
+static bool inverse_in_shared(const InverseJob& j) { return j.a <= (j.X ? kInvShared : kMaxDesign); }
 
 void launch_inverses(Ctx& c, const InverseJob* jobs, int n) {
     SLFMM_REQUIRE(n <= kMaxInverseJobs, SLFMM_ERR_BAD_ARG, "too many matrices for one inversion launch");

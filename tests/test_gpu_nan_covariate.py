@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
-@pytest.mark.parametrize("d,j", [(1, 0), (3, 1), (20, 7), (40, 39), (45, 7), (45, 0), (120, 100), (200, 3)])
+@pytest.mark.parametrize("d,j", [(1, 0), (3, 1), (20, 7), (40, 39), (45, 7), (113, 0), (120, 100),
+                                 (200, 3)])
 def test_not_finite_covariate(engine, capfd, d, j, bad):
     import schnellfmm_gb300 as sg
     c = simdata.simulate(400, 1500, k_pop=3, fst=0.1, miss=0.01, d=d, n_causal=10, seed=d)
@@ -35,4 +36,30 @@ def test_not_finite_covariate(engine, capfd, d, j, bad):
     # the same context on the covariates without it
     good = sg.fit_lfmm2(geno, sg.SubsetSpec.all(), geno, c.x, cfg, omega=omega, engine=engine)
     assert np.isfinite(good.beta).all() and np.abs(good.tstat).max() > 1
+    geno.free()
+
+
+def test_nothing_left_to_invert(engine):
+    """NaN from the first column on is refused (to 112 columns: the LU of wider
+    matrices passes it on): the factors of a sketch that broke down are NaN
+    altogether, and a fit on them has no tests to give."""
+    import schnellfmm_gb300 as sg
+    rng = np.random.default_rng(4)
+    c = simdata.simulate(300, 1500, k_pop=3, fst=0.1, miss=0.01, d=45, n_causal=10, seed=4)
+    geno = engine.upload(c.packed, c.n)
+    for d in (2, 20, 45):
+        x = c.x[:, :d].copy()
+        x[5, 0] = np.nan
+        with pytest.raises(sg.SchnelGpuError, match=r"X\^T X \+ .* inversion failed") as e:
+            sg.fit_lfmm2(geno, sg.SubsetSpec.all(), geno, x, sg.Lfmm2Config(k=3), engine=engine)
+        assert e.value.code == sg.ERR_SINGULAR
+    for k in (2, 16, 41):
+        u = rng.standard_normal((c.n, k))
+        u[7] = np.nan
+        with pytest.raises(sg.SchnelGpuError, match=r"U_hat\^T U_hat inversion failed") as e:
+            sg.test_associations(geno, c.x[:, :2], u, sg.Lfmm2Config(k=k), engine=engine)
+        assert e.value.code == sg.ERR_SINGULAR
+        u[7, 0] = 1.0
+        res = sg.test_associations(geno, c.x[:, :2], u, sg.Lfmm2Config(k=k), engine=engine)
+        assert (res.tstat == 0).all() and np.isnan(res.beta[res.beta != 0]).all()
     geno.free()
