@@ -216,6 +216,11 @@ __global__ void __launch_bounds__(kDrawThreads) k_draw_place(const double* __res
     for (unsigned i = threadIdx.x; i < n && before + i < count; i += kDrawThreads) out[before + i] = v[i];
 }
 
+// A draw of up to this many values that nobody has started ahead is the host's: the
+// device's takes two trips whatever its size (generate_omega of 16, 2 048, 4 096 and
+// 8 192 values: 59, 60, 64 and 63 us by the device, 32, 48, 63 and 94 by the host).
+constexpr uint64_t kDrawHost = 4096;
+
 // tail entries to expect among `count` draws, with room: 2.6 in 10 000
 unsigned tail_cap(uint64_t count) { return (unsigned)(count / 2000 + 64); }
 }  // namespace
@@ -296,7 +301,8 @@ void draw_normal(Ctx& c, uint64_t seed, uint64_t rows, int cols, double* out) {
     if (!count) return;
     std::shared_ptr<Ctx::PendingNormal> p = std::move(c.pending_normal);
     c.pending_normal.reset();
-    if (!p || p->seed != seed || p->rows != rows || p->cols != cols) p = start_draw(c, seed, rows, cols);
+    if (!p || p->seed != seed || p->rows != rows || p->cols != cols)
+        p = count > kDrawHost ? start_draw(c, seed, rows, cols) : nullptr;
     bool made = false;
     if (p) {
         SLFMM_CUDA(cudaEventSynchronize(c.draw_done));
