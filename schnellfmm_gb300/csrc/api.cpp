@@ -231,7 +231,7 @@ void upload_geno(Ctx& c, Geno& g, const uint8_t* packed, uint64_t n_phys, uint64
             SLFMM_REQUIRE(keep[i] < n_phys, SLFMM_ERR_BAD_ARG, "sample index out of range");
             k32[i] = (uint32_t)keep[i];
         }
-        keep_d = upload(c, k32.data(), n_keep);
+        keep_d = upload(c, std::move(k32));
         sync(c);
     }
     if (g.p) {
@@ -270,6 +270,7 @@ void upload_geno(Ctx& c, Geno& g, const uint8_t* packed, uint64_t n_phys, uint64
             std::vector<cudaEvent_t>& b;
             ~Cleanup() {
                 for (size_t i = 0; i < h.size(); ++i) {
+                    if (a[i]) cudaEventSynchronize(a[i]);  // the copies, where an error ends the upload
                     if (h[i]) cudaFreeHost(h[i]);
                     if (a[i]) cudaEventDestroy(a[i]);
                     if (b[i]) cudaEventDestroy(b[i]);
@@ -1011,13 +1012,13 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     const std::vector<double> Graw = Gh;  // unnormalised C^T C
     std::vector<double> f(w);
     for (int k = 0; k < w; ++k) f[k] = Gh[k * w + k] > 0 ? 1.0 / std::sqrt(Gh[k * w + k]) : 0.0;
-    DBuf<double> fd = upload(c, f.data(), w);
+    DBuf<double> fd = upload(c, std::vector<double>(f));
     launch_scale_cols(c, C.get(), n, w, w, fd.get());
     for (int i = 0; i < w; ++i)
         for (int j = 0; j < w; ++j) Gh[i * w + j] *= f[i] * f[j];
     for (int k = 0; k < w; ++k)
         if (f[k] == 0.0) Gh[k * w + k] = 0.0;
-    DBuf<double> L = upload(c, Gh.data(), Gh.size());
+    DBuf<double> L = upload(c, std::move(Gh));
     DBuf<int> st1(1, c.stream), dropped(w, c.stream);
     DBuf<double> Linv(w * w, c.stream);
     launch_chol_inv(c, L.get(), w, Linv.get(), false, st1.get(), 1e-10, dropped.get());
@@ -1033,7 +1034,7 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     std::vector<double> LiT((size_t)w * w);
     for (int i = 0; i < w; ++i)
         for (int j = 0; j < w; ++j) LiT[j * w + i] = Li[i * w + j];
-    DBuf<double> LiTd = upload(c, LiT.data(), LiT.size());
+    DBuf<double> LiTd = upload(c, std::move(LiT));
     DBuf<double> QC(n * w, c.stream);
     launch_gemm_small(c, C.get(), w, n, w, LiTd.get(), w, w, 1.0, 0.0, QC.get(), w);
     // theta rows and c_jj (coefficients of the X columns, src/testing.rs:1036-1048)
@@ -1137,9 +1138,9 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
         for (int jj = 0; jj < d; ++jj)
             for (int k = 1; k < w; ++k) bt[jj * wu + (k - 1)] = (float)Bh[jj * w + k];
     }
-    DBuf<float> thd = upload(c, th.data(), th.size()), btd = upload(c, bt.data(), bt.size());
-    DBuf<double> cjjd = upload(c, cjj.data(), cjj.size());
-    DBuf<uint8_t> dxd = upload(c, drop_x.data(), drop_x.size());
+    DBuf<float> thd = upload(c, std::move(th)), btd = upload(c, std::move(bt));
+    DBuf<double> cjjd = upload(c, std::move(cjj));
+    DBuf<uint8_t> dxd = upload(c, std::move(drop_x));
     AssocConsts k{d, wu, df, thd.get(), btd.get(), cjjd.get(), dxd.get(), st.zero_var.get()};
     const uint64_t pp = std::max<uint64_t>(p, 1);
     DBuf<double> beta(pp * d, c.stream), r2(pp * 3, c.stream), t64(pp * d, c.stream), pv(pp * d, c.stream);
@@ -1225,7 +1226,7 @@ void assoc(Ctx& c, const Geno& g, const SnpStd& st, const Step0& s0, const doubl
     }
     out.gif = gsum / d;
     if (out.gif_per_trait) std::copy(gpt.begin(), gpt.end(), out.gif_per_trait);
-    DBuf<double> gptd = upload(c, gpt.data(), gpt.size());
+    DBuf<double> gptd = upload(c, std::move(gpt));
     // t64 is already widened (and being copied out) when the pass ran in chunks
     launch_calibrate(c, p, d, t32.get(), gptd.get(), copied && out.tstat ? nullptr : t64.get(), pv.get());
     phase(c, "association statistics, GIF");
@@ -2081,7 +2082,7 @@ void geno_subset_samples(Ctx& c, const Geno& src, const std::vector<uint64_t>& k
         SLFMM_REQUIRE(keep[i] < src.n, SLFMM_ERR_BAD_ARG, "sample index out of range");
         k32[i] = (uint32_t)keep[i];
     }
-    DBuf<uint32_t> keep_d = upload(c, k32.data(), k32.size());
+    DBuf<uint32_t> keep_d = upload(c, std::move(k32));
     dst.n = keep.size();
     dst.p = src.p;
     dst.stride = round_up(ceil_div(dst.n, 4), 128);
@@ -2117,13 +2118,17 @@ void fit_trait(Ctx& c, const Geno& g, const double* y, const uint8_t* masks, uin
             keep.push_back(i);
             xt.push_back(y[i * n_traits + t]);
         }
+    struct Wait {  // the copy of xt is over before xt is, however the fit ends
+        Ctx& c;
+        ~Wait() { cudaStreamSynchronize(c.stream); }
+    } const wait{c};
     try {
         SLFMM_REQUIRE(!keep.empty(), SLFMM_ERR_BAD_ARG, "no samples");
         Geno sub;
         phase(c, "", true);
         if (tiles_only_fit(c, cfg, keep.size(), g.p)) {
             std::vector<uint32_t> k32(keep.begin(), keep.end());
-            DBuf<uint32_t> keep_d = upload(c, k32.data(), k32.size());
+            DBuf<uint32_t> keep_d = upload(c, std::move(k32));
             tiles_subset_samples(c, g, keep_d.get(), keep.size(), sub);
             sync(c);
         } else {

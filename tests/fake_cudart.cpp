@@ -30,7 +30,8 @@ std::vector<Copy>& copies() { static std::vector<Copy> v; return v; }
 std::map<const void*, std::string>& names() { static std::map<const void*, std::string> m; return m; }
 std::map<std::string, long>& launches() { static std::map<std::string, long> m; return m; }
 std::map<char*, size_t>& pinned() { static std::map<char*, size_t> m; return m; }
-long changed = 0, read_back = 0;
+long changed = 0, read_back = 0, allocations = 0, fail_in = 0;
+thread_local cudaError_t last_error = cudaSuccess;
 struct Call { dim3 grid, block; size_t smem; void* stream; };
 thread_local std::vector<Call> calls;
 
@@ -84,6 +85,9 @@ extern "C" {
 long fake_changed_sources() { return changed; }
 long fake_sources_compared() { return read_back; }
 long fake_pending() { return (long)copies().size(); }
+// the n-th allocation of device memory from here on fails (0: none)
+void fake_fail_allocation(long n) { allocations = 0, fail_in = n; }
+long fake_allocations() { return allocations; }
 long fake_launches(const char* part) {
     std::lock_guard<std::mutex> lock(mu);
     long n = 0;
@@ -150,10 +154,18 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
     return cudaErrorNotSupported;
 }
 const char* cudaGetErrorString(cudaError_t) { return "error of the stand-in runtime"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last_error;
+    last_error = cudaSuccess;
+    return e;
+}
+cudaError_t cudaPeekAtLastError() { return last_error; }
 
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) {
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (++allocations == fail_in) return last_error = cudaErrorMemoryAllocation;
+    }
     *p = std::calloc(1, n + 4096);
     return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }

@@ -110,6 +110,7 @@ def attempt(what, d, want, n=400, fit=True, tests=True, **cfg):
         rc = call(r)
         assert rc == want, f"{what}, call {i}: {rc}"
         assert fake.fake_pending() == 0, f"{what}, call {i}: copies in flight when the call returned"
+        assert fake.fake_changed_sources() == 0, f"{what}, call {i}: a source was gone before its copy was over"
         for f, m, buf in maps:
             there = (C.c_ubyte * (size // mmap.PAGESIZE))()
             assert libc.mincore(C.c_void_p(C.addressof(buf)), C.c_size_t(size), there) == 0
@@ -135,3 +136,51 @@ def test_refused_calls_leave_the_results_alone(fake):
     call runs: not by a call that is refused, whose arrays may be smaller than
     its d says."""
     run_with(fake, REFUSED)
+
+
+SCARCE = r'''
+import ctypes as C, sys
+import numpy as np
+import schnellfmm_gb300 as sg
+fake = C.CDLL(sys.argv[1])
+rng = np.random.default_rng(3)
+n, p, d = 400, 2000, 2
+packed = rng.integers(0, 256, size=(p, n // 4), dtype=np.uint8)
+x, u, mask = rng.standard_normal((n, d)), rng.standard_normal((n, 3)), rng.random((n, d)) < 0.9
+cfg, alls = sg.Lfmm2Config(k=3, oversampling=5), sg.SubsetSpec.all()
+calls = {
+    "fit": lambda: sg.fit_lfmm2(geno, alls, geno, x, cfg, engine=eng),
+    "fit from the host": lambda: sg.fit_lfmm2_host(packed, n, x, cfg, engine=eng),
+    "tests": lambda: sg.test_associations(geno, x, u, cfg, engine=eng),
+    "traits": lambda: sg.fit_lfmm2_traits(geno, x, mask, cfg, engine=eng),
+    "draw": lambda: eng.generate_omega(3, 10_000, 3),
+}
+with sg.Engine() as eng:
+    for name, call in calls.items():
+        geno = eng.upload(packed, n)
+        fake.fake_fail_allocation(0)
+        call()
+        count = fake.fake_allocations()
+        refused = 0
+        for k in range(1, count + 1):
+            fake.fake_fail_allocation(k)
+            try:
+                call()
+            except sg.SchnelGpuError as e:
+                assert e.code == sg.ERR_NOMEM, f"{name}, allocation {k}: {e}"
+                refused += 1
+            fake.fake_fail_allocation(0)
+            assert fake.fake_pending() == 0, f"{name}, allocation {k}: copies in flight when the call returned"
+            assert fake.fake_changed_sources() == 0, f"{name}, allocation {k}: a source was gone before its copy"
+            call()   # the context goes on
+        # the sketch's scratch is done without
+        assert refused >= count - 8 and refused > 0, (name, refused, count)
+        geno.free()
+print("ran")
+'''
+
+
+def test_every_allocation_may_fail(fake):
+    """A call that runs out of device memory, at any of its allocations, says so
+    and leaves neither copies in flight nor an error behind."""
+    run_with(fake, SCARCE)
