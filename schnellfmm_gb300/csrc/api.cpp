@@ -1818,6 +1818,7 @@ void ctx_close(Ctx& c) {
     if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
     c.copy_stream = nullptr;
     c.stream = nullptr;
+    cudaGetLastError();  // of a context that could not be opened
 }
 }  // namespace
 }  // namespace slfmm
@@ -1837,6 +1838,7 @@ int slfmm_create(int device, const slfmm_opts* opts, slfmm_ctx** out) {
     } catch (const slfmm::Error& e) {
         fprintf(stderr, "schnelgpu: %s\n", e.what());
         const int code = e.code;
+        ctx_close(*c);
         delete c;
         return code;
     }
@@ -2194,6 +2196,7 @@ int slfmm_fit_many(slfmm_ctx* c, const slfmm_problem* problems, uint32_t n_probl
             w.autotune = c->autotune;
             w.rng = c->rng;
         } catch (const Error& e) {
+            ctx_close(w);
             for (uint32_t i = next.fetch_add(1); i < n_problems; i = next.fetch_add(1)) {
                 st[i] = e.code;
                 msg[i] = e.what();

@@ -153,6 +153,7 @@ calls = {
     "fit from the host": lambda: sg.fit_lfmm2_host(packed, n, x, cfg, engine=eng),
     "tests": lambda: sg.test_associations(geno, x, u, cfg, engine=eng),
     "traits": lambda: sg.fit_lfmm2_traits(geno, x, mask, cfg, engine=eng),
+    "many fits": lambda: sg.fit_lfmm2_many([(packed, n, x, cfg)], engine=eng, n_streams=1),
     "draw": lambda: eng.generate_omega(3, 10_000, 3),
 }
 with sg.Engine() as eng:
