@@ -594,9 +594,11 @@ void fp8_row_run(Ctx& c, const Geno& g, const SnpStd& s, const Fp8RowPass& rp, u
 void row_contract_base(Ctx& c, const Geno& g, const SnpStd& s, const double* W, int w, int ldw,
                        DBuf<float>& out, int& wp, bool sketch = false) {
     wp = pad16(w);
-    if (wp > kMaxW) {
+    if (wp > kMaxW && c.precision != SLFMM_PREC_SPLIT_FP8) {
         // wider operands (association designs with many covariates): blocks
         // of 128 columns, each contracted as above and placed in its columns
+        // (the split-FP8 pass has column blocks of its own, the same ones
+        // whether its rows go in chunks or at once)
         out.alloc(std::max<uint64_t>(g.p, 1) * wp, c.stream);
         for (int c0 = 0; c0 < w; c0 += kMaxW) {
             const int wb = std::min(kMaxW, w - c0);

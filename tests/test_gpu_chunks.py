@@ -1,7 +1,8 @@
 """Association statistics that leave in chunks of SNPs (page-locked results)
 against the same pass in one piece (pageable results), bit for bit, in every
 form of the statistics: the thread per SNP (to 4 covariates), the 16-trait and
-the 64-trait tiles, with the indicator operand (to 32 columns) and without.
+the 64-trait tiles, with the indicator operand (to 32 columns) and without, designs of
+more than 128 columns among them.
 The sizes follow the rule for the chunks (whole waves of one 128-row tile per
 SM, 8 MB of results at least in each); the number of launches is checked, so
 that a change of the rule cannot leave nothing to compare.  SNPs without
@@ -15,10 +16,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("d,p", [(1, 700_001), (3, 470_000), (5, 300_007), (12, 200_000), (16, 190_123), (17, 150_000),
-                                 (40, 100_001), (70, 60_000)])
+                                 (40, 100_001), (70, 60_000), (127, 60_000), (140, 60_000), (200, 60_000)])
 def test_chunks_equal_one_piece(engine, d, p):
     import schnellfmm_gb300 as sg
-    n, k, apart = 96, 2, 4999
+    n, k, apart = 96 if d < 90 else 260, 2, 4999
     rng = np.random.default_rng(d)
     codes = rng.choice(np.array([0, 1, 2, 3], dtype=np.uint8), size=(p, n), p=[0.4, 0.02, 0.38, 0.2])
     codes[::apart] = rng.choice(np.array([0, 2, 3], dtype=np.uint8), size=(len(codes[::apart]), 1))
